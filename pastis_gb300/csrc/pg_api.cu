@@ -18,6 +18,7 @@
 #include "pg_stat.h"
 #include "pg_kernels.cuh"
 #include "pg_kernels_xd.cuh"
+#include "pg_lin.cuh"
 
 namespace {
 
@@ -102,6 +103,12 @@ struct Side {
     uint32_t maxlen = 0;
 };
 
+// bucket counts, bucket cursors and totals of the linear-gap alignment
+constexpr size_t LIN_BLOCK = 2 * pg::LIN_NB * sizeof(uint32_t) + sizeof(pg::LinTotals);
+
+// bytes kept readable past a side's last residue (pg_lin.cuh reads aligned words)
+constexpr size_t SEQ_PAD = 16;
+
 size_t next_pow2(size_t x)
 {
     size_t p = 1;
@@ -151,6 +158,16 @@ struct pg_ctx {
     void *d_scan = nullptr;
     size_t scan_bytes = 0;
     uint64_t dirb_cap = 0;
+    // linear-gap alignment (pg_lin.cuh): bucket counts, cursors and totals in
+    // one block, the list with its per-entry words, the X-drop walks' counts
+    bool lin_ok = false;
+    int lin_smax = 0, lin_bps = 1;
+    uint8_t *d_lin = nullptr;
+    pg::LinTotals *h_lin = nullptr;     // pinned
+    uint8_t *d_list = nullptr;
+    uint64_t list_cap = 0;
+    int4 *d_walk = nullptr;
+    uint64_t walk_cap = 0;
     // staging for the host-buffer entry point
     pg_pair *d_pairs = nullptr;
     pg_result *d_out = nullptr;
@@ -239,6 +256,8 @@ void pg_destroy(pg_ctx *ctx)
     cudaFree(ctx->d_xorder);
     cudaFree(ctx->d_dir); cudaFree(ctx->d_dbytes); cudaFree(ctx->d_doff); cudaFree(ctx->d_t1);
     cudaFree(ctx->d_dsc); cudaFree(ctx->d_scan);
+    cudaFree(ctx->d_lin); cudaFree(ctx->d_list); cudaFree(ctx->d_walk);
+    cudaFreeHost(ctx->h_lin);
     cudaFree(ctx->d_pairs);
     cudaFree(ctx->d_out);
     for (int k = 0; k < 3; ++k)
@@ -291,6 +310,9 @@ int pg_create(const pg_config *cfg, pg_ctx **out)
         int maxabs = std::max(std::abs(c->go), std::abs(c->ge));
         for (int k = 0; k < PG_NRES * PG_NRES; ++k) maxabs = std::max(maxabs, std::abs((int)c->sm[k]));
         c->lim16 = pg::dir16_limit(maxabs);
+        const auto mm = std::minmax_element(c->sm, c->sm + PG_NRES * PG_NRES);
+        c->lin_ok = pg::lin_supported(c->go, c->ge, *mm.first, *mm.second);
+        c->lin_smax = *mm.second;
     }
 #define CUD(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { pg_destroy(c); \
         return fail(e_ == cudaErrorMemoryAllocation ? PG_ERR_OOM : PG_ERR_CUDA, "%s: %s", #call, \
@@ -311,6 +333,9 @@ int pg_create(const pg_config *cfg, pg_ctx **out)
     }
     CUD(pg::stat_set_attributes());
     CUD(pg::dir_set_attributes());
+    CUD(cfg->mode == PG_MODE_XDROP ? pg::lin_attributes<true>(&c->lin_bps) : pg::lin_attributes<false>(&c->lin_bps));
+    CUD(cudaMalloc(&c->d_lin, LIN_BLOCK));
+    CUD(cudaMallocHost(&c->h_lin, sizeof(pg::LinTotals)));
     {
         // the direction arena may take up to a third of the device memory
         size_t fr = 0, tot = 0;
@@ -435,7 +460,7 @@ int pg_set_seqs(pg_ctx *c, int32_t side, const char *residues, const uint64_t *o
     if (side == 0 && c->cols_share_rows) { c->side[1] = Side(); c->cols_share_rows = false; }
     cudaFree(s.seq); cudaFree(s.offs);
     s = Side();
-    cudaError_t e1 = cudaMalloc(&s.seq, total ? total : 1);
+    cudaError_t e1 = cudaMalloc(&s.seq, total + SEQ_PAD);
     cudaError_t e2 = e1 == cudaSuccess ? cudaMalloc(&s.offs, (n + 1) * sizeof(uint64_t)) : e1;
     cudaError_t e3 = e2 == cudaSuccess ? cudaMemcpy(s.seq, codes, total, cudaMemcpyHostToDevice) : e2;
     cudaError_t e4 = e3 == cudaSuccess ? cudaMemcpy(s.offs, offs, (n + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice) : e3;
@@ -462,6 +487,95 @@ int pg_share_row_seqs(pg_ctx *c)
     c->cols_share_rows = true;
     ++c->epoch;
     return ensure_scratch(c);
+}
+
+static uint64_t arena_budget(const pg_ctx *c)
+{
+    return c->tune.dir_arena_mb > 0 ? ((uint64_t)c->tune.dir_arena_mb << 20) : c->dir_budget;
+}
+
+// the direction arena for a batch that needs `total` bytes: all of them, or the budget
+static int ensure_arena(pg_ctx *c, uint64_t total, uint64_t budget)
+{
+    if (c->dir_cap > budget) {           // a smaller cap than the arena held so far
+        cudaFree(c->d_dir);
+        c->d_dir = nullptr; c->dir_cap = 0;
+    }
+    // grow at least twofold (up to the cap): a stream of batches of growing
+    // need reallocates a few times, not once per batch
+    const uint64_t need = std::max<uint64_t>(16, std::min<uint64_t>(total, budget));
+    const uint64_t want = need > c->dir_cap ? std::min<uint64_t>(budget, std::max<uint64_t>(need, 2 * c->dir_cap))
+                                            : need;
+    if (want > c->dir_cap) {
+        cudaFree(c->d_dir);
+        c->d_dir = nullptr; c->dir_cap = 0;
+        CU(cudaMalloc(&c->d_dir, want));
+        c->dir_cap = want;
+    }
+    return PG_OK;
+}
+
+// The linear-gap alignment (pg_lin.cuh) of the pairs [p0, p1): their classes are
+// counted, the arena need is read back (one synchronization), then list, DP,
+// traceback and results.  A range that needs more than the arena's budget is
+// halved; one pair that does gets an arena of its own size.  Returns the launches.
+static int run_lin(pg_ctx *c, const pg::KParams &kp, uint64_t p0, uint64_t p1, cudaStream_t st)
+{
+    const bool xdrop = c->cfg.mode == PG_MODE_XDROP;
+    pg::LinParams lp;
+    lp.kp = kp;
+    lp.p0 = p0; lp.p1 = p1;
+    lp.cnt = reinterpret_cast<uint32_t *>(c->d_lin);
+    lp.cur = lp.cnt + pg::LIN_NB;
+    lp.tot = reinterpret_cast<pg::LinTotals *>(lp.cur + pg::LIN_NB);
+    lp.smax = c->lin_smax;
+    lp.e_first = (c->cfg.tie & PG_TIE_H_E_BEFORE_F) ? 1 : 0;
+    lp.list = nullptr; lp.dp = nullptr; lp.prog = nullptr; lp.arena = nullptr; lp.walk = nullptr;
+    CU(cudaMemsetAsync(c->d_lin, 0, LIN_BLOCK, st));
+    if (xdrop) pg::lin_count<true>(lp, c->nsm, st);
+    else pg::lin_count<false>(lp, c->nsm, st);
+    CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(c->h_lin, lp.tot, sizeof(pg::LinTotals), cudaMemcpyDeviceToHost, st));
+    CU(cudaStreamSynchronize(st));
+    const uint64_t total = (uint64_t)c->h_lin->units * 32u;
+    // offsets are 32-bit counts of 32 bytes
+    const uint64_t budget = std::min<uint64_t>(arena_budget(c), (uint64_t)1 << 37);
+    int launches = 2;
+    if (total > budget && p1 - p0 > 1) {
+        const uint64_t mid = p0 + (p1 - p0) / 2;
+        const int a = run_lin(c, kp, p0, mid, st);
+        if (a < 0) return a;
+        const int b = run_lin(c, kp, mid, p1, st);
+        return b < 0 ? b : launches + a + b;
+    }
+    int rc = ensure_arena(c, total, std::max(budget, total));
+    if (rc) return rc;
+    const uint64_t entries = c->h_lin->entries;
+    if (entries > c->list_cap || !c->d_list) {
+        cudaFree(c->d_list);
+        c->d_list = nullptr; c->list_cap = 0;
+        const uint64_t cap = std::max<uint64_t>(256, entries + entries / 4);
+        CU(cudaMalloc(&c->d_list, cap * (sizeof(pg::LinReg) + sizeof(int4) + sizeof(uint32_t))));
+        c->list_cap = cap;
+    }
+    if (xdrop && kp.n > c->walk_cap) {
+        cudaFree(c->d_walk);
+        c->d_walk = nullptr; c->walk_cap = 0;
+        CU(cudaMalloc(&c->d_walk, 2 * kp.n * sizeof(int4)));
+        c->walk_cap = kp.n;
+    }
+    lp.list = reinterpret_cast<pg::LinReg *>(c->d_list);
+    lp.dp = reinterpret_cast<int4 *>(lp.list + c->list_cap);
+    lp.prog = reinterpret_cast<uint32_t *>(lp.dp + c->list_cap);
+    lp.arena = c->d_dir;
+    lp.walk = c->d_walk;
+    const int per_sm = c->tune.dp_blocks_per_sm > 0 ? std::min(c->lin_bps, c->tune.dp_blocks_per_sm) : c->lin_bps;
+    const int blocks = c->nsm * std::max(per_sm, 1);
+    const uint32_t jobs = c->h_lin->jobs;
+    launches += xdrop ? pg::lin_align<true>(lp, (uint32_t)entries, jobs, c->nsm, blocks, st)
+                      : pg::lin_align<false>(lp, (uint32_t)entries, jobs, c->nsm, blocks, st);
+    CU(cudaGetLastError());
+    return launches;
 }
 
 // The traceback form of the DP phase: direction bytes per task, their
@@ -495,22 +609,8 @@ static int run_dir(pg_ctx *c, const pg::KParams &kp, uint64_t n, int grid, cudaS
     CU(cudaMemcpyAsync(&total, c->d_doff + n, sizeof total, cudaMemcpyDeviceToHost, st));
     CU(cudaMemcpyAsync(&nchk, d_nchk, sizeof nchk, cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
-    const uint64_t budget = c->tune.dir_arena_mb > 0 ? ((uint64_t)c->tune.dir_arena_mb << 20) : c->dir_budget;
-    if (c->dir_cap > budget) {           // a smaller cap than the arena held so far
-        cudaFree(c->d_dir);
-        c->d_dir = nullptr; c->dir_cap = 0;
-    }
-    // grow at least twofold (up to the cap): a stream of batches of growing
-    // need reallocates a few times, not once per batch
-    const uint64_t need = std::max<uint64_t>(16, std::min<uint64_t>(total, budget));
-    const uint64_t want = need > c->dir_cap ? std::min<uint64_t>(budget, std::max<uint64_t>(need, 2 * c->dir_cap))
-                                            : need;
-    if (want > c->dir_cap) {
-        cudaFree(c->d_dir);
-        c->d_dir = nullptr; c->dir_cap = 0;
-        CU(cudaMalloc(&c->d_dir, want));
-        c->dir_cap = want;
-    }
+    int rc = ensure_arena(c, total, arena_budget(c));
+    if (rc) return rc;
     const int dyn = kp.dir16_lim > 0 ? pg::DIR16_DYN_SMEM : pg::DP_DYN_SMEM;
     const int tie = c->cfg.tie;
     int launches = 1;
@@ -591,6 +691,10 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
         if (c->cfg.mode == PG_MODE_SW || gmax >= 0) kp.dir16_side = 65535;
         else kp.dir16_side = std::min(65535, (pg::SAT16_DP - std::abs(c->go)) / -gmax);
     }
+    // gap scores whose affine recurrence is a linear one: the default form runs
+    // them through pg_lin.cuh (the scheduling options that have no meaning there
+    // select the kernels they were made for)
+    const bool lin = c->lin_ok && c->tune.dp_traceback == 3 && c->tune.rows_max == 8 && c->tune.bucket_order;
     CU(cudaMemsetAsync(c->d_counter, 0, (4 + pg::SCHED_WORDS + pg::XSCHED_WORDS) * sizeof(unsigned int), st));
     CU(cudaMemsetAsync(c->d_status, 0, sizeof(int), st));
     const uint64_t need_blocks = (n + pg::WARPS - 1) / pg::WARPS;
@@ -643,13 +747,17 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
             else pg::k_xd<<<gx, pg::XT, 0, st>>>(kp);
             pg::k_xd_wide<<<c->grid_wide, blk, 0, st>>>(kp);
         }
-        if (kp.order) {
+        if (kp.order && !lin) {
             pg::k_hist<true><<<gsched, 256, 0, st>>>(kp);
             pg::k_bucket<true><<<gsched, 256, 0, st>>>(kp);
         }
         CU(record_event(c, c->ev[1], st));
         const int dyn = pg::DP_DYN_SMEM;
-        if (kp.dir) {
+        if (lin) {
+            const int l = run_lin(c, kp, 0, n, st);
+            if (l < 0) return l;
+            c->last_launches = 2 + l + xlaunch;
+        } else if (kp.dir) {
             const int l = run_dir(c, kp, n, (int)gmax, st);
             if (l < 0) return l;
             c->last_launches = (kp.order ? 4 : 2) + l + xlaunch;
@@ -658,13 +766,17 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
             c->last_launches = (kp.order ? 5 : 3) + xlaunch;
         }
     } else {
-        if (kp.order) {
+        if (kp.order && !lin) {
             pg::k_hist<false><<<gsched, 256, 0, st>>>(kp);
             pg::k_bucket<false><<<gsched, 256, 0, st>>>(kp);
         }
         CU(record_event(c, c->ev[1], st));
         const int dyn = pg::DP_DYN_SMEM;
-        if (kp.dir) {
+        if (lin) {
+            const int l = run_lin(c, kp, 0, n, st);
+            if (l < 0) return l;
+            c->last_launches = l;
+        } else if (kp.dir) {
             const int l = run_dir(c, kp, n, (int)gmax, st);
             if (l < 0) return l;
             c->last_launches = (kp.order ? 2 : 0) + l;
@@ -717,6 +829,7 @@ static int check_status(pg_ctx *c)
     int st = 0;
     CU(cudaMemcpy(&st, c->d_status, sizeof st, cudaMemcpyDeviceToHost));
     if (st & pg::ST_BAD_INDEX) return fail(PG_ERR_ARG, "a pair refers to a sequence index out of range");
+    if (st & pg::ST_WAIT) return fail(PG_ERR_CUDA, "internal: a stripe's wait ran out");
     if (st & pg::ST_BAD_SCHED) return fail(PG_ERR_CUDA, "internal: inconsistent bucket schedule");
     return PG_OK;
 }

@@ -292,7 +292,7 @@ extern "C" int pg_set_seqs_fasta(pg_ctx *ctx, int32_t side, const char *fasta, u
         return pg_internal_fail(PG_ERR_RANGE, "pg_set_seqs_fasta: a sequence has more than 65535 residues");
     }
     uint8_t *d_codes = nullptr;
-    if (cudaMalloc(&d_codes, total ? total : 1) != cudaSuccess) {
+    if (cudaMalloc(&d_codes, total + 16) != cudaSuccess) {   // 16: aligned words are read (pg_lin.cuh)
         cudaFree(d_offs);
         return pg_internal_fail(PG_ERR_OOM, "pg_set_seqs_fasta: residues");
     }

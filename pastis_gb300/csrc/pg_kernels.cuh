@@ -47,6 +47,7 @@ constexpr int ST_BAD_INDEX = 1;
 constexpr int ST_TOO_LONG = 2;    // a sequence beyond a kernel's length bound
 constexpr int ST_BAD_SCHED = 4;   // bucket order inconsistent (never expected)
 constexpr int ST_BAD_CODE = 8;    // a residue code outside 0..24
+constexpr int ST_WAIT = 16;       // a stripe gave up waiting for the one above it (never expected)
 
 // extension of one (pair, seed)
 constexpr uint32_t XF_NONE = 1;    // seed not tried (seed_count / spurious switch)
@@ -89,6 +90,7 @@ struct KParams {
     int dir16_pair = 0;              // 1: 16-bit regions of up to 32 x rows_cap rows two per warp
     const uint32_t *xorder = nullptr; // X-drop extension tasks, longest length bound first (null: t)
     unsigned int *xsched = nullptr;   // [0, XBUCKET) task bucket sizes, [XBUCKET, 2*XBUCKET) cursors
+    int four = 4;                     // a 4 the compiler cannot see (pg_lin.cuh)
 };
 
 __device__ __forceinline__ void load_sm(int *ssm, const int8_t *sm)

@@ -1,0 +1,1039 @@
+// pg_lin.cuh -- the alignment DP and its traceback when the affine recurrence
+// collapses to a linear one (sm_103a).
+//
+// With a first gap position that costs less than the further ones (go > ge,
+// what PASTIS's parameters become when they are passed as it passes them),
+// E(i, j) = max(E(i, j-1) + ge, H(i, j-1) + go) is always H(i, j-1) + go,
+// strictly: E <= H and ge < go.  The same holds for F.  So
+//     H(i, j) = max(H(i-1, j-1) + s, H(i-1, j) + go, H(i, j-1) + go [, 0])
+// and every gap of the traceback was opened, whatever the tie policy says of
+// gap ties.  What bounds the DP is the integer ALU pipe (two cycles a warp
+// instruction), so the form below is built to need few ALU operations:
+//
+//  - two cells per 32-bit register (int16 halves: the low half R rows, the
+//    high half the R rows below them one column behind), values scaled by 4;
+//  - the decision rides in the two free bits: a term carries its tag (diagonal
+//    3 on identical residues, 2 otherwise; of F and E the one the tie policy
+//    prefers 1, the other 0), so the maximum picks the larger H and on a tie
+//    the larger tag, and no comparison is needed to know which term won;
+//  - per row and two cells: one prmt (score), one add, two DPX add-max, one
+//    logic op to clear the tag; the tags are gathered by multiply-adds on the
+//    FMA pipe (the sum of the tagged minus the sum of the cleared values).
+// That is 5 ALU operations for 2 cells against 17 in the affine form.
+//
+// A direction word holds 2 bits per cell: the 2 x 8 rows of a lane's two
+// virtual lanes at one wavefront step in one 32-bit word; eight steps of a
+// lane fill a 32-byte sector, written as two 16-byte stores.
+//
+// Work units.  Regions are listed by class (lanes L x rows per lane R) and
+// column count.  A region of up to 16 R rows takes 8 lanes, 32 R rows 16 lanes,
+// 64 R rows a warp, so that a warp works 4, 2 or 1 regions of the same class
+// and nearly the same column count together: a wavefront spends a step per
+// virtual lane filling and another draining, and the fewer lanes a region has
+// the shorter those ramps, at 8 rows per lane that spread a step's fixed cost
+// (shuffle, residue, profile reads, store) over 16 cells.  Taller regions, and
+// those whose scaled values could leave int16, run as stripes of 64 R rows, one
+// warp each, pipelined: a stripe waits for the stripe above only 32 columns at
+// a time (boundary row and progress word in HBM), and its lanes keep their
+// values relative to a base that follows them, so no region is too large.
+#pragma once
+#include <cstdint>
+
+#include "pg_kernels.cuh"
+#include "pg_lin.h"
+
+namespace pg {
+
+// ------------------------------------------------------------- host rule
+// scores the tagged 16-bit form takes: gap scores as above; substitution
+// scores that fit an int8 profile after scaling; a gap that costs less than the
+// sentinel's -128 after scaling.  H moves by at most 31 + 31 from a neighbour,
+// so a lane's values stay inside int16 for 64 columns between two base moves
+// ((64 + 16) columns x 4 x 62 = 19840)
+constexpr int LIN_SMAX = 31;
+__host__ __forceinline__ bool lin_supported(int go, int ge, int smin, int smax)
+{
+    return go > ge && go < 0 && go >= -LIN_SMAX && smin >= -LIN_SMAX - 1 && smax <= LIN_SMAX;
+}
+
+// ------------------------------------------------------------- work list
+// one region, or one stripe of a region that runs in stripes (its stripes are
+// consecutive entries)
+struct LinReg {
+    uint64_t v, h;        // first row / column residue (offsets into the sides' residues)
+    uint32_t key;         // X-drop: 2 * pair + seed; SW: pair
+    uint32_t off;         // its direction words, in 32-byte units of the arena
+    uint16_t m, n;
+    uint16_t stripe, nstripe;
+};
+static_assert(sizeof(LinReg) == 32, "two 16-byte loads");
+
+// classes: 0-3 stripes with R = 8..5; 4-7 a warp, R = 8..5; 8-11 16 lanes,
+// R = 8..5; 12-17 8 lanes, R = 8, 7, 6, 5, 4, 2.  The costly ones first.
+constexpr int LIN_SEG = 18;
+constexpr int LIN_LEV = 48;                        // column-count levels per class, long first
+constexpr int LIN_NB = LIN_SEG * LIN_LEV;
+
+struct LinTotals {
+    unsigned long long units;                      // arena need in 32-byte units
+    unsigned long long cursor;                     // arena units handed out by k_lin_place
+    uint32_t entries, jobs;
+    uint32_t next_job, pad;                        // work counter of k_lin_dp
+    uint32_t seg[3 * LIN_SEG];                     // per class: first list entry, entries, first job
+};
+
+struct LinParams {
+    KParams kp;
+    uint64_t p0, p1;                               // pairs of this pass
+    uint32_t *cnt;                                 // LIN_NB bucket sizes
+    uint32_t *cur;                                 // LIN_NB bucket cursors
+    LinTotals *tot;
+    LinReg *list;
+    int4 *dp;                                      // per entry: score, end row, end column, have
+    uint32_t *prog;                                // per entry: columns of its boundary row written
+    uint8_t *arena;
+    int4 *walk;                                    // X-drop, per key: score, matches, diagonals, gap runs
+    int smax;
+    int e_first;                                   // H ties: E before F
+};
+
+__host__ __device__ __forceinline__ int lin_seg_lanes(int seg) { return seg < 8 ? 32 : seg < 12 ? 16 : 8; }
+__host__ __device__ __forceinline__ int lin_seg_rows(int seg)
+{
+    return seg < 16 ? 8 - (seg & 3) : seg == 16 ? 4 : 2;
+}
+__host__ __device__ __forceinline__ int lin_seg_group(int seg) { return seg < 8 ? 1 : seg < 12 ? 2 : 4; }
+
+__device__ __forceinline__ int lin_seg(const LinParams &lp, bool local, int m, int n)
+{
+    // every scaled value of the region provably inside int16 (no base):
+    // above smax per diagonal, below the all-gaps path plus the rows past m
+    const int lo = local ? 0 : -lp.kp.go * (m + n + 20);
+    const bool plain = 4 * lp.smax * min(m, n) <= 31000 && 4 * lo <= 30000;
+    if (m > 512 || !plain) {
+        const int stripes = (m + 511) >> 9;
+        const int r = (m + 64 * stripes - 1) / (64 * stripes);
+        return r <= 5 ? 3 : 8 - r;
+    }
+    if (m > 256) { const int r = (m + 63) >> 6; return 4 + 8 - r; }
+    if (m > 128) { const int r = (m + 31) >> 5; return 8 + 8 - r; }
+    const int r = (m + 15) >> 4;
+    return r <= 2 ? 17 : r <= 4 ? 16 : 12 + 8 - r;
+}
+__device__ __forceinline__ int lin_level(int n)
+{
+    const int l = n < 256 ? n >> 3 : n < 1024 ? 32 + ((n - 256) >> 6) : n < 4096 ? 44 + ((n - 1024) >> 10) : 47;
+    return LIN_LEV - 1 - l;
+}
+// stripes of a region (1 for the classes that do not run in stripes)
+__host__ __device__ __forceinline__ int lin_stripes(int seg, int m)
+{
+    return seg < 4 ? (m + 64 * lin_seg_rows(seg) - 1) / (64 * lin_seg_rows(seg)) : 1;
+}
+// 8-step tiles of one stripe, in 32-byte units; boundary row of one stripe
+__host__ __device__ __forceinline__ uint32_t lin_tile_units(int lanes, int n)
+{
+    return (uint32_t)((n + 2 * lanes - 1 + 7) >> 3) * (uint32_t)lanes;
+}
+__host__ __device__ __forceinline__ uint32_t lin_row_units(int n) { return (uint32_t)((n + 1 + 7) >> 3); }
+__host__ __device__ __forceinline__ uint32_t lin_units(int seg, int m, int n)
+{
+    const int s = lin_stripes(seg, m);
+    return (uint32_t)s * lin_tile_units(lin_seg_lanes(seg), n) + (uint32_t)(s - 1) * lin_row_units(n);
+}
+
+// the DP regions of pair p: X-drop up to two (one per seed), SW one
+struct LinPair {
+    uint64_t v[2], h[2];
+    int m[2], n[2];
+    bool dp[2];
+    bool bad;              // a sequence index out of range
+};
+template <bool XDROP>
+__device__ __forceinline__ LinPair lin_pair(const KParams &kp, uint64_t p)
+{
+    LinPair lp;
+    lp.dp[0] = lp.dp[1] = false;
+    lp.m[0] = lp.m[1] = lp.n[0] = lp.n[1] = 0;
+    lp.v[0] = lp.v[1] = lp.h[0] = lp.h[1] = 0;
+    const pg_pair pr = kp.pairs[p];
+    const uint64_t r = (uint64_t)pr.row + kp.roff, c = (uint64_t)pr.col + kp.coff;
+    lp.bad = r >= kp.nr || c >= kp.nc;
+    if (lp.bad) return lp;
+    const uint64_t r0 = kp.roffs[r], c0 = kp.coffs[c];
+    if (XDROP) {
+        const XdRec a = kp.xd[2 * p], b = kp.xd[2 * p + 1];
+        lp.dp[0] = !(a.flags & (XF_NONE | XF_BADIDX)) && a.ev > a.bv && a.eh > a.bh;
+        const bool same = !(a.flags & XF_NONE) && b.bv == a.bv && b.ev == a.ev && b.bh == a.bh && b.eh == a.eh;
+        lp.dp[1] = !(b.flags & (XF_NONE | XF_SAME | XF_BADIDX)) && !same && b.ev > b.bv && b.eh > b.bh;
+        lp.v[0] = r0 + a.bv; lp.h[0] = c0 + a.bh; lp.m[0] = a.ev - a.bv; lp.n[0] = a.eh - a.bh;
+        lp.v[1] = r0 + b.bv; lp.h[1] = c0 + b.bh; lp.m[1] = b.ev - b.bv; lp.n[1] = b.eh - b.bh;
+    } else {
+        lp.v[0] = r0; lp.h[0] = c0;
+        lp.m[0] = (int)(kp.roffs[r + 1] - r0);
+        lp.n[0] = (int)(kp.coffs[c + 1] - c0);
+        lp.dp[0] = lp.m[0] > 0 && lp.n[0] > 0;
+    }
+    return lp;
+}
+
+constexpr int LIN_PT = 256;                        // threads of the list kernels
+constexpr int LIN_PP = 4;                          // pairs per thread and pass
+
+// bucket sizes and arena need of the pass
+template <bool XDROP>
+__global__ void __launch_bounds__(LIN_PT) k_lin_hist(const LinParams lp)
+{
+    __shared__ uint32_t h[LIN_NB];
+    __shared__ unsigned long long su;
+    for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT) h[b] = 0;
+    if (threadIdx.x == 0) su = 0;
+    __syncthreads();
+    unsigned long long units = 0;
+    for (uint64_t p = lp.p0 + (uint64_t)blockIdx.x * LIN_PT + threadIdx.x; p < lp.p1;
+         p += (uint64_t)gridDim.x * LIN_PT) {
+        const LinPair r = lin_pair<XDROP>(lp.kp, p);
+#pragma unroll
+        for (int s = 0; s < (XDROP ? 2 : 1); ++s) {
+            if (!r.dp[s]) continue;
+            const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
+            atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])], (uint32_t)lin_stripes(seg, r.m[s]));
+            units += lin_units(seg, r.m[s], r.n[s]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) units += __shfl_xor_sync(FULL, units, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&su, units);
+    __syncthreads();
+    for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT)
+        if (h[b]) atomicAdd(&lp.cnt[b], h[b]);
+    if (threadIdx.x == 0 && su) atomicAdd(&lp.tot->units, su);
+}
+
+// bucket starts (exclusive prefix) and the classes' places in the list and in
+// the job order; one block of 1024 threads
+static __global__ void __launch_bounds__(1024) k_lin_scan(const LinParams lp)
+{
+    static_assert(LIN_NB <= 1024, "one bucket per thread");
+    __shared__ uint32_t w[32], start[LIN_NB + 1];
+    const int t = threadIdx.x, lane = t & 31;
+    const uint32_t c = t < LIN_NB ? lp.cnt[t] : 0;
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) w[t >> 5] = x;
+    __syncthreads();
+    if (t < 32) {
+        uint32_t y = w[t];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t z = __shfl_up_sync(FULL, y, o);
+            if (lane >= o) y += z;
+        }
+        w[t] = y;
+    }
+    __syncthreads();
+    const uint32_t inc = x + (t >= 32 ? w[(t >> 5) - 1] : 0);
+    if (t < LIN_NB) { start[t] = inc - c; lp.cur[t] = inc - c; }
+    if (t == LIN_NB - 1) start[LIN_NB] = inc;
+    __syncthreads();
+    if (t == 0) {
+        uint32_t job = 0;
+        for (int s = 0; s < LIN_SEG; ++s) {
+            const uint32_t b = start[s * LIN_LEV], n = start[(s + 1) * LIN_LEV] - b;
+            const uint32_t g = (uint32_t)lin_seg_group(s);
+            lp.tot->seg[s] = b;
+            lp.tot->seg[LIN_SEG + s] = n;
+            lp.tot->seg[2 * LIN_SEG + s] = job;
+            job += (n + g - 1) / g;
+        }
+        lp.tot->entries = start[LIN_NB];
+        lp.tot->jobs = job;
+    }
+}
+
+// the list, in bucket order; arena units by one atomic per block and pass.  A
+// pair without a region in SW gets its (empty) result here.
+template <bool XDROP>
+__global__ void __launch_bounds__(LIN_PT) k_lin_place(const LinParams lp)
+{
+    __shared__ uint32_t h[LIN_NB];
+    __shared__ uint32_t su;
+    __shared__ unsigned long long ubase;
+    const uint64_t step = (uint64_t)LIN_PT * LIN_PP;
+    unsigned long long cells = 0;
+    for (uint64_t c0 = lp.p0 + blockIdx.x * step; c0 < lp.p1; c0 += gridDim.x * step) {
+        for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT) h[b] = 0;
+        if (threadIdx.x == 0) su = 0;
+        __syncthreads();
+        constexpr int NS = XDROP ? 2 : 1;
+        uint32_t rank[LIN_PP * NS], off[LIN_PP * NS];
+#pragma unroll
+        for (int q = 0; q < LIN_PP; ++q) {
+            const uint64_t p = c0 + (uint64_t)q * LIN_PT + threadIdx.x;
+            LinPair r;
+            r.dp[0] = r.dp[1] = false;
+            if (p < lp.p1) r = lin_pair<XDROP>(lp.kp, p);
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                rank[q * NS + s] = off[q * NS + s] = 0;
+                if (!r.dp[s]) continue;
+                const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
+                rank[q * NS + s] = atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])],
+                                             (uint32_t)lin_stripes(seg, r.m[s]));
+                off[q * NS + s] = atomicAdd(&su, lin_units(seg, r.m[s], r.n[s]));
+                cells += (unsigned long long)r.m[s] * (unsigned long long)r.n[s];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) ubase = su ? atomicAdd(&lp.tot->cursor, (unsigned long long)su) : 0;
+        for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT) {
+            const uint32_t k = h[b];
+            if (k) h[b] = atomicAdd(&lp.cur[b], k);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < LIN_PP; ++q) {
+            const uint64_t p = c0 + (uint64_t)q * LIN_PT + threadIdx.x;
+            if (p >= lp.p1) continue;
+            const LinPair r = lin_pair<XDROP>(lp.kp, p);
+            if (!XDROP && !r.dp[0]) {
+                pg_result o = empty_result();
+                if (r.bad) atomicOr(lp.kp.status, ST_BAD_INDEX);
+                else apply_filter(o, r.m[0], r.n[0], lp.kp.cov_thr, lp.kp.ani_thr);
+                lp.kp.out[p] = o;
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                if (!r.dp[s]) continue;
+                const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
+                const int ns = lin_stripes(seg, r.m[s]);
+                uint32_t pos = h[seg * LIN_LEV + lin_level(r.n[s])] + rank[q * NS + s];
+                LinReg e;
+                e.v = r.v[s]; e.h = r.h[s];
+                e.key = XDROP ? (uint32_t)(2 * p + s) : (uint32_t)p;
+                e.off = (uint32_t)(ubase + off[q * NS + s]);
+                e.m = (uint16_t)r.m[s]; e.n = (uint16_t)r.n[s];
+                e.nstripe = (uint16_t)ns;
+                for (int k = 0; k < ns; ++k, ++pos) {
+                    e.stripe = (uint16_t)k;
+                    const uint4 *src = reinterpret_cast<const uint4 *>(&e);
+                    uint4 *dst = reinterpret_cast<uint4 *>(lp.list + pos);
+                    dst[0] = src[0];
+                    dst[1] = src[1];
+                    lp.prog[pos] = 0;
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cells += __shfl_xor_sync(FULL, cells, o);
+    if ((threadIdx.x & 31) == 0 && cells) atomicAdd(lp.kp.exec_cells + 1, cells);
+}
+
+// ------------------------------------------------------------------ the DP
+constexpr int LIN_ROWB = 36;                       // byte stride of a score-table row: 9 words spread the banks
+constexpr int LIN_NC = NCODES + 1;                 // the residues and the sentinel past either end
+constexpr int LIN_PROF = 2 * LIN_NC * 32 * 8;      // bytes per warp
+constexpr int LIN_DYN = WARPS * LIN_PROF;
+constexpr uint32_t LIN_CLR = 0xFFFCFFFCu;          // clears both halves' tags
+constexpr int LIN_NEG = -32000;
+
+// tagged score table: row a, byte b = 4 * s(a, b) + (a == b ? 3 : 2); the
+// sentinel row and the sentinel column -128
+__device__ __forceinline__ void lin_table(int8_t *t, const int8_t *sm)
+{
+    for (int k = threadIdx.x; k < LIN_NC * LIN_ROWB; k += blockDim.x) {
+        const int a = k / LIN_ROWB, b = k - a * LIN_ROWB;
+        t[k] = a < PG_NRES && b < PG_NRES ? (int8_t)(4 * (int)sm[a * PG_NRES + b] + (a == b ? 3 : 2)) : (int8_t)-128;
+    }
+}
+
+// This lane's score profile for rows row0 .. row0 + 2R - 1 of V (0-based; rows
+// past m: sentinel): for each residue code, NG words per half, byte r of word g
+// = the tagged score of row 4 g + r.  Four rows' table words (four codes each)
+// are transposed with 8 byte permutes, 28 prmt per code group in place of a
+// table read and four logic ops per entry.
+template <int R>
+__device__ __forceinline__ void lin_profile(const uint32_t *tab, const uint8_t *V, int row0, int m,
+                                            bool on, uint32_t *prof)
+{
+    constexpr int NG = (R + 3) / 4;
+    const int lane = threadIdx.x & 31;
+    uint32_t a[2 * NG * 4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < NG * 4; ++r) {
+            const int i = row0 + h * R + r;
+            a[h * NG * 4 + r] = (uint32_t)(r < R && on && i < m ? (int)__ldg(V + i) : PG_NRES) * (LIN_ROWB / 4);
+        }
+    for (int w = 0; w < (LIN_NC + 3) / 4; ++w) {
+        uint32_t y[4][2 * NG];
+#pragma unroll
+        for (int g = 0; g < 2 * NG; ++g) {
+            const uint32_t x0 = tab[a[4 * g] + w], x1 = tab[a[4 * g + 1] + w];
+            const uint32_t x2 = tab[a[4 * g + 2] + w], x3 = tab[a[4 * g + 3] + w];
+            const uint32_t t0 = prmt(x0, x1, 0x5140u), t1 = prmt(x2, x3, 0x5140u);
+            const uint32_t t2 = prmt(x0, x1, 0x7362u), t3 = prmt(x2, x3, 0x7362u);
+            y[0][g] = prmt(t0, t1, 0x5410u);
+            y[1][g] = prmt(t0, t1, 0x7632u);
+            y[2][g] = prmt(t2, t3, 0x5410u);
+            y[3][g] = prmt(t2, t3, 0x7632u);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int c = 4 * w + q;
+            if (c >= LIN_NC) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t *d = prof + ((h * LIN_NC + c) * 32 + lane) * NG;
+                if (NG == 2) *reinterpret_cast<uint2 *>(d) = make_uint2(y[q][h * NG], y[q][h * NG + 1]);
+                else *d = y[q][h];
+            }
+        }
+    }
+}
+
+// the column residues of a lane, four at a time from aligned words; bytes past
+// the sequence read as the sentinel
+struct LinCols {
+    const uint32_t *w;      // word of the next group's upper bytes
+    int y, n;               // that word's first byte, as a column index
+    uint32_t cur, nxt;
+    uint32_t sh;
+    __device__ __forceinline__ uint32_t load() const
+    {
+        uint32_t v = 0x19191919u;
+        if (n > 0 && (unsigned)(y + 3) < (unsigned)(n + 3)) {
+            v = __ldg(w);
+            if (y + 4 > n) {
+                const uint32_t keep = (1u << (8 * (n - y))) - 1u;      // 1..3 bytes
+                v = (v & keep) | (0x19191919u & ~keep);
+            }
+        }
+        return v;
+    }
+    // x0: column index (0-based) of the first residue wanted
+    __device__ __forceinline__ void init(const uint8_t *H, int n_, int x0)
+    {
+        static_assert(NCODES == 25, "0x19 is the sentinel's code");
+        n = n_;
+        const uint8_t *p = H + x0;
+        const int a = (int)(reinterpret_cast<uintptr_t>(p) & 3u);
+        sh = 8u * (uint32_t)a;
+        w = reinterpret_cast<const uint32_t *>(p - a);
+        y = x0 - a;
+        cur = load();
+        ++w; y += 4;
+        nxt = load();
+    }
+    __device__ __forceinline__ uint32_t next()
+    {
+        const uint32_t r = __funnelshift_r(cur, nxt, sh);
+        cur = nxt;
+        ++w; y += 4;
+        nxt = load();
+        return r;
+    }
+};
+
+// best cell of a lane's two halves (local form): the running maximum, and
+// for each half the column and row of its first occurrence
+struct LinBest {
+    uint32_t sbs, seen;
+    int p0, p1;             // column << 3 | row of the lane
+};
+template <int R>
+__device__ __forceinline__ void lin_best(LinBest &b, const uint32_t (&H)[R], int j)
+{
+    uint32_t s = b.sbs;
+#pragma unroll
+    for (int r = 0; r + 1 < R; r += 2) s = __vimax3_s16x2(s, H[r], H[r + 1]);
+    if (R & 1) s = v16max(s, H[R - 1]);
+    b.sbs = s;
+    if (s != b.seen) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int v = half16(s, h);
+            if (v != half16(b.seen, h)) {
+                int rr = R - 1;
+#pragma unroll
+                for (int r = R - 1; r >= 0; --r)
+                    if (half16(H[r], h) == v) rr = r;
+                const int p = ((j - h) << 3) | rr;
+                if (h) b.p1 = p; else b.p0 = p;
+            }
+        }
+        b.seen = s;
+    }
+}
+
+struct LinConst {
+    uint32_t goL, goU;      // packed 4 go + tag of E / F
+    uint32_t four;          // 4, from memory: the multiply-adds below stay on the FMA pipe
+    int go4;
+};
+
+// one column of the lane's 2R rows; returns the direction word
+template <int R, bool LOCAL, bool BASE>
+__device__ __forceinline__ uint32_t lin_rows(uint32_t (&H)[R], uint32_t dgH, uint32_t in_h,
+                                             const uint32_t *pl, const uint32_t *ph,
+                                             const LinConst &c, uint32_t floor2)
+{
+    constexpr int NG = (R + 3) / 4;
+    uint32_t lo[NG], hi[NG];
+    if (NG == 2) {
+        const uint2 a = *reinterpret_cast<const uint2 *>(pl), b = *reinterpret_cast<const uint2 *>(ph);
+        lo[0] = a.x; lo[NG - 1] = a.y; hi[0] = b.x; hi[NG - 1] = b.y;
+    } else {
+        lo[0] = *pl; hi[0] = *ph;
+    }
+    uint32_t dl[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t s2 = prmt(lo[r >> 2], hi[r >> 2], sx_sel(r & 3));
+        uint32_t dg = v16add(r ? H[r ? r - 1 : 0] : dgH, s2);
+        if (LOCAL && BASE) dg = v16max(dg, floor2);
+        dl[r] = __viaddmax_s16x2(H[r], c.goL, dg);
+    }
+    uint32_t up = in_h, wa = 0, wb = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t t = LOCAL && !BASE ? __viaddmax_s16x2_relu(up, c.goU, dl[r])
+                                          : __viaddmax_s16x2(up, c.goU, dl[r]);
+        up = t & LIN_CLR;
+        H[r] = up;
+        wa = wa * c.four + t;
+        wb = wb * c.four + up;
+    }
+    return wa - wb;
+}
+
+// Regions of the L-lane classes: each L lanes of the warp pass their own region
+// (m = 0: none).  The result is that of the lane's region.
+template <bool LOCAL, int L, int R>
+__device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, const LinConst &c,
+                                        const uint8_t *V, int m, const uint8_t *Hs, int n, uint8_t *dir)
+{
+    constexpr int NG = (R + 3) / 4;
+    const int lane = threadIdx.x & 31;
+    const int sl = lane & (L - 1);
+    const bool has = m > 0 && n > 0;
+    const int v_last = has ? (m - 1) / R : -1;       // <= 2L - 1
+    const int t_last = v_last >> 1;
+    const bool on = sl <= t_last;
+    const int hi_on = 2 * sl + 1 <= v_last ? 1 : 0;
+    const int i_base = 2 * sl * R;
+    const int own = has ? n + v_last : 0;            // this region's steps
+    const unsigned lim = on ? (unsigned)(n + hi_on) : 0u;
+    __syncwarp();
+    lin_profile<R>(tab, V, i_base, m, on, prof);
+    __syncwarp();
+    // column 0 of the low half's rows, column -1 (sentinels) of the high half's
+    uint32_t H[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) H[r] = pk16(LOCAL ? 0 : c.go4 * (i_base + r + 1), LIN_NEG);
+    const int up0 = LOCAL ? 0 : c.go4 * i_base, lo0 = LOCAL ? 0 : c.go4 * (i_base + R);
+    const int hi0 = LOCAL ? 0 : c.go4 * (i_base + 2 * R);
+    uint32_t in_h = pk16(up0, lo0), out_h = pk16(lo0, hi0);
+    uint32_t bord = LOCAL ? 0u : (uint32_t)c.go4 << 16;       // H(0, j) of the first lane, in the high half
+    const uint32_t bstep = LOCAL ? 0u : (uint32_t)c.go4 << 16;
+    LinCols cols;
+    cols.init(Hs, has ? n : 0, -2 * sl);
+    const char *lbase = reinterpret_cast<const char *>(prof + lane * NG);
+    const char *pa = lbase + PG_NRES * (128 * NG);   // the sentinel's profile: column 0 of the high half
+    LinBest best{0u, 0u, 0, 0};
+    int nsteps = own;
+#pragma unroll
+    for (int o = L; o < 32; o <<= 1) nsteps = max(nsteps, __shfl_xor_sync(FULL, nsteps, o));
+    uint8_t *dst = dir + sl * 32;
+    for (int k0 = 0; k0 < nsteps; k0 += 4) {
+        const uint32_t res4 = cols.next();
+        const int x0 = k0 - 2 * sl;                  // low half's column at the first step, 0-based
+        uint32_t w[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t rh = __shfl_up_sync(FULL, out_h, 1, L);
+            const uint32_t dgH = in_h;
+            const uint32_t th = sl == 0 ? bord : rh;
+            if (!LOCAL) bord += bstep;
+            in_h = prmt(th, out_h, 0x5432u);
+            w[s] = 0;
+            if ((unsigned)(x0 + s) < lim) {
+                const char *ph = pa + LIN_NC * (128 * NG);
+                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
+                w[s] = lin_rows<R, LOCAL, false>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
+                                                 reinterpret_cast<const uint32_t *>(ph), c, 0u);
+                out_h = H[R - 1];
+                if (LOCAL) lin_best<R>(best, H, x0 + s + 1);
+            }
+        }
+        if (on && k0 < own)
+            *reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * (L * 32) + (k0 & 4) * 4) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    int4 res = make_int4(0, 0, 0, 0);
+    if (LOCAL) {
+        // first maximum in column-major order: the low half's rows before the
+        // high half's in a column, then the smaller column, then the smaller row
+        int bs = 0, bi = 0, bj = 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int s = half16(best.sbs, h);
+            const int sp = h ? best.p1 : best.p0;
+            const int sj = sp >> 3;
+            if (s > 0 && (s > bs || (s == bs && sj < bj))) { bs = s; bj = sj; bi = i_base + h * R + (sp & 7) + 1; }
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+            const int os = __shfl_xor_sync(FULL, bs, o);
+            const int oi = __shfl_xor_sync(FULL, bi, o);
+            const int oj = __shfl_xor_sync(FULL, bj, o);
+            if (os > bs || (os == bs && (oj < bj || (oj == bj && oi < bi)))) { bs = os; bi = oi; bj = oj; }
+        }
+        res = make_int4(bs >> 2, bi, bj, bs > 0 ? 1 : 0);
+    } else {
+        const int rl = has ? (m - 1) % R : -1, h = v_last & 1;
+        int hs = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r == rl) hs = half16(H[r], h);
+        res.x = __shfl_sync(FULL, hs, (lane & ~(L - 1)) + (t_last > 0 ? t_last : 0)) >> 2;
+    }
+    return res;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
+{
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(uint32_t *p, uint32_t v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
+}
+
+// Wait (one lane) until the stripe above has written `need` columns of its
+// boundary row.  Stripes are taken in list order, so the one waited for is
+// already running or done and the wait ends; after 2^24 polls (seconds) it
+// gives up, sets ST_WAIT, and the batch fails with an error.
+__device__ __forceinline__ void lin_wait(const uint32_t *p, uint32_t need, int *status)
+{
+    for (int it = 0; ld_acquire(p) < need; ++it) {
+        __nanosleep(64);
+        if ((it & 1023) == 1023 && (*(volatile int *)status & ST_WAIT)) return;
+        if (it >= (1 << 24)) { atomicOr(status, ST_WAIT); return; }
+    }
+}
+
+// One stripe of 64 R rows (the last: what is left) of a region on a warp.
+// Values are relative to the lane's base B (a multiple of 4, moved every 64
+// steps to the lane's current values).  V: the region's first row; rows rb ..
+// of it are this stripe's.  bin / bout: boundary rows (4 H of columns 1..n) of
+// the stripe above and of this one (null: none), pin / pout their progress.
+template <bool LOCAL, int R>
+__device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, const LinConst &c,
+                                           const uint8_t *V, int m, int rb, const uint8_t *Hs, int n,
+                                           uint8_t *dir, const int *bin, const uint32_t *pin, int *bout,
+                                           uint32_t *pout, int *status)
+{
+    constexpr int NG = (R + 3) / 4;
+    const int lane = threadIdx.x & 31;
+    const int rows = min(64 * R, m - rb);
+    const int v_last = (rows - 1) / R;
+    const int t_last = v_last >> 1;
+    const bool on = lane <= t_last;
+    const int hi_on = 2 * lane + 1 <= v_last ? 1 : 0;
+    const int i_base = rb + 2 * lane * R;
+    const unsigned lim = on ? (unsigned)(n + hi_on) : 0u;
+    __syncwarp();
+    lin_profile<R>(tab, V, i_base, m, on, prof);
+    __syncwarp();
+    // column 0, relative to the lane's first row there
+    int B = LOCAL ? 0 : c.go4 * i_base;
+    uint32_t H[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) H[r] = pk16(LOCAL ? 0 : c.go4 * (r + 1), LIN_NEG);
+    const int lo0 = LOCAL ? 0 : c.go4 * R, hi0 = LOCAL ? 0 : c.go4 * 2 * R;
+    uint32_t in_h = pk16(0, lo0), out_h = pk16(lo0, hi0);
+    LinCols cols;
+    cols.init(Hs, n, -2 * lane);
+    const char *lbase = reinterpret_cast<const char *>(prof + lane * NG);
+    const char *pa = lbase + PG_NRES * (128 * NG);
+    LinBest best{0u, 0u, 0, 0};
+    int abs0 = 0, abs1 = 0;                          // best 4 H of the low and high half's rows so far
+    uint32_t floor2 = 0, d2 = 0;
+    int bval = 0;
+    const int nsteps = n + v_last;
+    uint8_t *dst = dir + lane * 32;
+    for (int k0 = 0; k0 < nsteps; k0 += 4) {
+        if ((k0 & 31) == 0) {
+            if ((k0 & 63) == 0) {
+                // move the base of the lanes whose two halves hold real columns
+                const int sh = k0 - 1 - 2 * lane >= 1 ? lo16(H[0]) & ~3 : 0;
+                const uint32_t s2 = pk16(-sh, -sh);
+                if (LOCAL) {
+                    abs0 = max(abs0, lo16(best.sbs) + B);
+                    abs1 = max(abs1, hi16(best.sbs) + B);
+                }
+                B += sh;
+#pragma unroll
+                for (int r = 0; r < R; ++r) H[r] = v16add(H[r], s2);
+                in_h = v16add(in_h, s2);
+                out_h = v16add(out_h, s2);
+                if (LOCAL) {
+                    const int f = max(-B, LIN_NEG);
+                    floor2 = pk16(f, f);
+                    best.sbs = pk16(min(max(abs0 - B, LIN_NEG), 32767), min(max(abs1 - B, LIN_NEG), 32767));
+                    best.seen = best.sbs;
+                }
+                const int d = __shfl_up_sync(FULL, B, 1) - B;
+                d2 = pk16(0, d);                     // the lane above hands its high half down
+            }
+            const int j = k0 + 1 + lane;             // boundary columns of the next 32 steps
+            const int b0 = __shfl_sync(FULL, B, 0);
+            int h = LOCAL ? 0 : c.go4 * j;
+            if (bin) {
+                const int need = min(n, k0 + 32);
+                if (lane == 0 && k0 < n) lin_wait(pin, (uint32_t)need, status);
+                __syncwarp();
+                h = j <= n ? __ldcg(bin + j) : 0;
+            }
+            bval = (j <= n ? h - b0 : 0) << 16;
+        }
+        const uint32_t res4 = cols.next();
+        const int x0 = k0 - 2 * lane;
+        uint32_t w[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t rh = v16add(__shfl_up_sync(FULL, out_h, 1), d2);
+            const uint32_t bh = (uint32_t)__shfl_sync(FULL, bval, (k0 + s) & 31);
+            const uint32_t dgH = in_h;
+            const uint32_t th = lane == 0 ? bh : rh;
+            in_h = prmt(th, out_h, 0x5432u);
+            w[s] = 0;
+            if ((unsigned)(x0 + s) < lim) {
+                const char *ph = pa + LIN_NC * (128 * NG);
+                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
+                w[s] = lin_rows<R, LOCAL, true>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
+                                                reinterpret_cast<const uint32_t *>(ph), c, floor2);
+                out_h = H[R - 1];
+                if (LOCAL) lin_best<R>(best, H, x0 + s + 1);
+                // the stripe's last row, 64 R - 1: the last lane's high half, column x0 + s
+                if (bout && lane == 31 && x0 + s >= 1) bout[x0 + s] = hi16(out_h) + B;
+            }
+        }
+        if (on) *reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * 1024 + (k0 & 4) * 4) =
+                make_uint4(w[0], w[1], w[2], w[3]);
+        if (bout && lane == 31 && (k0 & 28) == 28 && x0 + 3 >= 1)
+            st_release(pout, (uint32_t)min(n, x0 + 3));
+    }
+    if (bout && lane == 31) st_release(pout, (uint32_t)n);
+    int4 res = make_int4(0, 0, 0, 0);
+    if (LOCAL) {
+        abs0 = max(abs0, lo16(best.sbs) + B);
+        abs1 = max(abs1, hi16(best.sbs) + B);
+        int bs = 0, bi = 0, bj = 0;
+        if (on) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int s = h ? abs1 : abs0;
+                const int sp = h ? best.p1 : best.p0;
+                const int sj = sp >> 3;
+                if (s > 0 && (s > bs || (s == bs && sj < bj))) { bs = s; bj = sj; bi = i_base + h * R + (sp & 7) + 1; }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int os = __shfl_xor_sync(FULL, bs, o);
+            const int oi = __shfl_xor_sync(FULL, bi, o);
+            const int oj = __shfl_xor_sync(FULL, bj, o);
+            if (os > bs || (os == bs && (oj < bj || (oj == bj && oi < bi)))) { bs = os; bi = oi; bj = oj; }
+        }
+        res = make_int4(bs >> 2, bi, bj, bs > 0 ? 1 : 0);
+    } else {
+        const int rl = (rows - 1) % R, h = v_last & 1;
+        int hs = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (r == rl) hs = half16(H[r], h) + B;
+        res.x = __shfl_sync(FULL, hs, t_last) >> 2;
+    }
+    return res;
+}
+
+// Jobs in list order from one counter: a group of 32 / L regions, or a stripe.
+template <bool LOCAL>
+__global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
+{
+    __shared__ __align__(16) int8_t tab8[LIN_NC * LIN_ROWB];
+    __shared__ uint32_t sl[3 * LIN_SEG + 1];
+    lin_table(tab8, lp.kp.sm);
+    for (int t = threadIdx.x; t < 3 * LIN_SEG; t += blockDim.x) sl[t] = lp.tot->seg[t];
+    if (threadIdx.x == 0) sl[3 * LIN_SEG] = lp.tot->jobs;
+    __syncthreads();
+    const uint32_t *tab = reinterpret_cast<const uint32_t *>(tab8);
+    const int lane = threadIdx.x & 31;
+    uint32_t *prof = reinterpret_cast<uint32_t *>(g_dyn_prof) + (threadIdx.x >> 5) * (LIN_PROF / 4);
+    LinConst c;
+    c.go4 = 4 * lp.kp.go;
+    c.goL = pk16(c.go4 + lp.e_first, c.go4 + lp.e_first);
+    c.goU = pk16(c.go4 + 1 - lp.e_first, c.go4 + 1 - lp.e_first);
+    c.four = (uint32_t)lp.kp.four;
+    int seg = 0;
+    for (;;) {
+        uint32_t job = 0;
+        if (lane == 0) job = atomicAdd(&lp.tot->next_job, 1u);
+        job = __shfl_sync(FULL, job, 0);
+        if (job >= sl[3 * LIN_SEG]) break;
+        while (seg + 1 < LIN_SEG && job >= sl[2 * LIN_SEG + seg + 1]) ++seg;
+        const int lanes = lin_seg_lanes(seg), group = lin_seg_group(seg);
+        const uint32_t q = (job - sl[2 * LIN_SEG + seg]) * (uint32_t)group + (uint32_t)(lane / lanes);
+        const bool has = q < sl[LIN_SEG + seg];
+        const uint32_t pos = sl[seg] + q;
+        LinReg e;
+        e.m = e.n = 0; e.v = e.h = 0; e.off = 0; e.stripe = 0; e.nstripe = 1;
+        if (has) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(lp.list + pos);
+            uint4 *d = reinterpret_cast<uint4 *>(&e);
+            d[0] = src[0];
+            d[1] = src[1];
+        }
+        const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
+        uint8_t *dir = lp.arena + (uint64_t)e.off * 32u;
+        int4 r;
+        if (seg < 4) {
+            const uint32_t tu = lin_tile_units(32, e.n), ru = lin_row_units(e.n);
+            uint8_t *rows = dir + (uint64_t)e.nstripe * tu * 32u;
+            const int *bin = e.stripe ? (const int *)(rows + (uint64_t)(e.stripe - 1) * ru * 32u) : nullptr;
+            int *bout = e.stripe + 1 < e.nstripe ? (int *)(rows + (uint64_t)e.stripe * ru * 32u) : nullptr;
+            uint8_t *d = dir + (uint64_t)e.stripe * tu * 32u;
+            const uint32_t *pin = lp.prog + pos - (e.stripe ? 1 : 0);
+            uint32_t *pout = lp.prog + pos;
+#define LIN_STRIPE(R_) lin_stripe<LOCAL, R_>(tab, prof, c, V, e.m, (int)e.stripe * 64 * R_, Hs, e.n, d, bin, pin, bout, pout, lp.kp.status)
+            switch (seg) {
+            case 0: r = LIN_STRIPE(8); break;
+            case 1: r = LIN_STRIPE(7); break;
+            case 2: r = LIN_STRIPE(6); break;
+            default: r = LIN_STRIPE(5); break;
+            }
+#undef LIN_STRIPE
+        } else {
+#define LIN_SUB(L_, R_) lin_sub<LOCAL, L_, R_>(tab, prof, c, V, e.m, Hs, e.n, dir)
+            switch (seg) {
+            case 4: r = LIN_SUB(32, 8); break;
+            case 5: r = LIN_SUB(32, 7); break;
+            case 6: r = LIN_SUB(32, 6); break;
+            case 7: r = LIN_SUB(32, 5); break;
+            case 8: r = LIN_SUB(16, 8); break;
+            case 9: r = LIN_SUB(16, 7); break;
+            case 10: r = LIN_SUB(16, 6); break;
+            case 11: r = LIN_SUB(16, 5); break;
+            case 12: r = LIN_SUB(8, 8); break;
+            case 13: r = LIN_SUB(8, 7); break;
+            case 14: r = LIN_SUB(8, 6); break;
+            case 15: r = LIN_SUB(8, 5); break;
+            case 16: r = LIN_SUB(8, 4); break;
+            default: r = LIN_SUB(8, 2); break;
+            }
+#undef LIN_SUB
+        }
+        if (has && (lane & (lanes - 1)) == 0) lp.dp[pos] = r;
+    }
+}
+
+// ------------------------------------------------------------ the traceback
+// One thread per region, in list order (neighbours of nearly equal length).  A
+// move has no branch: the tag says which of row and column step back.  Counts
+// what computeAlignmentStats counts (src/align/SeqanFullAligner.cpp:238-246).
+template <bool LOCAL>
+__global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
+{
+    __shared__ int8_t sm[PG_NRES * 32];
+    if (LOCAL) {
+        for (int t = threadIdx.x; t < PG_NRES * 32; t += blockDim.x)
+            sm[t] = (t & 31) < PG_NRES ? lp.kp.sm[(t >> 5) * PG_NRES + (t & 31)] : (int8_t)0;
+        __syncthreads();
+    }
+    const uint32_t entries = lp.tot->entries;
+    const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pos >= entries) return;
+    LinReg e;
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(lp.list + pos);
+        uint4 *d = reinterpret_cast<uint4 *>(&e);
+        d[0] = src[0];
+        d[1] = src[1];
+    }
+    if (e.stripe) return;
+    const int m = e.m, n = e.n, ns = e.nstripe;
+    int seg = 0;
+    while (seg + 1 < LIN_SEG && pos >= lp.tot->seg[seg + 1]) ++seg;
+    const int L = lin_seg_lanes(seg), R = lin_seg_rows(seg);
+    int4 d = lp.dp[pos + (LOCAL ? 0 : ns - 1)];
+    if (LOCAL)
+        for (int s = 1; s < ns; ++s) {               // ties: smaller column, then smaller row
+            const int4 o = lp.dp[pos + s];
+            if (o.w && (!d.w || o.x > d.x || (o.x == d.x && o.z < d.z))) d = o;
+        }
+    int i = LOCAL ? d.y : m, j = LOCAL ? d.z : n;
+    uint32_t M = 0, D = 0, G = 0;
+    int last = 0;
+    if (!LOCAL || d.w) {
+        const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
+        const uint32_t tile_row = (uint32_t)L * 8u;  // words per 8 steps
+        const int e_tag = lp.e_first, f_tag = 1 - lp.e_first, go = lp.kp.go;
+        const uint32_t stripe_words = lin_tile_units(L, n) * 8u;
+        int st = (i - 1) / (2 * L * R);
+        int v = (i - 1 - st * 2 * L * R) / R;
+        int sh = 2 * (R - 1 - (i - 1 - st * 2 * L * R - v * R));   // the row's bits in its half
+        const uint32_t *base = reinterpret_cast<const uint32_t *>(lp.arena + (uint64_t)e.off * 32u) +
+                               (uint64_t)st * stripe_words;
+        int h = LOCAL ? d.x : 1;
+        while (i > 0 && j > 0 && h > 0) {
+            const int k = j - 1 + v;
+            const uint32_t *w = base + (uint32_t)(k >> 3) * tile_row + (uint32_t)((v >> 1) * 8 + (k & 7));
+            const uint32_t word = __ldg(w);
+            // the tile before this one along the lane: in L1 by the time the walk gets there
+            if ((k & 7) == 7 && k > 7) asm volatile("prefetch.global.L1 [%0];" :: "l"(w - tile_row));
+            int sab = 0;
+            if (LOCAL) sab = sm[__ldg(V + i - 1) * 32 + __ldg(Hs + j - 1)];
+            const int tag = (int)(word >> (16 * (v & 1) + sh)) & 3;
+            const bool up = tag != e_tag, left = tag != f_tag;
+            const int mv = tag >= 2 ? 0 : tag == f_tag ? 1 : 2;
+            M += tag == 3 ? 1u : 0u;
+            D += tag >= 2 ? 1u : 0u;
+            G += mv != 0 && mv != last ? 1u : 0u;
+            last = mv;
+            if (LOCAL) h -= mv ? go : sab;
+            i -= up ? 1 : 0;
+            j -= left ? 1 : 0;
+            sh += up ? 2 : 0;
+            if (sh == 2 * R) {
+                sh = 0;
+                if (--v < 0) { v = 2 * L - 1; base -= stripe_words; }
+            }
+        }
+        if (!LOCAL && ((i > 0 && last != 1) || (j > 0 && last != 2))) ++G;
+    }
+    if (!LOCAL) {
+        lp.walk[e.key] = make_int4(d.x, (int)M, (int)D, (int)G);
+        return;
+    }
+    pg_result o = empty_result();
+    o.cells = sat_u32((uint64_t)m * (uint64_t)n);
+    if (d.w) {
+        const uint32_t len = (uint32_t)((d.y - i) + (d.z - j)) - D;
+        o.score = d.x;
+        o.aln_len = len; o.matches = M; o.gap_opens = G;
+        o.beg_v = (uint16_t)i; o.end_v = (uint16_t)d.y;
+        o.beg_h = (uint16_t)j; o.end_h = (uint16_t)d.z;
+        if (len > 0) { o.identity = identity_of(M, len); o.flags = 0; }
+    }
+    apply_filter(o, m, n, lp.kp.cov_thr, lp.kp.ani_thr);
+    lp.kp.out[e.key] = o;
+}
+
+// X-drop: the record of each pair from its regions' walks (the better seed by
+// identity, as SeqanXdropAligner.cpp:303-354), one thread per pair
+static __global__ void __launch_bounds__(256) k_lin_finish(const LinParams lp)
+{
+    const KParams &kp = lp.kp;
+    const int gmax = kp.go;                          // go > ge
+    for (uint64_t p = lp.p0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < lp.p1;
+         p += (uint64_t)gridDim.x * blockDim.x) {
+        const LinPair r = lin_pair<true>(kp, p);
+        pg_result best = empty_result();
+        if (r.bad) {
+            atomicOr(kp.status, ST_BAD_INDEX);
+            kp.out[p] = best;
+            continue;
+        }
+        const pg_pair pr = kp.pairs[p];
+        const uint64_t ri = (uint64_t)pr.row + kp.roff, ci = (uint64_t)pr.col + kp.coff;
+        const XdRec rec0 = kp.xd[2 * p], rec1 = kp.xd[2 * p + 1];
+        uint64_t cells = 0;
+        bool bad = false, have = false;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const XdRec &rec = s ? rec1 : rec0;
+            if (rec.flags & XF_NONE) continue;
+            if (rec.flags & XF_SAME) {
+                cells += (uint64_t)rec0.cells + (uint64_t)(rec0.ev - rec0.bv) * (uint64_t)(rec0.eh - rec0.bh);
+                continue;
+            }
+            if (rec.flags & XF_BAD) bad = true;
+            const int rm = rec.ev - rec.bv, rn = rec.eh - rec.bh;
+            cells += rec.cells + (uint64_t)rm * (uint64_t)rn;
+            if (s == 1 && !(rec0.flags & XF_NONE) && rec.bv == rec0.bv && rec.ev == rec0.ev &&
+                rec.bh == rec0.bh && rec.eh == rec0.eh) continue;   // the first seed's region again
+            int score = 0;
+            uint32_t M = 0, D = 0, G = 0;
+            if (r.dp[s]) {
+                const int4 w = lp.walk[2 * p + s];
+                score = w.x; M = (uint32_t)w.y; D = (uint32_t)w.z; G = (uint32_t)w.w;
+            } else if (rm + rn > 0) {
+                score = kp.go + (rm + rn - 1) * gmax;               // one gap run
+                G = 1;
+            }
+            const uint32_t L = (uint32_t)(rm + rn) - D;
+            pg_result cur;
+            cur.score = score; cur.aln_len = L; cur.matches = M; cur.gap_opens = G;
+            cur.beg_v = rec.bv; cur.end_v = rec.ev;
+            cur.beg_h = rec.bh; cur.end_h = rec.eh;
+            cur.seed_used = (uint8_t)s; cur.pad = 0; cur.cells = 0; cur.score_aln = 0.0f;
+            if (L == 0) { cur.identity = 0.0f; cur.flags = PG_RF_EMPTY; }
+            else { cur.identity = identity_of(M, L); cur.flags = 0; }
+            const bool nan = ((cur.flags | best.flags) & PG_RF_EMPTY) != 0;
+            if (!have || (!nan && cur.identity > best.identity)) { best = cur; have = true; }
+        }
+        best.cells = sat_u32(cells);
+        if (bad) best.flags |= PG_RF_BAD_SEED;
+        apply_filter(best, (int)(kp.roffs[ri + 1] - kp.roffs[ri]), (int)(kp.coffs[ci + 1] - kp.coffs[ci]),
+                     kp.cov_thr, kp.ani_thr);
+        kp.out[p] = best;
+    }
+}
+
+// ------------------------------------------------------------ host launches
+template <bool XDROP>
+cudaError_t lin_attributes(int *blocks_per_sm)
+{
+    cudaError_t e = cudaFuncSetAttribute(k_lin_dp<!XDROP>, cudaFuncAttributeMaxDynamicSharedMemorySize, LIN_DYN);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k_lin_dp<!XDROP>, WARPS * 32, LIN_DYN);
+    return e;
+}
+// class sizes and totals of the pairs [p0, p1): 2 launches
+template <bool XDROP>
+void lin_count(const LinParams &lp, int nsm, cudaStream_t st)
+{
+    const uint64_t n = lp.p1 - lp.p0;
+    const uint64_t grid = (n + LIN_PT - 1) / LIN_PT;
+    k_lin_hist<XDROP><<<(int)(grid < (uint64_t)nsm * 8 ? grid : (uint64_t)nsm * 8), LIN_PT, 0, st>>>(lp);
+    k_lin_scan<<<1, 1024, 0, st>>>(lp);
+}
+// list, DP, traceback and results; returns the launches
+template <bool XDROP>
+int lin_align(const LinParams &lp, uint32_t entries, uint32_t jobs, int nsm, int max_blocks, cudaStream_t st)
+{
+    const uint64_t n = lp.p1 - lp.p0;
+    const uint64_t gp = (n + LIN_PT * LIN_PP - 1) / (LIN_PT * LIN_PP);
+    k_lin_place<XDROP><<<(int)(gp < (uint64_t)nsm * 8 ? gp : (uint64_t)nsm * 8), LIN_PT, 0, st>>>(lp);
+    const int gd = (int)(jobs < (uint32_t)max_blocks ? (jobs ? jobs : 1) : (uint32_t)max_blocks);
+    k_lin_dp<!XDROP><<<gd, WARPS * 32, LIN_DYN, st>>>(lp);
+    k_lin_walk<!XDROP><<<entries ? (entries + 255) / 256 : 1, 256, 0, st>>>(lp);
+    if (XDROP) {
+        const uint64_t gf = (n + 255) / 256;
+        k_lin_finish<<<(int)(gf < (uint64_t)nsm * 8 ? gf : (uint64_t)nsm * 8), 256, 0, st>>>(lp);
+    }
+    return XDROP ? 4 : 3;
+}
+
+}  // namespace pg
