@@ -38,6 +38,7 @@
 // values relative to a base that follows them, so no region is too large.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "pg_kernels.cuh"
 #include "pg_lin.h"
@@ -89,7 +90,7 @@ struct LinParams {
     uint32_t *cur;                                 // LIN_NB bucket cursors
     LinTotals *tot;
     LinReg *list;
-    int4 *dp;                                      // per entry: score, end row, end column, have
+    int4 *dp;                                      // per entry: score; local: low / high halves that reach it, have
     uint32_t *prog;                                // per entry: columns of its boundary row written
     uint8_t *arena;
     int4 *walk;                                    // X-drop, per key: score, matches, diagonals, gap runs
@@ -136,10 +137,32 @@ __host__ __device__ __forceinline__ uint32_t lin_tile_units(int lanes, int n)
     return (uint32_t)((n + 2 * lanes - 1 + 7) >> 3) * (uint32_t)lanes;
 }
 __host__ __device__ __forceinline__ uint32_t lin_row_units(int n) { return (uint32_t)((n + 1 + 7) >> 3); }
-__host__ __device__ __forceinline__ uint32_t lin_units(int seg, int m, int n)
+// 32-step chunks of one stripe
+__host__ __device__ __forceinline__ uint32_t lin_chunks(int lanes, int n) { return (uint32_t)((n + 2 * lanes - 1 + 31) >> 5); }
+// Arena of a region, planes of `ns` stripes each, in 32-byte units: direction
+// words; in the local form the lanes' edge words (same layout), their rows'
+// values at each chunk's start, the bases those are relative to (stripes) and the
+// chunk of each half's maximum; last, the boundary rows between stripes.
+struct LinPlanes {
+    uint32_t tile, snap, base, ids;                  // units of one stripe
+    __host__ __device__ __forceinline__ LinPlanes(bool local, int seg, int n)
+    {
+        const int l = lin_seg_lanes(seg);
+        const uint32_t ch = local ? lin_chunks(l, n) : 0;
+        tile = lin_tile_units(l, n);
+        snap = ch * (uint32_t)l;
+        base = seg < 4 ? ch * 4u : 0u;
+        ids = local ? (uint32_t)l / 8u : 0u;
+    }
+    __host__ __device__ __forceinline__ uint32_t stripe(bool local) const
+    {
+        return tile * (local ? 2u : 1u) + snap + base + ids;
+    }
+};
+__host__ __device__ __forceinline__ uint32_t lin_units(bool local, int seg, int m, int n)
 {
-    const int s = lin_stripes(seg, m);
-    return (uint32_t)s * lin_tile_units(lin_seg_lanes(seg), n) + (uint32_t)(s - 1) * lin_row_units(n);
+    const uint32_t s = (uint32_t)lin_stripes(seg, m);
+    return s * LinPlanes(local, seg, n).stripe(local) + (s - 1) * lin_row_units(n);
 }
 
 // the DP regions of pair p: X-drop up to two (one per seed), SW one
@@ -198,7 +221,7 @@ __global__ void __launch_bounds__(LIN_PT) k_lin_hist(const LinParams lp)
             if (!r.dp[s]) continue;
             const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
             atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])], (uint32_t)lin_stripes(seg, r.m[s]));
-            units += lin_units(seg, r.m[s], r.n[s]);
+            units += lin_units(!XDROP, seg, r.m[s], r.n[s]);
         }
     }
 #pragma unroll
@@ -284,7 +307,7 @@ __global__ void __launch_bounds__(LIN_PT) k_lin_place(const LinParams lp)
                 const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
                 rank[q * NS + s] = atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])],
                                              (uint32_t)lin_stripes(seg, r.m[s]));
-                off[q * NS + s] = atomicAdd(&su, lin_units(seg, r.m[s], r.n[s]));
+                off[q * NS + s] = atomicAdd(&su, lin_units(!XDROP, seg, r.m[s], r.n[s]));
                 cells += (unsigned long long)r.m[s] * (unsigned long long)r.n[s];
             }
         }
@@ -400,21 +423,24 @@ __device__ __forceinline__ void lin_profile(const uint32_t *tab, const uint8_t *
 }
 
 // the column residues of a lane, four at a time from aligned words; bytes past
-// the sequence read as the sentinel
+// the sequence read as the sentinel.  A word is loaded a group ahead and masked
+// only when it is used, so that nothing waits on the load in between.
 struct LinCols {
-    const uint32_t *w;      // word of the next group's upper bytes
-    int y, n;               // that word's first byte, as a column index
+    const uint32_t *w;      // the word last loaded
+    int y, n;               // its first byte, as a column index
     uint32_t cur, nxt;
     uint32_t sh;
     __device__ __forceinline__ uint32_t load() const
     {
         uint32_t v = 0x19191919u;
-        if (n > 0 && (unsigned)(y + 3) < (unsigned)(n + 3)) {
-            v = __ldg(w);
-            if (y + 4 > n) {
-                const uint32_t keep = (1u << (8 * (n - y))) - 1u;      // 1..3 bytes
-                v = (v & keep) | (0x19191919u & ~keep);
-            }
+        if (n > 0 && (unsigned)(y + 3) < (unsigned)(n + 3)) v = __ldg(w);
+        return v;
+    }
+    __device__ __forceinline__ uint32_t masked(uint32_t v) const
+    {
+        if (y + 4 > n && y < n) {
+            const uint32_t keep = (1u << (8 * (n - y))) - 1u;      // 1..3 bytes
+            v = (v & keep) | (0x19191919u & ~keep);
         }
         return v;
     }
@@ -428,49 +454,52 @@ struct LinCols {
         sh = 8u * (uint32_t)a;
         w = reinterpret_cast<const uint32_t *>(p - a);
         y = x0 - a;
-        cur = load();
+        cur = masked(load());
         ++w; y += 4;
         nxt = load();
     }
     __device__ __forceinline__ uint32_t next()
     {
-        const uint32_t r = __funnelshift_r(cur, nxt, sh);
-        cur = nxt;
+        const uint32_t v = masked(nxt);
+        const uint32_t r = __funnelshift_r(cur, v, sh);
+        cur = v;
         ++w; y += 4;
         nxt = load();
         return r;
     }
 };
 
-// best cell of a lane's two halves (local form): the running maximum, and
-// for each half the column and row of its first occurrence
-struct LinBest {
-    uint32_t sbs, seen;
-    int p0, p1;             // column << 3 | row of the lane
-};
+// maximum of a column's rows, per half, with a running one
 template <int R>
-__device__ __forceinline__ void lin_best(LinBest &b, const uint32_t (&H)[R], int j)
+__device__ __forceinline__ uint32_t lin_max(uint32_t s, const uint32_t (&H)[R])
 {
-    uint32_t s = b.sbs;
 #pragma unroll
     for (int r = 0; r + 1 < R; r += 2) s = __vimax3_s16x2(s, H[r], H[r + 1]);
-    if (R & 1) s = v16max(s, H[R - 1]);
-    b.sbs = s;
-    if (s != b.seen) {
+    return R & 1 ? v16max(s, H[R - 1]) : s;
+}
+
+// where a lane of the local form leaves what lin_locate needs
+struct LinTrack {
+    uint8_t *snap;          // [chunk][lane] 32 bytes: its rows at the chunk's start
+    int *base;              // [chunk][lane] their base (stripes)
+    uint32_t *ids;          // [lane] chunk of the low and the high half's maximum
+};
+template <int R>
+__device__ __forceinline__ void lin_snap(uint8_t *dst, const uint32_t (&H)[R])
+{
+    uint32_t v[8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int v = half16(s, h);
-            if (v != half16(b.seen, h)) {
-                int rr = R - 1;
-#pragma unroll
-                for (int r = R - 1; r >= 0; --r)
-                    if (half16(H[r], h) == v) rr = r;
-                const int p = ((j - h) << 3) | rr;
-                if (h) b.p1 = p; else b.p0 = p;
-            }
-        }
-        b.seen = s;
-    }
+    for (int r = 0; r < 8; ++r) v[r] = r < R ? H[r < R ? r : 0] : 0u;
+    reinterpret_cast<uint4 *>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    if (R > 4) reinterpret_cast<uint4 *>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+}
+// the halves whose maximum rose during chunk c
+__device__ __forceinline__ void lin_chunk(uint32_t sbs, uint32_t &seen, uint32_t &cid, int c)
+{
+    const uint32_t x = sbs ^ seen;
+    if (x & 0xffffu) cid = (cid & 0xffff0000u) | (uint32_t)c;
+    if (x >> 16) cid = (cid & 0xffffu) | ((uint32_t)c << 16);
+    seen = sbs;
 }
 
 struct LinConst {
@@ -518,7 +547,8 @@ __device__ __forceinline__ uint32_t lin_rows(uint32_t (&H)[R], uint32_t dgH, uin
 // (m = 0: none).  The result is that of the lane's region.
 template <bool LOCAL, int L, int R>
 __device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, const LinConst &c,
-                                        const uint8_t *V, int m, const uint8_t *Hs, int n, uint8_t *dir)
+                                        const uint8_t *V, int m, const uint8_t *Hs, int n, uint8_t *dir,
+                                        const LinTrack &tr)
 {
     constexpr int NG = (R + 3) / 4;
     const int lane = threadIdx.x & 31;
@@ -547,15 +577,24 @@ __device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, con
     cols.init(Hs, has ? n : 0, -2 * sl);
     const char *lbase = reinterpret_cast<const char *>(prof + lane * NG);
     const char *pa = lbase + PG_NRES * (128 * NG);   // the sentinel's profile: column 0 of the high half
-    LinBest best{0u, 0u, 0, 0};
-    int nsteps = own;
+    uint32_t sbs = 0, seen = 0, cid = 0;
+    // steps of the longest region; the steps where every lane that holds rows is
+    // inside its columns need no test per lane (the others compute in vain there):
+    // with the residues masked at their use, 400k X-drop pairs' DP 5.83 -> 4.82 ms
+    int nsteps = own, ks = on ? 2 * sl : 0, ke = has ? n : 0x7fffffff;
 #pragma unroll
-    for (int o = L; o < 32; o <<= 1) nsteps = max(nsteps, __shfl_xor_sync(FULL, nsteps, o));
+    for (int o = 16; o > 0; o >>= 1) {
+        nsteps = max(nsteps, __shfl_xor_sync(FULL, nsteps, o));
+        ks = max(ks, __shfl_xor_sync(FULL, ks, o));
+        ke = min(ke, __shfl_xor_sync(FULL, ke, o));
+    }
     uint8_t *dst = dir + sl * 32;
-    for (int k0 = 0; k0 < nsteps; k0 += 4) {
+    const size_t plane = (size_t)lin_tile_units(L, n) * 32u;
+    // four steps (a lambda, for its two uses)
+    auto group = [&](const int k0, auto test) {
         const uint32_t res4 = cols.next();
         const int x0 = k0 - 2 * sl;                  // low half's column at the first step, 0-based
-        uint32_t w[4];
+        uint32_t w[4], e[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             const uint32_t rh = __shfl_up_sync(FULL, out_h, 1, L);
@@ -564,39 +603,43 @@ __device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, con
             if (!LOCAL) bord += bstep;
             in_h = prmt(th, out_h, 0x5432u);
             w[s] = 0;
-            if ((unsigned)(x0 + s) < lim) {
+            if (!decltype(test)::value || (unsigned)(x0 + s) < lim) {
                 const char *ph = pa + LIN_NC * (128 * NG);
                 pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
                 w[s] = lin_rows<R, LOCAL, false>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
                                                  reinterpret_cast<const uint32_t *>(ph), c, 0u);
                 out_h = H[R - 1];
-                if (LOCAL) lin_best<R>(best, H, x0 + s + 1);
+                if (LOCAL) sbs = lin_max<R>(sbs, H);
             }
+            e[s] = out_h;
         }
-        if (on && k0 < own)
-            *reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * (L * 32) + (k0 & 4) * 4) =
-                make_uint4(w[0], w[1], w[2], w[3]);
+        if (on && k0 < own) {
+            uint4 *d = reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * (L * 32) + (k0 & 4) * 4);
+            *d = make_uint4(w[0], w[1], w[2], w[3]);
+            if (LOCAL) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(d) + plane) = make_uint4(e[0], e[1], e[2], e[3]);
+        }
+    };
+    for (int k0 = 0; k0 < nsteps; k0 += 4) {
+        if (LOCAL && (k0 & 31) == 0 && k0) {
+            lin_chunk(sbs, seen, cid, (k0 >> 5) - 1);
+            if (on && k0 < own) lin_snap<R>(tr.snap + ((size_t)(k0 >> 5) * L + sl) * 32, H);
+        }
+        if (k0 >= ks && k0 + 4 <= ke) group(k0, std::false_type());
+        else group(k0, std::true_type());
     }
     int4 res = make_int4(0, 0, 0, 0);
     if (LOCAL) {
-        // first maximum in column-major order: the low half's rows before the
-        // high half's in a column, then the smaller column, then the smaller row
-        int bs = 0, bi = 0, bj = 0;
+        lin_chunk(sbs, seen, cid, (nsteps - 1) >> 5);
+        if (has) tr.ids[sl] = cid;
+        if (!on) sbs = 0;
+        int bs = max(lo16(sbs), hi16(sbs));
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int s = half16(best.sbs, h);
-            const int sp = h ? best.p1 : best.p0;
-            const int sj = sp >> 3;
-            if (s > 0 && (s > bs || (s == bs && sj < bj))) { bs = s; bj = sj; bi = i_base + h * R + (sp & 7) + 1; }
-        }
-#pragma unroll
-        for (int o = L / 2; o > 0; o >>= 1) {
-            const int os = __shfl_xor_sync(FULL, bs, o);
-            const int oi = __shfl_xor_sync(FULL, bi, o);
-            const int oj = __shfl_xor_sync(FULL, bj, o);
-            if (os > bs || (os == bs && (oj < bj || (oj == bj && oi < bi)))) { bs = os; bi = oi; bj = oj; }
-        }
-        res = make_int4(bs >> 2, bi, bj, bs > 0 ? 1 : 0);
+        for (int o = L / 2; o > 0; o >>= 1) bs = max(bs, __shfl_xor_sync(FULL, bs, o));
+        const int g = lane & ~(L - 1);
+        const uint32_t lm = L == 32 ? FULL : (1u << (L & 31)) - 1u;
+        const uint32_t m0 = __ballot_sync(FULL, lo16(sbs) == bs) >> g & lm;
+        const uint32_t m1 = __ballot_sync(FULL, hi16(sbs) == bs) >> g & lm;
+        res = make_int4(bs >> 2, bs > 0 ? (int)m0 : 0, bs > 0 ? (int)m1 : 0, bs > 0 ? 1 : 0);
     } else {
         const int rl = has ? (m - 1) % R : -1, h = v_last & 1;
         int hs = 0;
@@ -641,7 +684,7 @@ template <bool LOCAL, int R>
 __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, const LinConst &c,
                                            const uint8_t *V, int m, int rb, const uint8_t *Hs, int n,
                                            uint8_t *dir, const int *bin, const uint32_t *pin, int *bout,
-                                           uint32_t *pout, int *status)
+                                           uint32_t *pout, size_t plane, const LinTrack &tr, int *status)
 {
     constexpr int NG = (R + 3) / 4;
     const int lane = threadIdx.x & 31;
@@ -666,23 +709,56 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
     cols.init(Hs, n, -2 * lane);
     const char *lbase = reinterpret_cast<const char *>(prof + lane * NG);
     const char *pa = lbase + PG_NRES * (128 * NG);
-    LinBest best{0u, 0u, 0, 0};
+    uint32_t sbs = 0, seen = 0, cid = 0;
     int abs0 = 0, abs1 = 0;                          // best 4 H of the low and high half's rows so far
-    uint32_t floor2 = 0, d2 = 0;
+    uint32_t floor2 = 0, d2 = 0, b2 = 0;
     int bval = 0;
     const int nsteps = n + v_last;
+    const int ks = 2 * t_last;
     uint8_t *dst = dir + lane * 32;
+    auto group = [&](const int k0, auto test) {
+        const uint32_t res4 = cols.next();
+        const int x0 = k0 - 2 * lane;
+        uint32_t w[4], e[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t rh = v16add(__shfl_up_sync(FULL, out_h, 1), d2);
+            const uint32_t bh = (uint32_t)__shfl_sync(FULL, bval, (k0 + s) & 31);
+            const uint32_t dgH = in_h;
+            const uint32_t th = lane == 0 ? bh : rh;
+            in_h = prmt(th, out_h, 0x5432u);
+            w[s] = 0;
+            if (!decltype(test)::value || (unsigned)(x0 + s) < lim) {
+                const char *ph = pa + LIN_NC * (128 * NG);
+                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
+                w[s] = lin_rows<R, LOCAL, true>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
+                                                reinterpret_cast<const uint32_t *>(ph), c, floor2);
+                out_h = H[R - 1];
+                if (LOCAL) sbs = lin_max<R>(sbs, H);
+                // the stripe's last row, 64 R - 1: the last lane's high half, column x0 + s
+                if (bout && lane == 31 && x0 + s >= 1) bout[x0 + s] = hi16(out_h) + B;
+            }
+            if (LOCAL) e[s] = v16add(out_h, b2);
+        }
+        if (on) {
+            uint4 *d = reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * 1024 + (k0 & 4) * 4);
+            *d = make_uint4(w[0], w[1], w[2], w[3]);
+            if (LOCAL) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(d) + plane) = make_uint4(e[0], e[1], e[2], e[3]);
+        }
+    };
     for (int k0 = 0; k0 < nsteps; k0 += 4) {
         if ((k0 & 31) == 0) {
+            if (LOCAL && k0) lin_chunk(sbs, seen, cid, (k0 >> 5) - 1);
             if ((k0 & 63) == 0) {
                 // move the base of the lanes whose two halves hold real columns
                 const int sh = k0 - 1 - 2 * lane >= 1 ? lo16(H[0]) & ~3 : 0;
                 const uint32_t s2 = pk16(-sh, -sh);
                 if (LOCAL) {
-                    abs0 = max(abs0, lo16(best.sbs) + B);
-                    abs1 = max(abs1, hi16(best.sbs) + B);
+                    abs0 = max(abs0, lo16(sbs) + B);
+                    abs1 = max(abs1, hi16(sbs) + B);
                 }
                 B += sh;
+                b2 = pk16(B, B);
 #pragma unroll
                 for (int r = 0; r < R; ++r) H[r] = v16add(H[r], s2);
                 in_h = v16add(in_h, s2);
@@ -690,11 +766,17 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
                 if (LOCAL) {
                     const int f = max(-B, LIN_NEG);
                     floor2 = pk16(f, f);
-                    best.sbs = pk16(min(max(abs0 - B, LIN_NEG), 32767), min(max(abs1 - B, LIN_NEG), 32767));
-                    best.seen = best.sbs;
+                    // the maximum so far, as far as the new base can tell it: past
+                    // int16 no value of the next 64 columns reaches it
+                    sbs = pk16(min(max(abs0 - B, LIN_NEG), 32767), min(max(abs1 - B, LIN_NEG), 32767));
+                    seen = sbs;
                 }
                 const int d = __shfl_up_sync(FULL, B, 1) - B;
                 d2 = pk16(0, d);                     // the lane above hands its high half down
+            }
+            if (LOCAL && k0 && on) {
+                lin_snap<R>(tr.snap + ((size_t)(k0 >> 5) * 32 + lane) * 32, H);
+                tr.base[(k0 >> 5) * 32 + lane] = B;
             }
             const int j = k0 + 1 + lane;             // boundary columns of the next 32 steps
             const int b0 = __shfl_sync(FULL, B, 0);
@@ -707,56 +789,23 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
             }
             bval = (j <= n ? h - b0 : 0) << 16;
         }
-        const uint32_t res4 = cols.next();
-        const int x0 = k0 - 2 * lane;
-        uint32_t w[4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const uint32_t rh = v16add(__shfl_up_sync(FULL, out_h, 1), d2);
-            const uint32_t bh = (uint32_t)__shfl_sync(FULL, bval, (k0 + s) & 31);
-            const uint32_t dgH = in_h;
-            const uint32_t th = lane == 0 ? bh : rh;
-            in_h = prmt(th, out_h, 0x5432u);
-            w[s] = 0;
-            if ((unsigned)(x0 + s) < lim) {
-                const char *ph = pa + LIN_NC * (128 * NG);
-                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
-                w[s] = lin_rows<R, LOCAL, true>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
-                                                reinterpret_cast<const uint32_t *>(ph), c, floor2);
-                out_h = H[R - 1];
-                if (LOCAL) lin_best<R>(best, H, x0 + s + 1);
-                // the stripe's last row, 64 R - 1: the last lane's high half, column x0 + s
-                if (bout && lane == 31 && x0 + s >= 1) bout[x0 + s] = hi16(out_h) + B;
-            }
-        }
-        if (on) *reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * 1024 + (k0 & 4) * 4) =
-                make_uint4(w[0], w[1], w[2], w[3]);
-        if (bout && lane == 31 && (k0 & 28) == 28 && x0 + 3 >= 1)
-            st_release(pout, (uint32_t)min(n, x0 + 3));
+        if (k0 >= ks && k0 + 4 <= n) group(k0, std::false_type());
+        else group(k0, std::true_type());
+        if (bout && lane == 31 && (k0 & 28) == 28 && k0 >= 60)
+            st_release(pout, (uint32_t)min(n, k0 + 3 - 62));
     }
     if (bout && lane == 31) st_release(pout, (uint32_t)n);
     int4 res = make_int4(0, 0, 0, 0);
     if (LOCAL) {
-        abs0 = max(abs0, lo16(best.sbs) + B);
-        abs1 = max(abs1, hi16(best.sbs) + B);
-        int bs = 0, bi = 0, bj = 0;
-        if (on) {
+        lin_chunk(sbs, seen, cid, (nsteps - 1) >> 5);
+        tr.ids[lane] = cid;
+        abs0 = on ? max(abs0, lo16(sbs) + B) : 0;
+        abs1 = on ? max(abs1, hi16(sbs) + B) : 0;
+        int bs = max(abs0, abs1);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int s = h ? abs1 : abs0;
-                const int sp = h ? best.p1 : best.p0;
-                const int sj = sp >> 3;
-                if (s > 0 && (s > bs || (s == bs && sj < bj))) { bs = s; bj = sj; bi = i_base + h * R + (sp & 7) + 1; }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const int os = __shfl_xor_sync(FULL, bs, o);
-            const int oi = __shfl_xor_sync(FULL, bi, o);
-            const int oj = __shfl_xor_sync(FULL, bj, o);
-            if (os > bs || (os == bs && (oj < bj || (oj == bj && oi < bi)))) { bs = os; bi = oi; bj = oj; }
-        }
-        res = make_int4(bs >> 2, bi, bj, bs > 0 ? 1 : 0);
+        for (int o = 16; o > 0; o >>= 1) bs = max(bs, __shfl_xor_sync(FULL, bs, o));
+        const uint32_t m0 = __ballot_sync(FULL, abs0 == bs), m1 = __ballot_sync(FULL, abs1 == bs);
+        res = make_int4(bs >> 2, bs > 0 ? (int)m0 : 0, bs > 0 ? (int)m1 : 0, bs > 0 ? 1 : 0);
     } else {
         const int rl = (rows - 1) % R, h = v_last & 1;
         int hs = 0;
@@ -808,15 +857,26 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
         const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
         uint8_t *dir = lp.arena + (uint64_t)e.off * 32u;
         int4 r;
+        const LinPlanes pl(LOCAL, seg, e.n);
+        LinTrack tr{nullptr, nullptr, nullptr};
+        if (LOCAL) {
+            uint8_t *q = dir + (uint64_t)e.nstripe * pl.tile * 64u;
+            tr.snap = q + (uint64_t)e.stripe * pl.snap * 32u;
+            q += (uint64_t)e.nstripe * pl.snap * 32u;
+            tr.base = (int *)(q + (uint64_t)e.stripe * pl.base * 32u);
+            q += (uint64_t)e.nstripe * pl.base * 32u;
+            tr.ids = (uint32_t *)(q + (uint64_t)e.stripe * pl.ids * 32u);
+        }
         if (seg < 4) {
-            const uint32_t tu = lin_tile_units(32, e.n), ru = lin_row_units(e.n);
-            uint8_t *rows = dir + (uint64_t)e.nstripe * tu * 32u;
+            const uint32_t ru = lin_row_units(e.n);
+            const size_t plane = (size_t)e.nstripe * pl.tile * 32u;
+            uint8_t *rows = dir + (uint64_t)e.nstripe * pl.stripe(LOCAL) * 32u;
             const int *bin = e.stripe ? (const int *)(rows + (uint64_t)(e.stripe - 1) * ru * 32u) : nullptr;
             int *bout = e.stripe + 1 < e.nstripe ? (int *)(rows + (uint64_t)e.stripe * ru * 32u) : nullptr;
-            uint8_t *d = dir + (uint64_t)e.stripe * tu * 32u;
+            uint8_t *d = dir + (uint64_t)e.stripe * pl.tile * 32u;
             const uint32_t *pin = lp.prog + pos - (e.stripe ? 1 : 0);
             uint32_t *pout = lp.prog + pos;
-#define LIN_STRIPE(R_) lin_stripe<LOCAL, R_>(tab, prof, c, V, e.m, (int)e.stripe * 64 * R_, Hs, e.n, d, bin, pin, bout, pout, lp.kp.status)
+#define LIN_STRIPE(R_) lin_stripe<LOCAL, R_>(tab, prof, c, V, e.m, (int)e.stripe * 64 * R_, Hs, e.n, d, bin, pin, bout, pout, plane, tr, lp.kp.status)
             switch (seg) {
             case 0: r = LIN_STRIPE(8); break;
             case 1: r = LIN_STRIPE(7); break;
@@ -825,7 +885,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
             }
 #undef LIN_STRIPE
         } else {
-#define LIN_SUB(L_, R_) lin_sub<LOCAL, L_, R_>(tab, prof, c, V, e.m, Hs, e.n, dir)
+#define LIN_SUB(L_, R_) lin_sub<LOCAL, L_, R_>(tab, prof, c, V, e.m, Hs, e.n, dir, tr)
             switch (seg) {
             case 4: r = LIN_SUB(32, 8); break;
             case 5: r = LIN_SUB(32, 7); break;
@@ -848,6 +908,72 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
     }
 }
 
+// -------------------------------------------------- the local form's end cell
+// The DP keeps only the running maximum of each virtual lane's R rows (half an
+// operation per row; following the cell itself, row by row at every new maximum,
+// took as many instructions as the recurrence: 130 a step against 77, 100k pairs
+// 5.58 -> 3.51 ms) and the 32-step chunk in which it last rose.  The end cell, the first maximum in column-major order, is found
+// here: the R rows of a virtual lane that reached the score are computed again
+// over that chunk, from their values at its start (the snapshots) and from the
+// row above them (the edge words: 4 H mod 2^16 of both halves' last rows at each
+// step), up to the first column that holds the score.  At most 32 columns, so a
+// thread does it.  Returns column << 3 | row; ~0: none up to column `last`.
+struct LinStrip {
+    const uint32_t *edge;   // edge words of the virtual lane above (null: row 0)
+    const uint32_t *snap;   // this lane's snapshot of the chunk (null: it starts at column 0)
+    int base;               // what that is relative to
+    int half;               // of the lane
+    int va;                 // the virtual lane above + 1, counted in its stripe
+    int col;                // column of the snapshot (0: none)
+};
+__device__ __forceinline__ uint32_t lin_edge(const LinStrip &s, uint32_t tile_row, int j)
+{
+    const int u = s.va - 1, k = j - 1 + u;
+    const uint32_t w = __ldg(s.edge + (uint32_t)(k >> 3) * tile_row + (uint32_t)((u >> 1) * 8 + (k & 7)));
+    return u & 1 ? w >> 16 : w & 0xffffu;
+}
+__device__ __forceinline__ uint32_t lin_locate(const int8_t *sm, const uint8_t *V, int m, int row0, int R,
+                                               const uint8_t *Hs, int last, int score, int go,
+                                               uint32_t tile_row, const LinStrip &s)
+{
+    int a[8], H[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        a[r] = (r < R && row0 + r < m ? (int)__ldg(V + row0 + r) : PG_NRES) * 32;
+        H[r] = s.col && r < R ? (half16(__ldg(s.snap + r), s.half) + s.base) >> 2 : 0;
+    }
+    uint32_t raw = 0;
+    int top = 0;
+    if (s.edge && s.col) {                             // neighbours differ by at most 62
+        raw = lin_edge(s, tile_row, s.col);
+        top = H[0] + ((int)(int16_t)(uint16_t)(raw - 4u * (uint32_t)H[0]) >> 2);
+    }
+    for (int j = s.col + 1; j <= last; ++j) {
+        int dg = top;
+        if (s.edge) {
+            const uint32_t x = lin_edge(s, tile_row, j);
+            top += (int)(int16_t)(uint16_t)(x - raw) >> 2;
+            raw = x;
+        }
+        const int b = __ldg(Hs + j - 1);
+        int up = top, mx = 0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int d = dg + sm[a[r] + b];
+            dg = H[r];
+            H[r] = __viaddmax_s32_relu(max(up, H[r]), go, d);
+            up = H[r];
+            mx = max(mx, up);
+        }
+        if (mx == score) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (H[r] == score) return ((uint32_t)j << 3) | (uint32_t)r;
+        }
+    }
+    return ~0u;
+}
+
 // ------------------------------------------------------------ the traceback
 // One thread per region, in list order (neighbours of nearly equal length).  A
 // move has no branch: the tag says which of row and column step back.  Counts
@@ -855,10 +981,11 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
 template <bool LOCAL>
 __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
 {
-    __shared__ int8_t sm[PG_NRES * 32];
+    __shared__ int8_t sm[LIN_NC * 32];
     if (LOCAL) {
-        for (int t = threadIdx.x; t < PG_NRES * 32; t += blockDim.x)
-            sm[t] = (t & 31) < PG_NRES ? lp.kp.sm[(t >> 5) * PG_NRES + (t & 31)] : (int8_t)0;
+        for (int t = threadIdx.x; t < LIN_NC * 32; t += blockDim.x)
+            sm[t] = t < PG_NRES * 32 ? ((t & 31) < PG_NRES ? lp.kp.sm[(t >> 5) * PG_NRES + (t & 31)] : (int8_t)0)
+                                     : (int8_t)-128;
         __syncthreads();
     }
     const uint32_t entries = lp.tot->entries;
@@ -876,25 +1003,61 @@ __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
     int seg = 0;
     while (seg + 1 < LIN_SEG && pos >= lp.tot->seg[seg + 1]) ++seg;
     const int L = lin_seg_lanes(seg), R = lin_seg_rows(seg);
+    const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
+    const uint32_t tile_row = (uint32_t)L * 8u;      // words per 8 steps
+    const uint32_t stripe_words = lin_tile_units(L, n) * 8u;
+    const uint32_t *dirs = reinterpret_cast<const uint32_t *>(lp.arena + (uint64_t)e.off * 32u);
     int4 d = lp.dp[pos + (LOCAL ? 0 : ns - 1)];
-    if (LOCAL)
-        for (int s = 1; s < ns; ++s) {               // ties: smaller column, then smaller row
+    int i = m, j = n;
+    if (LOCAL) {
+        for (int s = 1; s < ns; ++s) {
             const int4 o = lp.dp[pos + s];
-            if (o.w && (!d.w || o.x > d.x || (o.x == d.x && o.z < d.z))) d = o;
+            if (o.x > d.x) d = o;
         }
-    int i = LOCAL ? d.y : m, j = LOCAL ? d.z : n;
+        // every virtual lane that reached the score: the smallest column, then row
+        const LinPlanes pl(true, seg, n);
+        const uint32_t *edges = dirs + (uint64_t)ns * stripe_words;
+        const uint32_t *snaps = edges + (uint64_t)ns * stripe_words;
+        const int *bases = reinterpret_cast<const int *>(snaps + (uint64_t)ns * pl.snap * 8u);
+        const uint32_t *ids = reinterpret_cast<const uint32_t *>(bases) + (uint64_t)ns * pl.base * 8u;
+        i = 0;
+        for (int s = 0; d.w && s < ns; ++s) {
+            const int4 o = lp.dp[pos + s];
+            if (o.x != d.x) continue;
+#pragma unroll 1
+            for (uint32_t m0 = (uint32_t)o.y, m1 = (uint32_t)o.z; m0 | m1;) {
+                const int f0 = m0 ? __ffs(m0) - 1 : 32, f1 = m1 ? __ffs(m1) - 1 : 32;
+                const int v = f0 <= f1 ? 2 * f0 : 2 * f1 + 1;
+                if (f0 <= f1) m0 &= m0 - 1; else m1 &= m1 - 1;
+                const int row0 = (s * 2 * L + v) * R, t = v >> 1;
+                LinStrip q;
+                q.half = v & 1;
+                // the row above: the virtual lane before, or the last one of the stripe above
+                q.edge = edges + (uint64_t)s * stripe_words;
+                q.va = v;
+                if (v == 0) { q.va = 2 * L; q.edge = s ? q.edge - stripe_words : nullptr; }
+                const int c = (int)((__ldg(ids + (uint64_t)s * pl.ids * 8u + t) >> (16 * q.half)) & 0xffffu);
+                const int start = 32 * c - 2 * t - q.half;       // its column before the chunk
+                q.col = max(0, start);
+                q.snap = snaps + ((uint64_t)s * pl.snap + (uint64_t)(c * L + t)) * 8u;
+                q.base = q.col && seg < 4 ? __ldg(bases + (uint64_t)s * pl.base * 8u + (uint64_t)(c * 32 + t)) : 0;
+                // an earlier find wins a tie (its rows are above)
+                const int lim = min(i ? j - 1 : n, start + 32);
+                const uint32_t z = lin_locate(sm, V, m, row0, R, Hs, lim, d.x, lp.kp.go, tile_row, q);
+                if (z != ~0u) { j = (int)(z >> 3); i = row0 + (int)(z & 7u) + 1; }
+            }
+        }
+        if (!i) d.w = 0;
+    }
+    const int end_i = i, end_j = j;
     uint32_t M = 0, D = 0, G = 0;
     int last = 0;
     if (!LOCAL || d.w) {
-        const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
-        const uint32_t tile_row = (uint32_t)L * 8u;  // words per 8 steps
         const int e_tag = lp.e_first, f_tag = 1 - lp.e_first, go = lp.kp.go;
-        const uint32_t stripe_words = lin_tile_units(L, n) * 8u;
         int st = (i - 1) / (2 * L * R);
         int v = (i - 1 - st * 2 * L * R) / R;
         int sh = 2 * (R - 1 - (i - 1 - st * 2 * L * R - v * R));   // the row's bits in its half
-        const uint32_t *base = reinterpret_cast<const uint32_t *>(lp.arena + (uint64_t)e.off * 32u) +
-                               (uint64_t)st * stripe_words;
+        const uint32_t *base = dirs + (uint64_t)st * stripe_words;
         int h = LOCAL ? d.x : 1;
         while (i > 0 && j > 0 && h > 0) {
             const int k = j - 1 + v;
@@ -929,11 +1092,11 @@ __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
     pg_result o = empty_result();
     o.cells = sat_u32((uint64_t)m * (uint64_t)n);
     if (d.w) {
-        const uint32_t len = (uint32_t)((d.y - i) + (d.z - j)) - D;
+        const uint32_t len = (uint32_t)((end_i - i) + (end_j - j)) - D;
         o.score = d.x;
         o.aln_len = len; o.matches = M; o.gap_opens = G;
-        o.beg_v = (uint16_t)i; o.end_v = (uint16_t)d.y;
-        o.beg_h = (uint16_t)j; o.end_h = (uint16_t)d.z;
+        o.beg_v = (uint16_t)i; o.end_v = (uint16_t)end_i;
+        o.beg_h = (uint16_t)j; o.end_h = (uint16_t)end_j;
         if (len > 0) { o.identity = identity_of(M, len); o.flags = 0; }
     }
     apply_filter(o, m, n, lp.kp.cov_thr, lp.kp.ani_thr);
