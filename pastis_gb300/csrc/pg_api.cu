@@ -530,7 +530,7 @@ static int run_lin(pg_ctx *c, const pg::KParams &kp, uint64_t p0, uint64_t p1, c
     lp.tot = reinterpret_cast<pg::LinTotals *>(lp.cur + pg::LIN_NB);
     lp.smax = c->lin_smax;
     lp.e_first = (c->cfg.tie & PG_TIE_H_E_BEFORE_F) ? 1 : 0;
-    lp.list = nullptr; lp.dp = nullptr; lp.prog = nullptr; lp.arena = nullptr; lp.walk = nullptr;
+    lp.list = nullptr; lp.dp = nullptr; lp.prog = nullptr; lp.wlist = nullptr; lp.arena = nullptr; lp.walk = nullptr;
     CU(cudaMemsetAsync(c->d_lin, 0, LIN_BLOCK, st));
     if (xdrop) pg::lin_count<true>(lp, c->nsm, st);
     else pg::lin_count<false>(lp, c->nsm, st);
@@ -555,7 +555,7 @@ static int run_lin(pg_ctx *c, const pg::KParams &kp, uint64_t p0, uint64_t p1, c
         cudaFree(c->d_list);
         c->d_list = nullptr; c->list_cap = 0;
         const uint64_t cap = std::max<uint64_t>(256, entries + entries / 4);
-        CU(cudaMalloc(&c->d_list, cap * (sizeof(pg::LinReg) + sizeof(int4) + sizeof(uint32_t))));
+        CU(cudaMalloc(&c->d_list, cap * (sizeof(pg::LinReg) + sizeof(int4) + 2 * sizeof(uint32_t))));
         c->list_cap = cap;
     }
     if (xdrop && kp.n > c->walk_cap) {
@@ -567,13 +567,14 @@ static int run_lin(pg_ctx *c, const pg::KParams &kp, uint64_t p0, uint64_t p1, c
     lp.list = reinterpret_cast<pg::LinReg *>(c->d_list);
     lp.dp = reinterpret_cast<int4 *>(lp.list + c->list_cap);
     lp.prog = reinterpret_cast<uint32_t *>(lp.dp + c->list_cap);
+    lp.wlist = lp.prog + c->list_cap;
     lp.arena = c->d_dir;
     lp.walk = c->d_walk;
     const int per_sm = c->tune.dp_blocks_per_sm > 0 ? std::min(c->lin_bps, c->tune.dp_blocks_per_sm) : c->lin_bps;
     const int blocks = c->nsm * std::max(per_sm, 1);
     const uint32_t jobs = c->h_lin->jobs;
-    launches += xdrop ? pg::lin_align<true>(lp, (uint32_t)entries, jobs, c->nsm, blocks, st)
-                      : pg::lin_align<false>(lp, (uint32_t)entries, jobs, c->nsm, blocks, st);
+    launches += xdrop ? pg::lin_align<true>(lp, (uint32_t)entries, c->h_lin->wide, jobs, c->nsm, blocks, st)
+                      : pg::lin_align<false>(lp, (uint32_t)entries, c->h_lin->wide, jobs, c->nsm, blocks, st);
     CU(cudaGetLastError());
     return launches;
 }

@@ -15,10 +15,13 @@
 //  - the decision rides in the two free bits: a term carries its tag (diagonal
 //    3 on identical residues, 2 otherwise; of F and E the one the tie policy
 //    prefers 1, the other 0), so the maximum picks the larger H and on a tie
-//    the larger tag, and no comparison is needed to know which term won;
+//    the larger tag, and no comparison is needed to know which term won.  The
+//    local form subtracts its tags (diagonal 1, F / E 2 and 3): at H = 0 the floor
+//    of the maximum, 0 itself, then wins every tie, and tag 0 marks the cells
+//    where a traceback ends;
 //  - per row and two cells: one prmt (score), one add, two DPX add-max, one
 //    logic op to clear the tag; the tags are gathered by multiply-adds on the
-//    FMA pipe (the sum of the tagged minus the sum of the cleared values).
+//    FMA pipe (the sum of the tagged against the sum of the cleared values).
 // That is 5 ALU operations for 2 cells against 17 in the affine form.
 //
 // A direction word holds 2 bits per cell: the 2 x 8 rows of a lane's two
@@ -49,12 +52,12 @@ namespace pg {
 // scores the tagged 16-bit form takes: gap scores as above; substitution
 // scores that fit an int8 profile after scaling; a gap that costs less than the
 // sentinel's -128 after scaling.  H moves by at most 31 + 31 from a neighbour,
-// so a lane's values stay inside int16 for 64 columns between two base moves
-// ((64 + 16) columns x 4 x 62 = 19840)
+// so a lane's values stay inside int16 and positive for the 32 columns between two
+// base moves (LIN_MID +- (32 + 16) cells x 4 x 62 = 11904)
 constexpr int LIN_SMAX = 31;
 __host__ __forceinline__ bool lin_supported(int go, int ge, int smin, int smax)
 {
-    return go > ge && go < 0 && go >= -LIN_SMAX && smin >= -LIN_SMAX - 1 && smax <= LIN_SMAX;
+    return go > ge && go < 0 && go >= -LIN_SMAX && smin >= -LIN_SMAX && smax <= LIN_SMAX;
 }
 
 // ------------------------------------------------------------- work list
@@ -70,19 +73,26 @@ struct LinReg {
 static_assert(sizeof(LinReg) == 32, "two 16-byte loads");
 
 // classes: 0-3 stripes with R = 8..5; 4-7 a warp, R = 8..5; 8-11 16 lanes,
-// R = 8..5; 12-17 8 lanes, R = 8, 7, 6, 5, 4, 2.  The costly ones first.
-constexpr int LIN_SEG = 18;
-constexpr int LIN_LEV = 48;                        // column-count levels per class, long first
-constexpr int LIN_NB = LIN_SEG * LIN_LEV;
+// R = 8..5; 12-17 8 lanes, R = 8, 7, 6, 5, 4, 2.  The list runs by class and in a
+// class by column count, the long first.
+constexpr int LIN_CLS = 18;
+constexpr int LIN_LEV = 48;                        // column-count levels per class
+constexpr int LIN_NB = LIN_CLS * LIN_LEV;
+// Columns from which a region's walk has a warp of its own.  The walk kernel, us:
+// 400k X-drop pairs 1068 / 861 / 839 / 1075 at 256 / 384 / 512 / 1024, 60k uneven
+// ones 373 / 365 / 405 / 598; 100k Smith-Waterman pairs 643 / 376 / 530 at 512 / 768 /
+// 1024, 8k uneven ones 512 / 527 / 530.
+__host__ __device__ __forceinline__ constexpr int lin_wide(bool local) { return local ? 768 : 384; }
 
 struct LinTotals {
     unsigned long long units;                      // arena need in 32-byte units
     unsigned long long cursor;                     // arena units handed out by k_lin_place
+    unsigned long long work[LIN_CLS];              // DP instructions of each class, about
     uint32_t entries, jobs;
-    uint32_t next_job, pad;                        // work counter of k_lin_dp
-    uint32_t seg[3 * LIN_SEG];                     // per class: first list entry, entries, first job
+    uint32_t wide, wcursor;                        // regions of lin_wide columns; their list's cursor
+    uint32_t next_job[LIN_CLS];                    // work counters of k_lin_dp
+    uint32_t cls[2 * LIN_CLS];                     // per class: first list entry, entries
 };
-
 struct LinParams {
     KParams kp;
     uint64_t p0, p1;                               // pairs of this pass
@@ -92,20 +102,21 @@ struct LinParams {
     LinReg *list;
     int4 *dp;                                      // per entry: score; local: low / high halves that reach it, have
     uint32_t *prog;                                // per entry: columns of its boundary row written
+    uint32_t *wlist;                               // list positions of the wide regions
     uint8_t *arena;
     int4 *walk;                                    // X-drop, per key: score, matches, diagonals, gap runs
     int smax;
     int e_first;                                   // H ties: E before F
 };
 
-__host__ __device__ __forceinline__ int lin_seg_lanes(int seg) { return seg < 8 ? 32 : seg < 12 ? 16 : 8; }
-__host__ __device__ __forceinline__ int lin_seg_rows(int seg)
+__host__ __device__ __forceinline__ int lin_seg_lanes(int cls) { return cls < 8 ? 32 : cls < 12 ? 16 : 8; }
+__host__ __device__ __forceinline__ int lin_seg_rows(int cls)
 {
-    return seg < 16 ? 8 - (seg & 3) : seg == 16 ? 4 : 2;
+    return cls < 16 ? 8 - (cls & 3) : cls == 16 ? 4 : 2;
 }
-__host__ __device__ __forceinline__ int lin_seg_group(int seg) { return seg < 8 ? 1 : seg < 12 ? 2 : 4; }
+__host__ __device__ __forceinline__ int lin_seg_group(int cls) { return cls < 8 ? 1 : cls < 12 ? 2 : 4; }
 
-__device__ __forceinline__ int lin_seg(const LinParams &lp, bool local, int m, int n)
+__device__ __forceinline__ int lin_class(const LinParams &lp, bool local, int m, int n)
 {
     // every scaled value of the region provably inside int16 (no base):
     // above smax per diagonal, below the all-gaps path plus the rows past m
@@ -121,15 +132,15 @@ __device__ __forceinline__ int lin_seg(const LinParams &lp, bool local, int m, i
     const int r = (m + 15) >> 4;
     return r <= 2 ? 17 : r <= 4 ? 16 : 12 + 8 - r;
 }
-__device__ __forceinline__ int lin_level(int n)
+__device__ __forceinline__ int lin_bucket(int cls, int n)
 {
     const int l = n < 256 ? n >> 3 : n < 1024 ? 32 + ((n - 256) >> 6) : n < 4096 ? 44 + ((n - 1024) >> 10) : 47;
-    return LIN_LEV - 1 - l;
+    return cls * LIN_LEV + LIN_LEV - 1 - l;
 }
 // stripes of a region (1 for the classes that do not run in stripes)
-__host__ __device__ __forceinline__ int lin_stripes(int seg, int m)
+__host__ __device__ __forceinline__ int lin_stripes(int cls, int m)
 {
-    return seg < 4 ? (m + 64 * lin_seg_rows(seg) - 1) / (64 * lin_seg_rows(seg)) : 1;
+    return cls < 4 ? (m + 64 * lin_seg_rows(cls) - 1) / (64 * lin_seg_rows(cls)) : 1;
 }
 // 8-step tiles of one stripe, in 32-byte units; boundary row of one stripe
 __host__ __device__ __forceinline__ uint32_t lin_tile_units(int lanes, int n)
@@ -145,13 +156,13 @@ __host__ __device__ __forceinline__ uint32_t lin_chunks(int lanes, int n) { retu
 // chunk of each half's maximum; last, the boundary rows between stripes.
 struct LinPlanes {
     uint32_t tile, snap, base, ids;                  // units of one stripe
-    __host__ __device__ __forceinline__ LinPlanes(bool local, int seg, int n)
+    __host__ __device__ __forceinline__ LinPlanes(bool local, int cls, int n)
     {
-        const int l = lin_seg_lanes(seg);
+        const int l = lin_seg_lanes(cls);
         const uint32_t ch = local ? lin_chunks(l, n) : 0;
         tile = lin_tile_units(l, n);
         snap = ch * (uint32_t)l;
-        base = seg < 4 ? ch * 4u : 0u;
+        base = cls < 4 ? ch * 4u : 0u;
         ids = local ? (uint32_t)l / 8u : 0u;
     }
     __host__ __device__ __forceinline__ uint32_t stripe(bool local) const
@@ -159,10 +170,10 @@ struct LinPlanes {
         return tile * (local ? 2u : 1u) + snap + base + ids;
     }
 };
-__host__ __device__ __forceinline__ uint32_t lin_units(bool local, int seg, int m, int n)
+__host__ __device__ __forceinline__ uint32_t lin_units(bool local, int cls, int m, int n)
 {
-    const uint32_t s = (uint32_t)lin_stripes(seg, m);
-    return s * LinPlanes(local, seg, n).stripe(local) + (s - 1) * lin_row_units(n);
+    const uint32_t s = (uint32_t)lin_stripes(cls, m);
+    return s * LinPlanes(local, cls, n).stripe(local) + (s - 1) * lin_row_units(n);
 }
 
 // the DP regions of pair p: X-drop up to two (one per seed), SW one
@@ -208,28 +219,39 @@ template <bool XDROP>
 __global__ void __launch_bounds__(LIN_PT) k_lin_hist(const LinParams lp)
 {
     __shared__ uint32_t h[LIN_NB];
-    __shared__ unsigned long long su;
+    __shared__ unsigned long long su, hw[LIN_CLS];
     for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT) h[b] = 0;
+    if (threadIdx.x < LIN_CLS) hw[threadIdx.x] = 0;
     if (threadIdx.x == 0) su = 0;
     __syncthreads();
     unsigned long long units = 0;
+    uint32_t wide = 0;
     for (uint64_t p = lp.p0 + (uint64_t)blockIdx.x * LIN_PT + threadIdx.x; p < lp.p1;
          p += (uint64_t)gridDim.x * LIN_PT) {
         const LinPair r = lin_pair<XDROP>(lp.kp, p);
 #pragma unroll
         for (int s = 0; s < (XDROP ? 2 : 1); ++s) {
             if (!r.dp[s]) continue;
-            const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
-            atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])], (uint32_t)lin_stripes(seg, r.m[s]));
-            units += lin_units(!XDROP, seg, r.m[s], r.n[s]);
+            const int cls = lin_class(lp, !XDROP, r.m[s], r.n[s]);
+            atomicAdd(&h[lin_bucket(cls, r.n[s])], (uint32_t)lin_stripes(cls, r.m[s]));
+            units += lin_units(!XDROP, cls, r.m[s], r.n[s]);
+            // a region's share of its warp's steps, about 20 + 8 R instructions each
+            atomicAdd(&hw[cls], (unsigned long long)(lin_stripes(cls, r.m[s]) * (r.n[s] + 2 * lin_seg_lanes(cls)) *
+                                                     (20 + 8 * lin_seg_rows(cls)) / lin_seg_group(cls)));
+            wide += r.n[s] >= lin_wide(!XDROP) ? 1u : 0u;
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) units += __shfl_xor_sync(FULL, units, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&su, units);
+    wide = __reduce_add_sync(FULL, wide);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&su, units);
+        if (wide) atomicAdd(&lp.tot->wide, wide);
+    }
     __syncthreads();
     for (int b = threadIdx.x; b < LIN_NB; b += LIN_PT)
         if (h[b]) atomicAdd(&lp.cnt[b], h[b]);
+    if (threadIdx.x < LIN_CLS && hw[threadIdx.x]) atomicAdd(&lp.tot->work[threadIdx.x], hw[threadIdx.x]);
     if (threadIdx.x == 0 && su) atomicAdd(&lp.tot->units, su);
 }
 
@@ -263,19 +285,13 @@ static __global__ void __launch_bounds__(1024) k_lin_scan(const LinParams lp)
     if (t < LIN_NB) { start[t] = inc - c; lp.cur[t] = inc - c; }
     if (t == LIN_NB - 1) start[LIN_NB] = inc;
     __syncthreads();
-    if (t == 0) {
-        uint32_t job = 0;
-        for (int s = 0; s < LIN_SEG; ++s) {
-            const uint32_t b = start[s * LIN_LEV], n = start[(s + 1) * LIN_LEV] - b;
-            const uint32_t g = (uint32_t)lin_seg_group(s);
-            lp.tot->seg[s] = b;
-            lp.tot->seg[LIN_SEG + s] = n;
-            lp.tot->seg[2 * LIN_SEG + s] = job;
-            job += (n + g - 1) / g;
-        }
-        lp.tot->entries = start[LIN_NB];
-        lp.tot->jobs = job;
+    if (t < LIN_CLS) {
+        const uint32_t b = start[t * LIN_LEV], n = start[(t + 1) * LIN_LEV] - b, g = (uint32_t)lin_seg_group(t);
+        lp.tot->cls[t] = b;
+        lp.tot->cls[LIN_CLS + t] = n;
+        atomicAdd(&lp.tot->jobs, (n + g - 1) / g);
     }
+    if (t == 0) lp.tot->entries = start[LIN_NB];
 }
 
 // the list, in bucket order; arena units by one atomic per block and pass.  A
@@ -304,10 +320,9 @@ __global__ void __launch_bounds__(LIN_PT) k_lin_place(const LinParams lp)
             for (int s = 0; s < NS; ++s) {
                 rank[q * NS + s] = off[q * NS + s] = 0;
                 if (!r.dp[s]) continue;
-                const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
-                rank[q * NS + s] = atomicAdd(&h[seg * LIN_LEV + lin_level(r.n[s])],
-                                             (uint32_t)lin_stripes(seg, r.m[s]));
-                off[q * NS + s] = atomicAdd(&su, lin_units(!XDROP, seg, r.m[s], r.n[s]));
+                const int cls = lin_class(lp, !XDROP, r.m[s], r.n[s]);
+                rank[q * NS + s] = atomicAdd(&h[lin_bucket(cls, r.n[s])], (uint32_t)lin_stripes(cls, r.m[s]));
+                off[q * NS + s] = atomicAdd(&su, lin_units(!XDROP, cls, r.m[s], r.n[s]));
                 cells += (unsigned long long)r.m[s] * (unsigned long long)r.n[s];
             }
         }
@@ -332,15 +347,16 @@ __global__ void __launch_bounds__(LIN_PT) k_lin_place(const LinParams lp)
 #pragma unroll
             for (int s = 0; s < NS; ++s) {
                 if (!r.dp[s]) continue;
-                const int seg = lin_seg(lp, !XDROP, r.m[s], r.n[s]);
-                const int ns = lin_stripes(seg, r.m[s]);
-                uint32_t pos = h[seg * LIN_LEV + lin_level(r.n[s])] + rank[q * NS + s];
+                const int cls = lin_class(lp, !XDROP, r.m[s], r.n[s]);
+                const int ns = lin_stripes(cls, r.m[s]);
+                uint32_t pos = h[lin_bucket(cls, r.n[s])] + rank[q * NS + s];
                 LinReg e;
                 e.v = r.v[s]; e.h = r.h[s];
                 e.key = XDROP ? (uint32_t)(2 * p + s) : (uint32_t)p;
                 e.off = (uint32_t)(ubase + off[q * NS + s]);
                 e.m = (uint16_t)r.m[s]; e.n = (uint16_t)r.n[s];
                 e.nstripe = (uint16_t)ns;
+                if (r.n[s] >= lin_wide(!XDROP)) lp.wlist[atomicAdd(&lp.tot->wcursor, 1u)] = pos;
                 for (int k = 0; k < ns; ++k, ++pos) {
                     e.stripe = (uint16_t)k;
                     const uint4 *src = reinterpret_cast<const uint4 *>(&e);
@@ -365,14 +381,15 @@ constexpr int LIN_PROF = 2 * LIN_NC * 32 * 8;      // bytes per warp
 constexpr int LIN_DYN = WARPS * LIN_PROF;
 constexpr uint32_t LIN_CLR = 0xFFFCFFFCu;          // clears both halves' tags
 constexpr int LIN_NEG = -32000;
+constexpr int LIN_MID = 16384;
 
-// tagged score table: row a, byte b = 4 * s(a, b) + (a == b ? 3 : 2); the
-// sentinel row and the sentinel column -128
-__device__ __forceinline__ void lin_table(int8_t *t, const int8_t *sm)
+// tagged score table: row a, byte b = 4 * s(a, b) + (a == b ? 3 : 2), in the local
+// form 4 * s(a, b) - 1; the sentinel row and the sentinel column -128
+__device__ __forceinline__ void lin_table(int8_t *t, const int8_t *sm, bool local)
 {
     for (int k = threadIdx.x; k < LIN_NC * LIN_ROWB; k += blockDim.x) {
         const int a = k / LIN_ROWB, b = k - a * LIN_ROWB;
-        t[k] = a < PG_NRES && b < PG_NRES ? (int8_t)(4 * (int)sm[a * PG_NRES + b] + (a == b ? 3 : 2)) : (int8_t)-128;
+        t[k] = a < PG_NRES && b < PG_NRES ? (int8_t)(4 * (int)sm[a * PG_NRES + b] + (local ? -1 : a == b ? 3 : 2)) : (int8_t)-128;
     }
 }
 
@@ -504,7 +521,7 @@ __device__ __forceinline__ void lin_chunk(uint32_t sbs, uint32_t &seen, uint32_t
 
 struct LinConst {
     uint32_t goL, goU;      // packed 4 go + tag of E / F
-    uint32_t four;          // 4, from memory: the multiply-adds below stay on the FMA pipe
+    uint32_t four, one;     // from memory: the multiply-adds below stay on the FMA pipe
     int go4;
 };
 
@@ -535,12 +552,14 @@ __device__ __forceinline__ uint32_t lin_rows(uint32_t (&H)[R], uint32_t dgH, uin
     for (int r = 0; r < R; ++r) {
         const uint32_t t = LOCAL && !BASE ? __viaddmax_s16x2_relu(up, c.goU, dl[r])
                                           : __viaddmax_s16x2(up, c.goU, dl[r]);
-        up = t & LIN_CLR;
+        // local: round up to the multiple of 4 (both halves of t are positive: no carry)
+        if (LOCAL) up = (t * c.one + 0x00030003u) & LIN_CLR;
+        else up = t & LIN_CLR;
         H[r] = up;
         wa = wa * c.four + t;
         wb = wb * c.four + up;
     }
-    return wa - wb;
+    return LOCAL ? wb - wa : wa - wb;
 }
 
 // Regions of the L-lane classes: each L lanes of the warp pass their own region
@@ -590,33 +609,40 @@ __device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, con
     }
     uint8_t *dst = dir + sl * 32;
     const size_t plane = (size_t)lin_tile_units(L, n) * 32u;
-    // four steps (a lambda, for its two uses)
-    auto group = [&](const int k0, auto test) {
-        const uint32_t res4 = cols.next();
-        const int x0 = k0 - 2 * sl;                  // low half's column at the first step, 0-based
+    // one step's inputs: the row above both halves; returns the diagonal's
+    auto step = [&]() {
+        const uint32_t rh = __shfl_up_sync(FULL, out_h, 1, L);
+        const uint32_t dgH = in_h;
+        const uint32_t th = sl == 0 ? bord : rh;
+        if (!LOCAL) bord += bstep;
+        in_h = prmt(th, out_h, 0x5432u);
+        return dgH;
+    };
+    auto rows_of = [&](const uint32_t dgH, const uint32_t code) {
+        const char *ph = pa + LIN_NC * (128 * NG);
+        pa = lbase + code * (128 * NG);
+        const uint32_t w = lin_rows<R, LOCAL, false>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
+                                                     reinterpret_cast<const uint32_t *>(ph), c, 0u);
+        out_h = H[R - 1];
+        if (LOCAL) sbs = lin_max<R>(sbs, H);
+        return w;
+    };
+    // four steps (a lambda, for its two uses: the steps where every lane that holds
+    // rows is inside its columns, and the ramps, where each lane is tested)
+    auto group = [&](const int k0, const uint32_t res4, auto test) {
         uint32_t w[4], e[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const uint32_t rh = __shfl_up_sync(FULL, out_h, 1, L);
-            const uint32_t dgH = in_h;
-            const uint32_t th = sl == 0 ? bord : rh;
-            if (!LOCAL) bord += bstep;
-            in_h = prmt(th, out_h, 0x5432u);
+            const uint32_t dgH = step();
             w[s] = 0;
-            if (!decltype(test)::value || (unsigned)(x0 + s) < lim) {
-                const char *ph = pa + LIN_NC * (128 * NG);
-                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
-                w[s] = lin_rows<R, LOCAL, false>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
-                                                 reinterpret_cast<const uint32_t *>(ph), c, 0u);
-                out_h = H[R - 1];
-                if (LOCAL) sbs = lin_max<R>(sbs, H);
-            }
+            if (!decltype(test)::value || (unsigned)(k0 + s - 2 * sl) < lim)
+                w[s] = rows_of(dgH, (res4 >> (8 * s)) & 0xffu);
             e[s] = out_h;
         }
         if (on && k0 < own) {
-            uint4 *d = reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * (L * 32) + (k0 & 4) * 4);
-            *d = make_uint4(w[0], w[1], w[2], w[3]);
-            if (LOCAL) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(d) + plane) = make_uint4(e[0], e[1], e[2], e[3]);
+            uint8_t *d = dst + (size_t)(k0 >> 3) * (L * 32) + (k0 & 4) * 4;
+            *reinterpret_cast<uint4 *>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (LOCAL) *reinterpret_cast<uint4 *>(d + plane) = make_uint4(e[0], e[1], e[2], e[3]);
         }
     };
     for (int k0 = 0; k0 < nsteps; k0 += 4) {
@@ -624,8 +650,9 @@ __device__ __forceinline__ int4 lin_sub(const uint32_t *tab, uint32_t *prof, con
             lin_chunk(sbs, seen, cid, (k0 >> 5) - 1);
             if (on && k0 < own) lin_snap<R>(tr.snap + ((size_t)(k0 >> 5) * L + sl) * 32, H);
         }
-        if (k0 >= ks && k0 + 4 <= ke) group(k0, std::false_type());
-        else group(k0, std::true_type());
+        const uint32_t res4 = cols.next();
+        if (k0 >= ks && k0 + 4 <= ke) group(k0, res4, std::false_type());
+        else group(k0, res4, std::true_type());
     }
     int4 res = make_int4(0, 0, 0, 0);
     if (LOCAL) {
@@ -676,8 +703,8 @@ __device__ __forceinline__ void lin_wait(const uint32_t *p, uint32_t need, int *
 }
 
 // One stripe of 64 R rows (the last: what is left) of a region on a warp.
-// Values are relative to the lane's base B (a multiple of 4, moved every 64
-// steps to the lane's current values).  V: the region's first row; rows rb ..
+// Values are relative to the lane's base B (a multiple of 4, moved every 32 steps
+// so that the lane's values lie around LIN_MID, all of them positive).  V: the region's first row; rows rb ..
 // of it are this stripe's.  bin / bout: boundary rows (4 H of columns 1..n) of
 // the stripe above and of this one (null: none), pin / pout their progress.
 template <bool LOCAL, int R>
@@ -698,13 +725,13 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
     __syncwarp();
     lin_profile<R>(tab, V, i_base, m, on, prof);
     __syncwarp();
-    // column 0, relative to the lane's first row there
-    int B = LOCAL ? 0 : c.go4 * i_base;
+    // column 0; the lane's first row there at LIN_MID
+    int B = (LOCAL ? 0 : c.go4 * i_base) - LIN_MID;
     uint32_t H[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) H[r] = pk16(LOCAL ? 0 : c.go4 * (r + 1), LIN_NEG);
-    const int lo0 = LOCAL ? 0 : c.go4 * R, hi0 = LOCAL ? 0 : c.go4 * 2 * R;
-    uint32_t in_h = pk16(0, lo0), out_h = pk16(lo0, hi0);
+    for (int r = 0; r < R; ++r) H[r] = pk16(LIN_MID + (LOCAL ? 0 : c.go4 * (r + 1)), LIN_NEG);
+    const int lo0 = LIN_MID + (LOCAL ? 0 : c.go4 * R), hi0 = LIN_MID + (LOCAL ? 0 : c.go4 * 2 * R);
+    uint32_t in_h = pk16(LIN_MID, lo0), out_h = pk16(lo0, hi0);
     LinCols cols;
     cols.init(Hs, n, -2 * lane);
     const char *lbase = reinterpret_cast<const char *>(prof + lane * NG);
@@ -714,44 +741,75 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
     uint32_t floor2 = 0, d2 = 0, b2 = 0;
     int bval = 0;
     const int nsteps = n + v_last;
-    const int ks = 2 * t_last;
+    const int ks = bout ? 64 : 2 * t_last;           // (a stripe with one below has all its lanes)
     uint8_t *dst = dir + lane * 32;
-    auto group = [&](const int k0, auto test) {
-        const uint32_t res4 = cols.next();
-        const int x0 = k0 - 2 * lane;
+    // one step: the low half's column x (0-based), its residue code
+    auto step = [&](const int k, const uint32_t code) {
+        const uint32_t rh = v16add(__shfl_up_sync(FULL, out_h, 1), d2);
+        const uint32_t bh = (uint32_t)__shfl_sync(FULL, bval, k & 31);
+        const uint32_t dgH = in_h;
+        const uint32_t th = lane == 0 ? bh : rh;
+        in_h = prmt(th, out_h, 0x5432u);
+        return dgH;
+    };
+    auto rows_of = [&](const uint32_t dgH, const uint32_t code) {
+        const char *ph = pa + LIN_NC * (128 * NG);
+        pa = lbase + code * (128 * NG);
+        const uint32_t w = lin_rows<R, LOCAL, true>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
+                                                    reinterpret_cast<const uint32_t *>(ph), c, floor2);
+        out_h = H[R - 1];
+        if (LOCAL) sbs = lin_max<R>(sbs, H);
+        return w;
+    };
+    // four steps with every lane inside its columns
+    auto group = [&](const int k0, const uint32_t res4) {
         uint32_t w[4], e[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const uint32_t rh = v16add(__shfl_up_sync(FULL, out_h, 1), d2);
-            const uint32_t bh = (uint32_t)__shfl_sync(FULL, bval, (k0 + s) & 31);
-            const uint32_t dgH = in_h;
-            const uint32_t th = lane == 0 ? bh : rh;
-            in_h = prmt(th, out_h, 0x5432u);
-            w[s] = 0;
-            if (!decltype(test)::value || (unsigned)(x0 + s) < lim) {
-                const char *ph = pa + LIN_NC * (128 * NG);
-                pa = lbase + ((res4 >> (8 * s)) & 0xffu) * (128 * NG);
-                w[s] = lin_rows<R, LOCAL, true>(H, dgH, in_h, reinterpret_cast<const uint32_t *>(pa),
-                                                reinterpret_cast<const uint32_t *>(ph), c, floor2);
-                out_h = H[R - 1];
-                if (LOCAL) sbs = lin_max<R>(sbs, H);
-                // the stripe's last row, 64 R - 1: the last lane's high half, column x0 + s
-                if (bout && lane == 31 && x0 + s >= 1) bout[x0 + s] = hi16(out_h) + B;
-            }
-            if (LOCAL) e[s] = v16add(out_h, b2);
+            const uint32_t code = (res4 >> (8 * s)) & 0xffu;
+            const uint32_t dgH = step(k0 + s, code);
+            w[s] = rows_of(dgH, code);
+            e[s] = LOCAL ? v16add(out_h, b2) : out_h;
         }
         if (on) {
-            uint4 *d = reinterpret_cast<uint4 *>(dst + (size_t)(k0 >> 3) * 1024 + (k0 & 4) * 4);
-            *d = make_uint4(w[0], w[1], w[2], w[3]);
-            if (LOCAL) *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(d) + plane) = make_uint4(e[0], e[1], e[2], e[3]);
+            uint8_t *d = dst + (size_t)(k0 >> 3) * 1024 + (k0 & 4) * 4;
+            *reinterpret_cast<uint4 *>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (LOCAL) *reinterpret_cast<uint4 *>(d + plane) = make_uint4(e[0], e[1], e[2], e[3]);
+        }
+        // the stripe's last row, 64 R - 1: the last lane's high half, columns
+        // k0 - 62 and on, two to a store
+        if (bout && lane == 31) {
+            int v[4];
+            // (local: e holds the values mod 2^16)
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+                v[s] = (LOCAL ? (int)(int16_t)(uint16_t)((e[s] >> 16) - (uint32_t)B) : hi16(e[s])) + B;
+            int2 *o = reinterpret_cast<int2 *>(bout + (k0 - 62));
+            o[0] = make_int2(v[0], v[1]);
+            o[1] = make_int2(v[2], v[3]);
+        }
+    };
+    // four steps, each lane tested: the ramps (a loop, to keep the code small)
+    auto ramp = [&](const int k0, const uint32_t res4) {
+#pragma unroll 1
+        for (int s = 0; s < 4; ++s) {
+            const uint32_t code = (res4 >> (8 * s)) & 0xffu;
+            const uint32_t dgH = step(k0 + s, code);
+            const int x = k0 + s - 2 * lane;
+            if ((unsigned)x < lim) {
+                uint32_t *d = reinterpret_cast<uint32_t *>(dst + (size_t)(k0 >> 3) * 1024 + ((k0 & 4) + s) * 4);
+                *d = rows_of(dgH, code);
+                if (LOCAL) *reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(d) + plane) = v16add(out_h, b2);
+                if (bout && lane == 31 && x >= 1) bout[x] = hi16(out_h) + B;
+            }
         }
     };
     for (int k0 = 0; k0 < nsteps; k0 += 4) {
         if ((k0 & 31) == 0) {
             if (LOCAL && k0) lin_chunk(sbs, seen, cid, (k0 >> 5) - 1);
-            if ((k0 & 63) == 0) {
+            {
                 // move the base of the lanes whose two halves hold real columns
-                const int sh = k0 - 1 - 2 * lane >= 1 ? lo16(H[0]) & ~3 : 0;
+                const int sh = k0 - 1 - 2 * lane >= 1 ? (lo16(H[0]) & ~3) - LIN_MID : 0;
                 const uint32_t s2 = pk16(-sh, -sh);
                 if (LOCAL) {
                     abs0 = max(abs0, lo16(sbs) + B);
@@ -767,7 +825,7 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
                     const int f = max(-B, LIN_NEG);
                     floor2 = pk16(f, f);
                     // the maximum so far, as far as the new base can tell it: past
-                    // int16 no value of the next 64 columns reaches it
+                    // int16 no value of the next 32 columns reaches it
                     sbs = pk16(min(max(abs0 - B, LIN_NEG), 32767), min(max(abs1 - B, LIN_NEG), 32767));
                     seen = sbs;
                 }
@@ -789,8 +847,12 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
             }
             bval = (j <= n ? h - b0 : 0) << 16;
         }
-        if (k0 >= ks && k0 + 4 <= n) group(k0, std::false_type());
-        else group(k0, std::true_type());
+        const uint32_t res4 = cols.next();
+        if (k0 >= ks && k0 + 4 <= n) {
+            group(k0, res4);
+        } else {
+            ramp(k0, res4);
+        }
         if (bout && lane == 31 && (k0 & 28) == 28 && k0 >= 60)
             st_release(pout, (uint32_t)min(n, k0 + 3 - 62));
     }
@@ -817,35 +879,71 @@ __device__ __forceinline__ int4 lin_stripe(const uint32_t *tab, uint32_t *prof, 
     return res;
 }
 
-// Jobs in list order from one counter: a group of 32 / L regions, or a stripe.
+// Each class has its own job counter (a job: a group of 32 / L regions, or a
+// stripe), its jobs taken in list order.  The global form goes through the classes
+// in order.  In the local form, whose loops are larger, an SM starts on the class
+// that holds its share of the batch's work and goes on with the classes after it:
+// an SM then runs one class's code at a time, and every class's long jobs start
+// early (8k uneven pairs: 5.74 ms in class order, where a late class's longest job
+// runs alone at the end; 7.35 ms with the longest jobs of all classes first, whose
+// loops together do not fit the instruction cache; 4.74 ms this way.  The global
+// form lost 6 % by it, its loops fit).
 template <bool LOCAL>
-__global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
+__global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp, int nsm)
 {
     __shared__ __align__(16) int8_t tab8[LIN_NC * LIN_ROWB];
-    __shared__ uint32_t sl[3 * LIN_SEG + 1];
-    lin_table(tab8, lp.kp.sm);
-    for (int t = threadIdx.x; t < 3 * LIN_SEG; t += blockDim.x) sl[t] = lp.tot->seg[t];
-    if (threadIdx.x == 0) sl[3 * LIN_SEG] = lp.tot->jobs;
+    __shared__ uint32_t sl[2 * LIN_CLS];
+    __shared__ int first;
+    lin_table(tab8, lp.kp.sm, LOCAL);
+    for (int t = threadIdx.x; t < 2 * LIN_CLS; t += blockDim.x) sl[t] = lp.tot->cls[t];
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x;
+        const double w = LOCAL && k < LIN_CLS ? (double)lp.tot->work[k] : 0.0;
+        double acc = w;                            // inclusive prefix over the classes
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double y = __shfl_up_sync(FULL, acc, o);
+            if (k >= o) acc += y;
+        }
+        uint32_t smid;
+        asm("mov.u32 %0, %%smid;" : "=r"(smid));
+        const double at = __shfl_sync(FULL, acc, 31) * (double)(smid % (uint32_t)nsm) / (double)nsm;
+        const uint32_t past = __ballot_sync(FULL, acc > at && w > 0.0);
+        if (k == 0) first = past ? __ffs(past) - 1 : 0;
+    }
     __syncthreads();
     const uint32_t *tab = reinterpret_cast<const uint32_t *>(tab8);
     const int lane = threadIdx.x & 31;
     uint32_t *prof = reinterpret_cast<uint32_t *>(g_dyn_prof) + (threadIdx.x >> 5) * (LIN_PROF / 4);
     LinConst c;
     c.go4 = 4 * lp.kp.go;
-    c.goL = pk16(c.go4 + lp.e_first, c.go4 + lp.e_first);
-    c.goU = pk16(c.go4 + 1 - lp.e_first, c.go4 + 1 - lp.e_first);
+    const int te = (LOCAL ? -3 : 0) + lp.e_first, tf = (LOCAL ? -3 : 0) + 1 - lp.e_first;
+    c.goL = pk16(c.go4 + te, c.go4 + te);
+    c.goU = pk16(c.go4 + tf, c.go4 + tf);
     c.four = (uint32_t)lp.kp.four;
-    int seg = 0;
+    c.one = c.four >> 2;
+    // lane k: the jobs of class k
+    const int mine = lane < LIN_CLS ? lane : 0;
+    const uint32_t my_jobs = (sl[LIN_CLS + mine] + (uint32_t)lin_seg_group(mine) - 1) / (uint32_t)lin_seg_group(mine);
+    int cls = first;
     for (;;) {
-        uint32_t job = 0;
-        if (lane == 0) job = atomicAdd(&lp.tot->next_job, 1u);
+        const int lanes = lin_seg_lanes(cls), group = lin_seg_group(cls);
+        const uint32_t jobs = __shfl_sync(FULL, my_jobs, cls);
+        uint32_t job = jobs;
+        if (lane == 0 && jobs) job = atomicAdd(&lp.tot->next_job[cls], 1u);
         job = __shfl_sync(FULL, job, 0);
-        if (job >= sl[3 * LIN_SEG]) break;
-        while (seg + 1 < LIN_SEG && job >= sl[2 * LIN_SEG + seg + 1]) ++seg;
-        const int lanes = lin_seg_lanes(seg), group = lin_seg_group(seg);
-        const uint32_t q = (job - sl[2 * LIN_SEG + seg]) * (uint32_t)group + (uint32_t)(lane / lanes);
-        const bool has = q < sl[LIN_SEG + seg];
-        const uint32_t pos = sl[seg] + q;
+        if (job >= jobs) {
+            // the next class with jobs left, around from this one
+            const bool any = lane < LIN_CLS && *(volatile uint32_t *)&lp.tot->next_job[mine] < my_jobs;
+            const uint32_t left = __ballot_sync(FULL, any);
+            if (!left) break;
+            const uint32_t after = left & ~((2u << cls) - 1u);
+            cls = __ffs(after ? after : left) - 1;
+            continue;
+        }
+        const uint32_t q = job * (uint32_t)group + (uint32_t)(lane / lanes);
+        const bool has = q < sl[LIN_CLS + cls];
+        const uint32_t pos = sl[cls] + q;
         LinReg e;
         e.m = e.n = 0; e.v = e.h = 0; e.off = 0; e.stripe = 0; e.nstripe = 1;
         if (has) {
@@ -857,7 +955,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
         const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
         uint8_t *dir = lp.arena + (uint64_t)e.off * 32u;
         int4 r;
-        const LinPlanes pl(LOCAL, seg, e.n);
+        const LinPlanes pl(LOCAL, cls, e.n);
         LinTrack tr{nullptr, nullptr, nullptr};
         if (LOCAL) {
             uint8_t *q = dir + (uint64_t)e.nstripe * pl.tile * 64u;
@@ -867,7 +965,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
             q += (uint64_t)e.nstripe * pl.base * 32u;
             tr.ids = (uint32_t *)(q + (uint64_t)e.stripe * pl.ids * 32u);
         }
-        if (seg < 4) {
+        if (cls < 4) {
             const uint32_t ru = lin_row_units(e.n);
             const size_t plane = (size_t)e.nstripe * pl.tile * 32u;
             uint8_t *rows = dir + (uint64_t)e.nstripe * pl.stripe(LOCAL) * 32u;
@@ -877,7 +975,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
             const uint32_t *pin = lp.prog + pos - (e.stripe ? 1 : 0);
             uint32_t *pout = lp.prog + pos;
 #define LIN_STRIPE(R_) lin_stripe<LOCAL, R_>(tab, prof, c, V, e.m, (int)e.stripe * 64 * R_, Hs, e.n, d, bin, pin, bout, pout, plane, tr, lp.kp.status)
-            switch (seg) {
+            switch (cls) {
             case 0: r = LIN_STRIPE(8); break;
             case 1: r = LIN_STRIPE(7); break;
             case 2: r = LIN_STRIPE(6); break;
@@ -886,7 +984,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_lin_dp(const LinParams lp)
 #undef LIN_STRIPE
         } else {
 #define LIN_SUB(L_, R_) lin_sub<LOCAL, L_, R_>(tab, prof, c, V, e.m, Hs, e.n, dir, tr)
-            switch (seg) {
+            switch (cls) {
             case 4: r = LIN_SUB(32, 8); break;
             case 5: r = LIN_SUB(32, 7); break;
             case 6: r = LIN_SUB(32, 6); break;
@@ -975,22 +1073,174 @@ __device__ __forceinline__ uint32_t lin_locate(const int8_t *sm, const uint8_t *
 }
 
 // ------------------------------------------------------------ the traceback
-// One thread per region, in list order (neighbours of nearly equal length).  A
-// move has no branch: the tag says which of row and column step back.  Counts
-// what computeAlignmentStats counts (src/align/SeqanFullAligner.cpp:238-246).
+// Counts what computeAlignmentStats counts (src/align/SeqanFullAligner.cpp:238-246):
+// diagonal columns (D), identical ones (M), gap runs (G).  A region's walk is
+// one chain of dependent reads, so its latency is what counts, in two forms:
+//
+//  - a thread per region, for the many short ones: moves have no branch on the
+//    tag, and locally the tags of four cells along the diagonal are read at once
+//    (100k pairs 0.79 -> 0.56 ms; the global form, with half the registers, ran
+//    faster one cell at a time, 1.06 against 1.29 ms on 400k X-drop pairs).  A
+//    warp waits for whichever of its 32 walks misses L1, about 400 cycles a move.
+//  - a warp per region, for regions in stripes and for batches too small to fill
+//    the chip with threads: 16 lanes read the next 16 cells of the diagonal, a
+//    ballot gives the run of diagonal moves, and the other lanes bring the
+//    sectors of the 16 cells after those into L1.
+struct LinPath {
+    int i, j;              // in: the end cell; out: the start cell
+    uint32_t M, D, G;
+};
+struct LinDirs {
+    const uint32_t *dirs;  // the region's direction words
+    uint32_t tile_row;     // words per 8 steps
+    uint32_t stripe_words;
+    int rows, R;           // of a stripe; per virtual lane
+    const uint8_t *V, *Hs;
+    int e_tag, f_tag;
+};
+
 template <bool LOCAL>
-__global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
+__device__ __forceinline__ void lin_walk_thread(const LinDirs &x, LinPath &p)
+{
+    constexpr int RUN = LOCAL ? 4 : 1;
+    const uint32_t inv = (65536u + (uint32_t)x.R - 1u) / (uint32_t)x.R;   // q / R for q < 8192
+    int st = (p.i - 1) / x.rows;
+    int q = p.i - 1 - st * x.rows;                 // row in the stripe
+    int j = p.j, last = 0;
+    const uint32_t *base = x.dirs + (uint64_t)st * x.stripe_words;
+    bool more = true;
+    while (j > 0 && more) {
+        if (q < 0) {
+            if (--st < 0) break;
+            q = x.rows - 1;
+            base -= x.stripe_words;
+        }
+        // the tags of the next cells along the diagonal, all loads in flight together
+        // (past the first row or column: the last valid cell again, not used)
+        const int len = min(RUN, min(q + 1, j));
+        uint32_t word[RUN];
+        int sh[RUN], ra[RUN], rb[RUN], tag[RUN];
+#pragma unroll
+        for (int t = 0; t < RUN; ++t) {
+            const int tt = RUN > 1 ? min(t, len - 1) : 0, qt = q - tt;
+            const int v = (int)((uint32_t)qt * inv >> 16);
+            const int k = j - 1 - tt + v;
+            word[t] = __ldg(base + (uint32_t)(k >> 3) * x.tile_row + (uint32_t)((v >> 1) * 8 + (k & 7)));
+            sh[t] = 16 * (v & 1) + 2 * (x.R - 1 - (qt - v * x.R));
+            if (LOCAL) { ra[t] = __ldg(x.V + st * x.rows + qt); rb[t] = __ldg(x.Hs + j - 1 - tt); }
+        }
+        // the diagonal run, then the gap (or the end) after it
+        int run = 0, gap = 0;
+        bool on = true;
+#pragma unroll
+        for (int t = 0; t < RUN; ++t) {
+            tag[t] = (int)(word[t] >> sh[t]) & 3;
+            on = on && t < len && (LOCAL ? tag[t] == 1 : tag[t] >= 2);
+            run += on ? 1 : 0;
+            p.M += on && (LOCAL ? ra[t] == rb[t] : tag[t] == 3) ? 1u : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < RUN; ++t)
+            if (t == run && t < len) {
+                gap = tag[t] == x.f_tag ? 1 : tag[t] == x.e_tag ? 2 : 0;
+                more = gap != 0;
+            }
+        p.D += (uint32_t)run;
+        last = run ? 0 : last;
+        p.G += gap && gap != last ? 1u : 0u;
+        last = gap ? gap : last;
+        q -= run + (gap == 1 ? 1 : 0);
+        j -= run + (gap == 2 ? 1 : 0);
+    }
+    p.i = st < 0 ? 0 : st * x.rows + q + 1;
+    p.j = j;
+    if (!LOCAL && ((p.i > 0 && last != 1) || (j > 0 && last != 2))) ++p.G;
+}
+
+// the same by a warp; dummy: this lane's 4 bytes of shared memory
+template <bool LOCAL>
+__device__ __forceinline__ void lin_walk_warp(const LinDirs &x, LinPath &p, uint32_t *dummy)
+{
+    constexpr int RUN = 16;
+    const int lane = threadIdx.x & 31;
+    const uint32_t inv = (65536u + (uint32_t)x.R - 1u) / (uint32_t)x.R;
+    const uint32_t sdummy = (uint32_t)__cvta_generic_to_shared(dummy);
+    int st = (p.i - 1) / x.rows;
+    int q = p.i - 1 - st * x.rows;
+    int j = p.j, last = 0;
+    const uint32_t *base = x.dirs + (uint64_t)st * x.stripe_words;
+    int ra = 0, rb = 1;                            // local: the residues of the run before, and its cells
+    uint32_t ran = 0;
+    bool more = true;
+    while (j > 0 && more) {
+        if (q < 0) {
+            if (--st < 0) break;
+            q = x.rows - 1;
+            base -= x.stripe_words;
+        }
+        const int len = min(RUN, min(q + 1, j));
+        // lane t: the cell t moves along the diagonal (lanes past the run's reach
+        // fetch ahead: a copy into shared memory that nothing waits for)
+        const int tt = min(lane, min(q, j - 1)), qt = q - tt;
+        const int v = (int)((uint32_t)qt * inv >> 16);
+        const int k = j - 1 - tt + v;
+        const uint32_t *w = base + (uint32_t)(k >> 3) * x.tile_row + (uint32_t)((v >> 1) * 8 + (k & 7));
+        uint32_t word = 0;
+        if (lane < RUN) {
+            word = __ldg(w);
+        } else {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(sdummy), "l"(w) : "memory");
+        }
+        if (LOCAL) {
+            p.M += (uint32_t)__popc(__ballot_sync(FULL, ra == rb) & ran);
+            ra = __ldg(x.V + st * x.rows + qt);
+            rb = __ldg(x.Hs + j - 1 - tt);
+        }
+        const int tag = (int)(word >> (16 * (v & 1) + 2 * (x.R - 1 - (qt - v * x.R)))) & 3;
+        const bool cell = lane < len && (LOCAL ? tag == 1 : tag >= 2);
+        const int run = __ffs(~__ballot_sync(FULL, cell)) - 1;     // lane RUN is never one of them
+        if (LOCAL) ran = (1u << run) - 1u;
+        else p.M += (uint32_t)__popc(__ballot_sync(FULL, cell && tag == 3) & ((1u << run) - 1u));
+        p.D += (uint32_t)run;
+        last = run ? 0 : last;
+        int gap = 0;
+        if (run < len) {
+            const int g = __shfl_sync(FULL, tag, run);
+            gap = g == x.f_tag ? 1 : g == x.e_tag ? 2 : 0;
+            more = gap != 0;
+        }
+        p.G += gap && gap != last ? 1u : 0u;
+        last = gap ? gap : last;
+        q -= run + (gap == 1 ? 1 : 0);
+        j -= run + (gap == 2 ? 1 : 0);
+    }
+    if (LOCAL) p.M += (uint32_t)__popc(__ballot_sync(FULL, ra == rb) & ran);
+    p.i = st < 0 ? 0 : st * x.rows + q + 1;
+    p.j = j;
+    if (!LOCAL && ((p.i > 0 && last != 1) || (j > 0 && last != 2))) ++p.G;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// regions per SM up to which every walk has a warp of its own
+constexpr uint32_t LIN_WALK_WARPS = 64;
+
+// blocks [0, warp_blocks): a warp for each wide region (all: for each entry of the
+// list); the rest: a thread per entry
+template <bool LOCAL>
+__global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp, uint32_t warp_blocks, bool all)
 {
     __shared__ int8_t sm[LIN_NC * 32];
+    __shared__ uint32_t dummy[256];
     if (LOCAL) {
         for (int t = threadIdx.x; t < LIN_NC * 32; t += blockDim.x)
             sm[t] = t < PG_NRES * 32 ? ((t & 31) < PG_NRES ? lp.kp.sm[(t >> 5) * PG_NRES + (t & 31)] : (int8_t)0)
                                      : (int8_t)-128;
         __syncthreads();
     }
-    const uint32_t entries = lp.tot->entries;
-    const uint32_t pos = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pos >= entries) return;
+    const bool warp = blockIdx.x < warp_blocks;
+    uint32_t pos = warp ? blockIdx.x * 8u + (threadIdx.x >> 5) : (blockIdx.x - warp_blocks) * 256u + threadIdx.x;
+    if (pos >= (warp && !all ? lp.tot->wide : lp.tot->entries)) return;
+    if (warp && !all) pos = lp.wlist[pos];
     LinReg e;
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(lp.list + pos);
@@ -998,29 +1248,32 @@ __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
         d[0] = src[0];
         d[1] = src[1];
     }
-    if (e.stripe) return;
+    if (e.stripe || (!warp && e.n >= lin_wide(LOCAL))) return;
     const int m = e.m, n = e.n, ns = e.nstripe;
-    int seg = 0;
-    while (seg + 1 < LIN_SEG && pos >= lp.tot->seg[seg + 1]) ++seg;
-    const int L = lin_seg_lanes(seg), R = lin_seg_rows(seg);
-    const uint8_t *V = lp.kp.rseq + e.v, *Hs = lp.kp.cseq + e.h;
-    const uint32_t tile_row = (uint32_t)L * 8u;      // words per 8 steps
-    const uint32_t stripe_words = lin_tile_units(L, n) * 8u;
-    const uint32_t *dirs = reinterpret_cast<const uint32_t *>(lp.arena + (uint64_t)e.off * 32u);
+    const int cls = lin_class(lp, LOCAL, m, n);
+    const int L = lin_seg_lanes(cls), R = lin_seg_rows(cls);
+    LinDirs x;
+    x.V = lp.kp.rseq + e.v; x.Hs = lp.kp.cseq + e.h;
+    x.tile_row = (uint32_t)L * 8u;
+    x.stripe_words = lin_tile_units(L, n) * 8u;
+    x.dirs = reinterpret_cast<const uint32_t *>(lp.arena + (uint64_t)e.off * 32u);
+    x.rows = 2 * L * R; x.R = R;
+    x.e_tag = LOCAL ? 3 - lp.e_first : lp.e_first;
+    x.f_tag = LOCAL ? 2 + lp.e_first : 1 - lp.e_first;
     int4 d = lp.dp[pos + (LOCAL ? 0 : ns - 1)];
-    int i = m, j = n;
+    LinPath p{m, n, 0u, 0u, 0u};
     if (LOCAL) {
         for (int s = 1; s < ns; ++s) {
             const int4 o = lp.dp[pos + s];
             if (o.x > d.x) d = o;
         }
         // every virtual lane that reached the score: the smallest column, then row
-        const LinPlanes pl(true, seg, n);
-        const uint32_t *edges = dirs + (uint64_t)ns * stripe_words;
-        const uint32_t *snaps = edges + (uint64_t)ns * stripe_words;
+        const LinPlanes pl(true, cls, n);
+        const uint32_t *edges = x.dirs + (uint64_t)ns * x.stripe_words;
+        const uint32_t *snaps = edges + (uint64_t)ns * x.stripe_words;
         const int *bases = reinterpret_cast<const int *>(snaps + (uint64_t)ns * pl.snap * 8u);
         const uint32_t *ids = reinterpret_cast<const uint32_t *>(bases) + (uint64_t)ns * pl.base * 8u;
-        i = 0;
+        p.i = 0;
         for (int s = 0; d.w && s < ns; ++s) {
             const int4 o = lp.dp[pos + s];
             if (o.x != d.x) continue;
@@ -1033,71 +1286,41 @@ __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp)
                 LinStrip q;
                 q.half = v & 1;
                 // the row above: the virtual lane before, or the last one of the stripe above
-                q.edge = edges + (uint64_t)s * stripe_words;
+                q.edge = edges + (uint64_t)s * x.stripe_words;
                 q.va = v;
-                if (v == 0) { q.va = 2 * L; q.edge = s ? q.edge - stripe_words : nullptr; }
+                if (v == 0) { q.va = 2 * L; q.edge = s ? q.edge - x.stripe_words : nullptr; }
                 const int c = (int)((__ldg(ids + (uint64_t)s * pl.ids * 8u + t) >> (16 * q.half)) & 0xffffu);
                 const int start = 32 * c - 2 * t - q.half;       // its column before the chunk
                 q.col = max(0, start);
                 q.snap = snaps + ((uint64_t)s * pl.snap + (uint64_t)(c * L + t)) * 8u;
-                q.base = q.col && seg < 4 ? __ldg(bases + (uint64_t)s * pl.base * 8u + (uint64_t)(c * 32 + t)) : 0;
+                q.base = q.col && cls < 4 ? __ldg(bases + (uint64_t)s * pl.base * 8u + (uint64_t)(c * 32 + t)) : 0;
                 // an earlier find wins a tie (its rows are above)
-                const int lim = min(i ? j - 1 : n, start + 32);
-                const uint32_t z = lin_locate(sm, V, m, row0, R, Hs, lim, d.x, lp.kp.go, tile_row, q);
-                if (z != ~0u) { j = (int)(z >> 3); i = row0 + (int)(z & 7u) + 1; }
+                const int lim = min(p.i ? p.j - 1 : n, start + 32);
+                const uint32_t z = lin_locate(sm, x.V, m, row0, R, x.Hs, lim, d.x, lp.kp.go, x.tile_row, q);
+                if (z != ~0u) { p.j = (int)(z >> 3); p.i = row0 + (int)(z & 7u) + 1; }
             }
         }
-        if (!i) d.w = 0;
+        if (!p.i) d.w = 0;
     }
-    const int end_i = i, end_j = j;
-    uint32_t M = 0, D = 0, G = 0;
-    int last = 0;
+    const int end_i = p.i, end_j = p.j;
     if (!LOCAL || d.w) {
-        const int e_tag = lp.e_first, f_tag = 1 - lp.e_first, go = lp.kp.go;
-        int st = (i - 1) / (2 * L * R);
-        int v = (i - 1 - st * 2 * L * R) / R;
-        int sh = 2 * (R - 1 - (i - 1 - st * 2 * L * R - v * R));   // the row's bits in its half
-        const uint32_t *base = dirs + (uint64_t)st * stripe_words;
-        int h = LOCAL ? d.x : 1;
-        while (i > 0 && j > 0 && h > 0) {
-            const int k = j - 1 + v;
-            const uint32_t *w = base + (uint32_t)(k >> 3) * tile_row + (uint32_t)((v >> 1) * 8 + (k & 7));
-            const uint32_t word = __ldg(w);
-            // the tile before this one along the lane: in L1 by the time the walk gets there
-            if ((k & 7) == 7 && k > 7) asm volatile("prefetch.global.L1 [%0];" :: "l"(w - tile_row));
-            int sab = 0;
-            if (LOCAL) sab = sm[__ldg(V + i - 1) * 32 + __ldg(Hs + j - 1)];
-            const int tag = (int)(word >> (16 * (v & 1) + sh)) & 3;
-            const bool up = tag != e_tag, left = tag != f_tag;
-            const int mv = tag >= 2 ? 0 : tag == f_tag ? 1 : 2;
-            M += tag == 3 ? 1u : 0u;
-            D += tag >= 2 ? 1u : 0u;
-            G += mv != 0 && mv != last ? 1u : 0u;
-            last = mv;
-            if (LOCAL) h -= mv ? go : sab;
-            i -= up ? 1 : 0;
-            j -= left ? 1 : 0;
-            sh += up ? 2 : 0;
-            if (sh == 2 * R) {
-                sh = 0;
-                if (--v < 0) { v = 2 * L - 1; base -= stripe_words; }
-            }
-        }
-        if (!LOCAL && ((i > 0 && last != 1) || (j > 0 && last != 2))) ++G;
+        if (warp) lin_walk_warp<LOCAL>(x, p, dummy + threadIdx.x);
+        else lin_walk_thread<LOCAL>(x, p);
     }
+    if (warp && (threadIdx.x & 31)) return;
     if (!LOCAL) {
-        lp.walk[e.key] = make_int4(d.x, (int)M, (int)D, (int)G);
+        lp.walk[e.key] = make_int4(d.x, (int)p.M, (int)p.D, (int)p.G);
         return;
     }
     pg_result o = empty_result();
     o.cells = sat_u32((uint64_t)m * (uint64_t)n);
     if (d.w) {
-        const uint32_t len = (uint32_t)((end_i - i) + (end_j - j)) - D;
+        const uint32_t len = (uint32_t)((end_i - p.i) + (end_j - p.j)) - p.D;
         o.score = d.x;
-        o.aln_len = len; o.matches = M; o.gap_opens = G;
-        o.beg_v = (uint16_t)i; o.end_v = (uint16_t)end_i;
-        o.beg_h = (uint16_t)j; o.end_h = (uint16_t)end_j;
-        if (len > 0) { o.identity = identity_of(M, len); o.flags = 0; }
+        o.aln_len = len; o.matches = p.M; o.gap_opens = p.G;
+        o.beg_v = (uint16_t)p.i; o.end_v = (uint16_t)end_i;
+        o.beg_h = (uint16_t)p.j; o.end_h = (uint16_t)end_j;
+        if (len > 0) { o.identity = identity_of(p.M, len); o.flags = 0; }
     }
     apply_filter(o, m, n, lp.kp.cov_thr, lp.kp.ani_thr);
     lp.kp.out[e.key] = o;
@@ -1164,7 +1387,10 @@ static __global__ void __launch_bounds__(256) k_lin_finish(const LinParams lp)
     }
 }
 
+#ifdef PG_LIN_UNIT
 // ------------------------------------------------------------ host launches
+// (only in the units that instantiate them: a second copy of the kernels would
+// come with every other include)
 template <bool XDROP>
 cudaError_t lin_attributes(int *blocks_per_sm)
 {
@@ -1184,19 +1410,28 @@ void lin_count(const LinParams &lp, int nsm, cudaStream_t st)
 }
 // list, DP, traceback and results; returns the launches
 template <bool XDROP>
-int lin_align(const LinParams &lp, uint32_t entries, uint32_t jobs, int nsm, int max_blocks, cudaStream_t st)
+int lin_align(const LinParams &lp, uint32_t entries, uint32_t wide, uint32_t jobs, int nsm, int max_blocks,
+              cudaStream_t st)
 {
     const uint64_t n = lp.p1 - lp.p0;
     const uint64_t gp = (n + LIN_PT * LIN_PP - 1) / (LIN_PT * LIN_PP);
     k_lin_place<XDROP><<<(int)(gp < (uint64_t)nsm * 8 ? gp : (uint64_t)nsm * 8), LIN_PT, 0, st>>>(lp);
-    const int gd = (int)(jobs < (uint32_t)max_blocks ? (jobs ? jobs : 1) : (uint32_t)max_blocks);
-    k_lin_dp<!XDROP><<<gd, WARPS * 32, LIN_DYN, st>>>(lp);
-    k_lin_walk<!XDROP><<<entries ? (entries + 255) / 256 : 1, 256, 0, st>>>(lp);
+    // fewer jobs than resident warps: as few warps per block as hold them, so that
+    // they spread over the SMs
+    const uint32_t want = (jobs + (uint32_t)max_blocks - 1) / (uint32_t)max_blocks;
+    const int warps = want < 1 ? 1 : want < (uint32_t)WARPS ? (int)want : WARPS;
+    k_lin_dp<!XDROP><<<max_blocks, warps * 32, warps * LIN_PROF, st>>>(lp, nsm);
+    // a warp per wide region, whose walk is long, and per region while that leaves
+    // SMs with no more than LIN_WALK_WARPS of them
+    const bool all = entries <= (uint32_t)nsm * LIN_WALK_WARPS;
+    const uint32_t wb = ((all ? entries : wide) + 7) / 8, tb = all ? 0 : (entries + 255) / 256;
+    k_lin_walk<!XDROP><<<wb + tb ? wb + tb : 1, 256, 0, st>>>(lp, wb, all);
     if (XDROP) {
         const uint64_t gf = (n + 255) / 256;
         k_lin_finish<<<(int)(gf < (uint64_t)nsm * 8 ? gf : (uint64_t)nsm * 8), 256, 0, st>>>(lp);
     }
     return XDROP ? 4 : 3;
 }
+#endif
 
 }  // namespace pg

@@ -16,8 +16,10 @@ cudaError_t lin_attributes(int *blocks_per_sm);
 // class sizes and totals (lp.tot) of the pairs [lp.p0, lp.p1); two launches
 template <bool XDROP>
 void lin_count(const LinParams &lp, int nsm, cudaStream_t st);
-// their list, DP, traceback and results, after lin_count; returns the launches
+// their list, DP, traceback and results, after lin_count, which found `entries`
+// list entries (`wide` regions among them of lin_wide columns) and `jobs`; returns the launches
 template <bool XDROP>
-int lin_align(const LinParams &lp, uint32_t entries, uint32_t jobs, int nsm, int max_blocks, cudaStream_t st);
+int lin_align(const LinParams &lp, uint32_t entries, uint32_t wide, uint32_t jobs, int nsm, int max_blocks,
+              cudaStream_t st);
 
 }  // namespace pg

@@ -17,12 +17,12 @@ COLS = [1, 2, 3, 4, 5, 7, 8, 9, 33, 61, 250, 700, 1500]
 
 
 def _extreme():
-    """Scores over the whole range the tagged int8 profile holds, -32 to 31."""
+    """Scores over the whole range the tagged int8 profile holds, -31 to 31."""
     rng = np.random.default_rng(5)
-    s = rng.integers(-32, 12, (25, 25))
+    s = rng.integers(-31, 12, (25, 25))
     s = np.minimum(s, s.T)
     s[np.arange(25), np.arange(25)] = rng.integers(5, 32, 25)
-    s[3, 4] = s[4, 3] = -32
+    s[3, 4] = s[4, 3] = -31
     s[0, 0] = 31
     return np.ascontiguousarray(s.astype(np.int8))
 
