@@ -168,6 +168,7 @@ struct pg_ctx {
     uint64_t list_cap = 0;
     int4 *d_walk = nullptr;
     uint64_t walk_cap = 0;
+    cudaMemPool_t pool = nullptr;       // scratch of the calls around the aligner (pg_kmer.cu, pg_fasta.cu)
     // staging for the host-buffer entry point
     pg_pair *d_pairs = nullptr;
     pg_result *d_out = nullptr;
@@ -258,6 +259,7 @@ void pg_destroy(pg_ctx *ctx)
     cudaFree(ctx->d_dsc); cudaFree(ctx->d_scan);
     cudaFree(ctx->d_lin); cudaFree(ctx->d_list); cudaFree(ctx->d_walk);
     cudaFreeHost(ctx->h_lin);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cudaFree(ctx->d_pairs);
     cudaFree(ctx->d_out);
     for (int k = 0; k < 3; ++k)
@@ -975,6 +977,33 @@ int pg_internal_adopt_side(pg_ctx *c, int side, uint8_t *d_codes, uint64_t *d_of
     if (n > 0) CU(cudaMemcpy(&s.nres, d_offs + n, sizeof s.nres, cudaMemcpyDeviceToHost));
     ++c->epoch;
     return ensure_scratch(c);
+}
+
+// internal: the context's own memory pool, made at its first use.  It keeps up to
+// POOL_KEEP bytes between calls: with the device's default pool, which gives all of
+// it back at every synchronization, mapping the candidate generator's scratch again
+// took half of its call.  pg_destroy gives it back.
+constexpr uint64_t POOL_KEEP = (uint64_t)8 << 30;
+int pg_internal_pool(pg_ctx *c, cudaMemPool_t *pool)
+{
+    if (!c) return fail(PG_ERR_ARG, "null context");
+    if (!c->pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->cfg.device;
+        cudaMemPool_t p = nullptr;
+        CU(cudaMemPoolCreate(&p, &props));
+        uint64_t keep = POOL_KEEP;
+        const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(p);
+            return fail(PG_ERR_CUDA, "cudaMemPoolSetAttribute: %s", cudaGetErrorString(e));
+        }
+        c->pool = p;
+    }
+    *pool = c->pool;
+    return PG_OK;
 }
 
 // internal: the context's substitution table on the device (25 x 25 int8)

@@ -2,19 +2,25 @@
 // PASTIS (src/kmer/KmerOps.cpp:31-245, src/sim_search.cpp:154-187) with the
 // KmerIntersectLoc semiring (inc/sr.hpp:30-117), restated as sort and join.
 //
-//   1. k-mers of every row and column sequence of the block: code over the
-//      alphabet (Horner, base = alphabet size, as KmerOps.cpp:60-62), offset;
-//      one warp per sequence, lanes across positions.
-//   2. radix sort of each side by code (the columns of A).
-//   3. join: every row occurrence meets the run of equal codes on the column
-//      side; each occurrence pair that survives the symmetric prune becomes a
-//      product (key = col << 32 | row, seed = code << 32 | row off << 16 | col off).
-//   4. radix sort of the products by key, run-length encoding, and per pair:
-//      count = run length, first / second seed = smallest / largest seed
-//      value, score = largest k-mer self score; ckthr / mosthr applied.
-// The products of one call live in HBM at once (16 B each plus the sort's
-// double buffer); max_products bounds them and callers block larger inputs,
-// as PASTIS blocks its SpGEMM.
+//   1. k-mers of every row sequence of the block: code over the alphabet
+//      (Horner, base = alphabet size, as KmerOps.cpp:60-62), offset; one warp per
+//      sequence, lanes across positions.
+//   2. radix sort of the row occurrences by a bijection of the code (a
+//      multiplication modulo a power of two, so that a table indexed by its top
+//      bits is evenly filled), and that table: first occurrence of each value.
+//   3. a block per column sequence: each of its k-mers finds its run of equal
+//      codes on the row side through the table; the occurrence pairs that survive
+//      the symmetric prune are counted per row in a hash table in shared memory.
+//      The rows whose count passes ckthr (a few: most pairs share one k-mer by
+//      chance) get their first / second seed (smallest / largest seed value) and
+//      score (largest k-mer self score) in a second sweep over the same runs, are
+//      ranked by row and written out.
+//   4. the columns' records are moved into place, column-major.
+// The product of a block is never written out or sorted: for 200k proteins that
+// was 58M 16-byte products through a 7-pass radix sort, a run-length encoding and
+// a reduction, 28.5 ms a call with the allocation of their buffers; 11.3 ms now.  A
+// column with more rows than the hash table holds goes through a dense array over
+// the rows in global memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,7 +29,6 @@
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_run_length_encode.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include "../../include/pastis_gb300.h"
@@ -33,6 +38,7 @@ int pg_internal_seqs(const pg_ctx *c, const uint8_t **rseq, const uint64_t **rof
                      void **stream, int *mode);
 int pg_internal_fail(int code, const char *msg);
 int pg_internal_score(const pg_ctx *c, const int8_t **d_sm);
+int pg_internal_pool(pg_ctx *c, cudaMemPool_t *pool);
 
 namespace {
 
@@ -56,7 +62,14 @@ struct KmerTab {
     int16_t cost[32];    // alphabet code -> self score of its letter
     uint32_t base;
     int k;
+    int bits;            // of the k-mer universe
 };
+
+// the bijection of a code the row side is sorted by
+__device__ __forceinline__ uint32_t kmer_mix(uint32_t code, int bits)
+{
+    return (code * 0x9E3779B1u) & (bits < 32 ? (1u << bits) - 1u : 0xffffffffu);
+}
 
 // k-mers of sequences [s0, s0 + ns) of one side; one warp per sequence
 __global__ void k_kmer_fill(const uint8_t *seq, const uint64_t *offs, uint64_t s0, uint64_t ns,
@@ -76,7 +89,7 @@ __global__ void k_kmer_fill(const uint8_t *seq, const uint64_t *offs, uint64_t s
             const int pos = q * stride;
             uint32_t code = 0;
             for (int j = 0; j < tab.k; ++j) code = code * tab.base + tab.map[seq[b + pos + j] & 31];
-            codes[o + q] = code;
+            codes[o + q] = kmer_mix(code, tab.bits);
             vals[o + q] = (s << 16) | (uint64_t)pos;
         }
     }
@@ -92,16 +105,6 @@ __global__ void k_kmer_count(const uint64_t *offs, uint64_t s0, uint64_t ns, int
     }
 }
 
-// first index in [lo, hi) with a[i] >= v
-__device__ __forceinline__ uint64_t lower(const uint32_t *a, uint64_t lo, uint64_t hi, uint32_t v)
-{
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-
 // PG_PRUNE_* on global indices (sim_search.cpp:172-186 and :403-412)
 __device__ __forceinline__ bool keep_pair(int prune, uint64_t r, uint64_t c)
 {
@@ -114,69 +117,439 @@ __device__ __forceinline__ bool keep_pair(int prune, uint64_t r, uint64_t c)
     return true;
 }
 
-// pass 1 (emit == false): products per row occurrence; pass 2: write them
-template <bool EMIT>
-__global__ void k_join(const uint32_t *rcode, const uint64_t *rval, uint64_t nrk,
-                       const uint32_t *ccode, const uint64_t *cval, uint64_t nck,
-                       uint64_t row_begin, uint64_t col_begin, int prune, uint64_t *cnt,
-                       const uint64_t *start, uint64_t *keys, uint64_t *seeds)
+// the distinct values of the sorted codes: their number per block of RB codes,
+// then (after a scan of those) their value and first occurrence (one entry more:
+// the end), for each value of their top bits the first distinct one (table, ~0:
+// none), and the occurrences' rows and offsets in arrays of their own (the sweeps
+// over a run read rows only)
+constexpr int RB = 2048;
+template <class I>
+struct KmerRun {
+    uint32_t h;
+    I start;
+};
+__global__ void __launch_bounds__(256) k_runs_count(const uint32_t *h, uint64_t n, uint32_t *cnt)
 {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nrk;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t code = rcode[i];
-        const uint64_t lo = lower(ccode, 0, nck, code);
-        const uint64_t rv = rval[i];
-        const uint64_t r = rv >> 16, rpos = rv & 0xffff;
-        uint64_t n = 0, o = EMIT ? start[i] : 0;
-        for (uint64_t j = lo; j < nck && ccode[j] == code; ++j) {
-            const uint64_t cv = cval[j];
-            const uint64_t c = cv >> 16, cpos = cv & 0xffff;
-            if (!keep_pair(prune, r + row_begin, c + col_begin)) continue;
-            if (EMIT) {
-                keys[o] = (c << 32) | r;
-                seeds[o] = ((uint64_t)code << 32) | (rpos << 16) | cpos;
-                ++o;
-            } else {
-                ++n;
-            }
+    const uint64_t i0 = (uint64_t)blockIdx.x * RB;
+    uint32_t c = 0;
+    for (uint64_t i = i0 + threadIdx.x; i < min(i0 + RB, n); i += 256)
+        c += i == 0 || h[i - 1] != h[i] ? 1u : 0u;
+    c = __reduce_add_sync(0xffffffffu, c);
+    __shared__ uint32_t w[8];
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) c += w[k];
+        cnt[blockIdx.x] = c;
+    }
+}
+template <class I>
+__global__ void __launch_bounds__(256) k_runs_write(const uint32_t *h, const uint64_t *val, uint64_t n,
+                                                    const uint64_t *first, int shift, KmerRun<I> *run, I *table,
+                                                    uint32_t *rrow, uint16_t *rpos)
+{
+    __shared__ uint32_t w[8];
+    const uint64_t i0 = (uint64_t)blockIdx.x * RB;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t o = first[blockIdx.x];
+    for (uint64_t q = i0; q < min(i0 + RB, n); q += 256) {
+        const uint64_t i = q + threadIdx.x;
+        const uint32_t v = i < n ? h[i] : 0u, u = i < n && i ? h[i - 1] : 0u;
+        const bool head = i < n && (i == 0 || u != v);
+        const uint32_t m = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) w[warp] = (uint32_t)__popc(m);
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+        for (int k = 0; k < 8; ++k) { before += k < warp ? w[k] : 0u; all += w[k]; }
+        if (head) {
+            const uint64_t x = o + before + (uint32_t)__popc(m & ((1u << lane) - 1u));
+            run[x] = KmerRun<I>{v, (I)i};
+            if (i == 0 || (u >> shift) != (v >> shift)) table[v >> shift] = (I)x;
         }
-        if (!EMIT) cnt[i] = n;
+        if (i < n) {
+            const uint64_t rv = val[i];
+            rrow[i] = (uint32_t)(rv >> 16);
+            rpos[i] = (uint16_t)rv;
+        }
+        if (i == n - 1) run[o + all] = KmerRun<I>{0u, (I)n};
+        o += all;
+        __syncthreads();
     }
 }
 
-// one pair per run of equal keys
-__global__ void k_reduce_pairs(const uint64_t *ukeys, const uint32_t *rlen, const uint64_t *rstart,
-                               const uint64_t *nruns, const uint64_t *seeds, KmerTab tab,
-                               int ckthr, int mosthr, pg_pair *out, uint32_t *keep)
+// the run of each column k-mer on the row side (length 0: none), in the order of
+// the columns; a warp per column, lanes across positions.  own: the columns are the
+// rows and a k-mer of its own sequence alone makes no pair.
+template <class I>
+__global__ void k_col_runs(const uint8_t *seq, const uint64_t *offs, uint64_t s0, uint64_t ns, int stride,
+                           const uint64_t *kstart, KmerTab tab, const I *table, int shift, const KmerRun<I> *run,
+                           uint64_t nu, bool own, I *first, uint32_t *len)
 {
-    const uint64_t nr = *nruns;
-    for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nr;
-         u += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t b = rstart[u];
-        const uint32_t len = rlen[u];
-        uint64_t mn = ~0ull, mx = 0;
-        int score = -32768;
-        for (uint32_t q = 0; q < len; ++q) {
-            const uint64_t sv = seeds[b + q];
-            mn = sv < mn ? sv : mn;
-            mx = sv > mx ? sv : mx;
-            uint32_t code = (uint32_t)(sv >> 32);
-            int cost = 0;
-            for (int j = 0; j < tab.k; ++j) { cost += tab.cost[code % tab.base]; code /= tab.base; }
-            score = cost > score ? cost : score;
+    __shared__ uint8_t map[32];
+    if (threadIdx.x < 32) map[threadIdx.x] = tab.map[threadIdx.x];
+    __syncthreads();
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    for (uint64_t s = warp; s < ns; s += nwarps) {
+        const uint64_t b = offs[s0 + s], o = kstart[s];
+        const int nk = (int)(kstart[s + 1] - o);
+        for (int q = lane; q < nk; q += 32) {
+            const uint8_t *p = seq + b + (uint64_t)q * (uint64_t)stride;
+            uint32_t code = 0;
+            for (int j = 0; j < tab.k; ++j) code = code * tab.base + map[__ldg(p + j) & 31];
+            const uint32_t h = kmer_mix(code, tab.bits);
+            I lo = 0, hi = 0;
+            const I t = __ldg(table + (h >> shift));
+            if (t != (I)~(I)0) {
+                uint64_t u = t;
+                KmerRun<I> e = run[u];
+                while (e.h < h && ++u < nu) e = run[u];
+                if (u < nu && e.h == h) { lo = e.start; hi = run[u + 1].start; }
+            }
+            if (own && hi - lo == 1) hi = lo;
+            first[o + q] = lo;
+            len[o + q] = (uint32_t)(hi - lo);
         }
-        const uint16_t count = (uint16_t)len;   // ushort arithmetic of the semiring
-        pg_pair p;
-        p.row = (uint32_t)(ukeys[u] & 0xffffffffu);
-        p.col = (uint32_t)(ukeys[u] >> 32);
-        p.rs0 = (uint16_t)((mn >> 16) & 0xffff);
-        p.cs0 = (uint16_t)(mn & 0xffff);
-        p.rs1 = len >= 2 ? (uint16_t)((mx >> 16) & 0xffff) : 0;
-        p.cs1 = len >= 2 ? (uint16_t)(mx & 0xffff) : 0;
-        p.count = count;
-        p.score = (int16_t)score;
-        out[u] = p;
-        keep[u] = ((int)count > ckthr && score > mosthr) ? 1u : 0u;
+    }
+}
+
+constexpr int CT = 128;              // threads per column block
+constexpr int CSLOT = 2048;          // hash slots: 6 blocks per SM with their tables
+constexpr int CLIST = 896;           // pairs kept for the second sweep
+constexpr int CROWS = 1536;          // distinct rows a block takes (CT inserts may be under way beyond)
+constexpr int CSURV = 320;           // rows that pass ckthr
+constexpr uint32_t CRUN = 1024;     // rows of a run that is expanded with its warp's others
+constexpr uint32_t CEMPTY = 0xffffffffu;
+constexpr uint32_t CMARK = 0x80000000u;
+
+// what the column kernels share
+template <class I>
+struct CandArgs {
+    const uint8_t *cseq;
+    const uint64_t *coffs;
+    uint64_t col_begin, ncols, row_begin, nrows;
+    KmerTab tab;
+    int stride, prune, ckthr, mosthr;
+    const uint32_t *rrow;            // row occurrences by mixed code: sequence, offset
+    const uint16_t *rpos;
+    const uint64_t *kstart;          // first k-mer of each column, and of its k-mers:
+    const I *first;                  // first row occurrence,
+    const uint32_t *len;             // their number
+    pg_pair *tmp;                    // records in any column order, tmp_cap of them
+    uint64_t tmp_cap;
+    uint64_t *start;                 // per column: its records in tmp, their number
+    uint32_t *cnt;
+    unsigned long long *tot;         // [0] products, [1] records, [2] overflowed columns, [3] next column
+    uint32_t *ovf;                   // overflowed columns
+};
+
+// Visits every occurrence pair of column c that survives the prune, in no order:
+// visit(valid, row, row occurrence j, k-mer number), called by whole warps (the
+// lanes without a pair pass valid = false).  The block's threads take the column's
+// k-mers, CQ each at a time, their reads in flight together.  Returns this thread's
+// number of pairs.
+constexpr int CQ = 3;
+template <class I, class F>
+__device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c, F visit)
+{
+    const uint64_t o = A.kstart[c];
+    const int nk = (int)(A.kstart[c + 1] - o);
+    const int lane = threadIdx.x & 31;
+    const uint64_t gc = c + A.col_begin;
+    uint64_t np = 0;
+    auto one = [&](bool in, uint64_t j, int q) {
+        const uint32_t r = in ? __ldg(A.rrow + j) : 0u;
+        const bool valid = in && keep_pair(A.prune, r + A.row_begin, gc);
+        np += valid ? 1 : 0;
+        visit(valid, r, j, q);
+    };
+    for (int q0 = 0; q0 < nk; q0 += (int)blockDim.x * CQ) {
+        __syncwarp();
+        I lo[CQ];
+        uint32_t ln[CQ];
+#pragma unroll
+        for (int r = 0; r < CQ; ++r) {
+            const int q = q0 + r * (int)blockDim.x + (int)threadIdx.x;
+            lo[r] = 0; ln[r] = 0;
+            if (q < nk) { lo[r] = __ldg(A.first + o + q); ln[r] = __ldg(A.len + o + q); }
+        }
+#pragma unroll
+        for (int r = 0; r < CQ; ++r) {
+            // the warp's runs end to end, a lane per occurrence pair (a lane per run left
+            // 3 of 32 lanes busy: a family's k-mer has tens of rows, a chance one one or
+            // two); runs of more than CRUN rows one at a time
+            const int q = q0 + r * (int)blockDim.x + (int)threadIdx.x;
+            const bool big = ln[r] > CRUN;
+            const uint32_t n = big ? 0u : ln[r];
+            uint32_t inc = n;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += y;
+            }
+            const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+            const I l0 = lo[r] - (I)(inc - n);     // run start less the pairs before it
+            for (uint32_t i0 = 0; i0 < all; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                int src = 0;                       // the lane whose run holds pair i
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1)
+                    if (__shfl_sync(0xffffffffu, inc, src + d - 1) <= i) src += d;
+                src = min(src, 31);
+                const I l = __shfl_sync(0xffffffffu, l0, src);
+                one(i < all, (uint64_t)(I)(l + (I)i), q - lane + src);
+            }
+            for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
+                const int src = __ffs(m) - 1;
+                const I l = __shfl_sync(0xffffffffu, lo[r], src);
+                const uint32_t u = __shfl_sync(0xffffffffu, ln[r], src);
+                for (uint32_t j = 0; j < u; j += 32) one(j + lane < u, (uint64_t)l + j + lane, q - lane + src);
+            }
+        }
+    }
+    return np;
+}
+
+// code and self score of the k-mer at p
+__device__ __forceinline__ uint32_t kmer_at(const uint8_t *p, const uint8_t *map, const int *cost, const KmerTab &tab,
+                                            int &score)
+{
+    uint32_t code = 0;
+    score = 0;
+    for (int j = 0; j < tab.k; ++j) {
+        const uint32_t a = map[__ldg(p + j) & 31];
+        code = code * tab.base + a;
+        score += cost[a];
+    }
+    return code;
+}
+__device__ __forceinline__ uint64_t seed_value(uint32_t code, uint32_t rpos, int cpos)
+{
+    return ((uint64_t)code << 32) | ((uint64_t)rpos << 16) | (uint64_t)cpos;
+}
+
+__device__ __forceinline__ pg_pair cand_record(uint32_t row, uint64_t c, uint32_t len, uint64_t mn, uint64_t mx,
+                                               int score)
+{
+    pg_pair p;
+    p.row = row;
+    p.col = (uint32_t)c;
+    p.rs0 = (uint16_t)((mn >> 16) & 0xffff);
+    p.cs0 = (uint16_t)(mn & 0xffff);
+    p.rs1 = len >= 2 ? (uint16_t)((mx >> 16) & 0xffff) : 0;
+    p.cs1 = len >= 2 ? (uint16_t)(mx & 0xffff) : 0;
+    p.count = (uint16_t)len;         // ushort arithmetic of the semiring
+    p.score = (int16_t)score;
+    return p;
+}
+__device__ __forceinline__ bool cand_count_ok(uint32_t len, int ckthr) { return (int)(uint16_t)len > ckthr; }
+
+// What bounds it: the latency of a column's chain of reads (table, code, run, row
+// values, all at random places in HBM or L2), hidden by the other columns of an
+// SM; hence small blocks, a hash table just large enough for the long proteins'
+// columns, and the second sweep from a list of the pairs kept in shared memory
+// (from the runs again where a column has more than CLIST of them).
+template <class I>
+__global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
+{
+    __shared__ uint32_t key[CSLOT], num[CSLOT];
+    __shared__ I list_j[CLIST];
+    __shared__ uint32_t list_qs[CLIST];          // k-mer number << 11 | hash slot
+    __shared__ uint16_t used[CROWS + CT];        // the slots in use
+    __shared__ unsigned long long smin[CSURV], smax[CSURV];
+    __shared__ uint32_t srow[CSURV], slen[CSURV];
+    __shared__ int sscore[CSURV], cost[32];
+    __shared__ uint8_t map[32];
+    __shared__ uint32_t ndist, nsurv, nkeep, nlist, over;
+    __shared__ unsigned long long base;
+    static_assert(CSLOT == 2048, "11 bits of a list word");
+    const int t = threadIdx.x;
+    if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
+    if (t == 0) ndist = 0;
+    for (int k = t; k < CSLOT; k += CT) { key[k] = CEMPTY; num[k] = 0; }
+    unsigned long long products = 0;
+    for (;;) {
+        // the next column: one counter for all blocks, columns differ in length
+        if (t == 0) base = atomicAdd(&A.tot[3], 1ull);
+        __syncthreads();
+        const uint64_t c = base;
+        if (c >= A.ncols) break;
+        for (uint32_t x = t; x < ndist; x += CT) { key[used[x]] = CEMPTY; num[used[x]] = 0; }
+        __syncthreads();
+        if (t == 0) { ndist = 0; nsurv = 0; nkeep = 0; nlist = 0; over = 0; }
+        __syncthreads();
+        products += cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
+            // a full table is left alone (its column goes the dense way): one lane's
+            // reading decides for the warp, which stays together for the ballots below
+            if (__shfl_sync(0xffffffffu, *(volatile uint32_t *)&ndist, 0) >= CROWS) { over = 1; return; }
+            uint32_t s = (r * 0x9E3779B1u) >> 21;
+            bool fresh = false;
+            while (valid) {
+                uint32_t k = *(volatile uint32_t *)&key[s];
+                if (k == CEMPTY) { k = atomicCAS(&key[s], CEMPTY, r); fresh = k == CEMPTY; }
+                if (fresh || k == r) break;
+                s = (s + 1) & (CSLOT - 1);
+            }
+            __syncwarp();
+            if (valid) atomicAdd(&num[s], 1u);
+            // one atomic a warp for the places in the two lists
+            const uint32_t mf = __ballot_sync(0xffffffffu, fresh), mv = __ballot_sync(0xffffffffu, valid);
+            const uint32_t below = (1u << (t & 31)) - 1u;
+            uint32_t bf = 0, bv = 0;
+            if ((t & 31) == 0) {
+                if (mf) bf = atomicAdd(&ndist, (uint32_t)__popc(mf));
+                if (mv) bv = atomicAdd(&nlist, (uint32_t)__popc(mv));
+            }
+            bf = __shfl_sync(0xffffffffu, bf, 0);
+            bv = __shfl_sync(0xffffffffu, bv, 0) + (uint32_t)__popc(mv & below);
+            if (fresh) used[bf + (uint32_t)__popc(mf & below)] = (uint16_t)s;
+            if (valid && bv < CLIST) { list_j[bv] = (I)j; list_qs[bv] = ((uint32_t)q << 11) | s; }
+        });
+        __syncthreads();
+        for (uint32_t x = t; x < ndist && !over; x += CT) {
+            const int s = used[x];
+            const uint32_t len = num[s];
+            uint32_t mark = 0;
+            if (cand_count_ok(len, A.ckthr)) {
+                const uint32_t u = atomicAdd(&nsurv, 1u);
+                if (u < CSURV) {
+                    srow[u] = key[s]; slen[u] = len;
+                    smin[u] = ~0ull; smax[u] = 0; sscore[u] = -32768;
+                    mark = CMARK | u;
+                }
+            }
+            num[s] = mark;
+        }
+        __syncthreads();
+        if (over || nsurv > CSURV) {
+            if (t == 0) A.ovf[atomicAdd(&A.tot[2], 1ull)] = (uint32_t)c;
+            continue;
+        }
+        const uint32_t ns = nsurv;
+        if (ns) {
+            const uint8_t *p = A.cseq + A.coffs[A.col_begin + c];
+            auto update = [&](uint32_t u, uint64_t j, int q) {
+                int sc;
+                const uint32_t code = kmer_at(p + (uint64_t)q * (uint64_t)A.stride, map, cost, A.tab, sc);
+                const uint64_t sv = seed_value(code, __ldg(A.rpos + j), q * A.stride);
+                if (sv < *(volatile unsigned long long *)&smin[u]) atomicMin(&smin[u], (unsigned long long)sv);
+                if (sv > *(volatile unsigned long long *)&smax[u]) atomicMax(&smax[u], (unsigned long long)sv);
+                if (sc > *(volatile int *)&sscore[u]) atomicMax(&sscore[u], sc);
+            };
+            if (nlist <= CLIST) {
+                for (uint32_t x = t; x < nlist; x += CT) {
+                    const uint32_t w = list_qs[x], mark = num[w & (CSLOT - 1)];
+                    if (mark & CMARK) update(mark & ~CMARK, list_j[x], (int)(w >> 11));
+                }
+            } else {
+                cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
+                    if (!valid) return;
+                    uint32_t s = (r * 0x9E3779B1u) >> 21;
+                    while (key[s] != r) s = (s + 1) & (CSLOT - 1);
+                    const uint32_t mark = num[s];
+                    if (mark & CMARK) update(mark & ~CMARK, j, q);
+                });
+            }
+            __syncthreads();
+            for (uint32_t u = t; u < ns; u += CT)
+                if (sscore[u] > A.mosthr) atomicAdd(&nkeep, 1u);
+            __syncthreads();
+            if (t == 0) base = nkeep ? atomicAdd(&A.tot[1], (unsigned long long)nkeep) : 0;
+            __syncthreads();
+            const bool fits = base + nkeep <= A.tmp_cap;
+            for (uint32_t u = t; u < ns && fits; u += CT) {
+                if (sscore[u] <= A.mosthr) continue;
+                uint32_t rank = 0;
+                for (uint32_t v = 0; v < ns; ++v)
+                    rank += srow[v] < srow[u] && sscore[v] > A.mosthr ? 1u : 0u;
+                A.tmp[base + rank] = cand_record(srow[u], c, slen[u], smin[u], smax[u], sscore[u]);
+            }
+        }
+        if (t == 0) { A.start[c] = base; A.cnt[c] = nkeep; }
+    }
+    if (products) atomicAdd(&A.tot[0], products);
+}
+
+// the overflowed columns: a dense array over the rows per block (count, smallest
+// and largest seed value, score), cleared, filled and read out in row order
+struct CandDense {
+    unsigned long long mn, mx;
+    uint32_t len;
+    int score;
+};
+template <class I>
+__global__ void __launch_bounds__(256) k_cand_dense(const CandArgs<I> A, CandDense *dense, uint64_t novf)
+{
+    __shared__ int cost[32];
+    __shared__ uint8_t map[32];
+    __shared__ uint32_t wsum[8], total;
+    __shared__ unsigned long long base;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
+    CandDense *D = dense + (uint64_t)blockIdx.x * A.nrows;
+    auto kept = [&](uint64_t r) {
+        return r < A.nrows && D[r].len && cand_count_ok(D[r].len, A.ckthr) && D[r].score > A.mosthr;
+    };
+    for (uint64_t x = blockIdx.x; x < novf; x += gridDim.x) {
+        const uint64_t c = A.ovf[x];
+        for (uint64_t r = t; r < A.nrows; r += blockDim.x) D[r] = CandDense{~0ull, 0ull, 0u, -32768};
+        if (t == 0) total = 0;
+        __syncthreads();
+        const uint8_t *p = A.cseq + A.coffs[A.col_begin + c];
+        cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
+            if (!valid) return;
+            int sc;
+            const uint32_t code = kmer_at(p + (uint64_t)q * (uint64_t)A.stride, map, cost, A.tab, sc);
+            const uint64_t sv = seed_value(code, __ldg(A.rpos + j), q * A.stride);
+            atomicAdd(&D[r].len, 1u);
+            atomicMin(&D[r].mn, (unsigned long long)sv);
+            atomicMax(&D[r].mx, (unsigned long long)sv);
+            atomicMax(&D[r].score, sc);
+        });
+        __threadfence_block();
+        __syncthreads();
+        uint32_t n = 0;
+        for (uint64_t r = t; r < A.nrows; r += blockDim.x) n += kept(r) ? 1u : 0u;
+        if (n) atomicAdd(&total, n);
+        __syncthreads();
+        if (t == 0) {
+            base = total ? atomicAdd(&A.tot[1], (unsigned long long)total) : 0;
+            A.start[c] = base;
+            A.cnt[c] = total;
+        }
+        __syncthreads();
+        const bool fits = base + total <= A.tmp_cap;
+        uint64_t o = base;
+        for (uint64_t r0 = 0; r0 < A.nrows && fits; r0 += blockDim.x) {
+            const uint64_t r = r0 + t;
+            const bool k = kept(r);
+            const uint32_t m = __ballot_sync(0xffffffffu, k);
+            if (lane == 0) wsum[w] = (uint32_t)__popc(m);
+            __syncthreads();
+            uint32_t before = 0, all = 0;
+            for (int i = 0; i < 8; ++i) { before += i < w ? wsum[i] : 0u; all += wsum[i]; }
+            if (k)
+                A.tmp[o + before + (uint32_t)__popc(m & ((1u << lane) - 1u))] =
+                    cand_record((uint32_t)r, c, D[r].len, D[r].mn, D[r].mx, D[r].score);
+            o += all;
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+}
+
+// the columns' records into place, a warp per column, as 32-bit words
+__global__ void k_cand_place(const pg_pair *tmp, const uint64_t *start, const uint32_t *cnt, const uint64_t *pos,
+                             uint64_t ncols, pg_pair *out)
+{
+    constexpr int W = sizeof(pg_pair) / 4;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t c = warp; c < ncols; c += nwarps) {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(tmp + start[c]);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(out + pos[c]);
+        for (uint64_t k = threadIdx.x & 31; k < (uint64_t)cnt[c] * W; k += 32) dst[k] = src[k];
     }
 }
 
@@ -201,19 +574,11 @@ __global__ void k_triple_write(const pg_pair *pairs, const pg_result *res, uint6
     }
 }
 
-__global__ void k_compact_pairs(const pg_pair *in, const uint32_t *keep, const uint64_t *pos,
-                                const uint64_t *nruns, pg_pair *out)
-{
-    const uint64_t nr = *nruns;
-    for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nr;
-         u += (uint64_t)gridDim.x * blockDim.x)
-        if (keep[u]) out[pos[u]] = in[u];
-}
-
 // device buffers of one call, freed on every exit path
 struct Bufs {
     std::vector<void *> ptrs;
     cudaStream_t st = nullptr;
+    cudaMemPool_t pool = nullptr;    // the context's; null: the device's default pool
     ~Bufs()
     {
         for (void *p : ptrs) cudaFreeAsync(p, st);
@@ -222,7 +587,8 @@ struct Bufs {
     cudaError_t get(T **p, size_t count)
     {
         void *q = nullptr;
-        const cudaError_t e = cudaMallocAsync(&q, std::max<size_t>(count * sizeof(T), 16), st);
+        const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
+        const cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, bytes, pool, st) : cudaMallocAsync(&q, bytes, st);
         if (e == cudaSuccess) ptrs.push_back(q);
         *p = (T *)q;
         return e;
@@ -239,11 +605,13 @@ uint64_t pow_u(uint64_t b, int k)
 struct SideKmers {
     uint32_t *code = nullptr;
     uint64_t *val = nullptr;
+    uint64_t *start = nullptr;       // first k-mer of each sequence (one more: n)
     uint64_t n = 0;
 };
 
+// k-mers of one side: how many per sequence, and (sorted) the occurrences by mixed code
 int side_kmers(Bufs &B, const uint8_t *seq, const uint64_t *offs, uint64_t s0, uint64_t ns,
-               const pg_kmer_config &kc, const KmerTab &tab, int nsm, SideKmers &out)
+               const pg_kmer_config &kc, const KmerTab &tab, int nsm, bool sorted, SideKmers &out)
 {
     cudaStream_t st = B.st;
     uint64_t *cnt, *start;
@@ -261,23 +629,120 @@ int side_kmers(Bufs &B, const uint8_t *seq, const uint64_t *offs, uint64_t s0, u
     KCU(cudaMemcpyAsync(&total, start + ns, sizeof total, cudaMemcpyDeviceToHost, st));
     KCU(cudaStreamSynchronize(st));
     out.n = total;
+    out.start = start;
+    if (!sorted) return PG_OK;
     uint32_t *c0, *c1;
     uint64_t *v0, *v1;
     KCU(B.get(&c0, total)); KCU(B.get(&c1, total));
     KCU(B.get(&v0, total)); KCU(B.get(&v1, total));
     if (total) k_kmer_fill<<<grid, 256, 0, st>>>(seq, offs, s0, ns, kc.stride, start, tab, c0, v0);
     KCU(cudaGetLastError());
-    int bits = 1;
-    while (bits < 32 && ((uint64_t)1 << bits) < pow_u(tab.base, tab.k)) ++bits;
     cub::DoubleBuffer<uint32_t> kb(c0, c1);
     cub::DoubleBuffer<uint64_t> vb(v0, v1);
     size_t sb = 0;
-    KCU(cub::DeviceRadixSort::SortPairs(nullptr, sb, kb, vb, (int64_t)total, 0, bits, st));
+    KCU(cub::DeviceRadixSort::SortPairs(nullptr, sb, kb, vb, (int64_t)total, 0, tab.bits, st));
     void *stmp;
     KCU(B.get((char **)&stmp, sb));
-    KCU(cub::DeviceRadixSort::SortPairs(stmp, sb, kb, vb, (int64_t)total, 0, bits, st));
+    KCU(cub::DeviceRadixSort::SortPairs(stmp, sb, kb, vb, (int64_t)total, 0, tab.bits, st));
     out.code = kb.Current();
     out.val = vb.Current();
+    return PG_OK;
+}
+
+// steps 2 (the table) to 4 on the sorted row occurrences; I holds their indices
+template <class I>
+int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const KmerTab &tab, int nsm,
+                  const uint8_t *cseq, const uint64_t *coffs, const SideKmers &C, uint64_t row_begin,
+                  uint64_t nrows, bool same, uint64_t col_begin, uint64_t ncols, uint64_t maxp, pg_pair *d_out, uint64_t cap,
+                  uint64_t *n_out)
+{
+    cudaStream_t st = B.st;
+    const int grid = nsm * 8;
+    // about two occurrences per table entry, at most 2^24 entries (64 MB: inside L2)
+    int tb = 1;
+    while (tb < 24 && tb < tab.bits && ((uint64_t)2 << tb) < R.n) ++tb;
+    const uint64_t rblocks = (R.n + RB - 1) / RB;
+    uint32_t *rcnt;
+    uint64_t *rfirst;
+    KCU(B.get(&rcnt, rblocks + 1));
+    KCU(B.get(&rfirst, rblocks + 1));
+    KCU(cudaMemsetAsync(rcnt + rblocks, 0, sizeof(uint32_t), st));
+    k_runs_count<<<(unsigned)rblocks, 256, 0, st>>>(R.code, R.n, rcnt);
+    size_t rb = 0;
+    KCU(cub::DeviceScan::ExclusiveSum(nullptr, rb, rcnt, rfirst, (int64_t)(rblocks + 1), st));
+    void *rtmp;
+    KCU(B.get((char **)&rtmp, rb));
+    KCU(cub::DeviceScan::ExclusiveSum(rtmp, rb, rcnt, rfirst, (int64_t)(rblocks + 1), st));
+    uint64_t nu = 0;
+    KCU(cudaMemcpyAsync(&nu, rfirst + rblocks, sizeof nu, cudaMemcpyDeviceToHost, st));
+    KCU(cudaStreamSynchronize(st));
+    KmerRun<I> *run;
+    uint32_t *rrow, *clen;
+    uint16_t *rpos;
+    I *cfirst;
+    KCU(B.get(&run, nu + 1));
+    KCU(B.get(&rrow, R.n));
+    KCU(B.get(&rpos, R.n));
+    KCU(B.get(&cfirst, C.n));
+    KCU(B.get(&clen, C.n));
+    CandArgs<I> A;
+    A.cseq = cseq; A.coffs = coffs;
+    A.col_begin = col_begin; A.ncols = ncols; A.row_begin = row_begin; A.nrows = nrows;
+    A.tab = tab;
+    A.stride = kc.stride; A.prune = kc.prune; A.ckthr = kc.ckthr; A.mosthr = kc.mosthr;
+    A.rrow = rrow; A.rpos = rpos; A.kstart = C.start; A.first = cfirst; A.len = clen;
+    const int shift = tab.bits - tb;
+    I *table;
+    KCU(B.get(&table, (size_t)1 << tb));
+    KCU(cudaMemsetAsync(table, 0xff, sizeof(I) << tb, st));
+    k_runs_write<I><<<(unsigned)rblocks, 256, 0, st>>>(R.code, R.val, R.n, rfirst, shift, run, table, rrow, rpos);
+    k_col_runs<I><<<grid, 256, 0, st>>>(cseq, coffs, col_begin, ncols, kc.stride, C.start, tab, table, shift, run,
+                                        nu, same && kc.prune != PG_PRUNE_NONE, cfirst, clen);
+    KCU(B.get(&A.start, ncols));
+    KCU(B.get(&A.cnt, ncols + 1));
+    KCU(B.get(&A.ovf, ncols));
+    KCU(B.get(&A.tot, 4));
+    // records of the call: room for 32 a column at first, or what the caller takes
+    A.tmp_cap = std::min<uint64_t>(cap, std::max<uint64_t>((uint64_t)1 << 20, 32 * ncols));
+    unsigned long long tot[4] = {0, 0, 0, 0};
+    for (;;) {
+        KCU(B.get(&A.tmp, A.tmp_cap));
+        KCU(cudaMemsetAsync(A.cnt, 0, (ncols + 1) * sizeof(uint32_t), st));
+        KCU(cudaMemsetAsync(A.tot, 0, sizeof tot, st));
+        const uint64_t blocks = std::min<uint64_t>(ncols, (uint64_t)nsm * 6);
+        k_cand<I><<<(unsigned)blocks, CT, 0, st>>>(A);
+        KCU(cudaGetLastError());
+        KCU(cudaMemcpyAsync(tot, A.tot, sizeof tot, cudaMemcpyDeviceToHost, st));
+        KCU(cudaStreamSynchronize(st));
+        if (tot[0] > maxp)
+            return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: too many k-mer occurrence pairs for one block");
+        if (tot[2]) {
+            // dense arrays for as many columns at a time as 4 GiB hold
+            const uint64_t fit = std::max<uint64_t>(1, ((uint64_t)4 << 30) / (nrows * sizeof(CandDense)));
+            const uint64_t slots = std::min<uint64_t>(std::min<uint64_t>(tot[2], fit), (uint64_t)nsm * 4);
+            CandDense *dense;
+            KCU(B.get(&dense, slots * nrows));
+            k_cand_dense<I><<<(unsigned)slots, 256, 0, st>>>(A, dense, tot[2]);
+            KCU(cudaGetLastError());
+            KCU(cudaMemcpyAsync(tot, A.tot, sizeof tot, cudaMemcpyDeviceToHost, st));
+            KCU(cudaStreamSynchronize(st));
+        }
+        *n_out = tot[1];
+        if (tot[1] > cap) return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: output capacity too small");
+        if (tot[1] <= A.tmp_cap) break;
+        A.tmp_cap = tot[1];          // more records than the first guess: once more with room for them
+    }
+    if (!tot[1]) return PG_OK;
+    uint64_t *pos;
+    KCU(B.get(&pos, ncols + 1));
+    size_t xb = 0;
+    KCU(cub::DeviceScan::ExclusiveSum(nullptr, xb, A.cnt, pos, (int64_t)(ncols + 1), st));
+    void *xtmp;
+    KCU(B.get((char **)&xtmp, xb));
+    KCU(cub::DeviceScan::ExclusiveSum(xtmp, xb, A.cnt, pos, (int64_t)(ncols + 1), st));
+    k_cand_place<<<grid, 256, 0, st>>>(A.tmp, A.start, A.cnt, pos, ncols, d_out);
+    KCU(cudaGetLastError());
+    KCU(cudaStreamSynchronize(st));
     return PG_OK;
 }
 
@@ -340,96 +805,30 @@ int pg_candidates(pg_ctx *ctx, const pg_kmer_config *kc, uint64_t row_begin, uin
     // the reference asserts the k-mer universe fits an int (KmerOps.cpp:117-120)
     if (pow_u(tab.base, tab.k) > (uint64_t)0x7fffffff)
         return pg_internal_fail(PG_ERR_ARG, "pg_candidates: alphabet^k exceeds 2^31");
+    tab.bits = 1;
+    while (tab.bits < 32 && ((uint64_t)1 << tab.bits) < pow_u(tab.base, tab.k)) ++tab.bits;
     int nsm = 0;
     KCU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     Bufs B;
     B.st = stream ? (cudaStream_t)stream : (cudaStream_t)cst;
-    cudaStream_t st = B.st;
-    SideKmers R, C;
-    rc = side_kmers(B, rseq, roffs, row_begin, row_end - row_begin, *kc, tab, nsm, R);
+    rc = pg_internal_pool(ctx, &B.pool);
     if (rc) return rc;
     const bool same = rseq == cseq && roffs == coffs && row_begin == col_begin && row_end == col_end;
+    SideKmers R, C;
+    rc = side_kmers(B, rseq, roffs, row_begin, row_end - row_begin, *kc, tab, nsm, true, R);
+    if (rc) return rc;
     if (same) C = R;
     else {
-        rc = side_kmers(B, cseq, coffs, col_begin, col_end - col_begin, *kc, tab, nsm, C);
+        rc = side_kmers(B, cseq, coffs, col_begin, col_end - col_begin, *kc, tab, nsm, false, C);
         if (rc) return rc;
     }
-    const int grid = nsm * 8;
-    // products per row occurrence, then their offsets
-    uint64_t *pcnt, *pstart;
-    KCU(B.get(&pcnt, R.n + 1));
-    KCU(B.get(&pstart, R.n + 1));
-    KCU(cudaMemsetAsync(pcnt + R.n, 0, sizeof(uint64_t), st));
-    if (R.n)
-        k_join<false><<<grid, 256, 0, st>>>(R.code, R.val, R.n, C.code, C.val, C.n, row_begin,
-                                            col_begin, kc->prune, pcnt, nullptr, nullptr, nullptr);
-    KCU(cudaGetLastError());
-    size_t tb = 0;
-    KCU(cub::DeviceScan::ExclusiveSum(nullptr, tb, pcnt, pstart, R.n + 1, st));
-    void *tmp;
-    KCU(B.get((char **)&tmp, tb));
-    KCU(cub::DeviceScan::ExclusiveSum(tmp, tb, pcnt, pstart, R.n + 1, st));
-    uint64_t P = 0;
-    KCU(cudaMemcpyAsync(&P, pstart + R.n, sizeof P, cudaMemcpyDeviceToHost, st));
-    KCU(cudaStreamSynchronize(st));
+    if (!R.n || !C.n) return PG_OK;
     const uint64_t maxp = kc->max_products ? kc->max_products : (1ull << 31);
-    if (P > maxp) return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: too many k-mer occurrence pairs for one block");
-    if (P == 0) return PG_OK;
-    uint64_t *k0, *k1, *s0, *s1;
-    KCU(B.get(&k0, P)); KCU(B.get(&k1, P));
-    KCU(B.get(&s0, P)); KCU(B.get(&s1, P));
-    k_join<true><<<grid, 256, 0, st>>>(R.code, R.val, R.n, C.code, C.val, C.n, row_begin, col_begin,
-                                       kc->prune, nullptr, pstart, k0, s0);
-    KCU(cudaGetLastError());
-    int cbits = 1;
-    while (cbits < 32 && (1ull << cbits) < (col_end - col_begin)) ++cbits;
-    cub::DoubleBuffer<uint64_t> kb(k0, k1), sb(s0, s1);
-    size_t sbytes = 0;
-    KCU(cub::DeviceRadixSort::SortPairs(nullptr, sbytes, kb, sb, (int64_t)P, 0, 32 + cbits, st));
-    void *stmp;
-    KCU(B.get((char **)&stmp, sbytes));
-    KCU(cub::DeviceRadixSort::SortPairs(stmp, sbytes, kb, sb, (int64_t)P, 0, 32 + cbits, st));
-    // runs of equal keys = candidate pairs
-    uint64_t *ukeys, *nruns, *rstart;
-    uint32_t *rlen, *keep;
-    KCU(B.get(&ukeys, P)); KCU(B.get(&rlen, P + 1)); KCU(B.get(&nruns, 1));
-    KCU(B.get(&rstart, P + 1)); KCU(B.get(&keep, P + 1));
-    size_t eb = 0;
-    KCU(cub::DeviceRunLengthEncode::Encode(nullptr, eb, kb.Current(), ukeys, rlen, nruns, (int64_t)P, st));
-    void *etmp;
-    KCU(B.get((char **)&etmp, eb));
-    KCU(cub::DeviceRunLengthEncode::Encode(etmp, eb, kb.Current(), ukeys, rlen, nruns, (int64_t)P, st));
-    uint64_t U = 0;
-    KCU(cudaMemcpyAsync(&U, nruns, sizeof U, cudaMemcpyDeviceToHost, st));
-    KCU(cudaStreamSynchronize(st));
-    KCU(cudaMemsetAsync(rlen + U, 0, sizeof(uint32_t), st));
-    size_t xb = 0;
-    KCU(cub::DeviceScan::ExclusiveSum(nullptr, xb, rlen, rstart, (int64_t)(U + 1), st));
-    void *xtmp;
-    KCU(B.get((char **)&xtmp, xb));
-    KCU(cub::DeviceScan::ExclusiveSum(xtmp, xb, rlen, rstart, (int64_t)(U + 1), st));
-    pg_pair *all;
-    KCU(B.get(&all, U));
-    k_reduce_pairs<<<grid, 256, 0, st>>>(ukeys, rlen, rstart, nruns, sb.Current(), tab, kc->ckthr,
-                                         kc->mosthr, all, keep);
-    KCU(cudaGetLastError());
-    uint64_t *kpos;
-    KCU(B.get(&kpos, U + 1));
-    KCU(cudaMemsetAsync(keep + U, 0, sizeof(uint32_t), st));
-    size_t qb = 0;
-    KCU(cub::DeviceScan::ExclusiveSum(nullptr, qb, keep, kpos, (int64_t)(U + 1), st));
-    void *qtmp;
-    KCU(B.get((char **)&qtmp, qb));
-    KCU(cub::DeviceScan::ExclusiveSum(qtmp, qb, keep, kpos, (int64_t)(U + 1), st));
-    uint64_t K = 0;
-    KCU(cudaMemcpyAsync(&K, kpos + U, sizeof K, cudaMemcpyDeviceToHost, st));
-    KCU(cudaStreamSynchronize(st));
-    *n_out = K;
-    if (K > cap) return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: output capacity too small");
-    k_compact_pairs<<<grid, 256, 0, st>>>(all, keep, kpos, nruns, d_out);
-    KCU(cudaGetLastError());
-    KCU(cudaStreamSynchronize(st));
-    return PG_OK;
+    if (R.n < 0xffffffffull)
+        return candidates_of<uint32_t>(B, R, *kc, tab, nsm, cseq, coffs, C, row_begin, row_end - row_begin, same,
+                                       col_begin, col_end - col_begin, maxp, d_out, cap, n_out);
+    return candidates_of<uint64_t>(B, R, *kc, tab, nsm, cseq, coffs, C, row_begin, row_end - row_begin, same,
+                                   col_begin, col_end - col_begin, maxp, d_out, cap, n_out);
 }
 
 int pg_triples(const pg_pair *d_pairs, const pg_result *d_res, uint64_t n, uint64_t bl_roffset,

@@ -120,3 +120,32 @@ def test_triples_are_the_nonzero_score_aln_entries(fam):
     assert np.array_equal(c[:k].cpu().numpy(), pairs["col"][sel].astype(np.int64) + cols[0])
     assert np.array_equal(v[:k].cpu().numpy(), res["score_aln"][sel])
     ctx.close()
+
+
+@pytest.mark.parametrize("k,ckthr,mosthr,cols", [(2, 0, -1, (0, 5)), (2, 3, -1, (2, 7)), (3, 0, 9, (0, 6)), (3, 1, -1, (1, 3))])
+def test_crowded_columns_match_oracle(native, k, ckthr, mosthr, cols):
+    """Columns that meet more rows than a block's hash table takes (1536), more
+    surviving rows than its list (384), runs longer than a warp, and one just
+    inside all of them (k = 3, ckthr = 1): short k-mers over 2200 sequences."""
+    from oracle import kmer_oracle as K
+    from oracle import oracle as O
+    from pastis_gb300 import capi
+    rng = np.random.default_rng(17)
+    lens = rng.integers(1, 60, 2200)
+    lens[:8] = [400, 3, 90, 1, 250, 700, 40, 2]
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    seq = rng.integers(0, 20, int(offs[-1])).astype(np.uint8)
+    seq[int(offs[5]):int(offs[5]) + 60] = 3          # a run of one residue
+    seq[int(offs[900]):int(offs[903])] = 3
+    ascii_ = np.frombuffer(b"ARNDCQEGHILKMFPSTWYV", dtype=np.uint8)[seq]
+    ctx = capi.Context(capi.config(capi.MODE_XDROP))
+    ctx.set_seqs(0, ascii_, offs)
+    ctx.share_row_seqs()
+    rows = (0, len(lens))
+    kc = capi.kmer_config(k=k, ckthr=ckthr, mosthr=mosthr)
+    got = ctx.candidates(kc, rows, cols)
+    exp = K.candidates(seq, offs, rows, cols, O.blosum62(), k=k, stride=1, alph=0, prune=0, ckthr=ckthr)
+    exp = [e for e in exp if e["score"] > mosthr]
+    assert len(exp) > 0
+    assert as_rows(got) == [tuple(e[f] for f in FIELDS) for e in exp]
+    ctx.close()
