@@ -147,7 +147,8 @@ struct pg_ctx {
     uint32_t *d_ovf = nullptr;          // overflowed extension tasks
     uint64_t xd_cap = 0;
     uint32_t *d_order = nullptr;        // bucket order of the pairs
-    uint32_t *d_xorder = nullptr;       // X-drop extension tasks, longest length bound first
+    uint32_t *d_xorder = nullptr;       // X-drop extension directions, longest length bound first
+    pg::XdSide *d_xdir = nullptr;        // their results (k_xdr)
     uint64_t order_cap = 0;
     // traceback form: direction arena, per-task byte counts / offsets,
     // per-pair scores and end cells, scan scratch
@@ -254,7 +255,7 @@ void pg_destroy(pg_ctx *ctx)
     cudaFree(ctx->d_xd);
     cudaFree(ctx->d_ovf);
     cudaFree(ctx->d_order);
-    cudaFree(ctx->d_xorder);
+    cudaFree(ctx->d_xorder); cudaFree(ctx->d_xdir);
     cudaFree(ctx->d_dir); cudaFree(ctx->d_dbytes); cudaFree(ctx->d_doff); cudaFree(ctx->d_t1);
     cudaFree(ctx->d_dsc); cudaFree(ctx->d_scan);
     cudaFree(ctx->d_lin); cudaFree(ctx->d_list); cudaFree(ctx->d_walk);
@@ -428,12 +429,13 @@ static int ensure_batch(pg_ctx *c, uint64_t n)
         c->order_cap = n;
     }
     if (c->cfg.mode != PG_MODE_XDROP || n <= c->xd_cap) return PG_OK;
-    cudaFree(c->d_xd); cudaFree(c->d_ovf); cudaFree(c->d_xorder);
-    c->d_xd = nullptr; c->d_ovf = nullptr; c->d_xorder = nullptr; c->xd_cap = 0;
+    cudaFree(c->d_xd); cudaFree(c->d_ovf); cudaFree(c->d_xorder); cudaFree(c->d_xdir);
+    c->d_xd = nullptr; c->d_ovf = nullptr; c->d_xorder = nullptr; c->d_xdir = nullptr; c->xd_cap = 0;
     ++c->epoch;
     CU(cudaMalloc(&c->d_xd, 2 * n * sizeof(pg::XdRec)));
-    CU(cudaMalloc(&c->d_ovf, 2 * n * sizeof(uint32_t)));
-    CU(cudaMalloc(&c->d_xorder, 2 * n * sizeof(uint32_t)));
+    CU(cudaMalloc(&c->d_ovf, 4 * n * sizeof(uint32_t)));
+    CU(cudaMalloc(&c->d_xorder, 4 * n * sizeof(uint32_t)));
+    CU(cudaMalloc(&c->d_xdir, 4 * n * sizeof(pg::XdSide)));
     c->xd_cap = n;
     return PG_OK;
 }
@@ -715,12 +717,15 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
         // (each task run to its end, more resident warps) when residues
         // stream from DRAM
         const uint64_t nres = c->side[0].nres + (c->cols_share_rows ? 0 : c->side[1].nres);
-        const bool reg_ok = pg::xdr_supported(kp.xg, c->cfg.xdrop);
+        // (k_xdr numbers directions, four to a pair, in 32 bits)
+        const bool reg_ok = pg::xdr_supported(kp.xg, c->cfg.xdrop) && n < (1ull << 30);
         int form = c->tune.xd_stepped;
         if (form < 0) form = reg_ok ? 2 : (nres <= c->l2_bytes / 2 ? 1 : 0);
         if (form == 2 && !reg_ok) form = 1;
         const bool int16 = c->tune.xd_int16 && c->cfg.xdrop <= pg::XMAX16;
-        const uint64_t need_xd = (2 * n + pg::XT - 1) / pg::XT;
+        // a thread per task; k_xdr in length order may give every direction a warp
+        const bool reg = form == 2 && !int16;
+        const uint64_t need_xd = ((reg ? 4 : 2) * n * (reg && c->tune.bucket_order ? 32 : 1) + pg::XT - 1) / pg::XT;
         uint64_t xmax = (uint64_t)(int16 ? c->grid_xd_run
                                          : form == 2 ? c->grid_xdr : form == 1 ? c->grid_xd : c->grid_xd_run);
         if (c->tune.xd_blocks_per_sm > 0)
@@ -741,6 +746,7 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
             kp.xorder = c->d_xorder;
             xlaunch = 2;
         }
+        if (!affine && !int16 && form == 2) kp.xdir = c->d_xdir;
         if (affine) {
             pg::k_xda<<<c->grid_wide, blk, 0, st>>>(kp);
         } else {

@@ -62,6 +62,13 @@ struct XdRec {
     uint32_t flags;
 };
 
+// extension of one direction of a (pair, seed) by k_xdr
+struct XdSide {
+    uint16_t dv, dh;
+    uint32_t cells;      // XDIR_OVF: the band outgrew the register window
+};
+constexpr uint32_t XDIR_OVF = 0x80000000u;
+
 struct KParams {
     const pg_pair *pairs;
     uint64_t n;
@@ -88,7 +95,8 @@ struct KParams {
     int dir16_lim = 0;               // traceback form: regions with m + n <= this on 16-bit lanes
     int dir16_side = 0;              // ... and larger ones with both sides <= this, checked
     int dir16_pair = 0;              // 1: 16-bit regions of up to 32 x rows_cap rows two per warp
-    const uint32_t *xorder = nullptr; // X-drop extension tasks, longest length bound first (null: t)
+    const uint32_t *xorder = nullptr; // X-drop extension directions, longest length bound first (null: t)
+    XdSide *xdir = nullptr;     // k_xdr's results: 4 per pair (seed, left / right)
     unsigned int *xsched = nullptr;   // [0, XBUCKET) task bucket sizes, [XBUCKET, 2*XBUCKET) cursors
     int four = 4;                     // a 4 the compiler cannot see (pg_lin.cuh)
 };
@@ -180,6 +188,17 @@ __device__ __forceinline__ bool seed_region(const KParams &kp, const pg_pair &pr
     return false;
 }
 
+// which (pair, seed) extensions run: XF_NONE / XF_SAME where none does, else its
+// seed region and XF_BAD or 0
+__device__ __forceinline__ uint32_t xd_seed(const KParams &kp, const pg_pair &pr, int s, int m, int n,
+                                            int &bv, int &ev, int &bh, int &eh)
+{
+    bv = ev = bh = eh = 0;
+    if (s >= kp.seed_count || (s == 1 && (kp.flags & PG_F_SKIP_SPURIOUS_SEED) && pr.count < 2)) return XF_NONE;
+    if (s == 1 && pr.rs1 == pr.rs0 && pr.cs1 == pr.cs0) return XF_SAME;
+    return seed_region(kp, pr, s, m, n, bv, ev, bh, eh) ? XF_BAD : 0u;
+}
+
 // ------------------------------------------------------------------ k_ga
 // Rows per lane by region height.  A stripe of 32*R rows costs (n + last
 // busy lane) column steps of R cells whatever number of its lanes hold rows,
@@ -228,7 +247,7 @@ __device__ __forceinline__ DpOut<S> dp_dispatch(const uint8_t *V, int m, const u
 constexpr int NBUCKET = 24;
 constexpr int SCHED_WORDS = 2 * NBUCKET;
 constexpr int XBUCKET = 72;          // extension task buckets: quarter octaves of the length bound
-constexpr int XSCHED_WORDS = 2 * XBUCKET;
+constexpr int XSCHED_WORDS = 2 * XBUCKET + 2;   // and two work counters: long directions, wide tasks
 constexpr int BUCKET_NONE = 23;   // no DP work
 
 // traceback form, lanes of a region's DP (pg_dpdir16.cuh): 0 32-bit; 1 16-bit,

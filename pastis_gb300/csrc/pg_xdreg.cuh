@@ -213,7 +213,7 @@ struct XrDirT {
         }
         uint32_t live = (lm | (lm >> 15)) & MASK;
         // the reference keeps a border cell only when d * g > best - X
-        if ((long long)d * g == (long long)(best + B) - X) {
+        if (d * g == best + B - X) {           // |d g| < 2^30, best + B < 2^24
             if (off3 == 0) { N[0] = prmt(N[0], XR_UND2, 0x3254u); live &= ~1u; }
             if (d - off3 < NS) {
                 const int sd = xr_mod<NS>(d);
@@ -325,5 +325,89 @@ struct XrDirT {
 };
 
 using XrDir = XrDirT<8>;
+
+// ------------------------------------------------------ a warp per direction
+// The same direction on a warp: anti-diagonal column c in lane c mod 32, a window of
+// up to 31 columns, 32-bit values, any gap and X.  A thread of k_xdr spends about
+// 370 instructions on a step, this about a fifth of that, but a warp's: several
+// times the issue slots for a band of a few columns.  Its step takes some 200 cycles
+// in place of 900 (2000 with the SM's other warps), so it serves where the longest
+// directions decide: a call of 256 pairs 650 -> 355 us, 60k pairs of very uneven
+// lengths 7.0 -> 6.5 ms.  (With two and four columns a lane for wider bands it was
+// no faster than the ring of xdrop_dir_warp: 20k pairs with a gap of -2 4.2 ms there,
+// 4.5 and 6.6 here.)
+// Cells outside the band are set dead at every step.  The score of a step is looked
+// up one step ahead and its residue read two ahead, for the column the lane then
+// holds: a lane whose column has just changed is outside the band for the next
+// step (the window is at least two columns longer, and the band grows by one a step).
+// tab: score table, rows of XR_STRIDE ints.
+__device__ __noinline__ XdOut xdrop_dir_regs(const uint8_t *__restrict__ V, int nv, int vstep,
+                                             const uint8_t *__restrict__ Hs, int nh, int hstep,
+                                             const int *__restrict__ tab, int g, int X)
+{
+    const int lane = threadIdx.x & 31;
+    XdOut o{0, 0, 0u, 1};
+    const int cols = nv + 1, rows = nh + 1;
+    if (cols == 1 || rows == 1) return o;
+    auto vres = [&](int c) { return c >= 1 && c <= nv ? (int)__ldg(V + vstep * (c - 1)) : 24; };
+    auto hres = [&](int i) { return i >= 0 && i < nh ? (int)__ldg(Hs + hstep * i) : 24; };
+    const int v1 = (-g > X) ? UND : g;
+    // the window at d = 2 starts at column 0
+    int P = lane <= 1 ? v1 : UND;                    // d = 1
+    int Q = lane == 0 ? 0 : UND, Q2 = UND;           // d = 0, and the one before
+    int D = lane == 1 ? 0 : UND;                     // (d - 2, c - 1) for d = 2
+    int col = lane, vr = vres(lane);
+    int s = tab[vr * XR_STRIDE + hres(1 - lane)], hr = hres(2 - lane);
+    int off1 = 0, len1 = 0, off2 = 0, len2 = 1, off3 = 0, len3 = 2;
+    int best = 0, d = 1, lo = 1, hi = 2;
+    while (lo < hi) {
+        ++d;
+        off1 = off2; len1 = len2;
+        off2 = off3; len2 = len3;
+        off3 = lo - 1; len3 = hi + 1 - off3;
+        if (len3 > 31) { o.ok = 0; return o; }
+        const int thr = best - X, db = d * g, span = hi - off3;
+        const int bval = db > thr ? db : UND;
+        const int left = __shfl_sync(FULL, P, (lane - 1) & 31);
+        const int p = (lane - off3) & 31, c = off3 + p;
+        const int v = max(max(left, P) + g, D + s);
+        int lb = db, tl = hi + 1, tu = off3;
+        int n = p >= 1 && p < span && v >= thr ? v : UND;
+        if (n != UND) lb = max(lb, n);
+        if ((p == 0 && off3 == 0) || (p == span && d == hi && hi < cols)) n = bval;   // the border cells
+        if (p >= 1 && p <= span && (n != UND || left != UND)) tl = min(tl, c);
+        if (p < span && (n != UND || P != UND)) tu = max(tu, c + 1);
+        D = left;
+        Q2 = Q;
+        Q = P;
+        P = n;
+        s = tab[vr * XR_STRIDE + hr];                // of d + 1
+        if (c != col) { col = c; vr = vres(c); }
+        hr = hres(d + 1 - c);                        // of d + 2
+        // best and band trims by reductions (by ballots, shifts and bit searches, one
+        // after the other, the step took a third longer)
+        best = max(best, __reduce_max_sync(FULL, lb));
+        o.cells += (uint32_t)(hi - lo);
+        lo = max(__reduce_min_sync(FULL, tl), d + 2 - rows);
+        hi = min(__reduce_max_sync(FULL, tu) + 1, cols);
+    }
+    // the end point (the rule of xdrop_dir_thread)
+    int lc = off3 + len3 - 2, lr = d - lc, ls = __shfl_sync(FULL, P, lc & 31);
+    if (ls == UND) {
+        const int ca = off2 + len2 - 2;
+        const int a0 = __shfl_sync(FULL, Q, ca & 31), a1 = __shfl_sync(FULL, Q, (ca - 1) & 31);
+        if (a0 != UND) { lc = ca; lr = d - 1 - lc; ls = a0; }
+        else if (len2 > 2 && a1 != UND) { lc = ca - 1; lr = d - 1 - lc; ls = a1; }
+    }
+    if (ls == UND) {
+        // the first maximum two anti-diagonals back
+        const int mx = __reduce_max_sync(FULL, Q2);
+        const int at = (lane - off1) & 31;
+        const int first = __reduce_min_sync(FULL, mx != UND && Q2 == mx ? at : 32);
+        if (first < len1) { ls = mx; lc = off1 + first; lr = d - 2 - lc; }
+    }
+    if (ls != UND) { o.dv = lc; o.dh = lr; }
+    return o;
+}
 
 }  // namespace pg
