@@ -80,61 +80,115 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 }
 
 __device__ __forceinline__ uint32_t ld_u32(const __nv_bfloat16 *p) { return *reinterpret_cast<const uint32_t *>(p); }
+__device__ __forceinline__ void st_bf16x2(__nv_bfloat16 *p, float lo, float hi)
+{
+    *reinterpret_cast<uint32_t *>(p) = pack_bf16(lo, hi);
+}
 
-// weights as the MLP kernels read them from shared memory
+// four 8x8 BF16 matrices; lanes 8i..8i+7 give the row addresses of matrix i
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16 *p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16 *p)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+
+// Weights as the MLP kernels read them from shared memory.  The rows are
+// padded to an odd number of 16-byte units, so that the eight rows of an
+// ldmatrix tile (and the rows of a tile's accumulator stores) meet eight
+// different bank groups.  The backward pass reads w2t transposed, so one copy
+// serves both directions.
+constexpr int LD1 = NF + 8, LD2 = NH + 8;
 struct SmemW {
-    __nv_bfloat16 w1t[NH * NF];   // [out][in]      layer-1 B operand
-    __nv_bfloat16 w2t[NH * NH];   // [out][in]      layer-2 B operand
-    __nv_bfloat16 w2[NH * NH];    // [in][out]      backward B operand
+    alignas(16) __nv_bfloat16 w1t[NH * LD1];   // [out][in]
+    alignas(16) __nv_bfloat16 w2t[NH * LD2];   // [out][in]
     float b1[NH], b2[NH], w3[NH], b3;
 };
 
-__device__ void load_weights(SmemW &s, const float *P)
+// Every load is issued before the first conversion: a block does one or two
+// tiles a warp, so the way of the weights through L2 is a good part of it.
+__device__ __forceinline__ void load_weights(SmemW &s, const float *P)
 {
-    for (int k = threadIdx.x; k < NH * NF; k += blockDim.x) s.w1t[k] = __float2bfloat16_rn(P[P_W1 + k]);
-    for (int k = threadIdx.x; k < NH * NH; k += blockDim.x) {
-        const int o = k / NH, i = k % NH;
-        const __nv_bfloat16 v = __float2bfloat16_rn(P[P_W2 + k]);
-        s.w2t[k] = v;
-        s.w2[i * NH + o] = v;
-    }
-    for (int k = threadIdx.x; k < NH; k += blockDim.x) {
+    static_assert(FWARPS * 32 == 128 && NH * NF == 2 * 512 && P_W2 % 4 == 0, "weight load split");
+    const int k = threadIdx.x;
+    float4 v1[2], v2[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v2[u] = reinterpret_cast<const float4 *>(P + P_W2)[k + u * 128];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) v1[u] = reinterpret_cast<const float4 *>(P + P_W1)[k + u * 128];
+    if (k < NH) {
         s.b1[k] = P[P_B1 + k];
         s.b2[k] = P[P_B2 + k];
         s.w3[k] = P[P_W3 + k];
     }
-    if (threadIdx.x == 0) s.b3 = P[P_B3];
+    if (k == 0) s.b3 = P[P_B3];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int e = (k + u * 128) * 4;
+        uint2 q = make_uint2(pack_bf16(v2[u].x, v2[u].y), pack_bf16(v2[u].z, v2[u].w));
+        *reinterpret_cast<uint2 *>(s.w2t + (e / NH) * LD2 + e % NH) = q;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int e = (k + u * 128) * 4;
+        uint2 q = make_uint2(pack_bf16(v1[u].x, v1[u].y), pack_bf16(v1[u].z, v1[u].w));
+        *reinterpret_cast<uint2 *>(s.w1t + (e / NF) * LD1 + e % NF) = q;
+    }
 }
 
-// Forward pass of 16 samples starting at row `base` of X (bf16 [n][16]).
-// Thread (g = lane/4, t = lane%4) ends up with the rows g and g+8 of h1 / h2 in
-// the mma accumulator layout, and the logits of those two rows.
+// Forward pass of 16 samples.  Thread (g = lane/4, t = lane%4) ends up with
+// the rows g and g+8 of h1 / h2 in the mma accumulator layout, and the logits
+// of those two rows.
 struct Tile {
     float h1[8][4];   // relu(x W1 + b1), fp32
     float h2[8][4];   // relu(h1_bf16 W2 + b2)
     float z0, z1;     // logits of rows g, g+8
 };
 
-__device__ __forceinline__ void forward_tile(const SmemW &s, const __nv_bfloat16 *X, uint64_t n,
-                                             uint64_t base, Tile &T)
+// the A fragment of 16 rows of X (bf16 [n][16]) from row `base`; rows past n are 0
+__device__ __forceinline__ void load_x(uint32_t (&a)[4], const __nv_bfloat16 *X, uint64_t n, uint64_t base)
 {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const uint64_t r0 = base + g, r1 = base + g + 8;
-    uint32_t a[4];
     a[0] = r0 < n ? ld_u32(X + r0 * NF + 2 * t) : 0u;
     a[1] = r1 < n ? ld_u32(X + r1 * NF + 2 * t) : 0u;
     a[2] = r0 < n ? ld_u32(X + r0 * NF + 2 * t + 8) : 0u;
     a[3] = r1 < n ? ld_u32(X + r1 * NF + 2 * t + 8) : 0u;
+}
+
+__device__ __forceinline__ void load_labels(float (&v)[4], const float *label, const float *wts, uint64_t n,
+                                            uint64_t base)
+{
+    const uint64_t r0 = base + ((threadIdx.x & 31) >> 2), r1 = r0 + 8;
+    v[0] = r0 < n ? label[r0] : 0.f;
+    v[1] = r1 < n ? label[r1] : 0.f;
+    v[2] = r0 < n ? wts[r0] : 0.f;
+    v[3] = r1 < n ? wts[r1] : 0.f;
+}
+
+__device__ __forceinline__ void forward_tile(const SmemW &s, const uint32_t (&a)[4], Tile &T)
+{
+    const int lane = threadIdx.x & 31, t = lane & 3;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        const __nv_bfloat16 *w = s.w1t + (nt * 8 + g) * NF + 2 * t;
-        mma16816(d, a, ld_u32(w), ld_u32(w + 8));
-        const int c = nt * 8 + 2 * t;
-        T.h1[nt][0] = fmaxf(d[0] + s.b1[c], 0.f);
-        T.h1[nt][1] = fmaxf(d[1] + s.b1[c + 1], 0.f);
-        T.h1[nt][2] = fmaxf(d[2] + s.b1[c], 0.f);
-        T.h1[nt][3] = fmaxf(d[3] + s.b1[c + 1], 0.f);
+    for (int np = 0; np < 4; ++np) {   // a pair of 8-unit tiles an ldmatrix
+        uint32_t b[4];
+        ldsm4(b, s.w1t + (np * 16 + (lane & 7) + (lane >> 4) * 8) * LD1 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int nt = 2 * np + q, c = nt * 8 + 2 * t;
+            float d[4] = {0.f, 0.f, 0.f, 0.f};
+            mma16816(d, a, b[2 * q], b[2 * q + 1]);
+            T.h1[nt][0] = fmaxf(d[0] + s.b1[c], 0.f);
+            T.h1[nt][1] = fmaxf(d[1] + s.b1[c + 1], 0.f);
+            T.h1[nt][2] = fmaxf(d[2] + s.b1[c], 0.f);
+            T.h1[nt][3] = fmaxf(d[3] + s.b1[c + 1], 0.f);
+        }
     }
     uint32_t a2[4][4];
 #pragma unroll
@@ -149,9 +203,11 @@ __device__ __forceinline__ void forward_tile(const SmemW &s, const __nv_bfloat16
     for (int nt = 0; nt < 8; ++nt) {
         float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int kc = 0; kc < 4; ++kc) {
-            const __nv_bfloat16 *w = s.w2t + (nt * 8 + g) * NH + kc * 16 + 2 * t;
-            mma16816(d, a2[kc], ld_u32(w), ld_u32(w + 8));
+        for (int kp = 0; kp < 2; ++kp) {
+            uint32_t b[4];
+            ldsm4(b, s.w2t + (nt * 8 + (lane & 7)) * LD2 + kp * 32 + (lane >> 3) * 8);
+            mma16816(d, a2[2 * kp], b[0], b[1]);
+            mma16816(d, a2[2 * kp + 1], b[2], b[3]);
         }
         const int c = nt * 8 + 2 * t;
         T.h2[nt][0] = fmaxf(d[0] + s.b2[c], 0.f);
@@ -170,56 +226,142 @@ __device__ __forceinline__ void forward_tile(const SmemW &s, const __nv_bfloat16
 }
 
 // ----------------------------------------------------------------- kernels
+// Residue-group fractions of every sequence, a warp a sequence: 16 bytes a
+// lane and load, counts in packed bytes of a 32-bit word (at most 16 of a group
+// a load, so they are unpacked after each).  Bound by instruction issue, two a
+// residue: 15 us for 30 thousand proteins of 280 residues (125 us with a thread
+// a sequence, whose byte loads shared no sector with its neighbours').
 __global__ void k_composition(const uint8_t *seq, const uint64_t *offs, uint64_t nseq, float4 *comp)
 {
-    // residue group of each code in ARNDCQEGHILKMFPSTWYVBZX*J; 4 = none
-    const uint8_t grp[25] = {0, 2, 1, 3, 0, 1, 3, 1, 2, 0, 0, 2, 0, 0, 1, 1, 1, 0, 1, 0, 4, 4, 4, 4, 4};
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nseq;
-         i += (uint64_t)gridDim.x * blockDim.x) {
+    // residue group of each code in ARNDCQEGHILKMFPSTWYVBZX*J as its counter's
+    // byte (hydrophobic, polar, positive, negative); codes past J have none
+    __shared__ uint32_t inc[32];
+    if (threadIdx.x < 32) {
+        const uint8_t grp[25] = {0, 2, 1, 3, 0, 1, 3, 1, 2, 0, 0, 2, 0, 0, 1, 1, 1, 0, 1, 0, 4, 4, 4, 4, 4};
+        const int g = threadIdx.x < 25 ? grp[threadIdx.x] : 4;
+        inc[threadIdx.x] = g < 4 ? 1u << (8 * g) : 0u;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < nseq; i += nw) {
         const uint64_t b = offs[i], e = offs[i + 1];
-        float c[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        for (uint64_t q = b; q < e; ++q) {
-            const uint8_t r = seq[q];
-            c[r < 25 ? grp[r] : 4] += 1.f;
+        uint32_t c[4] = {0, 0, 0, 0};
+        // whole aligned 16-byte units inside [b, e); the ends by bytes
+        const uint64_t base = (uint64_t)(uintptr_t)seq;
+        const uint64_t ab = (base + b + 15) & ~15ull, ae = (base + e) & ~15ull;
+        const uint64_t hb = ab > base + e ? e : ab - base;        // end of the head
+        const uint64_t tb = ae < ab ? e : ae - base;              // start of the tail
+        uint32_t acc = 0;
+        if (b + lane < hb) { const uint8_t r = seq[b + lane]; acc += r < 32 ? inc[r] : 0u; }
+        if (tb + lane < e) { const uint8_t r = seq[tb + lane]; acc += r < 32 ? inc[r] : 0u; }
+        c[0] = acc & 0xff; c[1] = acc >> 8 & 0xff; c[2] = acc >> 16 & 0xff; c[3] = acc >> 24;
+        for (uint64_t q = ab + 16 * lane; q < ae; q += 512) {
+            const uint4 v = *reinterpret_cast<const uint4 *>((uintptr_t)q);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            acc = 0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+                const uint32_t r = w[k >> 2] >> (8 * (k & 3)) & 0xff;
+                acc += r < 32 ? inc[r] : 0u;
+            }
+            c[0] += acc & 0xff; c[1] += acc >> 8 & 0xff; c[2] += acc >> 16 & 0xff; c[3] += acc >> 24;
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] = __reduce_add_sync(0xffffffffu, c[k]);
         const float inv = e > b ? 1.f / (float)(e - b) : 0.f;
-        comp[i] = make_float4(c[0] * inv, c[1] * inv, c[2] * inv, c[3] * inv);
+        if (lane == 0)
+            comp[i] = make_float4((float)c[0] * inv, (float)c[1] * inv, (float)c[2] * inv, (float)c[3] * inv);
     }
 }
 
 constexpr int WIN_BEFORE = 32, WIN_LEN = 64;
 
-__device__ float diag_window(const uint8_t *V, int m, const uint8_t *H, int n, int r0, int c0,
-                             const int8_t *sm)
-{
-    int s = 0, cnt = 0;
-    for (int t = -WIN_BEFORE; t < WIN_LEN - WIN_BEFORE; ++t) {
-        const int i = r0 + t, j = c0 + t;
-        if (i < 0 || j < 0 || i >= m || j >= n) continue;
-        s += sm[V[i] * PG_NRES + H[j]];
-        ++cnt;
-    }
-    return cnt ? (float)s / (4.f * (float)cnt) : 0.f;
-}
-
-__global__ void k_features(const pg_pair *pairs, uint64_t n, uint64_t roff, uint64_t coff,
+// Features of 32 pairs a warp.  The two seeds' diagonal windows are summed by
+// the whole warp for one pair after the other (lanes 0-15 the first seed, 16-31
+// the second; position t of the window on lane t % 16), so that a window is
+// four coalesced loads of each sequence; then every lane forms its own pair's
+// row.  Bound by instruction issue, 180 a pair: 37 us for 150 thousand pairs (55
+// us with a thread a pair walking its windows by bytes).
+__global__ void __launch_bounds__(256) k_features(const pg_pair *pairs, uint64_t n, uint64_t roff, uint64_t coff,
                            const uint8_t *rseq, const uint64_t *roffs, uint64_t nr,
                            const uint8_t *cseq, const uint64_t *coffs, uint64_t nc,
                            const int8_t *sm, const float4 *rcomp, const float4 *ccomp,
                            __nv_bfloat16 *X, int *status)
 {
-    for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < n;
-         p += (uint64_t)gridDim.x * blockDim.x) {
-        const pg_pair pr = pairs[p];
-        const uint64_t r = pr.row + roff, c = pr.col + coff;
+    __shared__ int8_t ssm[PG_NRES * PG_NRES];
+    for (int k = threadIdx.x; k < PG_NRES * PG_NRES; k += blockDim.x) ssm[k] = sm[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = (uint64_t)gridDim.x * (blockDim.x >> 5), groups = (n + 31) / 32;
+    for (uint64_t grp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; grp < groups; grp += nw) {
+        const uint64_t p = grp * 32 + lane;
+        pg_pair pr = {};
+        uint64_t r = 0, c = 0, rb = 0, cb = 0;
+        int mi = 0, ni = 0;
+        float4 ca = make_float4(0.f, 0.f, 0.f, 0.f), cc = ca;
+        bool ok = false;
+        if (p < n) {
+            pr = pairs[p];
+            r = pr.row + roff;
+            c = pr.col + coff;
+            ok = r < nr && c < nc;
+            if (ok) {
+                rb = roffs[r];
+                cb = coffs[c];
+                mi = (int)(roffs[r + 1] - rb);
+                ni = (int)(coffs[c + 1] - cb);
+                ca = rcomp[r];
+                cc = ccomp[c];
+            } else atomicOr(status, 1);
+        }
+        const bool two = pr.count >= 2;
+        const bool win2 = two && (pr.rs1 != pr.rs0 || pr.cs1 != pr.cs0);
+        float win = 0.f;
+        const unsigned live = __ballot_sync(0xffffffffu, ok);
+        const int h = lane >> 4, l16 = lane & 15;
+        for (unsigned rest = live; rest; rest &= rest - 1) {
+            const int src = __ffs(rest) - 1;
+            const uint8_t *V = rseq + __shfl_sync(0xffffffffu, rb, src);
+            const uint8_t *H = cseq + __shfl_sync(0xffffffffu, cb, src);
+            const int m = __shfl_sync(0xffffffffu, mi, src), nn = __shfl_sync(0xffffffffu, ni, src);
+            const int a0 = __shfl_sync(0xffffffffu, (int)pr.rs0, src), a1 = __shfl_sync(0xffffffffu, (int)pr.rs1, src);
+            const int b0 = __shfl_sync(0xffffffffu, (int)pr.cs0, src), b1 = __shfl_sync(0xffffffffu, (int)pr.cs1, src);
+            const bool both = __shfl_sync(0xffffffffu, (int)win2, src);
+            int sum = 0, cnt = 0;
+            if (h == 0 || both) {
+                const int i0 = (h ? a1 : a0) - WIN_BEFORE + l16, j0 = (h ? b1 : b0) - WIN_BEFORE + l16;
+                uint8_t v[WIN_LEN / 16], w[WIN_LEN / 16];
+                bool in[WIN_LEN / 16];
+#pragma unroll
+                for (int q = 0; q < WIN_LEN / 16; ++q) {
+                    const int i = i0 + 16 * q, j = j0 + 16 * q;
+                    in[q] = i >= 0 && j >= 0 && i < m && j < nn;
+                    v[q] = in[q] ? V[i] : 0;
+                    w[q] = in[q] ? H[j] : 0;
+                }
+#pragma unroll
+                for (int q = 0; q < WIN_LEN / 16; ++q) {
+                    sum += in[q] ? (int)ssm[v[q] * PG_NRES + w[q]] : 0;
+                    cnt += in[q];
+                }
+            }
+            // |sum| <= 64 * 128 and cnt <= 64 of a half: both in one word
+            int pk = (sum << 8) + cnt;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) pk += __shfl_xor_sync(0xffffffffu, pk, o);
+            const int c1 = pk & 0xff, s1 = (pk - c1) >> 8;
+            const float mine = c1 ? (float)s1 / (4.f * (float)c1) : 0.f;
+            const float x0 = __shfl_sync(0xffffffffu, mine, 0), x1 = __shfl_sync(0xffffffffu, mine, 16);
+            if (lane == src) win = both ? fmaxf(x0, x1) : x0;
+        }
+        if (p >= n) continue;
         float f[NF];
-        if (r >= nr || c >= nc) {
-            atomicOr(status, 1);
-            for (int k = 0; k < NF; ++k) f[k] = 0.f;
-        } else {
-            const float m = (float)(roffs[r + 1] - roffs[r]), nn = (float)(coffs[c + 1] - coffs[c]);
+#pragma unroll
+        for (int k = 0; k < NF; ++k) f[k] = 0.f;
+        if (ok) {
+            const float m = (float)(uint64_t)(unsigned)mi, nn = (float)(uint64_t)(unsigned)ni;
             const float mm = fmaxf(m, 1.f), n1 = fmaxf(nn, 1.f), L = fmaxf(mm, n1);
-            const bool two = pr.count >= 2;
             const float d0 = ((float)pr.cs0 - (float)pr.rs0) / L;
             const float d1 = ((float)pr.cs1 - (float)pr.rs1) / L;
             f[0] = log2f(1.f + (float)pr.count) * 0.25f;
@@ -230,31 +372,28 @@ __global__ void k_features(const pg_pair *pairs, uint64_t n, uint64_t roff, uint
             f[5] = two ? fabsf(d0 - d1) : 0.f;
             f[6] = (float)pr.rs0 / mm;
             f[7] = (float)pr.cs0 / n1;
-            {
-                const uint8_t *V = rseq + roffs[r], *H = cseq + coffs[c];
-                const int mi = (int)(roffs[r + 1] - roffs[r]), ni = (int)(coffs[c + 1] - coffs[c]);
-                float w = diag_window(V, mi, H, ni, pr.rs0, pr.cs0, sm);
-                if (two && (pr.rs1 != pr.rs0 || pr.cs1 != pr.cs0))
-                    w = fmaxf(w, diag_window(V, mi, H, ni, pr.rs1, pr.cs1, sm));
-                f[8] = w;
-            }
+            f[8] = win;
             f[9] = log2f(mm) * (1.f / 12.f);
             f[10] = log2f(n1) * (1.f / 12.f);
             f[11] = fabsf(log2f(mm / n1));
-            const float4 a = rcomp[r], b = ccomp[c];
-            f[12] = fabsf(a.x - b.x);
-            f[13] = fabsf(a.y - b.y);
-            f[14] = fabsf(a.z - b.z);
-            f[15] = fabsf(a.w - b.w);
+            f[12] = fabsf(ca.x - cc.x);
+            f[13] = fabsf(ca.y - cc.y);
+            f[14] = fabsf(ca.z - cc.z);
+            f[15] = fabsf(ca.w - cc.w);
         }
-        __nv_bfloat16 *o = X + p * NF;
+        uint32_t o[8];
 #pragma unroll
-        for (int k = 0; k < NF; k += 2) {
-            *reinterpret_cast<__nv_bfloat162 *>(o + k) = __floats2bfloat162_rn(f[k], f[k + 1]);
-        }
+        for (int k = 0; k < 8; ++k) o[k] = pack_bf16(f[2 * k], f[2 * k + 1]);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(X + p * NF);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dst[k] = o[k];
     }
 }
 
+// Logits, 16 rows a warp and step.  Bound by the latency of the weights' way into
+// shared memory for a mini-batch and by issue above it: 8192 rows 4.4 us, 150
+// thousand 10 us (10 and 60 us with strided weight reads, eight to a bank, and
+// scalar conversions into two layouts).
 __global__ void __launch_bounds__(FWARPS * 32) k_mlp_forward(const float *P, const __nv_bfloat16 *X,
                                                               uint64_t n, float *logits)
 {
@@ -265,8 +404,10 @@ __global__ void __launch_bounds__(FWARPS * 32) k_mlp_forward(const float *P, con
     const uint64_t tiles = (n + 15) / 16;
     for (uint64_t tile = blockIdx.x * (uint64_t)FWARPS + (threadIdx.x >> 5); tile < tiles;
          tile += (uint64_t)gridDim.x * FWARPS) {
+        uint32_t a[4];
+        load_x(a, X, n, tile * 16);
         Tile T;
-        forward_tile(s, X, n, tile * 16, T);
+        forward_tile(s, a, T);
         if (t == 0) {
             const uint64_t r0 = tile * 16 + g, r1 = r0 + 8;
             if (r0 < n) logits[r0] = T.z0;
@@ -275,191 +416,205 @@ __global__ void __launch_bounds__(FWARPS * 32) k_mlp_forward(const float *P, con
     }
 }
 
-// Per-warp staging for the weight-gradient GEMMs (all [row][sample], bf16)
-struct WarpStage {
-    __nv_bfloat16 dh2t[NH * 16];   // dL/d(pre-activation 2), [unit][sample]
-    __nv_bfloat16 h1t[NH * 16];    // h1 as layer 2 saw it, [unit][sample]
-    __nv_bfloat16 dh1t[NH * 16];   // dL/d(pre-activation 1), [unit][sample]
-    __nv_bfloat16 xt[NF * 16];     // x, [feature][sample]
+// A block's 64 samples as the weight-gradient products read them, [sample][unit]
+constexpr int FROWS = FWARPS * 16;
+struct Stage {
+    alignas(16) __nv_bfloat16 dh2[FROWS * LD2];   // dL/d(pre-activation 2)
+    alignas(16) __nv_bfloat16 h1[FROWS * LD2];    // h1 as layer 2 saw it
+    alignas(16) __nv_bfloat16 dh1[FROWS * LD2];   // dL/d(pre-activation 1)
+    alignas(16) __nv_bfloat16 x[FROWS * LD1];
 };
 
-struct GradAcc {
-    float w1t[NH * NF], b1[NH], w2t[NH * NH], b2[NH], w3[NH], b3, loss;
-};
+// Sum N values a lane over the eight lanes with the same t: each step sends
+// half of what is left, so N/8 values remain: those from index g * N/8 on.
+template <int N> __device__ __forceinline__ void sum_rows(float (&v)[N], int lane)
+{
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        const int o = 16 >> s, half = N >> (s + 1);
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < half; ++k) {
+            const float send = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+}
+
+// four neighbouring gradients from a pair of lanes' accumulators: the even lane
+// takes row g, the odd one row g + 8
+__device__ __forceinline__ void add_tile(float *G, int ld, const float (&d)[4], int lane)
+{
+    const int g = lane >> 2, t = lane & 3;
+    const bool odd = t & 1;
+    const float s0 = odd ? d[0] : d[2], s1 = odd ? d[1] : d[3];
+    const float r0 = __shfl_xor_sync(0xffffffffu, s0, 1), r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+    const float4 v = odd ? make_float4(r0, r1, d[2], d[3]) : make_float4(d[0], d[1], r0, r1);
+    atomicAdd(reinterpret_cast<float4 *>(G + (g + 8 * odd) * ld + 4 * (t >> 1)), v);
+}
 
 // One pass over a mini-batch: forward, binary cross-entropy with logits
 // (weighted by wts, averaged by inv_norm), backward, and gradient
-// accumulation into G (same layout as P) and *loss.
+// accumulation into G (same layout as P) and the loss after it.
+//
+// Bound by latency: at 8192 rows a block has one 64-row step.  The four warps
+// take 16 rows each through both layers and back; then the block's activations
+// stand in shared memory as [sample][unit], and warp w forms rows 16w..16w+15
+// of both weight gradients over all 64 samples, in registers that live as long
+// as the block.  Nothing is added in shared memory (an FP32 add there is a
+// compare-and-swap loop): a block ends in one vector reduction to G.
+// 8192 rows: 6.9 us (30 us with every 16x8 product added to shared memory).
 __global__ void __launch_bounds__(FWARPS * 32) k_mlp_backward(const float *P, const __nv_bfloat16 *X,
                                                                const float *label, const float *wts,
                                                                uint64_t n, float inv_norm, float *G)
 {
-    extern __shared__ unsigned char fsm[];
-    SmemW &s = *reinterpret_cast<SmemW *>(fsm);
-    GradAcc &acc = *reinterpret_cast<GradAcc *>(fsm + sizeof(SmemW));
-    WarpStage *stages = reinterpret_cast<WarpStage *>(fsm + sizeof(SmemW) + sizeof(GradAcc));
-    load_weights(s, P);
-    {
-        float *a = reinterpret_cast<float *>(&acc);
-        for (int k = threadIdx.x; k < (int)(sizeof(GradAcc) / sizeof(float)); k += blockDim.x) a[k] = 0.f;
-    }
-    __syncthreads();
+    __shared__ SmemW s;
+    __shared__ Stage st;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, wib = threadIdx.x >> 5;
-    WarpStage &st = stages[wib];
-    const uint64_t tiles = (n + 15) / 16;
-    for (uint64_t tile = blockIdx.x * (uint64_t)FWARPS + wib; tile < tiles;
-         tile += (uint64_t)gridDim.x * FWARPS) {
-        const uint64_t base = tile * 16;
-        Tile T;
-        forward_tile(s, X, n, base, T);
+    uint64_t base = blockIdx.x * (uint64_t)FROWS + wib * 16;
+    uint32_t a[4];
+    float lw[4];   // labels and weights of rows g, g + 8
+    load_x(a, X, n, base);
+    load_labels(lw, label, wts, n, base);
+    load_weights(s, P);
+    float dw2[8][4] = {}, dw1[2][4] = {};
+    float pw3[16] = {}, pb2[16] = {}, pb1[16] = {}, pb3 = 0.f, ploss = 0.f;
+    __syncthreads();
+    const uint64_t steps = (n + FROWS - 1) / FROWS;
+    for (uint64_t step = blockIdx.x; step < steps; step += gridDim.x) {
         const uint64_t r0 = base + g, r1 = r0 + 8;
-        const float y0 = r0 < n ? label[r0] : 0.f, y1 = r1 < n ? label[r1] : 0.f;
-        const float w0 = r0 < n ? wts[r0] : 0.f, w1 = r1 < n ? wts[r1] : 0.f;
+        const float y0 = lw[0], y1 = lw[1], w0 = lw[2], w1 = lw[3];
+        __nv_bfloat16 *sx = st.x + (wib * 16 + g) * LD1 + 2 * t;
+        *reinterpret_cast<uint32_t *>(sx) = a[0];
+        *reinterpret_cast<uint32_t *>(sx + 8 * LD1) = a[1];
+        *reinterpret_cast<uint32_t *>(sx + 8) = a[2];
+        *reinterpret_cast<uint32_t *>(sx + 8 * LD1 + 8) = a[3];
+        Tile T;
+        forward_tile(s, a, T);
         const float p0 = 1.f / (1.f + __expf(-T.z0)), p1 = 1.f / (1.f + __expf(-T.z1));
-        const float dz0 = w0 * (p0 - y0) * inv_norm, dz1 = w1 * (p1 - y1) * inv_norm;
+        const float dz0 = r0 < n ? w0 * (p0 - y0) * inv_norm : 0.f;
+        const float dz1 = r1 < n ? w1 * (p1 - y1) * inv_norm : 0.f;
         if (t == 0) {
             const float l0 = fmaxf(T.z0, 0.f) - T.z0 * y0 + log1pf(__expf(-fabsf(T.z0)));
             const float l1 = fmaxf(T.z1, 0.f) - T.z1 * y1 + log1pf(__expf(-fabsf(T.z1)));
-            atomicAdd(&acc.loss, (w0 * l0 + w1 * l1) * inv_norm);
-            atomicAdd(&acc.b3, dz0 + dz1);
+            ploss += ((r0 < n ? w0 * l0 : 0.f) + (r1 < n ? w1 * l1 : 0.f)) * inv_norm;
+            pb3 += dz0 + dz1;
         }
         // layer 3 and the pre-activation gradient of layer 2
         float dh2[8][4];
+        __nv_bfloat16 *sh = st.h1 + (wib * 16 + g) * LD2 + 2 * t;
+        __nv_bfloat16 *s2 = st.dh2 + (wib * 16 + g) * LD2 + 2 * t;
+        __nv_bfloat16 *s1 = st.dh1 + (wib * 16 + g) * LD2 + 2 * t;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             const int c = nt * 8 + 2 * t;
-            float gw0 = dz0 * T.h2[nt][0] + dz1 * T.h2[nt][2];
-            float gw1 = dz0 * T.h2[nt][1] + dz1 * T.h2[nt][3];
+            pw3[2 * nt] += dz0 * T.h2[nt][0] + dz1 * T.h2[nt][2];
+            pw3[2 * nt + 1] += dz0 * T.h2[nt][1] + dz1 * T.h2[nt][3];
             dh2[nt][0] = T.h2[nt][0] > 0.f ? dz0 * s.w3[c] : 0.f;
             dh2[nt][1] = T.h2[nt][1] > 0.f ? dz0 * s.w3[c + 1] : 0.f;
             dh2[nt][2] = T.h2[nt][2] > 0.f ? dz1 * s.w3[c] : 0.f;
             dh2[nt][3] = T.h2[nt][3] > 0.f ? dz1 * s.w3[c + 1] : 0.f;
-            float gb0 = dh2[nt][0] + dh2[nt][2], gb1 = dh2[nt][1] + dh2[nt][3];
-            // sum over the 8 row groups (lanes with the same t)
-#pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                gw0 += __shfl_xor_sync(0xffffffffu, gw0, o);
-                gw1 += __shfl_xor_sync(0xffffffffu, gw1, o);
-                gb0 += __shfl_xor_sync(0xffffffffu, gb0, o);
-                gb1 += __shfl_xor_sync(0xffffffffu, gb1, o);
-            }
-            if (g == 0) {
-                atomicAdd(&acc.w3[c], gw0);
-                atomicAdd(&acc.w3[c + 1], gw1);
-                atomicAdd(&acc.b2[c], gb0);
-                atomicAdd(&acc.b2[c + 1], gb1);
-            }
+            pb2[2 * nt] += dh2[nt][0] + dh2[nt][2];
+            pb2[2 * nt + 1] += dh2[nt][1] + dh2[nt][3];
+            st_bf16x2(sh + nt * 8, T.h1[nt][0], T.h1[nt][1]);
+            st_bf16x2(sh + 8 * LD2 + nt * 8, T.h1[nt][2], T.h1[nt][3]);
         }
         // dh1 = dh2 W2 (tensor cores), masked by the layer-1 ReLU
-        uint32_t a[4][4];
+        uint32_t a2[4][4];
 #pragma unroll
         for (int kc = 0; kc < 4; ++kc) {
-            a[kc][0] = pack_bf16(dh2[2 * kc][0], dh2[2 * kc][1]);
-            a[kc][1] = pack_bf16(dh2[2 * kc][2], dh2[2 * kc][3]);
-            a[kc][2] = pack_bf16(dh2[2 * kc + 1][0], dh2[2 * kc + 1][1]);
-            a[kc][3] = pack_bf16(dh2[2 * kc + 1][2], dh2[2 * kc + 1][3]);
+            a2[kc][0] = pack_bf16(dh2[2 * kc][0], dh2[2 * kc][1]);
+            a2[kc][1] = pack_bf16(dh2[2 * kc][2], dh2[2 * kc][3]);
+            a2[kc][2] = pack_bf16(dh2[2 * kc + 1][0], dh2[2 * kc + 1][1]);
+            a2[kc][3] = pack_bf16(dh2[2 * kc + 1][2], dh2[2 * kc + 1][3]);
+            *reinterpret_cast<uint32_t *>(s2 + kc * 16) = a2[kc][0];
+            *reinterpret_cast<uint32_t *>(s2 + 8 * LD2 + kc * 16) = a2[kc][1];
+            *reinterpret_cast<uint32_t *>(s2 + kc * 16 + 8) = a2[kc][2];
+            *reinterpret_cast<uint32_t *>(s2 + 8 * LD2 + kc * 16 + 8) = a2[kc][3];
         }
-        float dh1[8][4];
+        // rows of a transposed tile pair: unit (lane & 7) + 8 * bit 3, columns 8 * bit 4
+        const int trow = (lane & 7) + (lane & 8), tcol = (lane >> 4) * 8;
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int np = 0; np < 4; ++np) {
+            float d[2][4] = {};
 #pragma unroll
             for (int kc = 0; kc < 4; ++kc) {
-                const __nv_bfloat16 *w = s.w2 + (nt * 8 + g) * NH + kc * 16 + 2 * t;
-                mma16816(d, a[kc], ld_u32(w), ld_u32(w + 8));
+                uint32_t b[4];
+                ldsm4t(b, s.w2t + (kc * 16 + trow) * LD2 + np * 16 + tcol);
+                mma16816(d[0], a2[kc], b[0], b[1]);
+                mma16816(d[1], a2[kc], b[2], b[3]);
             }
-            dh1[nt][0] = T.h1[nt][0] > 0.f ? d[0] : 0.f;
-            dh1[nt][1] = T.h1[nt][1] > 0.f ? d[1] : 0.f;
-            dh1[nt][2] = T.h1[nt][2] > 0.f ? d[2] : 0.f;
-            dh1[nt][3] = T.h1[nt][3] > 0.f ? d[3] : 0.f;
-            const int c = nt * 8 + 2 * t;
-            float gb0 = dh1[nt][0] + dh1[nt][2], gb1 = dh1[nt][1] + dh1[nt][3];
 #pragma unroll
-            for (int o = 4; o < 32; o <<= 1) {
-                gb0 += __shfl_xor_sync(0xffffffffu, gb0, o);
-                gb1 += __shfl_xor_sync(0xffffffffu, gb1, o);
-            }
-            if (g == 0) {
-                atomicAdd(&acc.b1[c], gb0);
-                atomicAdd(&acc.b1[c + 1], gb1);
+            for (int q = 0; q < 2; ++q) {
+                const int nt = 2 * np + q;
+                const float e0 = T.h1[nt][0] > 0.f ? d[q][0] : 0.f, e1 = T.h1[nt][1] > 0.f ? d[q][1] : 0.f;
+                const float e2 = T.h1[nt][2] > 0.f ? d[q][2] : 0.f, e3 = T.h1[nt][3] > 0.f ? d[q][3] : 0.f;
+                pb1[2 * nt] += e0 + e2;
+                pb1[2 * nt + 1] += e1 + e3;
+                st_bf16x2(s1 + nt * 8, e0, e1);
+                st_bf16x2(s1 + 8 * LD2 + nt * 8, e2, e3);
             }
         }
-        // stage the transposed operands of the weight-gradient GEMMs
+        base += (uint64_t)gridDim.x * FROWS;
+        load_x(a, X, n, base);   // the next step's rows
+        load_labels(lw, label, wts, n, base);
+        __syncthreads();
+        // dW2[o][i] = sum_s dh2[s][o] h1[s][i], dW1[o][f] = sum_s dh1[s][o] x[s][f]:
+        // M = this warp's 16 o, N = i or f, K = the samples
+        const int arow = (lane & 7) + (lane >> 4) * 8, acol = wib * 16 + (lane & 8);
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            const int c = nt * 8 + 2 * t;
-            st.dh2t[c * 16 + g] = __float2bfloat16_rn(dh2[nt][0]);
-            st.dh2t[(c + 1) * 16 + g] = __float2bfloat16_rn(dh2[nt][1]);
-            st.dh2t[c * 16 + g + 8] = __float2bfloat16_rn(dh2[nt][2]);
-            st.dh2t[(c + 1) * 16 + g + 8] = __float2bfloat16_rn(dh2[nt][3]);
-            st.h1t[c * 16 + g] = __float2bfloat16_rn(T.h1[nt][0]);
-            st.h1t[(c + 1) * 16 + g] = __float2bfloat16_rn(T.h1[nt][1]);
-            st.h1t[c * 16 + g + 8] = __float2bfloat16_rn(T.h1[nt][2]);
-            st.h1t[(c + 1) * 16 + g + 8] = __float2bfloat16_rn(T.h1[nt][3]);
-            st.dh1t[c * 16 + g] = __float2bfloat16_rn(dh1[nt][0]);
-            st.dh1t[(c + 1) * 16 + g] = __float2bfloat16_rn(dh1[nt][1]);
-            st.dh1t[c * 16 + g + 8] = __float2bfloat16_rn(dh1[nt][2]);
-            st.dh1t[(c + 1) * 16 + g + 8] = __float2bfloat16_rn(dh1[nt][3]);
-        }
-        for (int k = lane; k < NF * 16; k += 32) {
-            const int f = k / 16, smp = k % 16;
-            const uint64_t r = base + smp;
-            st.xt[k] = r < n ? X[r * NF + f] : __float2bfloat16_rn(0.f);
-        }
-        __syncwarp();
-        // dW2[o][i] = sum_s dh2[s][o] h1[s][i]:  M = o, N = i, K = the 16 samples
+        for (int kc = 0; kc < FWARPS; ++kc) {
+            uint32_t am[4], b[4];
+            ldsm4t(am, st.dh2 + (kc * 16 + arow) * LD2 + acol);
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-            uint32_t am[4];
-            am[0] = ld_u32(st.dh2t + (mt * 16 + g) * 16 + 2 * t);
-            am[1] = ld_u32(st.dh2t + (mt * 16 + g + 8) * 16 + 2 * t);
-            am[2] = ld_u32(st.dh2t + (mt * 16 + g) * 16 + 2 * t + 8);
-            am[3] = ld_u32(st.dh2t + (mt * 16 + g + 8) * 16 + 2 * t + 8);
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                float d[4] = {0.f, 0.f, 0.f, 0.f};
-                const __nv_bfloat16 *b = st.h1t + (nt * 8 + g) * 16 + 2 * t;
-                mma16816(d, am, ld_u32(b), ld_u32(b + 8));
-                const int o0 = mt * 16 + g, i0 = nt * 8 + 2 * t;
-                atomicAdd(&acc.w2t[o0 * NH + i0], d[0]);
-                atomicAdd(&acc.w2t[o0 * NH + i0 + 1], d[1]);
-                atomicAdd(&acc.w2t[(o0 + 8) * NH + i0], d[2]);
-                atomicAdd(&acc.w2t[(o0 + 8) * NH + i0 + 1], d[3]);
+            for (int np = 0; np < 4; ++np) {
+                ldsm4t(b, st.h1 + (kc * 16 + trow) * LD2 + np * 16 + tcol);
+                mma16816(dw2[2 * np], am, b[0], b[1]);
+                mma16816(dw2[2 * np + 1], am, b[2], b[3]);
             }
+            ldsm4t(am, st.dh1 + (kc * 16 + arow) * LD2 + acol);
+            ldsm4t(b, st.x + (kc * 16 + trow) * LD1 + tcol);
+            mma16816(dw1[0], am, b[0], b[1]);
+            mma16816(dw1[1], am, b[2], b[3]);
         }
-        // dW1[o][f] = sum_s dh1[s][o] x[s][f]:  M = o, N = f, K = samples
+        __syncthreads();
+    }
+    float *G2 = G + P_W2 + wib * 16 * NH, *G1 = G + P_W1 + wib * 16 * NF;
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-            uint32_t am[4];
-            am[0] = ld_u32(st.dh1t + (mt * 16 + g) * 16 + 2 * t);
-            am[1] = ld_u32(st.dh1t + (mt * 16 + g + 8) * 16 + 2 * t);
-            am[2] = ld_u32(st.dh1t + (mt * 16 + g) * 16 + 2 * t + 8);
-            am[3] = ld_u32(st.dh1t + (mt * 16 + g + 8) * 16 + 2 * t + 8);
+    for (int nt = 0; nt < 8; ++nt) add_tile(G2 + nt * 8, NH, dw2[nt], lane);
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                float d[4] = {0.f, 0.f, 0.f, 0.f};
-                const __nv_bfloat16 *b = st.xt + (nt * 8 + g) * 16 + 2 * t;
-                mma16816(d, am, ld_u32(b), ld_u32(b + 8));
-                const int o0 = mt * 16 + g, f0 = nt * 8 + 2 * t;
-                atomicAdd(&acc.w1t[o0 * NF + f0], d[0]);
-                atomicAdd(&acc.w1t[o0 * NF + f0 + 1], d[1]);
-                atomicAdd(&acc.w1t[(o0 + 8) * NF + f0], d[2]);
-                atomicAdd(&acc.w1t[(o0 + 8) * NF + f0 + 1], d[3]);
-            }
-        }
-        __syncwarp();
+    for (int nt = 0; nt < 2; ++nt) add_tile(G1 + nt * 8, NF, dw1[nt], lane);
+    // the vectors: over the warp's rows, then over the warps
+    float *sum = reinterpret_cast<float *>(st.dh2);          // [warp][w3, b2, b1][unit], b3, loss
+    sum_rows(pw3, lane);
+    sum_rows(pb2, lane);
+    sum_rows(pb1, lane);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+        pb3 += __shfl_xor_sync(0xffffffffu, pb3, o);
+        ploss += __shfl_xor_sync(0xffffffffu, ploss, o);
+    }
+    // values 2g and 2g + 1 of the 16 are units 8g + 2t and the next
+    const int unit = g * 8 + 2 * t;
+    constexpr int WS = 3 * NH + 2;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        sum[wib * WS + unit + k] = pw3[k];
+        sum[wib * WS + NH + unit + k] = pb2[k];
+        sum[wib * WS + 2 * NH + unit + k] = pb1[k];
+    }
+    if (lane == 0) {
+        sum[wib * WS + 3 * NH] = pb3;
+        sum[wib * WS + 3 * NH + 1] = ploss;
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < NH * NF; k += blockDim.x) atomicAdd(&G[P_W1 + k], acc.w1t[k]);
-    for (int k = threadIdx.x; k < NH * NH; k += blockDim.x) atomicAdd(&G[P_W2 + k], acc.w2t[k]);
-    for (int k = threadIdx.x; k < NH; k += blockDim.x) {
-        atomicAdd(&G[P_B1 + k], acc.b1[k]);
-        atomicAdd(&G[P_B2 + k], acc.b2[k]);
-        atomicAdd(&G[P_W3 + k], acc.w3[k]);
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(&G[P_B3], acc.b3);
-        atomicAdd(&G[NPARAM], acc.loss);
+    for (int k = threadIdx.x; k < WS; k += FWARPS * 32) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < FWARPS; ++w) v += sum[w * WS + k];
+        const int at = k < NH ? P_W3 + k : k < 2 * NH ? P_B2 + k - NH : k < 3 * NH ? P_B1 + k - 2 * NH
+                     : k == 3 * NH ? P_B3 : NPARAM;
+        atomicAdd(G + at, v);
     }
 }
 
@@ -518,8 +673,6 @@ __global__ void k_scatter(const pg_result *kept_res, const uint32_t *kept_idx, c
         out[kept_idx[q]] = kept_res[q];
 }
 
-size_t backward_smem() { return sizeof(SmemW) + sizeof(GradAcc) + FWARPS * sizeof(WarpStage); }
-
 }  // namespace
 
 struct pg_filter {
@@ -576,9 +729,6 @@ int pg_filter_create(int device, uint64_t seed, pg_filter **out)
     if (e == cudaSuccess) e = cudaMemset(f->d_G, 0, (NPARAM + 1) * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(f->d_M1, 0, NPARAM * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(f->d_M2, 0, NPARAM * sizeof(float));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)backward_smem());
     if (e != cudaSuccess) {
         pg_filter_destroy(f);
         return pg_internal_fail(e == cudaErrorMemoryAllocation ? PG_ERR_OOM : PG_ERR_CUDA,
@@ -637,10 +787,12 @@ int pg_filter_features(pg_filter *f, pg_ctx *ctx, const pg_pair *d_pairs, uint64
     }
     const int grid = f->nsm * 8;
     k_composition<<<grid, 256, 0, st>>>(rseq, roffs, nr, f->d_rcomp);
-    k_composition<<<grid, 256, 0, st>>>(cseq, coffs, nc, f->d_ccomp);
+    // a block of the search against itself has one set on both sides
+    const bool same = rseq == cseq && roffs == coffs && nr == nc;
+    if (!same) k_composition<<<grid, 256, 0, st>>>(cseq, coffs, nc, f->d_ccomp);
     FCU(cudaMemsetAsync(f->d_status, 0, sizeof(int), st));
     if (n) k_features<<<grid, 256, 0, st>>>(d_pairs, n, bl_roffset, bl_coffset, rseq, roffs, nr,
-                                           cseq, coffs, nc, d_sm, f->d_rcomp, f->d_ccomp,
+                                           cseq, coffs, nc, d_sm, f->d_rcomp, same ? f->d_rcomp : f->d_ccomp,
                                            (__nv_bfloat16 *)d_features, f->d_status);
     FCU(cudaGetLastError());
     int status = 0;
@@ -656,7 +808,7 @@ int pg_filter_predict(pg_filter *f, const void *d_features, uint64_t n, float *d
     if (!n) return PG_OK;
     FCU(cudaSetDevice(f->device));
     const uint64_t tiles = (n + 15) / 16;
-    const uint64_t blocks = std::min<uint64_t>((tiles + FWARPS - 1) / FWARPS, (uint64_t)f->nsm * 16);
+    const uint64_t blocks = std::min<uint64_t>((tiles + FWARPS - 1) / FWARPS, (uint64_t)f->nsm * 8);
     k_mlp_forward<<<(unsigned)blocks, FWARPS * 32, 0, (cudaStream_t)stream>>>(
         f->d_P, (const __nv_bfloat16 *)d_features, n, d_logits);
     FCU(cudaGetLastError());
@@ -671,9 +823,8 @@ int pg_filter_gradients(pg_filter *f, const void *d_features, const float *d_lab
     FCU(cudaSetDevice(f->device));
     cudaStream_t st = (cudaStream_t)stream;
     FCU(cudaMemsetAsync(f->d_G, 0, (NPARAM + 1) * sizeof(float), st));
-    const uint64_t tiles = (n + 15) / 16;
-    const uint64_t blocks = std::min<uint64_t>((tiles + FWARPS - 1) / FWARPS, (uint64_t)f->nsm * 4);
-    k_mlp_backward<<<(unsigned)blocks, FWARPS * 32, backward_smem(), st>>>(
+    const uint64_t blocks = std::min<uint64_t>((n + FROWS - 1) / FROWS, (uint64_t)f->nsm * 2);
+    k_mlp_backward<<<(unsigned)blocks, FWARPS * 32, 0, st>>>(
         f->d_P, (const __nv_bfloat16 *)d_features, d_labels, d_weights, n, 1.0f / (float)n, f->d_G);
     FCU(cudaGetLastError());
     if (host_grad_and_loss) {

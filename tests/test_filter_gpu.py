@@ -155,3 +155,78 @@ def test_features_match_oracle(native):
     assert win[w.homolog == 1].mean() > win[w.homolog == 0].mean() + 0.2
     f.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [1, 15, 17, 63, 65, 129, 64 * 304 + 1, 64 * 608 + 79])
+def test_gradients_at_step_edges(native, n):
+    """Rows that end inside a warp's 16, a block's 64 and a block's second
+    step; the bounds are those of test_forward_and_gradients_match_reference
+    (same rounding points, float32 sums in another order)."""
+    import torch
+    from oracle import mlp_oracle as M
+    from pastis_gb300.filter import Filter
+    rng = np.random.default_rng(n)
+    f = Filter(0, seed=3)
+    P = rng.normal(0, 0.25, M.NPARAM).astype(np.float32)
+    f.set_params(P)
+    Xb, Xr = _dev_features(rng.random((n, M.NF)) * 2 - 0.5)
+    y = (rng.random(n) < 0.3).astype(np.float32)
+    w = rng.uniform(0.5, 3.0, n).astype(np.float32)
+    z = torch.full((n + 64,), 7.0, dtype=torch.float32, device="cuda:0")
+    f.predict(Xb.data_ptr(), n, z.data_ptr())
+    torch.cuda.synchronize()
+    z_ref, _ = M.forward(P, Xr, bf16_ops=True)
+    assert np.allclose(z[:n].cpu().numpy(), z_ref, rtol=2e-3, atol=2e-3)
+    assert (z[n:] == 7.0).all()
+    yd, wd = torch.from_numpy(y).cuda(), torch.from_numpy(w).cuda()
+    g, loss = f.gradients(Xb.data_ptr(), yd.data_ptr(), wd.data_ptr(), n)
+    loss_ref, g_ref = M.loss_and_grad(P, Xr, y, w, bf16_ops=True)
+    assert abs(loss - loss_ref) <= 1e-3 * max(1.0, abs(loss_ref))
+    for a, b in ((M.P_W1, M.P_B1), (M.P_B1, M.P_W2), (M.P_W2, M.P_B2), (M.P_B2, M.P_W3),
+                 (M.P_W3, M.P_B3), (M.P_B3, M.NPARAM)):
+        # a bf16 rounding tie may fall either way once in many thousand rows:
+        # one step (2^-8) of one of n rows' terms
+        err = np.abs(g[a:b] - g_ref[a:b]).max() / (np.abs(g_ref[a:b]).max() + 1e-12)
+        assert err < 1e-5 + 2.0 ** -8 / max(n, 1) ** 0.5, (a, err)
+    f.close()
+
+
+@pytest.mark.parametrize("shared", [True, False])
+def test_features_of_short_and_odd_sequences(native, shared):
+    """Lengths 1..70 at every byte offset, seeds at the ends, 1 to 33 pairs in
+    a group of 32, rows and columns as one set or as two equal ones."""
+    import torch
+    from oracle import mlp_oracle as M
+    from oracle import oracle as O
+    from pastis_gb300 import capi
+    from pastis_gb300.filter import Filter
+    rng = np.random.default_rng(5)
+    lens = np.concatenate([np.arange(1, 71), [511, 512, 513, 1030]])
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    ascii_ = np.frombuffer(b"ARNDCQEGHILKMFPSTWYVBZX*J", np.uint8)[rng.integers(0, 25, int(offs[-1]))]
+    ctx = capi.Context(capi.config(capi.MODE_XDROP))
+    ctx.set_seqs(0, ascii_, offs)
+    if shared:
+        ctx.share_row_seqs()
+    else:
+        ctx.set_seqs(1, ascii_, offs)
+    codes, _ = ctx.get_seqs(0)
+    f = Filter(0, seed=1)
+    for n in (1, 31, 33, 400):
+        p = np.zeros(n, dtype=capi.PAIR_DTYPE)
+        p["row"], p["col"] = rng.integers(0, len(lens), n), rng.integers(0, len(lens), n)
+        for a, b in (("rs0", "row"), ("rs1", "row"), ("cs0", "col"), ("cs1", "col")):
+            p[a] = rng.integers(0, lens[p[b]])
+        p["count"], p["score"] = rng.integers(1, 4, n), rng.integers(-5, 60, n)
+        d = torch.from_numpy(p.view(np.uint8).copy()).cuda()
+        feats = torch.empty(n * 32, dtype=torch.uint8, device="cuda:0")
+        f.features(ctx, d.data_ptr(), n, feats.data_ptr())
+        torch.cuda.synchronize()
+        got = feats.cpu().numpy().view(np.uint16).reshape(n, 16).astype(np.int64)
+        ref = M.features(p, codes, offs, O.blosum62().reshape(-1))
+        bits = (M.bf16(ref).astype(np.float32).view(np.uint32) >> 16).astype(np.int64)
+        assert np.abs(got - bits).max() <= 1
+        whole = got[:, [2, 8, 12, 13, 14, 15]] == bits[:, [2, 8, 12, 13, 14, 15]]
+        assert whole.mean() > 0.99
+    f.close()
+    ctx.close()
