@@ -18,6 +18,7 @@
 #include "pg_stat.h"
 #include "pg_kernels.cuh"
 #include "pg_kernels_xd.cuh"
+#include "pg_dptag.cuh"
 #include "pg_lin.cuh"
 
 namespace {
@@ -162,7 +163,7 @@ struct pg_ctx {
     // linear-gap alignment (pg_lin.cuh): bucket counts, cursors and totals in
     // one block, the list with its per-entry words, the X-drop walks' counts
     bool lin_ok = false;
-    int lin_smax = 0, lin_bps = 1;
+    int smin = 0, smax = 0, lin_bps = 1;
     uint8_t *d_lin = nullptr;
     pg::LinTotals *h_lin = nullptr;     // pinned
     uint8_t *d_list = nullptr;
@@ -315,7 +316,8 @@ int pg_create(const pg_config *cfg, pg_ctx **out)
         c->lim16 = pg::dir16_limit(maxabs);
         const auto mm = std::minmax_element(c->sm, c->sm + PG_NRES * PG_NRES);
         c->lin_ok = pg::lin_supported(c->go, c->ge, *mm.first, *mm.second);
-        c->lin_smax = *mm.second;
+        c->smin = *mm.first;
+        c->smax = *mm.second;
     }
 #define CUD(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { pg_destroy(c); \
         return fail(e_ == cudaErrorMemoryAllocation ? PG_ERR_OOM : PG_ERR_CUDA, "%s: %s", #call, \
@@ -382,8 +384,9 @@ static int ensure_scratch(pg_ctx *c)
 {
     const uint32_t rmax = c->side[0].maxlen;
     const uint32_t cmax = c->cols_share_rows ? rmax : c->side[1].maxlen;
-    // one DP row of the widest edge type (local statistics, 3 words)
-    const size_t per_warp = ((size_t)cmax + 1) * sizeof(pg::Edge<pg::L2>);
+    // one DP row of the widest edge type (local statistics, 3 words), in whole 16
+    // bytes: the tagged form reads and writes 8 bytes at a time
+    const size_t per_warp = (((size_t)cmax + 1) * sizeof(pg::Edge<pg::L2>) + 15) & ~(size_t)15;
     // keep the row scratch within 8 GiB: fewer resident warps for very long sequences
     size_t warps = (size_t)c->grid * pg::WARPS;
     const size_t budget = (size_t)8 << 30;
@@ -532,7 +535,7 @@ static int run_lin(pg_ctx *c, const pg::KParams &kp, uint64_t p0, uint64_t p1, c
     lp.cnt = reinterpret_cast<uint32_t *>(c->d_lin);
     lp.cur = lp.cnt + pg::LIN_NB;
     lp.tot = reinterpret_cast<pg::LinTotals *>(lp.cur + pg::LIN_NB);
-    lp.smax = c->lin_smax;
+    lp.smax = c->smax;
     lp.e_first = (c->cfg.tie & PG_TIE_H_E_BEFORE_F) ? 1 : 0;
     lp.list = nullptr; lp.dp = nullptr; lp.prog = nullptr; lp.wlist = nullptr; lp.arena = nullptr; lp.walk = nullptr;
     CU(cudaMemsetAsync(c->d_lin, 0, LIN_BLOCK, st));
@@ -695,6 +698,18 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
         const int gmax = std::max(c->go, c->ge);
         if (c->cfg.mode == PG_MODE_SW || gmax >= 0) kp.dir16_side = 65535;
         else kp.dir16_side = std::min(65535, (pg::SAT16_DP - std::abs(c->go)) / -gmax);
+    }
+    // tagged 16-bit form: scores that fit its int8 profile with their tags; m + n
+    // whose path of gaps stays in range after scaling by 4 (local: any).  Not
+    // where that would take regions the untagged form proves in range.
+    kp.tag = kp.tag_sum = kp.tag_min = 0;
+    if (kp.dir16_lim > 0 && c->go < 0 && c->ge < 0 && c->go >= -pg::TAG_SMAX && c->ge >= -pg::TAG_SMAX &&
+        c->smin >= -pg::TAG_SMAX && c->smax <= pg::TAG_SMAX) {
+        const int gmax = std::max(c->go, c->ge);
+        kp.tag_sum = c->cfg.mode == PG_MODE_SW ? 1 << 30
+                                               : (pg::SAT16_DP / 4 - 2 * std::abs(c->go)) / -gmax - 20;
+        kp.tag_min = pg::TAG_MAX / (4 * std::max(1, c->smax));
+        kp.tag = kp.tag_sum >= kp.dir16_lim ? 1 : 0;
     }
     // gap scores whose affine recurrence is a linear one: the default form runs
     // them through pg_lin.cuh (the scheduling options that have no meaning there

@@ -8,40 +8,45 @@ namespace pg {
 
 cudaError_t dir_set_attributes_ga()
 {
-    const void *k[12] = {(const void *)k_ga_dir<0, false>, (const void *)k_ga_dir<1, false>,
-                         (const void *)k_ga_dir<2, false>, (const void *)k_ga_dir<3, false>,
-                         (const void *)k_ga_dir<0, true>, (const void *)k_ga_dir<1, true>,
-                         (const void *)k_ga_dir<2, true>, (const void *)k_ga_dir<3, true>,
-                         (const void *)k_ga_pair<0>, (const void *)k_ga_pair<1>,
-                         (const void *)k_ga_pair<2>, (const void *)k_ga_pair<3>};
+    const void *k[20] = {(const void *)k_ga_dir<0, false, false>, (const void *)k_ga_dir<1, false, false>,
+                         (const void *)k_ga_dir<2, false, false>, (const void *)k_ga_dir<3, false, false>,
+                         (const void *)k_ga_dir<0, true, false>, (const void *)k_ga_dir<1, true, false>,
+                         (const void *)k_ga_dir<2, true, false>, (const void *)k_ga_dir<3, true, false>,
+                         (const void *)k_ga_dir<0, false, true>, (const void *)k_ga_dir<1, false, true>,
+                         (const void *)k_ga_dir<2, false, true>, (const void *)k_ga_dir<3, false, true>,
+                         (const void *)k_ga_pair<0, false>, (const void *)k_ga_pair<1, false>,
+                         (const void *)k_ga_pair<2, false>, (const void *)k_ga_pair<3, false>,
+                         (const void *)k_ga_pair<0, true>, (const void *)k_ga_pair<1, true>,
+                         (const void *)k_ga_pair<2, true>, (const void *)k_ga_pair<3, true>};
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 12 && e == cudaSuccess; ++i)
+    for (int i = 0; i < 20 && e == cudaSuccess; ++i)
         e = cudaFuncSetAttribute(k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, DIR16_DYN_SMEM);
     return e;
 }
 
-template <bool CHK>
+template <bool CHK, bool TAG>
 static void dp_ga(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint64_t *doff,
                    uint8_t *arena, int *dsc, int grid, int dyn, cudaStream_t st)
 {
     const dim3 blk(WARPS * 32);
     switch (tie) {
-    case 0: k_ga_dir<0, CHK><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    case 1: k_ga_dir<1, CHK><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    case 2: k_ga_dir<2, CHK><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    default: k_ga_dir<3, CHK><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 0: k_ga_dir<0, CHK, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 1: k_ga_dir<1, CHK, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 2: k_ga_dir<2, CHK, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    default: k_ga_dir<3, CHK, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
     }
 }
 
+template <bool TAG>
 static void pair_ga(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint64_t *doff,
                     uint8_t *arena, int *dsc, int grid, int dyn, cudaStream_t st)
 {
     const dim3 blk(WARPS * 32);
     switch (tie) {
-    case 0: k_ga_pair<0><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    case 1: k_ga_pair<1><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    case 2: k_ga_pair<2><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
-    default: k_ga_pair<3><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 0: k_ga_pair<0, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 1: k_ga_pair<1, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    case 2: k_ga_pair<2, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
+    default: k_ga_pair<3, TAG><<<grid, blk, dyn, st>>>(kp, t0, t1, doff, arena, dsc); break;
     }
 }
 
@@ -49,15 +54,17 @@ int dir_run_ga(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint6
                uint8_t *arena, int *dsc, int grid, int dyn, int grid_tb, bool chk, cudaStream_t st)
 {
     int launches = 2;
-    dp_ga<false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+    if (kp.tag) dp_ga<false, true>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+    else dp_ga<false, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
     if (kp.dir16_pair) {
         cudaMemsetAsync(kp.counter, 0, sizeof(unsigned int), st);
-        pair_ga(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        if (kp.tag) pair_ga<true>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        else pair_ga<false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
         ++launches;
     }
     if (chk) {
         cudaMemsetAsync(kp.counter, 0, sizeof(unsigned int), st);
-        dp_ga<true>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        dp_ga<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
         ++launches;
     }
     k_tb_ga<<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);

@@ -19,8 +19,8 @@
 //
 // Decisions come from equalities on the packed values, not from predicates:
 // min.u16x2(x ^ y, 1) is 1 in the halves where x != y.  Nibble of cell (i, j):
-//   bit 0   H is not the diagonal (diagonal wins every tie)
-//   bit 1   with bit 0: H is E (else F), under the tie policy's order of F and E
+//   bit 1   H is not the diagonal (diagonal wins every tie)
+//   bit 0   with bit 1: H is E (else F), under the tie policy's order of F and E
 //   bit 2   E(i, j) was opened from H(i, j-1)
 //   bit 3   F(i, j) was opened from H(i-1, j)
 // A local alignment's floor needs no bit: the traceback carries the score of
@@ -275,7 +275,7 @@ __device__ DirOut dp_warp_dir16(const uint8_t *__restrict__ V, int m,
                     const uint32_t Hv = LOCAL ? __vimax_s16x2_relu(X, F) : v16max(X, F);
                     const uint32_t nd = v16ne(Hv, dg);
                     const uint32_t ne = E_FIRST ? (v16ne(Hv, E) ^ ONE2) : v16ne(Hv, F);
-                    const uint32_t nib = nd + 2u * ne + 4u * pe + 8u * pf;
+                    const uint32_t nib = ne + 2u * nd + 4u * pe + 8u * pf;
                     if (r < 4) W0 += nib << (4 * (r & 3));
                     else W1 += nib << (4 * (r & 3));
                     const uint32_t G = v16add(Hv, go2);
@@ -531,7 +531,7 @@ __device__ DirOut dp_pair_dir16(const uint8_t *__restrict__ V, int m,
                 const uint32_t Hv = LOCAL ? __vimax_s16x2_relu(X, F) : v16max(X, F);
                 const uint32_t nd = v16ne(Hv, dg);
                 const uint32_t ne = E_FIRST ? (v16ne(Hv, E) ^ ONE2) : v16ne(Hv, F);
-                const uint32_t nib = nd + 2u * ne + 4u * pe + 8u * pf;
+                const uint32_t nib = ne + 2u * nd + 4u * pe + 8u * pf;
                 if (r < 4) W0 += nib << (4 * (r & 3));
                 else W1 += nib << (4 * (r & 3));
                 const uint32_t G = v16add(Hv, go2);

@@ -3,7 +3,8 @@
 // on 16-bit lanes for the regions that fit them (dp_traceback 2; one warp per
 // region, direction nibbles into an HBM arena); with dp_traceback 3 the 16-bit
 // regions of up to 256 rows run two per warp in dp_pair_dir16 (X-drop: in
-// k_ga_pair, SW: inside k_sw_dir).  k_tb_ga / k_tb_sw trace them back (one
+// k_ga_pair, SW: inside k_sw_dir).  With kernel parameter TAG the 16-bit regions
+// run dp_tag16 instead (pg_dptag.cuh).  k_tb_ga / k_tb_sw trace them back (one
 // thread per pair, pg_trace.cuh) and write the same pg_result records k_ga /
 // k_sw write.  A batch whose direction matrices exceed the arena runs in
 // chunks of consecutive tasks (bucket order), each chunk DP then traceback.
@@ -12,6 +13,7 @@
 
 #include "pg_dpdir.cuh"
 #include "pg_dpdir16.cuh"
+#include "pg_dptag.cuh"
 #include "pg_kernels.cuh"
 #include "pg_trace.cuh"
 
@@ -128,21 +130,59 @@ static __global__ void k_chunk_end(const uint64_t *doff, uint64_t t0, uint64_t n
     *t1 = lo;
 }
 
+// the score table of the tagged form and its parameters in a warp
+struct TagArgs {
+    const uint32_t *tab;
+    int go, ge;
+    uint32_t four;
+};
+template <int TIE, bool LOCAL, int L>
+__device__ __forceinline__ DirOut dp_dispatch_tag(const TagArgs &ta, int R, const uint8_t *V, int m,
+                                                  const uint8_t *Hs, int n, uint2 *prof, void *bnd,
+                                                  uint32_t *dir)
+{
+    uint32_t *pf = reinterpret_cast<uint32_t *>(prof);
+    uint2 *b = (uint2 *)bnd;
+    switch (R) {
+    case 1: return dp_tag16<TIE, 1, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 2: return dp_tag16<TIE, 2, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 3: return dp_tag16<TIE, 3, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 4: return dp_tag16<TIE, 4, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 5: return dp_tag16<TIE, 5, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 6: return dp_tag16<TIE, 6, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 7: return dp_tag16<TIE, 7, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    default: return dp_tag16<TIE, 8, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    }
+}
+// loads the tables of a DP kernel
+template <int TIE, bool TAG>
+__device__ __forceinline__ TagArgs dir_tables(const KParams &kp, int *ssm, uint32_t *tab)
+{
+    load_sm(ssm, kp.sm);
+    if (TAG) tag_table<TIE>(reinterpret_cast<int8_t *>(tab), kp.sm);
+    __syncthreads();
+    return TagArgs{tab, kp.go, kp.ge, (uint32_t)kp.four};
+}
+constexpr int TAG_TABW = LIN_NC * LIN_ROWB / 4;
+
 // The DP of one region.  CHK false: a region on 16-bit lanes with every value
 // provably in range (mode 1) or on 32-bit lanes (mode 0); CHK true: a checked
 // region (mode 2), the checked 16-bit form and, if a value left the range, the
 // 32-bit form after it (sat = 1: the traceback walks the 32-bit layout).  The
 // kernels take checked regions in a pass of their own, so the common pass's
 // code stays free of the checked form.
-template <int TIE, bool LOCAL, bool CHK>
-__device__ __forceinline__ DirOut dp_dispatch_dir(const KParams &kp, const uint8_t *V, int m,
+template <int TIE, bool LOCAL, bool CHK, bool TAG>
+__device__ __forceinline__ DirOut dp_dispatch_dir(const KParams &kp, const TagArgs &ta, const uint8_t *V, int m,
                                                   const uint8_t *Hs, int n, const int *ssm,
                                                   uint2 *prof, void *bnd, uint32_t *dir)
 {
+    static_assert(!(CHK && TAG), "the checked pass is the untagged form");
     EdgeD *b = (EdgeD *)bnd;
     const int go = kp.go, ge = kp.ge, cap = kp.rows_cap;
     DirOut d;
-    if (CHK || dir16_mode(kp, m, n) == 1) {
+    if (TAG && dir16_tagged(kp, m, n))
+        return dp_dispatch_tag<TIE, LOCAL, 32>(ta, dir16_rows(m, cap), V, m, Hs, n, prof, bnd, dir);
+    if (!TAG && (CHK || dir16_mode(kp, m, n) == 1)) {
         switch (dir16_rows(m, cap)) {
         case 1: d = dp_warp_dir16<TIE, 1, LOCAL, CHK>(V, m, Hs, n, ssm, prof, go, ge, b, dir); break;
         case 2: d = dp_warp_dir16<TIE, 2, LOCAL, CHK>(V, m, Hs, n, ssm, prof, go, ge, b, dir); break;
@@ -173,11 +213,12 @@ __device__ __forceinline__ DirOut dp_dispatch_dir(const KParams &kp, const uint8
 
 // the DP of two regions of R rows per lane on the two halves of the warp (each
 // lane passes its own half's region; m = 0: none)
-template <int TIE, bool LOCAL>
-__device__ __forceinline__ DirOut dp_dispatch_pair(const KParams &kp, int R, const uint8_t *V, int m,
+template <int TIE, bool LOCAL, bool TAG>
+__device__ __forceinline__ DirOut dp_dispatch_pair(const KParams &kp, const TagArgs &ta, int R, const uint8_t *V, int m,
                                                    const uint8_t *Hs, int n, const int *ssm,
                                                    uint2 *prof, uint32_t *dir)
 {
+    if (TAG) return dp_dispatch_tag<TIE, LOCAL, 16>(ta, R, V, m, Hs, n, prof, nullptr, dir);
     const int go = kp.go, ge = kp.ge;
     switch (R) {
     case 1: return dp_pair_dir16<TIE, 1, LOCAL>(V, m, Hs, n, ssm, prof, go, ge, dir);
@@ -229,8 +270,8 @@ __device__ __forceinline__ bool ga_region(const KParams &kp, uint64_t t, int s, 
 }
 
 // the DP of two waiting X-drop regions (keys a and b, + 1; b = 0: none)
-template <int TIE>
-__device__ __forceinline__ void ga_pair(const KParams &kp, int R, uint64_t a1, uint64_t b1, uint64_t t0,
+template <int TIE, bool TAG>
+__device__ __forceinline__ void ga_pair(const KParams &kp, const TagArgs &ta, int R, uint64_t a1, uint64_t b1, uint64_t t0,
                                         const uint64_t *doff, uint64_t base, uint8_t *arena,
                                         const int *ssm, uint2 *prof, int *dsc)
 {
@@ -241,21 +282,22 @@ __device__ __forceinline__ void ga_pair(const KParams &kp, int R, uint64_t a1, u
     int m = 0, n = 0;
     const int s = k1 ? (int)((k1 - 1) & 1) : 0;
     if (!k1 || !ga_region(kp, t0 + ((k1 - 1) >> 1), s, doff, base, p, V, m, Hs, n, off)) m = n = 0;
-    const DirOut d = dp_dispatch_pair<TIE, false>(kp, R, V, m, Hs, n, ssm, prof, (uint32_t *)(arena + off));
+    const DirOut d = dp_dispatch_pair<TIE, false, TAG>(kp, ta, R, V, m, Hs, n, ssm, prof, (uint32_t *)(arena + off));
     if ((lane & 15) == 0 && m > 0) { dsc[2 * p + s] = d.score; dsc[2 * kp.n + 2 * p + s] = 0; }
 }
 
 // ---------------------------------------------------------------- X-drop
 // DP of each seed region of the tasks [t0, t1); a task's regions sit at
 // arena + doff[t] - doff[t0] (seed 0 first).  dsc[2p + s] = global score,
-// dsc[2n + 2p + s] = 1 where a checked 16-bit region was redone on 32-bit lanes.
-template <int TIE, bool CHK>
+// dsc[2n + 2p + s] = 1 where a checked 16-bit region was redone on 32-bit lanes, 2
+// where the common pass leaves a tagged one to the checked pass.
+template <int TIE, bool CHK, bool TAG>
 __global__ void __launch_bounds__(WARPS * 32, 2) k_ga_dir(const KParams kp, uint64_t t0, uint64_t t1,
                                                          const uint64_t *doff, uint8_t *arena, int *dsc)
 {
     __shared__ int ssm[32 * 32];
-    load_sm(ssm, kp.sm);
-    __syncthreads();
+    __shared__ __align__(16) uint32_t tab[TAG ? TAG_TABW : 1];
+    const TagArgs ta = dir_tables<TIE, TAG>(kp, ssm, tab);
     const uint64_t gw = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
     void *bnd = (char *)kp.bnd + gw * kp.bnd_bytes;
     uint2 *prof = dir_prof(kp);
@@ -281,11 +323,18 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_ga_dir(const KParams kp, uint
             const XdRec &r = sp.rec[s];
             const int rm = r.ev - r.bv, rn = r.eh - r.bh;
             // this pass's regions only (the half-warp ones run in k_ga_pair)
-            if ((dir16_mode(kp, rm, rn) == 2) == CHK && (CHK || !dir16_paired(kp, rm, rn))) {
-                const DirOut d = dp_dispatch_dir<TIE, false, CHK>(kp, V + r.bv, rm, Hs + r.bh, rn, ssm,
-                                                                  prof, bnd, (uint32_t *)(arena + off));
-                if (lane == 0) { dsc[2 * p + s] = d.score; dsc[2 * kp.n + 2 * p + s] = d.sat; }
-                exec += (uint64_t)rm * (uint64_t)rn;
+            const bool tagged = dir16_tagged(kp, rm, rn);
+            const bool mine = CHK ? dir16_mode(kp, rm, rn) == 2 && (!tagged || dsc[2 * kp.n + 2 * p + s] == 2)
+                                  : (tagged || dir16_mode(kp, rm, rn) != 2) && !dir16_paired(kp, rm, rn);
+            if (mine) {
+                const DirOut d = dp_dispatch_dir<TIE, false, CHK, TAG>(kp, ta, V + r.bv, rm, Hs + r.bh, rn, ssm,
+                                                                       prof, bnd, (uint32_t *)(arena + off));
+                __syncwarp();
+                if (lane == 0) {
+                    dsc[2 * p + s] = d.score;
+                    dsc[2 * kp.n + 2 * p + s] = !CHK && tagged ? 2 * d.sat : d.sat;
+                }
+                if (!CHK || !tagged) exec += (uint64_t)rm * (uint64_t)rn;
             }
             off += region_bytes(kp, rm, rn);
         }
@@ -297,13 +346,13 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_ga_dir(const KParams kp, uint
 // warp: a region waits for a partner of the same rows per lane, and those left
 // without one when the queue runs dry run alone.  A kernel of its own: with
 // both in k_ga_dir, its whole-warp regions ran 26 % slower.
-template <int TIE>
+template <int TIE, bool TAG>
 __global__ void __launch_bounds__(WARPS * 32, 2) k_ga_pair(const KParams kp, uint64_t t0, uint64_t t1,
                                                           const uint64_t *doff, uint8_t *arena, int *dsc)
 {
     __shared__ int ssm[32 * 32];
-    load_sm(ssm, kp.sm);
-    __syncthreads();
+    __shared__ __align__(16) uint32_t tab[TAG ? TAG_TABW : 1];
+    const TagArgs ta = dir_tables<TIE, TAG>(kp, ssm, tab);
     uint2 *prof = dir_prof(kp);
     const int lane = threadIdx.x & 31;
     unsigned long long exec = 0;
@@ -343,7 +392,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_ga_pair(const KParams kp, uin
             a1 = __shfl_sync(FULL, slots.pend, R);
             if (!a1) continue;
         }
-        ga_pair<TIE>(kp, R, a1, b1, t0, doff, base, arena, ssm, prof, dsc);
+        ga_pair<TIE, TAG>(kp, ta, R, a1, b1, t0, doff, base, arena, ssm, prof, dsc);
     }
     if (lane == 0 && exec) atomicAdd(kp.exec_cells + 1, exec);
 }
@@ -476,8 +525,8 @@ static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint6
 
 // ---------------------------------------------------------------- SW
 // the DP of two waiting SW pairs (task keys a and b, + 1; b = 0: none)
-template <int TIE>
-__device__ __forceinline__ void sw_pair(const KParams &kp, int R, uint64_t a1, uint64_t b1, uint64_t t0,
+template <int TIE, bool TAG>
+__device__ __forceinline__ void sw_pair(const KParams &kp, const TagArgs &ta, int R, uint64_t a1, uint64_t b1, uint64_t t0,
                                         const uint64_t *doff, uint64_t base, uint8_t *arena,
                                         const int *ssm, uint2 *prof, int *dsc)
 {
@@ -493,7 +542,7 @@ __device__ __forceinline__ void sw_pair(const KParams &kp, int R, uint64_t a1, u
         if (!pair_seqs(kp, pr, V, m, Hs, n)) m = n = 0;
         off = doff[t] - base;
     }
-    const DirOut d = dp_dispatch_pair<TIE, true>(kp, R, V, m, Hs, n, ssm, prof, (uint32_t *)(arena + off));
+    const DirOut d = dp_dispatch_pair<TIE, true, TAG>(kp, ta, R, V, m, Hs, n, ssm, prof, (uint32_t *)(arena + off));
     if ((lane & 15) == 0 && m > 0) {
         int4 *o = reinterpret_cast<int4 *>(dsc) + p;
         *o = make_int4(d.score, d.ei, d.ej, d.have);
@@ -501,18 +550,19 @@ __device__ __forceinline__ void sw_pair(const KParams &kp, int R, uint64_t a1, u
 }
 
 // local DP of the tasks [t0, t1); dsc[4p ..] = score, end row, end column,
-// have | 2 if a checked 16-bit region was redone on 32-bit lanes.  The
+// have | 2 if a checked 16-bit region was redone on 32-bit lanes, | 4 if the common
+// pass leaves a tagged one to the checked pass.  The
 // half-warp pairs (dir16_paired) run here too, two per warp: a pair waits for
 // a partner of the same rows per lane, and those left without one run alone
 // at the end.  (A pass of their own, as X-drop's k_ga_pair, measured 5 %
 // slower here: sw100k is 10 ms, and a second pass adds a second tail.)
-template <int TIE, bool CHK>
+template <int TIE, bool CHK, bool TAG>
 __global__ void __launch_bounds__(WARPS * 32, 2) k_sw_dir(const KParams kp, uint64_t t0, uint64_t t1,
                                                       const uint64_t *doff, uint8_t *arena, int *dsc)
 {
     __shared__ int ssm[32 * 32];
-    load_sm(ssm, kp.sm);
-    __syncthreads();
+    __shared__ __align__(16) uint32_t tab[TAG ? TAG_TABW : 1];
+    const TagArgs ta = dir_tables<TIE, TAG>(kp, ssm, tab);
     const uint64_t gw = (uint64_t)blockIdx.x * WARPS + (threadIdx.x >> 5);
     void *bnd = (char *)kp.bnd + gw * kp.bnd_bytes;
     uint2 *prof = dir_prof(kp);
@@ -530,23 +580,28 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_sw_dir(const KParams kp, uint
         const uint8_t *V, *Hs;
         int m, n;
         if (!pair_seqs(kp, pr, V, m, Hs, n)) continue;
-        if ((dir16_mode(kp, m, n) == 2) != CHK) continue;   // this pass's pairs only
-        exec += (unsigned long long)m * (unsigned long long)n;
+        // this pass's pairs only
+        const bool tagged = dir16_tagged(kp, m, n);
+        if (CHK ? dir16_mode(kp, m, n) != 2 || (tagged && !(reinterpret_cast<const int4 *>(dsc)[p].w & 4))
+                : dir16_mode(kp, m, n) == 2 && !tagged)
+            continue;
+        if (!CHK || !tagged) exec += (unsigned long long)m * (unsigned long long)n;
         if (!CHK && dir16_paired(kp, m, n)) {
             // half a warp: wait for a partner of the same rows per lane
             const int R = dir16_pair_rows(m);
             const uint64_t w1 = slots.swap(R, u + 1);
-            if (w1) sw_pair<TIE>(kp, R, w1, u + 1, t0, doff, base, arena, ssm, prof, dsc);
+            if (w1) sw_pair<TIE, TAG>(kp, ta, R, w1, u + 1, t0, doff, base, arena, ssm, prof, dsc);
             continue;
         }
         DirOut d;
         d.score = 0; d.ei = 0; d.ej = 0; d.have = 0;
         if (m > 0 && n > 0)
-            d = dp_dispatch_dir<TIE, true, CHK>(kp, V, m, Hs, n, ssm, prof, bnd,
+            d = dp_dispatch_dir<TIE, true, CHK, TAG>(kp, ta, V, m, Hs, n, ssm, prof, bnd,
                                                 (uint32_t *)(arena + (doff[t] - base)));
+        __syncwarp();
         if (lane == 0) {
             int4 *o = reinterpret_cast<int4 *>(dsc) + p;
-            *o = make_int4(d.score, d.ei, d.ej, d.have | (d.sat << 1));
+            *o = make_int4(d.score, d.ei, d.ej, d.have | (d.sat << (!CHK && tagged ? 2 : 1)));
         }
     }
     if (!CHK && kp.dir16_pair) {
@@ -554,7 +609,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_sw_dir(const KParams kp, uint
 #pragma unroll 1
         for (int R = 1; R <= 8; ++R) {
             const uint64_t w1 = __shfl_sync(FULL, slots.pend, R);
-            if (w1) sw_pair<TIE>(kp, R, w1, 0, t0, doff, base, arena, ssm, prof, dsc);
+            if (w1) sw_pair<TIE, TAG>(kp, ta, R, w1, 0, t0, doff, base, arena, ssm, prof, dsc);
         }
     }
     if (lane == 0 && exec) atomicAdd(kp.exec_cells + 1, exec);

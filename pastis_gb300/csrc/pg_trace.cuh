@@ -34,7 +34,7 @@ struct TraceOut {
 };
 
 // A walker over one region.  W16: the nibbles of dp_warp_dir16 or
-// dp_pair_dir16 (bit 0: not the diagonal, bit 1: E rather than F; a local walk
+// dp_pair_dir16 (bit 1: not the diagonal, bit 0: E rather than F; a local walk
 // carries the score of the cell it stands on, h, and stops where it is 0).
 // Otherwise the nibbles of dp_warp_dir (bits 0-1: diagonal, F, E or the local
 // floor).  Words: (s * (n + vl - 1) + k) * vl + v for stripe s, wavefront step
@@ -107,8 +107,8 @@ struct Walker {
         if (state == 0) {
             bool diag;
             if (W16) {
-                diag = !(nib & 1u);
-                if (!diag) state = (nib & 2u) ? 2 : 1;
+                diag = !(nib & 2u);
+                if (!diag) state = (nib & 1u) ? 2 : 1;
             } else {
                 const uint32_t hs = nib & 3u;
                 if (hs == DIR_ZERO) { done = true; return false; }
