@@ -645,7 +645,7 @@ static int run_dir(pg_ctx *c, const pg::KParams &kp, uint64_t n, int grid, cudaS
         CU(cudaMemsetAsync(c->d_counter + 3, 0, sizeof(unsigned int), st));
         const uint64_t nt = t1 - t0;
         const int g = (int)std::min<uint64_t>((uint64_t)grid, (nt + pg::WARPS - 1) / pg::WARPS);
-        const int gt = (int)std::min<uint64_t>((uint64_t)c->nsm * 8, (nt + 255) / 256);
+        const int gt = (int)std::min<uint64_t>((uint64_t)c->nsm * 8, ((pg::dir_walk_warps(kp, nt) ? 32 : 1) * nt + 255) / 256);
         launches += pg::dir_run(xdrop, tie, kp, t0, t1, c->d_doff, c->d_dir, c->d_dsc, g, dyn, gt, nchk > 0, st);
         CU(cudaGetLastError());
         t0 = t1;

@@ -20,6 +20,17 @@ void dir_sizes(bool xdrop, const KParams &kp, uint64_t *bytes, unsigned long lon
 // *t1 = end of the arena chunk that starts at task t0
 void dir_chunk_end(const uint64_t *doff, uint64_t t0, uint64_t n, uint64_t budget, uint64_t *t1,
                    cudaStream_t st);
+// A chunk's traceback takes a warp per task (trace_walk_warp) rather than a thread
+// while the chunk has few enough tasks that a walk's waits decide: a warp takes about
+// twice a thread's share of the issue slots, but a run of moves a turn.  Whole calls
+// with gaps of -11 / -2, thread / warp, us: X-drop 1750 / 1097 at 300 pairs, 7807 /
+// 6416 at 20k, 20627 / 19769 at 80k, 69759 / 70014 at 300k; Smith-Waterman 537 / 287,
+// 2383 / 1872, 5067 / 4780, 16864 / 17135.
+constexpr uint64_t DIR_WALK_WARPS = 1u << 17;
+__host__ __forceinline__ bool dir_walk_warps(const KParams &kp, uint64_t tasks)
+{
+    return kp.dir16_lim > 0 && tasks <= DIR_WALK_WARPS;
+}
 // DP of the tasks [t0, t1) (grid blocks, dyn bytes of dynamic shared memory),
 // with kp.dir16_pair (X-drop) a pass over their half-warp regions (SW runs
 // them in its common pass), with chk a pass over

@@ -67,7 +67,8 @@ int dir_run_ga(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint6
         dp_ga<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
         ++launches;
     }
-    k_tb_ga<<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);
+    if (dir_walk_warps(kp, t1 - t0)) k_tb_ga<true><<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);
+    else k_tb_ga<false><<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);
     return launches;
 }
 

@@ -5,7 +5,7 @@
 // regions of up to 256 rows run two per warp in dp_pair_dir16 (X-drop: in
 // k_ga_pair, SW: inside k_sw_dir).  With kernel parameter TAG the 16-bit regions
 // run dp_tag16 instead (pg_dptag.cuh).  k_tb_ga / k_tb_sw trace them back (one
-// thread per pair, pg_trace.cuh) and write the same pg_result records k_ga /
+// thread or warp per pair, pg_trace.cuh) and write the same pg_result records k_ga /
 // k_sw write.  A batch whose direction matrices exceed the arena runs in
 // chunks of consecutive tasks (bucket order), each chunk DP then traceback.
 #pragma once
@@ -417,11 +417,12 @@ __device__ __forceinline__ void walk_both(const KParams &kp, const uint32_t *con
     tr[1] = b.out();
 }
 
-// traceback and result of the tasks [t0, t1), one thread per task: the same
-// record k_ga writes.  Five resident blocks per SM (48 registers, a few
+// traceback and result of the tasks [t0, t1), a thread or (WARP) a warp per task
+// (dir_walk_warps): the same record k_ga writes.  By threads:  Five resident blocks per SM (48 registers, a few
 // spilled) measured 1 % faster than four: the walks wait on memory, so more
 // of them in flight count for more than the spills.
-static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint64_t t0, uint64_t t1,
+template <bool WARP>
+__global__ void __launch_bounds__(256, WARP ? 4 : 5) k_tb_ga(const KParams kp, uint64_t t0, uint64_t t1,
                                                const uint64_t *doff, const uint8_t *arena,
                                                const int *dsc)
 {
@@ -430,8 +431,10 @@ static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint6
     __syncthreads();
     const uint64_t base = doff[t0];
     const int gmax = kp.go > kp.ge ? kp.go : kp.ge;
-    for (uint64_t t = t0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < t1;
-         t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t sh = WARP ? 5 : 0;
+    const bool writes = !WARP || (threadIdx.x & 31) == 0;
+    for (uint64_t t = t0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> sh); t < t1;
+         t += ((uint64_t)gridDim.x * blockDim.x) >> sh) {
         const uint64_t p = kp.order ? (uint64_t)kp.order[t] : t;
         if (p >= kp.n) { atomicOr(kp.status, ST_BAD_SCHED); continue; }
         const pg_pair pr = kp.pairs[p];
@@ -440,7 +443,7 @@ static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint6
         pg_result best = empty_result();
         if (!pair_seqs(kp, pr, Vs, m, Hss, n)) {
             atomicOr(kp.status, ST_BAD_INDEX);
-            kp.out[p] = best;
+            if (writes) kp.out[p] = best;
             continue;
         }
         const SeedPlan sp = seed_plan(kp, p);
@@ -481,7 +484,19 @@ static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint6
             }
         }
         TraceOut tr[2];
-        if (w16[0] && w16[1]) walk_both<true, true>(kp, dm, rm, rn, V, Hs, ssm, act, tr);
+        if (WARP) {
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                tr[s] = TraceOut{0, 0, 0, 0, 0};
+                if (!act[s]) continue;
+                int R, vl;
+                region_layout(kp, rm[s], rn[s], w16[s], R, vl);
+                tr[s] = w16[s] ? trace_walk_warp<false>(dm[s], rn[s], R, vl, rm[s], rn[s], V[s], Hs[s], ssm,
+                                                        kp.go, kp.ge, 0)
+                               : trace_walk<false, false>(dm[s], rn[s], R, vl, rm[s], rn[s], V[s], Hs[s], ssm,
+                                                          kp.go, kp.ge, 0);
+            }
+        } else if (w16[0] && w16[1]) walk_both<true, true>(kp, dm, rm, rn, V, Hs, ssm, act, tr);
         else if (w16[0]) walk_both<true, false>(kp, dm, rm, rn, V, Hs, ssm, act, tr);
         else if (w16[1]) walk_both<false, true>(kp, dm, rm, rn, V, Hs, ssm, act, tr);
         else walk_both<false, false>(kp, dm, rm, rn, V, Hs, ssm, act, tr);
@@ -519,7 +534,7 @@ static __global__ void __launch_bounds__(256, 5) k_tb_ga(const KParams kp, uint6
         best.cells = sat_u32(cells);
         if (bad) best.flags |= PG_RF_BAD_SEED;
         apply_filter(best, m, n, kp.cov_thr, kp.ani_thr);
-        kp.out[p] = best;
+        if (writes) kp.out[p] = best;
     }
 }
 
@@ -615,9 +630,10 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_sw_dir(const KParams kp, uint
     if (lane == 0 && exec) atomicAdd(kp.exec_cells + 1, exec);
 }
 
-// traceback and result of the tasks [t0, t1), one thread per task: the same
-// record k_sw writes
-static __global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t t0, uint64_t t1,
+// traceback and result of the tasks [t0, t1), a thread or (WARP) a warp per task:
+// the same record k_sw writes
+template <bool WARP>
+__global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t t0, uint64_t t1,
                                                const uint64_t *doff, const uint8_t *arena,
                                                const int *dsc)
 {
@@ -625,8 +641,10 @@ static __global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t
     load_sm(ssm, kp.sm);
     __syncthreads();
     const uint64_t base = doff[t0];
-    for (uint64_t t = t0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < t1;
-         t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t sh = WARP ? 5 : 0;
+    const bool writes = !WARP || (threadIdx.x & 31) == 0;
+    for (uint64_t t = t0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> sh); t < t1;
+         t += ((uint64_t)gridDim.x * blockDim.x) >> sh) {
         const uint64_t p = kp.order ? (uint64_t)kp.order[t] : t;
         if (p >= kp.n) { atomicOr(kp.status, ST_BAD_SCHED); continue; }
         const pg_pair pr = kp.pairs[p];
@@ -635,7 +653,7 @@ static __global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t
         pg_result o = empty_result();
         if (!pair_seqs(kp, pr, V, m, Hs, n)) {
             atomicOr(kp.status, ST_BAD_INDEX);
-            kp.out[p] = o;
+            if (writes) kp.out[p] = o;
             continue;
         }
         o.cells = sat_u32((uint64_t)m * (uint64_t)n);
@@ -645,7 +663,8 @@ static __global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t
             const bool w16 = region16(kp, m, n, d.w >> 1);
             int R, vl;
             region_layout(kp, m, n, w16, R, vl);
-            const TraceOut tr = w16 ? trace_walk<true, true>(dm, n, R, vl, d.y, d.z, V, Hs, ssm, kp.go, kp.ge, d.x)
+            const TraceOut tr = w16 && WARP ? trace_walk_warp<true>(dm, n, R, vl, d.y, d.z, V, Hs, ssm, kp.go, kp.ge, d.x)
+                                : w16 ? trace_walk<true, true>(dm, n, R, vl, d.y, d.z, V, Hs, ssm, kp.go, kp.ge, d.x)
                                     : trace_walk<true, false>(dm, n, R, vl, d.y, d.z, V, Hs, ssm, kp.go, kp.ge, d.x);
             const uint32_t L = (uint32_t)((d.y - tr.i0) + (d.z - tr.j0)) - tr.D;
             o.score = d.x;
@@ -655,7 +674,7 @@ static __global__ void __launch_bounds__(256) k_tb_sw(const KParams kp, uint64_t
             if (L > 0) { o.identity = identity_of(tr.M, L); o.flags = 0; }
         }
         apply_filter(o, m, n, kp.cov_thr, kp.ani_thr);
-        kp.out[p] = o;
+        if (writes) kp.out[p] = o;
     }
 }
 

@@ -13,12 +13,11 @@
 // column 0 finishes along it in one gap run; a local alignment stops there,
 // or at a cell whose H fell to 0, and starts at that cell.
 //
-// One thread walks one region, one 4-byte direction word per step (the
-// words sit in HBM: the DP of a whole chunk writes them first).  Two
-// read-ahead schemes measured slower and were dropped: a per-thread tile of
-// 8 steps x 4 lanes (a refill somewhere in the warp at nearly every step,
-// and 8 sectors read per refill), and one warp per region reading 32-step x
-// 8-lane tiles through shuffles (a 32nd of the walks in flight).
+// In large batches one thread walks one region, one 4-byte direction word per
+// step (the words sit in HBM: the DP of a whole chunk writes them first); a
+// per-thread tile of 8 steps x 4 lanes measured slower there (a refill somewhere
+// in the warp at nearly every step, and 8 sectors read per refill).  Smaller
+// batches take a warp per region (trace_walk_warp).
 #pragma once
 #include <cstdint>
 
@@ -157,6 +156,94 @@ __device__ __forceinline__ TraceOut trace_walk(const uint32_t *dir, int n, int R
     Walker<LOCAL, W16> w(dir, n, R, vl, i, j, V, Hs, ssm, go, ge, h);
     while (w.step()) {}
     return w.out();
+}
+
+// The same walk of a 16-bit region by a warp (all lanes pass the same region and
+// get the same result): 32 cells of the diagonal, the row or the column ahead are
+// read at once and a run of moves is taken in one turn, so that the walk waits on
+// memory once a run and not at every other move.  A turn is about 100 instructions
+// and takes the whole run up to 32 moves.
+template <bool LOCAL>
+__device__ __forceinline__ TraceOut trace_walk_warp(const uint32_t *dir, int n, int R, int vl, int i, int j,
+                                                    const uint8_t *V, const uint8_t *Hs, const int *ssm,
+                                                    int go, int ge, int h)
+{
+    const int lane = threadIdx.x & 31;
+    const int vsh = vl == 32 ? 5 : 6;
+    TraceOut o{0, 0, 0, 0, 0};
+    int state = 0, last = 0;                       // as in Walker
+    auto nibble = [&](int ci, int cj) -> uint32_t {
+        const unsigned va = (unsigned)(ci - 1) / (unsigned)R;
+        const int r = ci - 1 - (int)va * R, s = (int)(va >> vsh), v = (int)(va & (unsigned)(vl - 1));
+        const uint64_t w = vl == 32 ? dir16_pair_word(cj - 1 + v, v) : dir16_warp_word(s, cj - 1 + v, v, n);
+        return (__ldg(dir + w) >> (4 * r)) & 15u;
+    };
+    for (;;) {
+        if (i == 0 || j == 0) {
+            if (!LOCAL) {
+                if (i > 0 && last != 1) ++o.G;
+                else if (j > 0 && last != 2) ++o.G;
+            }
+            break;
+        }
+        if (state == 0) {
+            if (LOCAL && h == 0) break;
+            const int ci = i - lane, cj = j - lane;
+            const bool in = ci >= 1 && cj >= 1;
+            uint32_t nib = 2u;
+            int a = 0, b = 0;
+            if (in) {
+                nib = nibble(ci, cj);
+                a = __ldg(V + ci - 1);
+                b = __ldg(Hs + cj - 1);
+            }
+            bool stop = (nib & 2u) != 0;
+            int sum = 0;                           // of the scores up to this lane's cell
+            if (LOCAL) {
+                const int sc = in ? ssm[a * 32 + b] : 0;
+                sum = sc;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(FULL, sum, d);
+                    if (lane >= d) sum += y;
+                }
+                stop = stop || h == sum - sc;
+            }
+            const unsigned bm = __ballot_sync(FULL, stop);
+            const int len = bm ? __ffs((int)bm) - 1 : 32;
+            const unsigned run = len == 32 ? FULL : (1u << len) - 1u;
+            o.D += (uint32_t)len;
+            o.M += (uint32_t)__popc(__ballot_sync(FULL, in && a == b) & run);
+            if (len > 0) {
+                last = 0;
+                if (LOCAL) h -= __shfl_sync(FULL, sum, len - 1);
+                i -= len;
+                j -= len;
+            }
+            if (len < 32) {
+                // the cell that ended the run (h and the borders: at the next turn)
+                const uint32_t w = __shfl_sync(FULL, nib, len);
+                if (i > 0 && j > 0 && (w & 2u) && !(LOCAL && h == 0)) state = (w & 1u) ? 2 : 1;
+            }
+        } else {
+            // a gap run up to the cell it was opened at
+            const bool up = state == 1;
+            const int ci = up ? i - lane : i, cj = up ? j : j - lane;
+            const bool in = ci >= 1 && cj >= 1;
+            const bool opened = in && (nibble(ci, cj) & (up ? DIR_FOPEN : DIR_EOPEN)) != 0;
+            const unsigned bm = __ballot_sync(FULL, opened);
+            const int len = bm ? __ffs((int)bm) : min(32, up ? i : j);
+            if (last != state) ++o.G;
+            last = state;
+            if (LOCAL) h -= bm ? (len - 1) * ge + go : len * ge;
+            if (up) i -= len;
+            else j -= len;
+            if (bm) state = 0;
+        }
+    }
+    o.i0 = i;
+    o.j0 = j;
+    return o;
 }
 
 }  // namespace pg

@@ -57,3 +57,42 @@ def test_tagged_edges(native, oracle_mod, mode, tie, first, further, table):
         ctx.set_tuning(dp_traceback=form, rows_max=rows, dir_arena_mb=mb)
         assert_same(ctx.align(pairs), exp, pairs)
     ctx.close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("batch", [131072, 131073])
+def test_walks_by_warp_and_by_thread(native, oracle_mod, mode, batch):
+    """Either side of the batch size from which the tracebacks take a thread per pair
+    in place of a warp."""
+    from pastis_gb300 import capi
+    O = oracle_mod
+    rng = np.random.default_rng(47)
+    alpha = np.frombuffer(b"ACDEFGHIKLMNPQRSTVWY", dtype=np.uint8)
+    root = rng.integers(0, 20, 80)
+    seqs = []
+    for L in [1, 2, 9, 31, 32, 33, 40, 57, 64, 65, 70] * 2:
+        s = root[:L].copy()
+        mut = rng.random(L) < 0.25
+        s[mut] = rng.integers(0, 20, int(mut.sum()))
+        cut = int(rng.integers(0, max(1, L // 2)))        # a gap
+        seqs.append(alpha[np.delete(s, slice(cut, cut + L // 8))].tobytes().decode())
+    w = _toy(seqs)
+    pairs = np.zeros(121, dtype=O.PAIR_DTYPE)
+    pairs["row"] = np.repeat(np.arange(11), 11)
+    pairs["col"] = 11 + np.tile(np.arange(11), 11)
+    pairs["count"] = 1
+    cfg = capi.config(mode, gap_semantics=capi.GAPS_NOMINAL)
+    if mode == capi.MODE_XDROP:
+        cfg.xdrop = 500
+    go, ge, xg = capi.resolved_gaps(cfg)
+    p = O.make_params(gap_first=go, gap_ext=ge, xdrop_gap=xg, xdrop=cfg.xdrop, seed_len=cfg.seed_len,
+                      seed_count=cfg.seed_count, tie=cfg.tie, flags=cfg.flags, cov_thr=cfg.cov_thr,
+                      ani_thr=cfg.ani_thr, sm=O.blosum62())
+    codes = O.encode(bytes(w.ascii))
+    exp = O.batch(mode, codes, w.offs, codes, w.offs, pairs, p)
+    at = np.arange(batch) % len(pairs)
+    ctx = capi.Context(cfg)
+    ctx.set_seqs(0, w.ascii, w.offs)
+    ctx.share_row_seqs()
+    assert_same(ctx.align(pairs[at]), exp[at], pairs[at])
+    ctx.close()
