@@ -274,14 +274,22 @@ __device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c,
             lo[r] = 0; ln[r] = 0;
             if (q < nk) { lo[r] = __ldg(A.first + o + q); ln[r] = __ldg(A.len + o + q); }
         }
-#pragma unroll
+        // (not unrolled: with three copies of the visits four of eighteen stall cycles an
+        // issue were waits for instructions, 0.3 so; reading the rows of two or three
+        // groups of pairs together was slower, 11.2 and 13.7 ms a call against 11.1)
+#pragma unroll 1
         for (int r = 0; r < CQ; ++r) {
             // the warp's runs end to end, a lane per occurrence pair (a lane per run left
             // 3 of 32 lanes busy: a family's k-mer has tens of rows, a chance one one or
             // two); runs of more than CRUN rows one at a time
             const int q = q0 + r * (int)blockDim.x + (int)threadIdx.x;
-            const bool big = ln[r] > CRUN;
-            const uint32_t n = big ? 0u : ln[r];
+            I lor = lo[0];
+            uint32_t lnr = ln[0];
+#pragma unroll
+            for (int x = 1; x < CQ; ++x)
+                if (r == x) { lor = lo[x]; lnr = ln[x]; }
+            const bool big = lnr > CRUN;
+            const uint32_t n = big ? 0u : lnr;
             uint32_t inc = n;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -289,7 +297,7 @@ __device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c,
                 if (lane >= d) inc += y;
             }
             const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
-            const I l0 = lo[r] - (I)(inc - n);     // run start less the pairs before it
+            const I l0 = lor - (I)(inc - n);     // run start less the pairs before it
             for (uint32_t i0 = 0; i0 < all; i0 += 32) {
                 const uint32_t i = i0 + lane;
                 int src = 0;                       // the lane whose run holds pair i
@@ -302,8 +310,8 @@ __device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c,
             }
             for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
                 const int src = __ffs(m) - 1;
-                const I l = __shfl_sync(0xffffffffu, lo[r], src);
-                const uint32_t u = __shfl_sync(0xffffffffu, ln[r], src);
+                const I l = __shfl_sync(0xffffffffu, lor, src);
+                const uint32_t u = __shfl_sync(0xffffffffu, lnr, src);
                 for (uint32_t j = 0; j < u; j += 32) one(j + lane < u, (uint64_t)l + j + lane, q - lane + src);
             }
         }
@@ -362,22 +370,26 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
     __shared__ int sscore[CSURV], cost[32];
     __shared__ uint8_t map[32];
     __shared__ uint32_t ndist, nsurv, nkeep, nlist, over;
-    __shared__ unsigned long long base;
+    __shared__ unsigned long long base, next;
     static_assert(CSLOT == 2048, "11 bits of a list word");
     const int t = threadIdx.x;
     if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
-    if (t == 0) ndist = 0;
+    if (t == 0) { ndist = 0; next = atomicAdd(&A.tot[3], 1ull); }
     for (int k = t; k < CSLOT; k += CT) { key[k] = CEMPTY; num[k] = 0; }
     unsigned long long products = 0;
     for (;;) {
-        // the next column: one counter for all blocks, columns differ in length
-        if (t == 0) base = atomicAdd(&A.tot[3], 1ull);
+        // the next column: one counter for all blocks, columns differ in length.  The
+        // one after it is taken below, so that no column waits for the counter
+        // (with the rounds of cand_visit not unrolled 6.50 -> 6.35 ms for 200k proteins)
         __syncthreads();
-        const uint64_t c = base;
+        const uint64_t c = next;
         if (c >= A.ncols) break;
         for (uint32_t x = t; x < ndist; x += CT) { key[used[x]] = CEMPTY; num[used[x]] = 0; }
         __syncthreads();
-        if (t == 0) { ndist = 0; nsurv = 0; nkeep = 0; nlist = 0; over = 0; }
+        if (t == 0) {
+            ndist = 0; nsurv = 0; nkeep = 0; nlist = 0; over = 0; base = 0;
+            next = atomicAdd(&A.tot[3], 1ull);
+        }
         __syncthreads();
         products += cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
             // a full table is left alone (its column goes the dense way): one lane's
