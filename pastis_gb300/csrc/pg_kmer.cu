@@ -179,15 +179,18 @@ __global__ void __launch_bounds__(256) k_runs_write(const uint32_t *h, const uin
 
 // the run of each column k-mer on the row side (length 0: none), in the order of
 // the columns; a warp per column, lanes across positions.  own: the columns are the
-// rows and a k-mer of its own sequence alone makes no pair.
+// rows and a k-mer of its own sequence alone makes no pair.  nu: the distinct values;
+// bound: the sum of the lengths, the block's occurrence pairs before the prune.
 template <class I>
 __global__ void k_col_runs(const uint8_t *seq, const uint64_t *offs, uint64_t s0, uint64_t ns, int stride,
                            const uint64_t *kstart, KmerTab tab, const I *table, int shift, const KmerRun<I> *run,
-                           uint64_t nu, bool own, I *first, uint32_t *len)
+                           const uint64_t *nu_, bool own, I *first, I *len, unsigned long long *bound)
 {
     __shared__ uint8_t map[32];
     if (threadIdx.x < 32) map[threadIdx.x] = tab.map[threadIdx.x];
     __syncthreads();
+    const uint64_t nu = *nu_;
+    unsigned long long sum = 0;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -209,9 +212,71 @@ __global__ void k_col_runs(const uint8_t *seq, const uint64_t *offs, uint64_t s0
             }
             if (own && hi - lo == 1) hi = lo;
             first[o + q] = lo;
-            len[o + q] = (uint32_t)(hi - lo);
+            len[o + q] = hi - lo;
+            sum += hi - lo;
         }
     }
+    __syncwarp();
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0 && sum) atomicAdd(bound, sum);
+}
+
+// first index of run [lo, hi) whose row is r or more (rows ascend within a run: the
+// occurrences were written by sequence and the sort is stable)
+template <class I>
+__device__ __forceinline__ I run_split(const uint32_t *rrow, I lo, I hi, uint64_t r)
+{
+    while (lo < hi) {
+        const I mid = lo + ((hi - lo) >> 1);
+        if (__ldg(rrow + mid) < r) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// 1 for the occurrences of odd rows (counted from the set's first), and a 0 at the end
+template <class I>
+__global__ void k_odd_rows(const uint32_t *rrow, uint64_t n, uint64_t row_begin, I *odd)
+{
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (uint64_t)gridDim.x * blockDim.x)
+        odd[i] = i < n ? (I)((rrow[i] + row_begin) & 1) : (I)0;
+}
+
+// The block's occurrence pairs after the prune, without a visit to each: from where
+// the column stands in each of its runs and, for the even/odd prune, the odd rows
+// before every occurrence (before: their exclusive prefix sum).  A block of a few
+// hundred low-complexity sequences has 1e11 pairs, which must be refused and not
+// walked.  The upper prune keeps the front of a run, which becomes its length.
+template <class I>
+__global__ void k_pairs_count(uint64_t col_begin, uint64_t ns, uint64_t row_begin, int prune, const uint64_t *kstart,
+                              const uint32_t *rrow, const I *before, const I *first, I *len, unsigned long long *tot)
+{
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    unsigned long long sum = 0;
+    for (uint64_t c = warp; c < ns; c += nwarps) {
+        const uint64_t gc = c + col_begin, o = kstart[c];
+        const uint64_t at = gc > row_begin ? gc - row_begin : 0;       // the row below which r < c
+        for (uint64_t x = o + lane; x < kstart[c + 1]; x += 32) {
+            const I lo = first[x], hi = lo + len[x];
+            if (lo == hi) continue;
+            const I s = run_split(rrow, lo, hi, at);
+            if (prune == PG_PRUNE_UPPER) {
+                len[x] = s - lo;
+                sum += s - lo;
+            } else {
+                // odd rows below and even ones above an even column, the others about an odd one
+                const I e = gc >= row_begin ? run_split(rrow, s, hi, at + 1) : s;
+                const uint64_t below = before[s] - before[lo], above = before[hi] - before[e];
+                sum += gc & 1 ? (uint64_t)(s - lo) - below + above : below + (uint64_t)(hi - e) - above;
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (lane == 0 && sum) atomicAdd(tot, sum);
 }
 
 constexpr int CT = 128;              // threads per column block
@@ -235,39 +300,35 @@ struct CandArgs {
     const uint16_t *rpos;
     const uint64_t *kstart;          // first k-mer of each column, and of its k-mers:
     const I *first;                  // first row occurrence,
-    const uint32_t *len;             // their number
+    const I *len;                    // their number
     pg_pair *tmp;                    // records in any column order, tmp_cap of them
     uint64_t tmp_cap;
     uint64_t *start;                 // per column: its records in tmp, their number
     uint32_t *cnt;
-    unsigned long long *tot;         // [0] products, [1] records, [2] overflowed columns, [3] next column
+    unsigned long long *tot;         // [0] pairs before the prune, or after it (k_pairs_count),
+                                     // [1] records, [2] overflowed columns, [3] next column
     uint32_t *ovf;                   // overflowed columns
 };
 
 // Visits every occurrence pair of column c that survives the prune, in no order:
 // visit(valid, row, row occurrence j, k-mer number), called by whole warps (the
 // lanes without a pair pass valid = false).  The block's threads take the column's
-// k-mers, CQ each at a time, their reads in flight together.  Returns this thread's
-// number of pairs.
+// k-mers, CQ each at a time, their reads in flight together.
 constexpr int CQ = 3;
 template <class I, class F>
-__device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c, F visit)
+__device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F visit)
 {
     const uint64_t o = A.kstart[c];
     const int nk = (int)(A.kstart[c + 1] - o);
     const int lane = threadIdx.x & 31;
     const uint64_t gc = c + A.col_begin;
-    uint64_t np = 0;
     auto one = [&](bool in, uint64_t j, int q) {
         const uint32_t r = in ? __ldg(A.rrow + j) : 0u;
-        const bool valid = in && keep_pair(A.prune, r + A.row_begin, gc);
-        np += valid ? 1 : 0;
-        visit(valid, r, j, q);
+        visit(in && keep_pair(A.prune, r + A.row_begin, gc), r, j, q);
     };
     for (int q0 = 0; q0 < nk; q0 += (int)blockDim.x * CQ) {
         __syncwarp();
-        I lo[CQ];
-        uint32_t ln[CQ];
+        I lo[CQ], ln[CQ];
 #pragma unroll
         for (int r = 0; r < CQ; ++r) {
             const int q = q0 + r * (int)blockDim.x + (int)threadIdx.x;
@@ -283,13 +344,12 @@ __device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c,
             // 3 of 32 lanes busy: a family's k-mer has tens of rows, a chance one one or
             // two); runs of more than CRUN rows one at a time
             const int q = q0 + r * (int)blockDim.x + (int)threadIdx.x;
-            I lor = lo[0];
-            uint32_t lnr = ln[0];
+            I lor = lo[0], lnr = ln[0];
 #pragma unroll
             for (int x = 1; x < CQ; ++x)
                 if (r == x) { lor = lo[x]; lnr = ln[x]; }
             const bool big = lnr > CRUN;
-            const uint32_t n = big ? 0u : lnr;
+            const uint32_t n = big ? 0u : (uint32_t)lnr;
             uint32_t inc = n;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -310,13 +370,12 @@ __device__ __forceinline__ uint64_t cand_visit(const CandArgs<I> &A, uint64_t c,
             }
             for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
                 const int src = __ffs(m) - 1;
-                const I l = __shfl_sync(0xffffffffu, lor, src);
-                const uint32_t u = __shfl_sync(0xffffffffu, lnr, src);
-                for (uint32_t j = 0; j < u; j += 32) one(j + lane < u, (uint64_t)l + j + lane, q - lane + src);
+                const uint64_t l = __shfl_sync(0xffffffffu, lor, src);
+                const uint64_t u = __shfl_sync(0xffffffffu, lnr, src);
+                for (uint64_t j = 0; j < u; j += 32) one(j + lane < u, l + j + lane, q - lane + src);
             }
         }
     }
-    return np;
 }
 
 // code and self score of the k-mer at p
@@ -376,7 +435,6 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
     if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
     if (t == 0) { ndist = 0; next = atomicAdd(&A.tot[3], 1ull); }
     for (int k = t; k < CSLOT; k += CT) { key[k] = CEMPTY; num[k] = 0; }
-    unsigned long long products = 0;
     for (;;) {
         // the next column: one counter for all blocks, columns differ in length.  The
         // one after it is taken below, so that no column waits for the counter
@@ -391,7 +449,7 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
             next = atomicAdd(&A.tot[3], 1ull);
         }
         __syncthreads();
-        products += cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
+        cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
             // a full table is left alone (its column goes the dense way): one lane's
             // reading decides for the warp, which stays together for the ballots below
             if (__shfl_sync(0xffffffffu, *(volatile uint32_t *)&ndist, 0) >= CROWS) { over = 1; return; }
@@ -480,7 +538,6 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
         }
         if (t == 0) { A.start[c] = base; A.cnt[c] = nkeep; }
     }
-    if (products) atomicAdd(&A.tot[0], products);
 }
 
 // the overflowed columns: a dense array over the rows per block (count, smallest
@@ -618,6 +675,7 @@ struct SideKmers {
     uint32_t *code = nullptr;
     uint64_t *val = nullptr;
     uint64_t *start = nullptr;       // first k-mer of each sequence (one more: n)
+    uint64_t *spare = nullptr;       // n + 1 words that the sort is done with
     uint64_t n = 0;
 };
 
@@ -646,7 +704,7 @@ int side_kmers(Bufs &B, const uint8_t *seq, const uint64_t *offs, uint64_t s0, u
     uint32_t *c0, *c1;
     uint64_t *v0, *v1;
     KCU(B.get(&c0, total)); KCU(B.get(&c1, total));
-    KCU(B.get(&v0, total)); KCU(B.get(&v1, total));
+    KCU(B.get(&v0, total + 1)); KCU(B.get(&v1, total + 1));
     if (total) k_kmer_fill<<<grid, 256, 0, st>>>(seq, offs, s0, ns, kc.stride, start, tab, c0, v0);
     KCU(cudaGetLastError());
     cub::DoubleBuffer<uint32_t> kb(c0, c1);
@@ -658,6 +716,7 @@ int side_kmers(Bufs &B, const uint8_t *seq, const uint64_t *offs, uint64_t s0, u
     KCU(cub::DeviceRadixSort::SortPairs(stmp, sb, kb, vb, (int64_t)total, 0, tab.bits, st));
     out.code = kb.Current();
     out.val = vb.Current();
+    out.spare = vb.Alternate();
     return PG_OK;
 }
 
@@ -685,14 +744,12 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
     void *rtmp;
     KCU(B.get((char **)&rtmp, rb));
     KCU(cub::DeviceScan::ExclusiveSum(rtmp, rb, rcnt, rfirst, (int64_t)(rblocks + 1), st));
-    uint64_t nu = 0;
-    KCU(cudaMemcpyAsync(&nu, rfirst + rblocks, sizeof nu, cudaMemcpyDeviceToHost, st));
-    KCU(cudaStreamSynchronize(st));
     KmerRun<I> *run;
-    uint32_t *rrow, *clen;
+    uint32_t *rrow;
     uint16_t *rpos;
-    I *cfirst;
-    KCU(B.get(&run, nu + 1));
+    I *cfirst, *clen;
+    if (sizeof(KmerRun<I>) <= sizeof *R.spare) run = reinterpret_cast<KmerRun<I> *>(R.spare);
+    else KCU(B.get(&run, std::min<uint64_t>(R.n, pow_u(tab.base, tab.k)) + 1));
     KCU(B.get(&rrow, R.n));
     KCU(B.get(&rpos, R.n));
     KCU(B.get(&cfirst, C.n));
@@ -708,12 +765,39 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
     KCU(B.get(&table, (size_t)1 << tb));
     KCU(cudaMemsetAsync(table, 0xff, sizeof(I) << tb, st));
     k_runs_write<I><<<(unsigned)rblocks, 256, 0, st>>>(R.code, R.val, R.n, rfirst, shift, run, table, rrow, rpos);
+    KCU(B.get(&A.tot, 4));
+    KCU(cudaMemsetAsync(A.tot, 0, sizeof(unsigned long long) * 4, st));
     k_col_runs<I><<<grid, 256, 0, st>>>(cseq, coffs, col_begin, ncols, kc.stride, C.start, tab, table, shift, run,
-                                        nu, same && kc.prune != PG_PRUNE_NONE, cfirst, clen);
+                                        rfirst + rblocks, same && kc.prune != PG_PRUNE_NONE, cfirst, clen, A.tot);
+    KCU(cudaGetLastError());
+    unsigned long long pairs = 0;
+    KCU(cudaMemcpyAsync(&pairs, A.tot, sizeof pairs, cudaMemcpyDeviceToHost, st));
+    KCU(cudaStreamSynchronize(st));
+    if (pairs > maxp && kc.prune != PG_PRUNE_NONE) {
+        // more than the caller allows before the prune: how many after it
+        I *before = nullptr;
+        if (kc.prune == PG_PRUNE_EVEN_ODD) {
+            KCU(B.get(&before, R.n + 1));
+            k_odd_rows<I><<<grid, 256, 0, st>>>(rrow, R.n, row_begin, before);
+            size_t ob = 0;
+            KCU(cub::DeviceScan::ExclusiveSum(nullptr, ob, before, before, (int64_t)(R.n + 1), st));
+            void *otmp;
+            KCU(B.get((char **)&otmp, ob));
+            KCU(cub::DeviceScan::ExclusiveSum(otmp, ob, before, before, (int64_t)(R.n + 1), st));
+        }
+        KCU(cudaMemsetAsync(A.tot, 0, sizeof pairs, st));
+        k_pairs_count<I><<<grid, 256, 0, st>>>(col_begin, ncols, row_begin, kc.prune, C.start, rrow, before, cfirst, clen,
+                                               A.tot);
+        KCU(cudaGetLastError());
+        KCU(cudaMemcpyAsync(&pairs, A.tot, sizeof pairs, cudaMemcpyDeviceToHost, st));
+        KCU(cudaStreamSynchronize(st));
+    }
+    if (pairs > maxp)
+        return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: too many k-mer occurrence pairs for one block");
+    if (!pairs) return PG_OK;
     KCU(B.get(&A.start, ncols));
     KCU(B.get(&A.cnt, ncols + 1));
     KCU(B.get(&A.ovf, ncols));
-    KCU(B.get(&A.tot, 4));
     // records of the call: room for 32 a column at first, or what the caller takes
     A.tmp_cap = std::min<uint64_t>(cap, std::max<uint64_t>((uint64_t)1 << 20, 32 * ncols));
     unsigned long long tot[4] = {0, 0, 0, 0};
@@ -726,8 +810,6 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
         KCU(cudaGetLastError());
         KCU(cudaMemcpyAsync(tot, A.tot, sizeof tot, cudaMemcpyDeviceToHost, st));
         KCU(cudaStreamSynchronize(st));
-        if (tot[0] > maxp)
-            return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: too many k-mer occurrence pairs for one block");
         if (tot[2]) {
             // dense arrays for as many columns at a time as 4 GiB hold
             const uint64_t fit = std::max<uint64_t>(1, ((uint64_t)4 << 30) / (nrows * sizeof(CandDense)));
