@@ -11,16 +11,16 @@
 //   3. a block per column sequence: each of its k-mers finds its run of equal
 //      codes on the row side through the table; the occurrence pairs that survive
 //      the symmetric prune are counted per row in a hash table in shared memory.
-//      The rows whose count passes ckthr (a few: most pairs share one k-mer by
-//      chance) get their first / second seed (smallest / largest seed value) and
+//      The rows whose count passes ckthr (few from ckthr = 1 on: most pairs share one
+//      k-mer by chance) get their first / second seed (smallest / largest seed value) and
 //      score (largest k-mer self score) in a second sweep over the same runs, are
 //      ranked by row and written out.
 //   4. the columns' records are moved into place, column-major.
 // The product of a block is never written out or sorted: for 200k proteins that
 // was 58M 16-byte products through a 7-pass radix sort, a run-length encoding and
-// a reduction, 28.5 ms a call with the allocation of their buffers; 11.3 ms now.  A
-// column with more rows than the hash table holds goes through a dense array over
-// the rows in global memory.
+// a reduction, 28.5 ms a call with the allocation of their buffers; 10.8 ms now (even/odd
+// prune, ckthr = 1).  A column that outgrows the tables of step 3, the usual one without
+// a threshold (ckthr = 0) or from about 500k rows on, goes through k_cand_parts.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -284,6 +284,7 @@ constexpr int CSLOT = 2048;          // hash slots: 6 blocks per SM with their t
 constexpr int CLIST = 896;           // pairs kept for the second sweep
 constexpr int CROWS = 1536;          // distinct rows a block takes (CT inserts may be under way beyond)
 constexpr int CSURV = 320;           // rows that pass ckthr
+constexpr uint32_t CHEAVY = 1u << 17;  // pairs of a column that one block takes
 constexpr uint32_t CRUN = 1024;     // rows of a run that is expanded with its warp's others
 constexpr uint32_t CEMPTY = 0xffffffffu;
 constexpr uint32_t CMARK = 0x80000000u;
@@ -306,14 +307,22 @@ struct CandArgs {
     uint64_t *start;                 // per column: its records in tmp, their number
     uint32_t *cnt;
     unsigned long long *tot;         // [0] pairs before the prune, or after it (k_pairs_count),
-                                     // [1] records, [2] overflowed columns, [3] next column
+                                     // [1] places in tmp, [2] overflowed columns, [3] next column,
+                                     // [4] next part, [5] records
     uint32_t *ovf;                   // overflowed columns
+    // parts of the overflowed columns: column, first row, end row, its column's first part
+    const uint4 *part;
+    uint64_t nparts;
+    uint64_t *pstart;                // per part: its records in tmp, their number
+    uint32_t *pcnt;
 };
+constexpr uint64_t CPARTS = ~0ull;   // start of a column whose records its parts hold
 
 // Visits every occurrence pair of column c that survives the prune, in no order:
 // visit(valid, row, row occurrence j, k-mer number), called by whole warps (the
-// lanes without a pair pass valid = false).  The block's threads take the column's
-// k-mers, CQ each at a time, their reads in flight together.
+// lanes without a pair pass valid = false); false, the same in all lanes, ends the
+// warp's visits.  The block's threads take the column's k-mers, CQ each at a time,
+// their reads in flight together.
 constexpr int CQ = 3;
 template <class I, class F>
 __device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F visit)
@@ -324,9 +333,10 @@ __device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F v
     const uint64_t gc = c + A.col_begin;
     auto one = [&](bool in, uint64_t j, int q) {
         const uint32_t r = in ? __ldg(A.rrow + j) : 0u;
-        visit(in && keep_pair(A.prune, r + A.row_begin, gc), r, j, q);
+        return visit(in && keep_pair(A.prune, r + A.row_begin, gc), r, j, q);
     };
-    for (int q0 = 0; q0 < nk; q0 += (int)blockDim.x * CQ) {
+    bool on = true;
+    for (int q0 = 0; q0 < nk && on; q0 += (int)blockDim.x * CQ) {
         __syncwarp();
         I lo[CQ], ln[CQ];
 #pragma unroll
@@ -339,7 +349,7 @@ __device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F v
         // issue were waits for instructions, 0.3 so; reading the rows of two or three
         // groups of pairs together was slower, 11.2 and 13.7 ms a call against 11.1)
 #pragma unroll 1
-        for (int r = 0; r < CQ; ++r) {
+        for (int r = 0; r < CQ && on; ++r) {
             // the warp's runs end to end, a lane per occurrence pair (a lane per run left
             // 3 of 32 lanes busy: a family's k-mer has tens of rows, a chance one one or
             // two); runs of more than CRUN rows one at a time
@@ -358,7 +368,7 @@ __device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F v
             }
             const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
             const I l0 = lor - (I)(inc - n);     // run start less the pairs before it
-            for (uint32_t i0 = 0; i0 < all; i0 += 32) {
+            for (uint32_t i0 = 0; i0 < all && on; i0 += 32) {
                 const uint32_t i = i0 + lane;
                 int src = 0;                       // the lane whose run holds pair i
 #pragma unroll
@@ -366,13 +376,13 @@ __device__ __forceinline__ void cand_visit(const CandArgs<I> &A, uint64_t c, F v
                     if (__shfl_sync(0xffffffffu, inc, src + d - 1) <= i) src += d;
                 src = min(src, 31);
                 const I l = __shfl_sync(0xffffffffu, l0, src);
-                one(i < all, (uint64_t)(I)(l + (I)i), q - lane + src);
+                on = one(i < all, (uint64_t)(I)(l + (I)i), q - lane + src);
             }
-            for (uint32_t m = __ballot_sync(0xffffffffu, big); m; m &= m - 1) {
+            for (uint32_t m = __ballot_sync(0xffffffffu, big); m && on; m &= m - 1) {
                 const int src = __ffs(m) - 1;
                 const uint64_t l = __shfl_sync(0xffffffffu, lor, src);
                 const uint64_t u = __shfl_sync(0xffffffffu, lnr, src);
-                for (uint64_t j = 0; j < u; j += 32) one(j + lane < u, l + j + lane, q - lane + src);
+                for (uint64_t j = 0; j < u && on; j += 32) on = one(j + lane < u, l + j + lane, q - lane + src);
             }
         }
     }
@@ -432,6 +442,8 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
     __shared__ unsigned long long base, next;
     static_assert(CSLOT == 2048, "11 bits of a list word");
     const int t = threadIdx.x;
+    // without a threshold every row survives, so that more than CSURV are too many
+    const uint32_t limit = A.ckthr <= 0 ? CSURV + 1 : CROWS;
     if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
     if (t == 0) { ndist = 0; next = atomicAdd(&A.tot[3], 1ull); }
     for (int k = t; k < CSLOT; k += CT) { key[k] = CEMPTY; num[k] = 0; }
@@ -450,9 +462,9 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
         }
         __syncthreads();
         cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
-            // a full table is left alone (its column goes the dense way): one lane's
-            // reading decides for the warp, which stays together for the ballots below
-            if (__shfl_sync(0xffffffffu, *(volatile uint32_t *)&ndist, 0) >= CROWS) { over = 1; return; }
+            // a column that outgrows the block is left to k_cand_parts: one lane's reading
+            // decides for the warp, which stays together for the ballots below
+            if (__shfl_sync(0xffffffffu, *(volatile uint32_t *)&over, 0)) return false;
             uint32_t s = (r * 0x9E3779B1u) >> 21;
             bool fresh = false;
             while (valid) {
@@ -470,11 +482,13 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
             if ((t & 31) == 0) {
                 if (mf) bf = atomicAdd(&ndist, (uint32_t)__popc(mf));
                 if (mv) bv = atomicAdd(&nlist, (uint32_t)__popc(mv));
+                if (bf + (uint32_t)__popc(mf) >= limit || bv >= CHEAVY) over = 1;
             }
             bf = __shfl_sync(0xffffffffu, bf, 0);
             bv = __shfl_sync(0xffffffffu, bv, 0) + (uint32_t)__popc(mv & below);
             if (fresh) used[bf + (uint32_t)__popc(mf & below)] = (uint16_t)s;
             if (valid && bv < CLIST) { list_j[bv] = (I)j; list_qs[bv] = ((uint32_t)q << 11) | s; }
+            return true;
         });
         __syncthreads();
         for (uint32_t x = t; x < ndist && !over; x += CT) {
@@ -493,7 +507,7 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
         }
         __syncthreads();
         if (over || nsurv > CSURV) {
-            if (t == 0) A.ovf[atomicAdd(&A.tot[2], 1ull)] = (uint32_t)c;
+            if (t == 0) { A.ovf[atomicAdd(&A.tot[2], 1ull)] = (uint32_t)c; A.start[c] = CPARTS; }
             continue;
         }
         const uint32_t ns = nsurv;
@@ -514,18 +528,22 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
                 }
             } else {
                 cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
-                    if (!valid) return;
+                    if (!valid) return true;
                     uint32_t s = (r * 0x9E3779B1u) >> 21;
                     while (key[s] != r) s = (s + 1) & (CSLOT - 1);
                     const uint32_t mark = num[s];
                     if (mark & CMARK) update(mark & ~CMARK, j, q);
+                    return true;
                 });
             }
             __syncthreads();
             for (uint32_t u = t; u < ns; u += CT)
                 if (sscore[u] > A.mosthr) atomicAdd(&nkeep, 1u);
             __syncthreads();
-            if (t == 0) base = nkeep ? atomicAdd(&A.tot[1], (unsigned long long)nkeep) : 0;
+            if (t == 0 && nkeep) {
+                base = atomicAdd(&A.tot[1], (unsigned long long)nkeep);
+                atomicAdd(&A.tot[5], (unsigned long long)nkeep);
+            }
             __syncthreads();
             const bool fits = base + nkeep <= A.tmp_cap;
             for (uint32_t u = t; u < ns && fits; u += CT) {
@@ -540,85 +558,297 @@ __global__ void __launch_bounds__(CT, 6) k_cand(const CandArgs<I> A)
     }
 }
 
-// the overflowed columns: a dense array over the rows per block (count, smallest
-// and largest seed value, score), cleared, filled and read out in row order
-struct CandDense {
-    unsigned long long mn, mx;
-    uint32_t len;
-    int score;
-};
-template <class I>
-__global__ void __launch_bounds__(256) k_cand_dense(const CandArgs<I> A, CandDense *dense, uint64_t novf)
+// -------------------------------------------------- columns that outgrow a block
+// A column with more rows than k_cand's table, survivors than its list or pairs than
+// one block should walk is done in parts of the row range.  Rows ascend within a run,
+// so a part is a contiguous piece of each of the column's runs, found by a search, and
+// goes through a table in shared memory that holds the seeds and the score of every
+// row it meets (a part visits its pairs once).  Parts are as many as give about WPART
+// rows and at most WWORK pairs each; a part that meets more than WROWS rows all the
+// same is done again in narrower ones, down to one row.  Against a dense array over
+// all rows of the block, 24 bytes a row to clear and to read twice: 200k proteins
+// without threshold or prune 855 -> 21 ms a call, 800k with ckthr = 1 and the even/odd
+// prune 7450 -> 170 ms (63 and 295 ms when the whole product was sorted).
+constexpr int WT = 256;              // threads of a block
+constexpr int WSLOT = 2048;          // hash slots: 3 blocks per SM
+constexpr int WROWS = 1536;          // distinct rows (WT inserts may be under way beyond)
+constexpr uint64_t WPART = 1000;
+constexpr uint64_t WWORK = 1u << 18;
+constexpr int WB = WT;               // buckets of the row order
+
+// parts of the x-th overflowed column: their number, and (EMIT) themselves from first[x] on
+template <class I, bool EMIT>
+__global__ void __launch_bounds__(256) k_parts(const CandArgs<I> A, uint64_t novf, uint32_t *num, const uint64_t *first,
+                                               uint4 *part)
 {
-    __shared__ int cost[32];
-    __shared__ uint8_t map[32];
-    __shared__ uint32_t wsum[8], total;
-    __shared__ unsigned long long base;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    if (t < 32) { map[t] = A.tab.map[t]; cost[t] = A.tab.cost[t]; }
-    CandDense *D = dense + (uint64_t)blockIdx.x * A.nrows;
-    auto kept = [&](uint64_t r) {
-        return r < A.nrows && D[r].len && cand_count_ok(D[r].len, A.ckthr) && D[r].score > A.mosthr;
-    };
-    for (uint64_t x = blockIdx.x; x < novf; x += gridDim.x) {
-        const uint64_t c = A.ovf[x];
-        for (uint64_t r = t; r < A.nrows; r += blockDim.x) D[r] = CandDense{~0ull, 0ull, 0u, -32768};
-        if (t == 0) total = 0;
-        __syncthreads();
-        const uint8_t *p = A.cseq + A.coffs[A.col_begin + c];
-        cand_visit(A, c, [&](bool valid, uint32_t r, uint64_t j, int q) {
-            if (!valid) return;
-            int sc;
-            const uint32_t code = kmer_at(p + (uint64_t)q * (uint64_t)A.stride, map, cost, A.tab, sc);
-            const uint64_t sv = seed_value(code, __ldg(A.rpos + j), q * A.stride);
-            atomicAdd(&D[r].len, 1u);
-            atomicMin(&D[r].mn, (unsigned long long)sv);
-            atomicMax(&D[r].mx, (unsigned long long)sv);
-            atomicMax(&D[r].score, sc);
-        });
-        __threadfence_block();
-        __syncthreads();
-        uint32_t n = 0;
-        for (uint64_t r = t; r < A.nrows; r += blockDim.x) n += kept(r) ? 1u : 0u;
-        if (n) atomicAdd(&total, n);
-        __syncthreads();
-        if (t == 0) {
-            base = total ? atomicAdd(&A.tot[1], (unsigned long long)total) : 0;
-            A.start[c] = base;
-            A.cnt[c] = total;
+    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    for (uint64_t x = warp; x < novf; x += nwarps) {
+        const uint64_t c = A.ovf[x], gc = c + A.col_begin;
+        // rows that the prune may keep
+        uint64_t nr = A.nrows;
+        if (A.prune == PG_PRUNE_UPPER) nr = min(nr, gc > A.row_begin ? gc - A.row_begin : (uint64_t)0);
+        uint64_t n;
+        if (EMIT) {
+            n = num[x];
+        } else {
+            uint64_t pairs = 0;
+            for (uint64_t q = A.kstart[c] + lane; q < A.kstart[c + 1]; q += 32) pairs += A.len[q];
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, d);
+            if (A.prune == PG_PRUNE_EVEN_ODD) pairs = (pairs + 1) / 2;
+            if (A.prune == PG_PRUNE_UPPER) pairs = (uint64_t)((double)pairs * (double)nr / (double)A.nrows);
+            n = max((min(pairs, nr) + WPART - 1) / WPART, (pairs + WWORK - 1) / WWORK);
+            n = max(min(n, nr), (uint64_t)1);
+            if (lane == 0) num[x] = (uint32_t)n;
         }
+        if (EMIT) {
+            const uint64_t f = first[x];
+            for (uint64_t k = lane; k < n; k += 32)
+                part[f + k] = make_uint4((uint32_t)c, (uint32_t)(nr * k / n), (uint32_t)(nr * (k + 1) / n), (uint32_t)f);
+        }
+    }
+}
+
+struct PartSmem {
+    unsigned long long mn[WSLOT], mx[WSLOT];
+    uint32_t key[WSLOT], num[WSLOT];
+    int score[WSLOT];
+    uint16_t used[WROWS + WT];       // the slots in use, in no order
+    uint16_t place[WROWS + WT];      // their places in their buckets (0xffff: not kept)
+    uint16_t grouped[WROWS + WT];    // the kept ones by bucket
+    uint16_t sorted[WROWS + WT];     // and by row
+    uint32_t hist[WB], bstart[WB + 1], wsum[WB / 32];
+    int cost[32];
+    uint8_t map[32];
+    uint32_t ndist, over;
+    unsigned long long next, base, pairs;
+    uint4 part;
+};
+
+template <class I>
+__global__ void __launch_bounds__(WT, 3) k_cand_parts(const CandArgs<I> A)
+{
+    extern __shared__ __align__(16) unsigned char part_smem[];
+    PartSmem &S = *reinterpret_cast<PartSmem *>(part_smem);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t < 32) { S.map[t] = A.tab.map[t]; S.cost[t] = A.tab.cost[t]; }
+    auto clear = [&](int s) {
+        S.key[s] = CEMPTY; S.num[s] = 0; S.mn[s] = ~0ull; S.mx[s] = 0; S.score[s] = -32768;
+    };
+    auto take = [&]() {              // thread 0
+        S.next = atomicAdd(&A.tot[4], 1ull);
+        if (S.next < A.nparts) S.part = A.part[S.next];
+    };
+    for (int s = t; s < WSLOT; s += WT) clear(s);
+    if (t == 0) { S.ndist = 0; S.over = 0; S.pairs = 0; take(); }
+    __syncthreads();
+    for (;;) {
+        const uint64_t id = S.next;
+        if (id >= A.nparts) break;
+        const uint64_t c = S.part.x, gc = c + A.col_begin;
+        const uint32_t r0 = S.part.y, r1 = S.part.z;
+        const uint64_t o = A.kstart[c];
+        const int nk = (int)(A.kstart[c + 1] - o);
+        const uint8_t *p = A.cseq + A.coffs[gc];
         __syncthreads();
-        const bool fits = base + total <= A.tmp_cap;
-        uint64_t o = base;
-        for (uint64_t r0 = 0; r0 < A.nrows && fits; r0 += blockDim.x) {
-            const uint64_t r = r0 + t;
-            const bool k = kept(r);
-            const uint32_t m = __ballot_sync(0xffffffffu, k);
-            if (lane == 0) wsum[w] = (uint32_t)__popc(m);
+        if (t == 0) take();          // the next part's, early
+        uint32_t kept = 0;           // records of the part so far
+        uint64_t base = 0;
+        bool room = true, whole = true;
+        uint32_t a = r0, width = r1 - r0;
+        while (a < r1) {
+            const uint32_t b = width < r1 - a ? a + width : r1;
+            const bool split = a != 0 || b != A.nrows;
+            // the pairs of rows [a, b)
+            bool on = true;
+            for (int q0 = 0; q0 < nk && on; q0 += WT) {
+                __syncwarp();
+                const int q = q0 + t;
+                I lo = 0, ln = 0;
+                uint32_t code = 0;
+                int sc = 0;
+                if (q < nk) { lo = __ldg(A.first + o + q); ln = __ldg(A.len + o + q); }
+                if (ln && split) {
+                    const I hi = run_split(A.rrow, lo, (I)(lo + ln), (uint64_t)b);
+                    lo = run_split(A.rrow, lo, hi, (uint64_t)a);
+                    ln = hi - lo;
+                }
+                if (ln) code = kmer_at(p + (uint64_t)q * (uint64_t)A.stride, S.map, S.cost, A.tab, sc);
+                // runs end to end, as in cand_visit
+                auto one = [&](bool in, uint64_t j, int src) {
+                    if (__shfl_sync(0xffffffffu, *(volatile uint32_t *)&S.over, 0)) return false;
+                    const uint32_t r = in ? __ldg(A.rrow + j) : 0u;
+                    const bool valid = in && keep_pair(A.prune, r + A.row_begin, gc);
+                    const uint32_t cd = __shfl_sync(0xffffffffu, code, src);
+                    const int s1 = __shfl_sync(0xffffffffu, sc, src);
+                    const int qs = q - lane + src;
+                    uint32_t s = (r * 0x9E3779B1u) >> 21;
+                    bool fresh = false;
+                    while (valid) {
+                        uint32_t k = *(volatile uint32_t *)&S.key[s];
+                        if (k == CEMPTY) { k = atomicCAS(&S.key[s], CEMPTY, r); fresh = k == CEMPTY; }
+                        if (fresh || k == r) break;
+                        s = (s + 1) & (WSLOT - 1);
+                    }
+                    __syncwarp();
+                    if (valid) {
+                        const uint64_t sv = seed_value(cd, __ldg(A.rpos + j), qs * A.stride);
+                        atomicAdd(&S.num[s], 1u);
+                        if (sv < *(volatile unsigned long long *)&S.mn[s]) atomicMin(&S.mn[s], (unsigned long long)sv);
+                        if (sv > *(volatile unsigned long long *)&S.mx[s]) atomicMax(&S.mx[s], (unsigned long long)sv);
+                        if (s1 > *(volatile int *)&S.score[s]) atomicMax(&S.score[s], s1);
+                    }
+                    const uint32_t mf = __ballot_sync(0xffffffffu, fresh);
+                    if (mf) {
+                        uint32_t bf = 0;
+                        if (lane == 0) {
+                            bf = atomicAdd(&S.ndist, (uint32_t)__popc(mf));
+                            if (bf + (uint32_t)__popc(mf) >= WROWS) S.over = 1;
+                        }
+                        bf = __shfl_sync(0xffffffffu, bf, 0);
+                        if (fresh) S.used[bf + (uint32_t)__popc(mf & ((1u << lane) - 1u))] = (uint16_t)s;
+                    }
+                    return true;
+                };
+                const bool big = ln > CRUN;
+                const uint32_t n = big ? 0u : (uint32_t)ln;
+                uint32_t inc = n;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+                    if (lane >= d) inc += y;
+                }
+                const uint32_t all = __shfl_sync(0xffffffffu, inc, 31);
+                const I l0 = lo - (I)(inc - n);
+                for (uint32_t i0 = 0; i0 < all && on; i0 += 32) {
+                    const uint32_t i = i0 + lane;
+                    int src = 0;
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1)
+                        if (__shfl_sync(0xffffffffu, inc, src + d - 1) <= i) src += d;
+                    src = min(src, 31);
+                    const I l = __shfl_sync(0xffffffffu, l0, src);
+                    on = one(i < all, (uint64_t)(I)(l + (I)i), src);
+                }
+                for (uint32_t m = __ballot_sync(0xffffffffu, big); m && on; m &= m - 1) {
+                    const int src = __ffs(m) - 1;
+                    const uint64_t l = __shfl_sync(0xffffffffu, lo, src), u = __shfl_sync(0xffffffffu, ln, src);
+                    for (uint64_t j = 0; j < u && on; j += 32) on = one(j + lane < u, l + j + lane, src);
+                }
+            }
             __syncthreads();
-            uint32_t before = 0, all = 0;
-            for (int i = 0; i < 8; ++i) { before += i < w ? wsum[i] : 0u; all += wsum[i]; }
-            if (k)
-                A.tmp[o + before + (uint32_t)__popc(m & ((1u << lane) - 1u))] =
-                    cand_record((uint32_t)r, c, D[r].len, D[r].mn, D[r].mx, D[r].score);
-            o += all;
+            const uint32_t nd = S.ndist;
+            if (S.over && b - a > 1) {
+                // too many rows: again in narrower ones.  The part's records stay together, in
+                // room for as many as it can have, one to a row and to ckthr + 1 pairs
+                if (whole) {
+                    uint64_t mine = 0;
+                    for (int q = t; q < nk; q += WT) {
+                        const I lo = __ldg(A.first + o + q);
+                        mine += run_split(A.rrow, lo, (I)(lo + __ldg(A.len + o + q)), (uint64_t)b) -
+                                run_split(A.rrow, lo, (I)(lo + __ldg(A.len + o + q)), (uint64_t)a);
+                    }
+                    atomicAdd(&S.pairs, (unsigned long long)mine);
+                    __syncthreads();
+                    const uint64_t most = min((uint64_t)(r1 - r0), (uint64_t)S.pairs / (uint64_t)(max(A.ckthr, 0) + 1));
+                    if (t == 0) S.base = atomicAdd(&A.tot[1], (unsigned long long)most);
+                    __syncthreads();
+                    base = S.base;
+                    room = base + most <= A.tmp_cap;
+                    whole = false;
+                }
+                width = (b - a) / 2;
+            } else {
+                // the rows that stay, ranked by row: grouped by its high bits first
+                const int sh = max(0, 24 - __clz((int)(b - a - 1)));
+                S.hist[t] = 0;
+                __syncthreads();
+                for (uint32_t x = t; x < nd; x += WT) {
+                    const int s = S.used[x];
+                    const bool keep = cand_count_ok(S.num[s], A.ckthr) && S.score[s] > A.mosthr;
+                    S.place[x] = keep ? (uint16_t)atomicAdd(&S.hist[(S.key[s] - a) >> sh], 1u) : (uint16_t)0xffff;
+                }
+                __syncthreads();
+                uint32_t inc = S.hist[t];
+                const uint32_t own = inc;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, d);
+                    if (lane >= d) inc += y;
+                }
+                if (lane == 31) S.wsum[warp] = inc;
+                __syncthreads();
+                for (int k = 0; k < warp; ++k) inc += S.wsum[k];
+                S.bstart[t] = inc - own;
+                if (t == WT - 1) {
+                    S.bstart[WB] = inc;
+                    if (whole) S.base = inc ? atomicAdd(&A.tot[1], (unsigned long long)inc) : 0;
+                }
+                __syncthreads();
+                const uint32_t nkeep = S.bstart[WB];
+                if (whole) { base = S.base; room = base + nkeep <= A.tmp_cap; }
+                for (uint32_t x = t; x < nd; x += WT)
+                    if (S.place[x] != 0xffff) {
+                        const int s = S.used[x];
+                        S.grouped[S.bstart[(S.key[s] - a) >> sh] + S.place[x]] = (uint16_t)s;
+                    }
+                __syncthreads();
+                for (uint32_t x = t; x < nkeep; x += WT) {
+                    const int s = S.grouped[x];
+                    const uint32_t r = S.key[s], g = (r - a) >> sh;
+                    uint32_t rank = S.bstart[g];
+                    for (uint32_t y = S.bstart[g]; y < S.bstart[g + 1]; ++y) rank += S.key[S.grouped[y]] < r ? 1u : 0u;
+                    S.sorted[rank] = (uint16_t)s;
+                }
+                __syncthreads();
+                for (uint32_t x = t; x < nkeep && room; x += WT) {
+                    const int s = S.sorted[x];
+                    A.tmp[base + kept + x] = cand_record(S.key[s], c, S.num[s], S.mn[s], S.mx[s], S.score[s]);
+                }
+                kept += nkeep;
+                a = b;
+            }
             __syncthreads();
+            for (uint32_t x = t; x < nd; x += WT) clear(S.used[x]);
+            if (t == 0) { S.ndist = 0; S.over = 0; S.pairs = 0; }
+            __syncthreads();
+        }
+        if (t == 0) {
+            A.pstart[id] = base;
+            A.pcnt[id] = kept;
+            if (kept) { atomicAdd(&A.cnt[c], kept); atomicAdd(&A.tot[5], (unsigned long long)kept); }
         }
         __syncthreads();
     }
 }
 
-// the columns' records into place, a warp per column, as 32-bit words
-__global__ void k_cand_place(const pg_pair *tmp, const uint64_t *start, const uint32_t *cnt, const uint64_t *pos,
-                             uint64_t ncols, pg_pair *out)
+// the columns' records into place, a warp per column or part (poff: the parts' records
+// before each), as 32-bit words
+template <class I>
+__global__ void k_cand_place(const CandArgs<I> A, const uint64_t *pos, const uint64_t *poff, pg_pair *out)
 {
     constexpr int W = sizeof(pg_pair) / 4;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t c = warp; c < ncols; c += nwarps) {
-        const uint32_t *src = reinterpret_cast<const uint32_t *>(tmp + start[c]);
-        uint32_t *dst = reinterpret_cast<uint32_t *>(out + pos[c]);
-        for (uint64_t k = threadIdx.x & 31; k < (uint64_t)cnt[c] * W; k += 32) dst[k] = src[k];
+    for (uint64_t x = warp; x < A.ncols + A.nparts; x += nwarps) {
+        uint64_t from, to, n;
+        if (x < A.ncols) {
+            from = A.start[x];
+            if (from == CPARTS) continue;
+            to = pos[x];
+            n = A.cnt[x];
+        } else {
+            const uint64_t id = x - A.ncols;
+            const uint4 p = A.part[id];
+            from = A.pstart[id];
+            to = pos[p.x] + poff[id] - poff[p.w];
+            n = A.pcnt[id];
+        }
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(A.tmp + from);
+        uint32_t *dst = reinterpret_cast<uint32_t *>(out + to);
+        for (uint64_t k = threadIdx.x & 31; k < n * W; k += 32) dst[k] = src[k];
     }
 }
 
@@ -765,8 +995,8 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
     KCU(B.get(&table, (size_t)1 << tb));
     KCU(cudaMemsetAsync(table, 0xff, sizeof(I) << tb, st));
     k_runs_write<I><<<(unsigned)rblocks, 256, 0, st>>>(R.code, R.val, R.n, rfirst, shift, run, table, rrow, rpos);
-    KCU(B.get(&A.tot, 4));
-    KCU(cudaMemsetAsync(A.tot, 0, sizeof(unsigned long long) * 4, st));
+    KCU(B.get(&A.tot, 6));
+    KCU(cudaMemsetAsync(A.tot, 0, sizeof(unsigned long long) * 6, st));
     k_col_runs<I><<<grid, 256, 0, st>>>(cseq, coffs, col_begin, ncols, kc.stride, C.start, tab, table, shift, run,
                                         rfirst + rblocks, same && kc.prune != PG_PRUNE_NONE, cfirst, clen, A.tot);
     KCU(cudaGetLastError());
@@ -798,35 +1028,56 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
     KCU(B.get(&A.start, ncols));
     KCU(B.get(&A.cnt, ncols + 1));
     KCU(B.get(&A.ovf, ncols));
-    // records of the call: room for 32 a column at first, or what the caller takes
-    A.tmp_cap = std::min<uint64_t>(cap, std::max<uint64_t>((uint64_t)1 << 20, 32 * ncols));
-    unsigned long long tot[4] = {0, 0, 0, 0};
+    // room for the records: as many as the caller takes, or as the pairs may give (one to
+    // ckthr + 1 of them; of the pairs before a prune about half are left)
+    const uint64_t most = (kc.prune == PG_PRUNE_NONE ? pairs : pairs / 2 + pairs / 16) / (uint64_t)(std::max(kc.ckthr, 0) + 1);
+    A.tmp_cap = std::min<uint64_t>(cap, most + 1024);
+    unsigned long long tot[6] = {};
+    uint64_t *poff = nullptr;
     for (;;) {
         KCU(B.get(&A.tmp, A.tmp_cap));
         KCU(cudaMemsetAsync(A.cnt, 0, (ncols + 1) * sizeof(uint32_t), st));
         KCU(cudaMemsetAsync(A.tot, 0, sizeof tot, st));
+        A.part = nullptr; A.nparts = 0; A.pstart = nullptr; A.pcnt = nullptr;
         const uint64_t blocks = std::min<uint64_t>(ncols, (uint64_t)nsm * 6);
         k_cand<I><<<(unsigned)blocks, CT, 0, st>>>(A);
         KCU(cudaGetLastError());
         KCU(cudaMemcpyAsync(tot, A.tot, sizeof tot, cudaMemcpyDeviceToHost, st));
         KCU(cudaStreamSynchronize(st));
-        if (tot[2]) {
-            // dense arrays for as many columns at a time as 4 GiB hold
-            const uint64_t fit = std::max<uint64_t>(1, ((uint64_t)4 << 30) / (nrows * sizeof(CandDense)));
-            const uint64_t slots = std::min<uint64_t>(std::min<uint64_t>(tot[2], fit), (uint64_t)nsm * 4);
-            CandDense *dense;
-            KCU(B.get(&dense, slots * nrows));
-            k_cand_dense<I><<<(unsigned)slots, 256, 0, st>>>(A, dense, tot[2]);
+        if (const uint64_t novf = tot[2]) {
+            uint32_t *pnum;
+            uint64_t *pfirst;
+            KCU(B.get(&pnum, novf + 1));
+            KCU(B.get(&pfirst, novf + 1));
+            KCU(cudaMemsetAsync(pnum + novf, 0, sizeof(uint32_t), st));
+            k_parts<I, false><<<grid, 256, 0, st>>>(A, novf, pnum, nullptr, nullptr);
+            size_t pb = 0;
+            KCU(cub::DeviceScan::ExclusiveSum(nullptr, pb, pnum, pfirst, (int64_t)(novf + 1), st));
+            void *ptmp;
+            KCU(B.get((char **)&ptmp, pb));
+            KCU(cub::DeviceScan::ExclusiveSum(ptmp, pb, pnum, pfirst, (int64_t)(novf + 1), st));
+            KCU(cudaMemcpyAsync(&A.nparts, pfirst + novf, sizeof A.nparts, cudaMemcpyDeviceToHost, st));
+            KCU(cudaStreamSynchronize(st));
+            uint4 *part;
+            KCU(B.get(&part, A.nparts));
+            KCU(B.get(&A.pstart, A.nparts));
+            KCU(B.get(&A.pcnt, A.nparts + 1));
+            KCU(B.get(&poff, A.nparts + 1));
+            KCU(cudaMemsetAsync(A.pcnt + A.nparts, 0, sizeof(uint32_t), st));
+            k_parts<I, true><<<grid, 256, 0, st>>>(A, novf, pnum, pfirst, part);
+            A.part = part;
+            KCU(cudaFuncSetAttribute(k_cand_parts<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PartSmem)));
+            k_cand_parts<I><<<(unsigned)std::min<uint64_t>(A.nparts, (uint64_t)nsm * 3), WT, sizeof(PartSmem), st>>>(A);
             KCU(cudaGetLastError());
             KCU(cudaMemcpyAsync(tot, A.tot, sizeof tot, cudaMemcpyDeviceToHost, st));
             KCU(cudaStreamSynchronize(st));
         }
-        *n_out = tot[1];
-        if (tot[1] > cap) return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: output capacity too small");
+        *n_out = tot[5];
+        if (tot[5] > cap) return pg_internal_fail(PG_ERR_RANGE, "pg_candidates: output capacity too small");
         if (tot[1] <= A.tmp_cap) break;
-        A.tmp_cap = tot[1];          // more records than the first guess: once more with room for them
+        A.tmp_cap = tot[1] + tot[1] / 8;     // more places than room: once more with room for them
     }
-    if (!tot[1]) return PG_OK;
+    if (!tot[5]) return PG_OK;
     uint64_t *pos;
     KCU(B.get(&pos, ncols + 1));
     size_t xb = 0;
@@ -834,7 +1085,14 @@ int candidates_of(Bufs &B, const SideKmers &R, const pg_kmer_config &kc, const K
     void *xtmp;
     KCU(B.get((char **)&xtmp, xb));
     KCU(cub::DeviceScan::ExclusiveSum(xtmp, xb, A.cnt, pos, (int64_t)(ncols + 1), st));
-    k_cand_place<<<grid, 256, 0, st>>>(A.tmp, A.start, A.cnt, pos, ncols, d_out);
+    if (A.nparts) {
+        size_t ob = 0;
+        KCU(cub::DeviceScan::ExclusiveSum(nullptr, ob, A.pcnt, poff, (int64_t)(A.nparts + 1), st));
+        void *otmp;
+        KCU(B.get((char **)&otmp, ob));
+        KCU(cub::DeviceScan::ExclusiveSum(otmp, ob, A.pcnt, poff, (int64_t)(A.nparts + 1), st));
+    }
+    k_cand_place<I><<<grid, 256, 0, st>>>(A, pos, poff, d_out);
     KCU(cudaGetLastError());
     KCU(cudaStreamSynchronize(st));
     return PG_OK;
