@@ -702,13 +702,16 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
     // tagged 16-bit form: scores that fit its int8 profile with their tags; m + n
     // whose path of gaps stays in range after scaling by 4 (local: any).  Not
     // where that would take regions the untagged form proves in range.
-    kp.tag = kp.tag_sum = kp.tag_min = 0;
+    kp.tag = kp.tag_sum = kp.tag_min = kp.tag_try = 0;
     if (kp.dir16_lim > 0 && c->go < 0 && c->ge < 0 && c->go >= -pg::TAG_SMAX && c->ge >= -pg::TAG_SMAX &&
         c->smin >= -pg::TAG_SMAX && c->smax <= pg::TAG_SMAX) {
         const int gmax = std::max(c->go, c->ge);
         kp.tag_sum = c->cfg.mode == PG_MODE_SW ? 1 << 30
                                                : (pg::SAT16_DP / 4 - 2 * std::abs(c->go)) / -gmax - 20;
         kp.tag_min = pg::TAG_MAX / (4 * std::max(1, c->smax));
+        // identical residues score about half of smax each, so homologs past twice
+        // tag_min leave the range as a rule
+        kp.tag_try = 2 * kp.tag_min;
         kp.tag = kp.tag_sum >= kp.dir16_lim ? 1 : 0;
     }
     // gap scores whose affine recurrence is a linear one: the default form runs

@@ -8,18 +8,20 @@ namespace pg {
 
 cudaError_t dir_set_attributes_ga()
 {
-    const void *k[20] = {(const void *)k_ga_dir<0, false, false>, (const void *)k_ga_dir<1, false, false>,
+    const void *k[24] = {(const void *)k_ga_dir<0, false, false>, (const void *)k_ga_dir<1, false, false>,
                          (const void *)k_ga_dir<2, false, false>, (const void *)k_ga_dir<3, false, false>,
                          (const void *)k_ga_dir<0, true, false>, (const void *)k_ga_dir<1, true, false>,
                          (const void *)k_ga_dir<2, true, false>, (const void *)k_ga_dir<3, true, false>,
                          (const void *)k_ga_dir<0, false, true>, (const void *)k_ga_dir<1, false, true>,
                          (const void *)k_ga_dir<2, false, true>, (const void *)k_ga_dir<3, false, true>,
+                         (const void *)k_ga_dir<0, true, true>, (const void *)k_ga_dir<1, true, true>,
+                         (const void *)k_ga_dir<2, true, true>, (const void *)k_ga_dir<3, true, true>,
                          (const void *)k_ga_pair<0, false>, (const void *)k_ga_pair<1, false>,
                          (const void *)k_ga_pair<2, false>, (const void *)k_ga_pair<3, false>,
                          (const void *)k_ga_pair<0, true>, (const void *)k_ga_pair<1, true>,
                          (const void *)k_ga_pair<2, true>, (const void *)k_ga_pair<3, true>};
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 20 && e == cudaSuccess; ++i)
+    for (int i = 0; i < 24 && e == cudaSuccess; ++i)
         e = cudaFuncSetAttribute(k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, DIR16_DYN_SMEM);
     return e;
 }
@@ -64,7 +66,8 @@ int dir_run_ga(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint6
     }
     if (chk) {
         cudaMemsetAsync(kp.counter, 0, sizeof(unsigned int), st);
-        dp_ga<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        if (kp.tag) dp_ga<true, true>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        else dp_ga<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
         ++launches;
     }
     if (dir_walk_warps(kp, t1 - t0)) k_tb_ga<true><<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);

@@ -8,14 +8,16 @@ namespace pg {
 
 cudaError_t dir_set_attributes_sw()
 {
-    const void *k[12] = {(const void *)k_sw_dir<0, false, false>, (const void *)k_sw_dir<1, false, false>,
+    const void *k[16] = {(const void *)k_sw_dir<0, false, false>, (const void *)k_sw_dir<1, false, false>,
                          (const void *)k_sw_dir<2, false, false>, (const void *)k_sw_dir<3, false, false>,
                          (const void *)k_sw_dir<0, true, false>, (const void *)k_sw_dir<1, true, false>,
                          (const void *)k_sw_dir<2, true, false>, (const void *)k_sw_dir<3, true, false>,
                          (const void *)k_sw_dir<0, false, true>, (const void *)k_sw_dir<1, false, true>,
-                         (const void *)k_sw_dir<2, false, true>, (const void *)k_sw_dir<3, false, true>};
+                         (const void *)k_sw_dir<2, false, true>, (const void *)k_sw_dir<3, false, true>,
+                         (const void *)k_sw_dir<0, true, true>, (const void *)k_sw_dir<1, true, true>,
+                         (const void *)k_sw_dir<2, true, true>, (const void *)k_sw_dir<3, true, true>};
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < 12 && e == cudaSuccess; ++i)
+    for (int i = 0; i < 16 && e == cudaSuccess; ++i)
         e = cudaFuncSetAttribute(k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, DIR16_DYN_SMEM);
     return e;
 }
@@ -42,7 +44,8 @@ int dir_run_sw(int tie, const KParams &kp, uint64_t t0, uint64_t t1, const uint6
     else dp_sw<false, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
     if (chk) {
         cudaMemsetAsync(kp.counter, 0, sizeof(unsigned int), st);
-        dp_sw<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        if (kp.tag) dp_sw<true, true>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
+        else dp_sw<true, false>(tie, kp, t0, t1, doff, arena, dsc, grid, dyn, st);
         ++launches;
     }
     if (dir_walk_warps(kp, t1 - t0)) k_tb_sw<true><<<grid_tb, 256, 0, st>>>(kp, t0, t1, doff, arena, dsc);

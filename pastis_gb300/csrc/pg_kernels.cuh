@@ -95,8 +95,9 @@ struct KParams {
     int dir16_lim = 0;               // traceback form: regions with m + n <= this on 16-bit lanes
     int dir16_side = 0;              // ... and larger ones with both sides <= this, checked
     // tagged 16-bit form (pg_dptag.cuh): 1 where the scores allow it; its regions have
-    // m + n <= tag_sum and, for every value provably in range, min(m, n) <= tag_min
-    int tag = 0, tag_sum = 0, tag_min = 0;
+    // m + n <= tag_sum and, for every value provably in range, min(m, n) <= tag_min;
+    // beyond it the common pass tries those up to tag_try
+    int tag = 0, tag_sum = 0, tag_min = 0, tag_try = 0;
     int dir16_pair = 0;              // 1: 16-bit regions of up to 32 x rows_cap rows two per warp
     const uint32_t *xorder = nullptr; // X-drop extension directions, longest length bound first (null: t)
     XdSide *xdir = nullptr;     // k_xdr's results: 4 per pair (seed, left / right)
@@ -272,7 +273,7 @@ __host__ __device__ __forceinline__ bool dir16_use(const KParams &kp, int m, int
 // checked pass does it again if its largest value left the range)
 __host__ __device__ __forceinline__ bool dir16_tagged(const KParams &kp, int m, int n)
 {
-    return kp.tag && m + n <= kp.tag_sum && dir16_mode(kp, m, n) != 0;
+    return kp.tag && m + n <= kp.tag_sum && min(m, n) <= kp.tag_try && dir16_mode(kp, m, n) != 0;
 }
 
 // a region whose DP runs on half a warp, two regions per warp (dp_pair_dir16):

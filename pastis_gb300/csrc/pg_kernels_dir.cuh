@@ -50,7 +50,7 @@ __device__ __forceinline__ uint64_t region_bytes(const KParams &kp, int m, int n
     if (dir16_paired(kp, m, n)) return dir16_pair_bytes(m, n);
     const int mode = dir16_mode(kp, m, n);
     const uint64_t b16 = mode ? dir16_bytes(m, n, dir16_rows(m, kp.rows_cap)) : 0;
-    const uint64_t b32 = mode != 1 ? dir_bytes(m, n, dir_rows(m, kp.rows_cap)) : 0;
+    const uint64_t b32 = mode == 0 || (mode == 2 && !kp.tag) ? dir_bytes(m, n, dir_rows(m, kp.rows_cap)) : 0;
     return b16 > b32 ? b16 : b32;
 }
 
@@ -136,7 +136,7 @@ struct TagArgs {
     int go, ge;
     uint32_t four;
 };
-template <int TIE, bool LOCAL, int L>
+template <int TIE, bool LOCAL, int L, bool BASE>
 __device__ __forceinline__ DirOut dp_dispatch_tag(const TagArgs &ta, int R, const uint8_t *V, int m,
                                                   const uint8_t *Hs, int n, uint2 *prof, void *bnd,
                                                   uint32_t *dir)
@@ -144,14 +144,14 @@ __device__ __forceinline__ DirOut dp_dispatch_tag(const TagArgs &ta, int R, cons
     uint32_t *pf = reinterpret_cast<uint32_t *>(prof);
     uint2 *b = (uint2 *)bnd;
     switch (R) {
-    case 1: return dp_tag16<TIE, 1, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 2: return dp_tag16<TIE, 2, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 3: return dp_tag16<TIE, 3, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 4: return dp_tag16<TIE, 4, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 5: return dp_tag16<TIE, 5, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 6: return dp_tag16<TIE, 6, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    case 7: return dp_tag16<TIE, 7, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
-    default: return dp_tag16<TIE, 8, LOCAL, L>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 1: return dp_tag16<TIE, 1, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 2: return dp_tag16<TIE, 2, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 3: return dp_tag16<TIE, 3, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 4: return dp_tag16<TIE, 4, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 5: return dp_tag16<TIE, 5, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 6: return dp_tag16<TIE, 6, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    case 7: return dp_tag16<TIE, 7, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
+    default: return dp_tag16<TIE, 8, LOCAL, L, BASE>(V, m, Hs, n, ta.tab, pf, ta.go, ta.ge, ta.four, b, dir);
     }
 }
 // loads the tables of a DP kernel
@@ -168,20 +168,20 @@ constexpr int TAG_TABW = LIN_NC * LIN_ROWB / 4;
 // The DP of one region.  CHK false: a region on 16-bit lanes with every value
 // provably in range (mode 1) or on 32-bit lanes (mode 0); CHK true: a checked
 // region (mode 2), the checked 16-bit form and, if a value left the range, the
-// 32-bit form after it (sat = 1: the traceback walks the 32-bit layout).  The
-// kernels take checked regions in a pass of their own, so the common pass's
-// code stays free of the checked form.
+// 32-bit form after it (sat = 1: the traceback walks the 32-bit layout), or with
+// TAG the tagged form on a base, which has no range to leave.  The kernels take
+// checked regions in a pass of their own, so the common pass's code stays free of
+// these forms.
 template <int TIE, bool LOCAL, bool CHK, bool TAG>
 __device__ __forceinline__ DirOut dp_dispatch_dir(const KParams &kp, const TagArgs &ta, const uint8_t *V, int m,
                                                   const uint8_t *Hs, int n, const int *ssm,
                                                   uint2 *prof, void *bnd, uint32_t *dir)
 {
-    static_assert(!(CHK && TAG), "the checked pass is the untagged form");
     EdgeD *b = (EdgeD *)bnd;
     const int go = kp.go, ge = kp.ge, cap = kp.rows_cap;
     DirOut d;
-    if (TAG && dir16_tagged(kp, m, n))
-        return dp_dispatch_tag<TIE, LOCAL, 32>(ta, dir16_rows(m, cap), V, m, Hs, n, prof, bnd, dir);
+    if (TAG && (CHK || dir16_tagged(kp, m, n)))
+        return dp_dispatch_tag<TIE, LOCAL, 32, CHK>(ta, dir16_rows(m, cap), V, m, Hs, n, prof, bnd, dir);
     if (!TAG && (CHK || dir16_mode(kp, m, n) == 1)) {
         switch (dir16_rows(m, cap)) {
         case 1: d = dp_warp_dir16<TIE, 1, LOCAL, CHK>(V, m, Hs, n, ssm, prof, go, ge, b, dir); break;
@@ -218,7 +218,7 @@ __device__ __forceinline__ DirOut dp_dispatch_pair(const KParams &kp, const TagA
                                                    const uint8_t *Hs, int n, const int *ssm,
                                                    uint2 *prof, uint32_t *dir)
 {
-    if (TAG) return dp_dispatch_tag<TIE, LOCAL, 16>(ta, R, V, m, Hs, n, prof, nullptr, dir);
+    if (TAG) return dp_dispatch_tag<TIE, LOCAL, 16, false>(ta, R, V, m, Hs, n, prof, nullptr, dir);
     const int go = kp.go, ge = kp.ge;
     switch (R) {
     case 1: return dp_pair_dir16<TIE, 1, LOCAL>(V, m, Hs, n, ssm, prof, go, ge, dir);
