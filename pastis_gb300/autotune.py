@@ -8,9 +8,10 @@ replay of the batch's launches.
 Candidates are timed with the library's own CUDA events (pg_kernel_ms) on a
 batch the caller supplies,
 normally a sample of the real one, and the winner is cached in a JSON file
-keyed by device and a workload signature (mode, batch size and length
-quantiles, rounded to powers of two) so later runs on the same kind of batch
-skip the search.
+keyed by device, build of the native library, scoring (gap scores, X, flags and
+score table: they decide which kernels the options reach) and a workload
+signature (mode, batch size and length quantiles, rounded to powers of two) so
+later runs on the same kind of batch skip the search.
 """
 import itertools
 import json
@@ -80,7 +81,10 @@ def tune(ctx, run, key=None, device=0, reps=3, grid=None, use_cache=True, log=No
     Returns (tuning dict, report)."""
     path = cache_path()
     dev = _device_name(device)
-    entry = "%s|%s" % (dev, key) if key else None
+    entry = None
+    if key:
+        scoring = ctx.scoring_key() if hasattr(ctx, "scoring_key") else ""
+        entry = "|".join((dev, capi.build_key(), scoring, key))
     if use_cache and entry and os.path.exists(path):
         try:
             cached = json.load(open(path)).get(entry)

@@ -4,7 +4,9 @@ The CUDA library must be present: loading raises if it is missing, there is no
 CPU fallback.
 """
 import ctypes
+import hashlib
 import os
+import zlib
 
 import numpy as np
 
@@ -216,6 +218,19 @@ def resolved_gaps(cfg):
     return cfg.gap_open, cfg.gap_ext, cfg.gap_ext
 
 
+def scoring_key(cfg):
+    """What of a configuration decides which kernels run: the gap scores as resolved, X,
+    the flags and the score table."""
+    table = zlib.crc32(ctypes.string_at(cfg.score_matrix, 25 * 25)) if cfg.score_matrix else 0
+    return "g%d.%d.%d-x%d-f%d-t%08x" % (*resolved_gaps(cfg), cfg.xdrop, cfg.flags, table)
+
+
+def build_key():
+    """Digest of the native library: which build of the kernels runs."""
+    with open(os.path.join(BUILD, "libpastis_gb300.so"), "rb") as f:
+        return hashlib.sha1(f.read()).hexdigest()[:12]
+
+
 def dpx_peak(device=0):
     """Measured DPX add-max instructions per second on a device."""
     v = ctypes.c_double()
@@ -233,6 +248,11 @@ class Context:
         h = ctypes.c_void_p()
         _check(self.lib.pg_create(ctypes.byref(cfg), ctypes.byref(h)))
         self.h = h
+        self._scoring = scoring_key(cfg)      # while cfg.score_matrix is known to be valid
+
+    def scoring_key(self):
+        """scoring_key() of the configuration this context was created with."""
+        return self._scoring
 
     def close(self):
         if getattr(self, "h", None):
