@@ -41,11 +41,40 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "GCUPS & alignments/s, batched SW/X-drop: GPU plain vs tuned+filtered vs CPU"
-# roofline model: E, F and H as add-max DPX-class ops plus the max with the
-# third term, per cell on 32-bit lanes
+# roofline model, DPX-class ops per cell.  Affine: E, F and H as add-max plus the max
+# with the third term.  Linear (a first gap position cheaper than the further ones): an
+# add-max with the cell to the left and one with the cell above
 DPX_OPS_PER_CELL = 4
+DPX_OPS_PER_CELL_LINEAR = 2
 SW_WORKLOADS = ("sw100k", "filter5m", "uneven10m_sw")
 SEED = 20260101
+
+
+def alignment_kernels(mode, gaps, tuning, scores=(-4, 11)):
+    """The kernels a batch's alignment runs on and their roofline model, by the rule of
+    launch() in pg_api.cu.  mode: PG_MODE_*; gaps: first and further position as resolved;
+    scores: the smallest and largest substitution score (BLOSUM62)."""
+    first, further = gaps
+    form = tuning["dp_traceback"]
+    xdrop = mode == 1
+    fits = min(scores) >= -31 and max(scores) <= 31           # an int8 profile of scores x 4
+    if (fits and -31 <= first < 0 and first > further and form == 3 and tuning["rows_max"] == 8
+            and tuning["bucket_order"]):
+        return {"kernel": "k_lin_dp + k_lin_walk", "cells_per_op": 2,
+                "ops_per_cell": DPX_OPS_PER_CELL_LINEAR,
+                "model": "linear gaps, values and decisions in tagged 16-bit lanes"}
+    name = {0: "k_ga" if xdrop else "k_sw",
+            1: "k_ga_dir + k_tb_ga" if xdrop else "k_sw_dir + k_tb_sw",
+            2: "k_ga_dir + k_tb_ga" if xdrop else "k_sw_dir + k_tb_sw",
+            3: "k_ga_dir + k_ga_pair + k_tb_ga" if xdrop else "k_sw_dir + k_tb_sw"}[form]
+    lanes16 = form >= 2 and max(abs(x) for x in (*scores, first, further)) <= 100
+    tagged = lanes16 and fits and -31 <= first < 0 and -31 <= further < 0
+    if lanes16:
+        name += " (%s16-bit lanes%s)" % ("tagged " if tagged else "",
+                                         ", two regions per warp" if form == 3 else "")
+    return {"kernel": name, "cells_per_op": 2 if lanes16 else 1, "ops_per_cell": DPX_OPS_PER_CELL,
+            "model": "affine gaps" + (", add-max with the decision in the value" if tagged else
+                                      ", the 16-bit kernels issue max and add" if lanes16 else "")}
 
 
 def parse():
@@ -419,20 +448,12 @@ def run_gpu(args, rank, world, local_rank):
     line = None
     if rank == 0:
         peak_ops = capi.dpx_peak(dev)
-        form = ctx.get_tuning().dp_traceback
-        # 16-bit lanes: each packed op advances two cells, so the same op rate
-        # bounds twice the cells (the conservative peak for a mixed batch)
-        cells_per_op = 2 if form >= 2 else 1
-        peak_gcups = peak_ops * cells_per_op / DPX_OPS_PER_CELL / 1e9
-        # dominant kernel: the alignment DP and its traceback, executed cells
+        dp = alignment_kernels(mode, capi.resolved_gaps(ctx.cfg)[:2], ctx.get_tuning().as_dict())
+        dp_kernel = dp["kernel"]
+        peak_gcups = peak_ops * dp["cells_per_op"] / dp["ops_per_cell"] / 1e9
+        # dominant kernels: the alignment DP and its traceback, executed cells
         achieved = exec_dp / (dp_ms * 1e-3) / 1e9
         traffic = None
-        dp_kernel = {0: "k_ga" if mode else "k_sw",
-                     1: "k_ga_dir + k_tb_ga" if mode else "k_sw_dir + k_tb_sw",
-                     2: ("k_ga_dir + k_tb_ga" if mode else "k_sw_dir + k_tb_sw")
-                     + " (16-bit lanes)",
-                     3: ("k_ga_dir + k_ga_pair + k_tb_ga" if mode else "k_sw_dir + k_tb_sw")
-                     + " (16-bit lanes, two regions per warp)"}[form]
         tpath = os.path.join(ROOT, "profiles", "traffic.json")
         if os.path.exists(tpath):
             # ncu DRAM bytes per pair of the same kernel on this workload
@@ -447,13 +468,11 @@ def run_gpu(args, rank, world, local_rank):
         alg_bytes = int((lens[w.pairs["row"]] + lens[w.pairs["col"]]).sum()) + n * (
             capi.PAIR_DTYPE.itemsize + capi.RESULT_DTYPE.itemsize)
         hbm_gbs = alg_bytes / (ms_step * 1e-3) / 1e9
-        if form >= 2:
-            peak_src = ("measured %.4g DPX add-max/s (pg_dpx_peak, int32) / %d DPX-class ops "
-                        "per cell x 2 cells per packed 16-bit op (model; the 16-bit kernels "
-                        "issue max/add.s16x2, not add-max)" % (peak_ops, DPX_OPS_PER_CELL))
-        else:
-            peak_src = ("measured %.4g DPX add-max/s (pg_dpx_peak, int32) / %d DPX-class ops "
-                        "per cell (model)" % (peak_ops, DPX_OPS_PER_CELL))
+        peak_src = "measured %.4g DPX add-max/s (pg_dpx_peak, int32) / %d DPX-class ops per cell" % (
+            peak_ops, dp["ops_per_cell"])
+        if dp["cells_per_op"] == 2:
+            peak_src += " x 2 cells per packed 16-bit op"
+        peak_src += " (model: %s)" % dp["model"]
         line = {
             "metric": METRIC, "value": gcups, "unit": "GCUPS", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
