@@ -860,6 +860,7 @@ static int check_status(pg_ctx *c)
     if (st & pg::ST_BAD_INDEX) return fail(PG_ERR_ARG, "a pair refers to a sequence index out of range");
     if (st & pg::ST_WAIT) return fail(PG_ERR_CUDA, "internal: a stripe's wait ran out");
     if (st & pg::ST_BAD_SCHED) return fail(PG_ERR_CUDA, "internal: inconsistent bucket schedule");
+    if (st & pg::ST_END) return fail(PG_ERR_CUDA, "internal: no cell holds the score found");
     return PG_OK;
 }
 

@@ -48,6 +48,7 @@ constexpr int ST_TOO_LONG = 2;    // a sequence beyond a kernel's length bound
 constexpr int ST_BAD_SCHED = 4;   // bucket order inconsistent (never expected)
 constexpr int ST_BAD_CODE = 8;    // a residue code outside 0..24
 constexpr int ST_WAIT = 16;       // a stripe gave up waiting for the one above it (never expected)
+constexpr int ST_END = 32;        // no cell holds the score found (never expected)
 
 // extension of one (pair, seed)
 constexpr uint32_t XF_NONE = 1;    // seed not tried (seed_count / spurious switch)

@@ -1300,7 +1300,11 @@ __global__ void __launch_bounds__(256) k_lin_walk(const LinParams lp, uint32_t w
                 if (z != ~0u) { p.j = (int)(z >> 3); p.i = row0 + (int)(z & 7u) + 1; }
             }
         }
-        if (!p.i) d.w = 0;
+        if (d.w && !p.i) {
+            // the DP saw the score in one of these lanes: not an empty result
+            atomicOr(lp.kp.status, ST_END);
+            d.w = 0;
+        }
     }
     const int end_i = p.i, end_j = p.j;
     if (!LOCAL || d.w) {
