@@ -175,7 +175,8 @@ typedef struct pg_tuning {
     int32_t dp_blocks_per_sm;   /* k_ga / k_sw resident blocks per SM; 0 = occupancy limit */
     int32_t xd_blocks_per_sm;   /* X-drop extension resident blocks per SM; 0 = occupancy limit */
     int32_t bucket_order;       /* 1: pairs in DP-bucket order, tallest first; 0: input order */
-    int32_t rows_max;           /* cap on DP rows per lane, 1..8 (wide statistics stop at 4) */
+    int32_t rows_max;           /* cap on DP rows per lane, 1..8 (wide statistics stop at 4);
+                                   8 is also a condition of the linear form, see dp_traceback */
     int32_t graph;              /* 1: pg_align / pg_align_device capture the batch's launches
                                    into a CUDA graph once per batch shape (pairs and output
                                    pointers, n, offsets, stream) and replay it after that */
@@ -192,13 +193,24 @@ typedef struct pg_tuning {
                                    32-bit lanes if a value leaves [-30000, 30000]; 32-bit
                                    lanes for the rest; 3: form 2, with the 16-bit regions
                                    of up to 32 * rows_max rows two per warp, each on half
-                                   of it; no graph capture in these forms */
+                                   of it; no graph capture in these forms.
+                                   Forms 2 and 3 with all scores within +-31 and both gap
+                                   scores negative keep the decision in the low bits of
+                                   scaled values (regions past their range on a moving base,
+                                   none on 32-bit lanes).  Form 3 with rows_max = 8 and
+                                   bucket_order = 1 runs gap scores whose first position is
+                                   the cheaper one (the default scores, as PASTIS passes
+                                   them) as linear gaps, 2 bits per cell: another value of
+                                   one of the three takes such batches to the affine form,
+                                   two to eight times slower */
     int32_t dir_arena_mb;       /* cap on that arena in MiB; 0 = a third of the device memory */
-    int32_t xd_stepped;         /* X-drop extension kernel, a thread per (pair, seed):
-                                   2 holds the band's 16-column window in registers and
-                                   computes it branch-free with packed 16-bit operations
-                                   (needs a linear X-drop gap of -1..-4096 and xdrop
-                                   <= 8192, else 1 runs); 1 steps one extension direction
+    int32_t xd_stepped;         /* X-drop extension kernel: 2 takes the directions of a
+                                   (pair, seed) apart, a thread each and a warp for the
+                                   longest, and holds the band's 16-column window in
+                                   registers, computed branch-free with packed 16-bit
+                                   operations (needs a linear X-drop gap of -1..-4096,
+                                   xdrop <= 8192 and fewer than 2^30 pairs, else 1 runs);
+                                   a thread per (pair, seed): 1 steps one extension direction
                                    at a time over a shared-memory ring and starts the next
                                    the moment one ends; 0 runs each task to its end over
                                    the ring (fewer registers, more resident warps);
@@ -314,7 +326,7 @@ typedef struct pg_kmer_config {
     int32_t  prune;          /* PG_PRUNE_*                                       */
     int32_t  ckthr;          /* drop pairs with count <= ckthr (0 keeps all)     */
     int32_t  mosthr;         /* drop pairs with score <= mosthr                  */
-    uint64_t max_products;   /* occurrence pairs one call may hold; 0 = 2^31     */
+    uint64_t max_products;   /* occurrence pairs one call may have after the prune; 0 = 2^31 */
 } pg_kmer_config;            /* 32 bytes */
 
 void pg_kmer_config_default(pg_kmer_config *kc);
@@ -322,8 +334,12 @@ void pg_kmer_config_default(pg_kmer_config *kc);
  * of the context's row and column sequences into d_out (device, cap records).
  * *n_out = pairs found.  PG_ERR_RANGE when they exceed cap (d_out untouched,
  * *n_out = the count needed) or the occurrence pairs exceed max_products
- * (*n_out = 0); PG_ERR_ARG when alphabet_size^k exceeds 2^31 (the reference's
- * own limit) or a range is out of bounds.  Synchronous. */
+ * (*n_out = 0; counted before any of them is visited); PG_ERR_ARG when
+ * alphabet_size^k exceeds 2^31 (the reference's own limit) or a range is out of
+ * bounds.  Synchronous.
+ * The context keeps up to 8 GiB of the call's scratch for the next one, until
+ * pg_destroy: a program with a context per host thread holds that per thread.
+ * (A cudaMalloc that found too little memory free was seen to get it.) */
 int pg_candidates(pg_ctx *ctx, const pg_kmer_config *kc, uint64_t row_begin, uint64_t row_end,
                   uint64_t col_begin, uint64_t col_end, pg_pair *d_out, uint64_t cap,
                   uint64_t *n_out, void *stream);

@@ -170,7 +170,7 @@ struct pg_ctx {
     uint64_t list_cap = 0;
     int4 *d_walk = nullptr;
     uint64_t walk_cap = 0;
-    cudaMemPool_t pool = nullptr;       // scratch of the calls around the aligner (pg_kmer.cu, pg_fasta.cu)
+    cudaMemPool_t pool = nullptr;       // scratch of pg_candidates (pg_kmer.cu)
     // staging for the host-buffer entry point
     pg_pair *d_pairs = nullptr;
     pg_result *d_out = nullptr;

@@ -1,7 +1,7 @@
 // pg_kernels_xd.cuh -- the X-drop extension kernels (one definition: only
-// pg_api.cu includes this file): k_xdr, thread per (pair, seed) task with the
-// band window in registers (pg_xdreg.cuh), the default; k_xdf and k_xd,
-// thread per task with the 32-bit band in a shared-memory ring (pg_xdrop.cuh),
+// pg_api.cu includes this file): k_xdr, a thread, for the longest a warp, per
+// direction of a (pair, seed) with the band window in registers (pg_xdreg.cuh), the
+// default; k_xdf and k_xd, thread per (pair, seed) task with the 32-bit band in a shared-memory ring (pg_xdrop.cuh),
 // stepping one direction at a time or running each task to its end (tuning
 // option xd_stepped); k_xd16, a thread per task on 16-bit lanes (tuning option
 // xd_int16); k_xd_wide, warp per task for the bands that overflow a thread's

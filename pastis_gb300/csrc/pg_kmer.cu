@@ -18,7 +18,7 @@
 //   4. the columns' records are moved into place, column-major.
 // The product of a block is never written out or sorted: for 200k proteins that
 // was 58M 16-byte products through a 7-pass radix sort, a run-length encoding and
-// a reduction, 28.5 ms a call with the allocation of their buffers; 10.8 ms now (even/odd
+// a reduction, 28.5 ms a call with the allocation of their buffers; 10.3 ms now (even/odd
 // prune, ckthr = 1).  A column that outgrows the tables of step 3, the usual one without
 // a threshold (ckthr = 0) or from about 500k rows on, goes through k_cand_parts.
 #include <cuda_runtime.h>

@@ -1082,8 +1082,8 @@ __device__ __forceinline__ uint32_t lin_locate(const int8_t *sm, const uint8_t *
 //    (100k pairs 0.79 -> 0.56 ms; the global form, with half the registers, ran
 //    faster one cell at a time, 1.06 against 1.29 ms on 400k X-drop pairs).  A
 //    warp waits for whichever of its 32 walks misses L1, about 400 cycles a move.
-//  - a warp per region, for regions in stripes and for batches too small to fill
-//    the chip with threads: 16 lanes read the next 16 cells of the diagonal, a
+//  - a warp per region, for regions of many columns (lin_wide) and for batches too
+//    small to fill the chip with threads: 16 lanes read the next 16 cells of the diagonal, a
 //    ballot gives the run of diagonal moves, and the other lanes bring the
 //    sectors of the 16 cells after those into L1.
 struct LinPath {
