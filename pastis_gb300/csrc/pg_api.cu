@@ -769,7 +769,8 @@ static int launch(pg_ctx *c, const pg_pair *d_pairs, uint64_t n, uint64_t roff, 
             pg::k_xda<<<c->grid_wide, blk, 0, st>>>(kp);
         } else {
             if (int16) pg::k_xd16<<<gx, pg::XT, 0, st>>>(kp);
-            else if (form == 2 && kp.xorder && 4 * n > pg::XDR_MIXED * (uint64_t)gx * (pg::XT / 32))
+            else if (form == 2 && kp.xorder && 4 * n > pg::XDR_MIXED * (uint64_t)gx * (pg::XT / 32) &&
+                     4 * n <= pg::XDR_MIXED_MAX * (uint64_t)gx * (pg::XT / 32))
                 pg::k_xdr<8, true><<<gx, pg::XT, 0, st>>>(kp);
             else if (form == 2) pg::k_xdr<8, false><<<gx, pg::XT, 0, st>>>(kp);
             else if (form == 1) pg::k_xdf<<<gx, pg::XT, 0, st>>>(kp);

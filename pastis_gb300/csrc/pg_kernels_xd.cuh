@@ -331,13 +331,15 @@ __global__ void __launch_bounds__(256) k_xtask_bucket(const KParams kp)
 // the warps, and the extension took 9.85 ms per 1M pairs against 9.3.
 // Needs xdr_supported(xg, xdrop) and direction ids in 32 bits (n < 2^30).
 //
-// MIXED (from XDR_MIXED directions a resident warp on): a quarter of the warps starts on
+// MIXED (XDR_MIXED to XDR_MIXED_MAX directions a resident warp): a quarter of the warps starts on
 // the threads' directions and helps with the long ones after.  With all warps on the long
 // ones first the two kinds run one after the other, the second with the machine half
 // empty: 12k pairs of ordinary lengths 0.92 -> 0.75 ms, 20k 1.53 -> 1.09, 60k 2.27 -> 1.51;
 // uneven ones 1.47 -> 1.14, 2.3 -> 1.52, 4.1 -> 2.69.  An instance of its own, as the loop
-// over the two parts made small batches 8 % slower (256 pairs 0.204 -> 0.220).
-constexpr uint64_t XDR_MIXED = 12;
+// over the two parts made small batches 8 % slower (256 pairs 0.204 -> 0.220).  In the largest
+// the mean load passes nearly every length, so that hardly any is long: 300k uneven pairs
+// 7.8 -> 7.1 ms, 400k 7.45 -> 7.55, 400k of ordinary lengths 4.31 -> 4.39.
+constexpr uint64_t XDR_MIXED = 12, XDR_MIXED_MAX = 576;
 // the first `first` directions of the order, a warp each
 __device__ __forceinline__ void xdr_long(const KParams &kp, const int *ssm, uint32_t first)
 {
@@ -366,49 +368,10 @@ __device__ __forceinline__ void xdr_long(const KParams &kp, const int *ssm, uint
     }
 }
 
-template <int NW, bool MIXED>
-__global__ void __launch_bounds__(XT) k_xdr(const KParams kp)
+// the directions after the first `first` ones, a thread each
+template <int NW>
+__device__ __forceinline__ void xdr_threads(const KParams &kp, const char *tbl, uint32_t ntask, uint32_t first)
 {
-    __shared__ int ssm[PG_NRES * XR_STRIDE];
-    __shared__ unsigned int total, nlong;
-    // where no gap fits into X a direction ends soon after its homology does, far below
-    // its bound: fewer long ones, beyond three times the mean load, on half of the warps
-    // (12k / 20k / 40k pairs 0.62 / 1.03 / 1.31 ms with the mean load as the line, 0.45 /
-    // 0.51 / 0.95 by threads alone, 0.36 / 0.52 / 0.69 so)
-    const bool narrow = MIXED && kp.xdrop < -kp.xg;
-    load_sm33(ssm, kp.sm);
-    if (threadIdx.x < 32) {
-        // the directions listed, and the long ones among them (a prefix of the order):
-        // those beyond the mean load of a thread, by the length bounds.  None where X
-        // lets a band outgrow a warp's window too (X / |g| gap steps to either side)
-        unsigned int t = 0, l = 0;
-        float load = 0.0f;
-        if (kp.xorder)
-            for (int b = threadIdx.x; b < XBUCKET; b += 32) {
-                t += kp.xsched[b];
-                load += (float)kp.xsched[b] * xdir_bucket_len(b);
-            }
-        t = __reduce_add_sync(FULL, t);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) load += __shfl_xor_sync(FULL, load, o);
-        const float lim = fmaxf(XDR_LONG, load / (float)(gridDim.x * blockDim.x) * (narrow ? 3.0f : 1.0f));
-        if (kp.xorder && 2 * kp.xdrop <= 20 * -kp.xg)
-            for (int b = threadIdx.x; b < XBUCKET; b += 32)
-                if (xdir_bucket_len(b) > lim) l += kp.xsched[b];
-        l = __reduce_add_sync(FULL, l);
-        if (threadIdx.x == 0) { total = kp.xorder ? t : (unsigned int)(4 * kp.n); nlong = l; }
-    }
-    __syncthreads();
-    const char *tbl = reinterpret_cast<const char *>(ssm);
-    const uint32_t ntask = total, first = nlong;
-    // (a loop over the two parts: with a second call after it, behind the same test, 12k to
-    // 40k uneven pairs ran 20 to 50 % slower)
-    const bool later = MIXED && (threadIdx.x >> 5) < (narrow ? XT / 64 : XT / 128);
-    for (int part = 0; part < (MIXED ? 2 : 1); ++part) {
-    if ((part == 0) != later) {
-        xdr_long(kp, ssm, first);
-        if (MIXED) continue;
-    }
     uint32_t ta, tb;
     pg_pair pb;
     XfReady c;
@@ -486,7 +449,55 @@ __global__ void __launch_bounds__(XT) k_xdr(const KParams kp)
         if (!x.ok) kp.ovf[atomicAdd(&kp.counter[2], 1u)] = task;
         run = false;
     }
-    __syncwarp();
+}
+
+template <int NW, bool MIXED>
+__global__ void __launch_bounds__(XT) k_xdr(const KParams kp)
+{
+    __shared__ int ssm[PG_NRES * XR_STRIDE];
+    __shared__ unsigned int total, nlong;
+    // where no gap fits into X a direction ends soon after its homology does, far below
+    // its bound: fewer long ones, beyond three times the mean load, on half of the warps
+    // (12k / 20k / 40k pairs 0.62 / 1.03 / 1.31 ms with the mean load as the line, 0.45 /
+    // 0.51 / 0.95 by threads alone, 0.36 / 0.52 / 0.69 so)
+    const bool narrow = MIXED && kp.xdrop < -kp.xg;
+    load_sm33(ssm, kp.sm);
+    if (threadIdx.x < 32) {
+        // the directions listed, and the long ones among them (a prefix of the order):
+        // those beyond the mean load of a thread, by the length bounds.  None where X
+        // lets a band outgrow a warp's window too (X / |g| gap steps to either side)
+        unsigned int t = 0, l = 0;
+        float load = 0.0f;
+        if (kp.xorder)
+            for (int b = threadIdx.x; b < XBUCKET; b += 32) {
+                t += kp.xsched[b];
+                load += (float)kp.xsched[b] * xdir_bucket_len(b);
+            }
+        t = __reduce_add_sync(FULL, t);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) load += __shfl_xor_sync(FULL, load, o);
+        const float lim = fmaxf(XDR_LONG, load / (float)(gridDim.x * blockDim.x) * (narrow ? 3.0f : 1.0f));
+        if (kp.xorder && 2 * kp.xdrop <= 20 * -kp.xg)
+            for (int b = threadIdx.x; b < XBUCKET; b += 32)
+                if (xdir_bucket_len(b) > lim) l += kp.xsched[b];
+        l = __reduce_add_sync(FULL, l);
+        if (threadIdx.x == 0) { total = kp.xorder ? t : (unsigned int)(4 * kp.n); nlong = l; }
+    }
+    __syncthreads();
+    const char *tbl = reinterpret_cast<const char *>(ssm);
+    const uint32_t ntask = total, first = nlong;
+    // (a loop over the two parts: with xdr_long called a second time after it, behind the
+    // same test, 12k to 40k uneven pairs ran 20 to 50 % slower)
+    const bool later = MIXED && (threadIdx.x >> 5) < (narrow ? XT / 64 : XT / 128);
+    if constexpr (MIXED) {
+        for (int part = 0; part < 2; ++part) {
+            if ((part == 0) != later) xdr_long(kp, ssm, first);
+            else xdr_threads<NW>(kp, tbl, ntask, first);
+            __syncwarp();
+        }
+    } else {
+        xdr_long(kp, ssm, first);
+        xdr_threads<NW>(kp, tbl, ntask, first);
     }
 }
 
